@@ -61,18 +61,29 @@ struct AcuIeee {
     using V = T;
     // CTAs per SM the kernel is compiled for: FP32 fits five (47 registers, no spills), FP64 four
     static constexpr int kMinBlocks = sizeof(T) == 4 ? 5 : 4;
+    static constexpr bool kRetest = true;  // quotients are taken before their dividends are tested
     struct C {
         T dtr, dtk;
         DivC<T> h[3];
+        uint32_t lo;  // the smallest dividend key all three take without a test
     };
     static __device__ __forceinline__ V in(S x, bool&) { return x; }
     static __device__ __forceinline__ V add(V a, V b) { return a + b; }
     static __device__ __forceinline__ V sub(V a, V b) { return a - b; }
     // `- dt/ρ*@d_i(P)/h`: dt/ρ is one host value (Julia evaluates dt/ρ first)
-    static __device__ __forceinline__ V vdel(V pa, V pb, const C& c, int d) { return -div_c(c.dtr * (pa - pb), c.h[d]); }
+    // FAST: without the dividend tests; *key keeps the smallest dividend key (see DivF)
+    template <bool FAST>
+    static __device__ __forceinline__ V dv(V a, const C& c, int d, uint32_t* key) {
+        return FAST ? dvd(a, DivF<T>{c.h[d], key}) : div_c(a, c.h[d]);
+    }
+    template <bool FAST>
+    static __device__ __forceinline__ V vdel(V pa, V pb, const C& c, int d, uint32_t* key) {
+        return -dv<FAST>(c.dtr * (pa - pb), c, d, key);
+    }
     // `- dt*k*(@d_xa(Vx)/dx + @d_ya(Vy)/dy + @d_za(Vz)/dz)`
-    static __device__ __forceinline__ V pdel(V ax, V ay, V az, const C& c) {
-        return -(c.dtk * ((div_c(ax, c.h[0]) + div_c(ay, c.h[1])) + div_c(az, c.h[2])));
+    template <bool FAST>
+    static __device__ __forceinline__ V pdel(V ax, V ay, V az, const C& c, uint32_t* key) {
+        return -(c.dtk * ((dv<FAST>(ax, c, 0, key) + dv<FAST>(ay, c, 1, key)) + dv<FAST>(az, c, 2, key)));
     }
     static __device__ __forceinline__ S store(S, V nv, V) { return nv; }
     static __device__ __forceinline__ V shfl_up(V v) { return __shfl_up_sync(0xFFFFFFFFu, v, 1); }
@@ -85,6 +96,7 @@ struct AcuSplit {
     using S = double;
     using V = dd;
     static constexpr int kMinBlocks = 4;
+    static constexpr bool kRetest = false;
     struct C {
         dd cv[3];  // (dt/ρ)/h_d as h + l, and its remainder r (h + l + r exact to ~2^-72)
         dd ck[3];  // (dt·k)/h_d
@@ -103,11 +115,13 @@ struct AcuSplit {
     static __device__ __forceinline__ V in(S x, bool& big) { return dd_split(x, big); }
     static __device__ __forceinline__ V add(V a, V b) { return dd_add(a, b); }
     static __device__ __forceinline__ V sub(V a, V b) { return dd_sub(a, b); }
-    static __device__ __forceinline__ V vdel(V pa, V pb, const C& c, int d) {
+    template <bool FAST>
+    static __device__ __forceinline__ V vdel(V pa, V pb, const C& c, int d, uint32_t*) {
         const V m = mulc(dd_sub(pa, pb), c.cv[d], c.cvr[d]);
         return {-m.h, -m.l};
     }
-    static __device__ __forceinline__ V pdel(V ax, V ay, V az, const C& c) {
+    template <bool FAST>
+    static __device__ __forceinline__ V pdel(V ax, V ay, V az, const C& c, uint32_t*) {
         const V m = dd_add(dd_add(mulc(ax, c.ck[0], c.ckr[0]), mulc(ay, c.ck[1], c.ckr[1])), mulc(az, c.ck[2], c.ckr[2]));
         return {-m.h, -m.l};
     }
@@ -162,7 +176,8 @@ __global__ void __launch_bounds__(32 * ACU_W, AR::kMinBlocks) acoustic_step_kern
         const S vo = xv ? a.Vz[oP] : S(0);
         const bool inner = m_vz && z0 >= 1;
         const S pm = (xv && inner) ? a.P[oP - sP] : S(0);
-        vzc = inner ? AR::add(AR::in(vo, big), AR::vdel(pc, AR::in(pm, big), c, 2)) : AR::in(vo, big);
+        vzc = inner ? AR::add(AR::in(vo, big), AR::template vdel<false>(pc, AR::in(pm, big), c, 2, nullptr))
+                    : AR::in(vo, big);
         if (xv && z0 == 0) a.Vz2[oP] = vo;  // face 0 is outside @inn(Vz)
     }
 
@@ -194,48 +209,58 @@ __global__ void __launch_bounds__(32 * ACU_W, AR::kMinBlocks) acoustic_step_kern
             f_xev = e_hi ? a.Vx[oX + sX + 1] : S(0);
         }
 
-        // Vy on faces y and y + 1
-        V vyn0 = AR::in(vy0, big), vyn1 = AR::in(vy1, big);
-        S st0 = vy0;
-        if (m_vy0 && zin) {
-            const V dl = AR::vdel(pc, AR::in(plo, big), c, 1);
-            vyn0 = AR::add(vyn0, dl);
-            st0 = AR::store(vy0, vyn0, dl);
-        }
-        if (m_vy1 && zin) {
-            const V dl = AR::vdel(AR::in(phi, big), pc, c, 1);
-            vyn1 = AR::add(vyn1, dl);
-            if (last_y) a.Vy2[oY + nx] = AR::store(vy1, vyn1, dl);
-        } else if (xv && last_y) {
-            a.Vy2[oY + nx] = vy1;  // face ny is outside @inn(Vy)
-        }
-        // Vx on face x (this lane) and face x + 1 (the next lane, or computed here at the edges)
-        V pxm = AR::shfl_up(pc);
-        if (lane == 0) pxm = AR::in(xep, big);
-        const bool in_x = m_vx && zin;
-        const V vxo_v = AR::in(vxo, big);
-        const V dlx = AR::vdel(pc, pxm, c, 0);
-        const V vxn = in_x ? AR::add(vxo_v, dlx) : vxo_v;
-        V vxp = AR::shfl_down(vxn);
-        if (e_hi) {
-            const V vo1 = AR::in(xev, big);
-            vxp = (m_vx1 && zin) ? AR::add(vo1, AR::vdel(AR::in(xep, big), pc, c, 0)) : vo1;
-            if (last_x) a.Vx2[oX + 1] = xev;  // face nx is outside @inn(Vx)
-        }
-        // Vz on face z + 1
-        const bool in_z = m_vz && z + 1 <= nz - 1;
-        const V vzo_v = AR::in(vzo, big);
-        const V pnv = AR::in(pn, big);
-        const V dlz = AR::vdel(pnv, pc, c, 2);
-        const V vzn = in_z ? AR::add(vzo_v, dlz) : vzo_v;
-        // P
-        const V dlp = AR::pdel(AR::sub(vxp, vxn), AR::sub(vyn1, vyn0), AR::sub(vzn, vzc), c);
-        if (xv) {
-            a.Vy2[oY] = st0;
-            a.Vx2[oX] = in_x ? AR::store(vxo, vxn, dlx) : vxo;
-            a.Vz2[oP + sP] = in_z ? AR::store(vzo, vzn, dlz) : vzo;
-            a.P2[oP] = AR::store(pr, AR::add(pc, dlp), dlp);
-        }
+        V vzn, pnv;
+        // the new faces of the plane and its P. Quotients are taken without testing their dividends;
+        // a warp that met one too small for that evaluates and stores the plane again with the tests.
+        auto plane = [&](auto fast, uint32_t* key) {
+            constexpr bool F = decltype(fast)::value;
+            // Vy on faces y and y + 1
+            V vyn0 = AR::in(vy0, big), vyn1 = AR::in(vy1, big);
+            S st0 = vy0;
+            if (m_vy0 && zin) {
+                const V dl = AR::template vdel<F>(pc, AR::in(plo, big), c, 1, key);
+                vyn0 = AR::add(vyn0, dl);
+                st0 = AR::store(vy0, vyn0, dl);
+            }
+            if (m_vy1 && zin) {
+                const V dl = AR::template vdel<F>(AR::in(phi, big), pc, c, 1, key);
+                vyn1 = AR::add(vyn1, dl);
+                if (last_y) a.Vy2[oY + nx] = AR::store(vy1, vyn1, dl);
+            } else if (xv && last_y) {
+                a.Vy2[oY + nx] = vy1;  // face ny is outside @inn(Vy)
+            }
+            // Vx on face x (this lane) and face x + 1 (the next lane, or computed here at the edges)
+            V pxm = AR::shfl_up(pc);
+            if (lane == 0) pxm = AR::in(xep, big);
+            const bool in_x = m_vx && zin;
+            const V vxo_v = AR::in(vxo, big);
+            const V dlx = AR::template vdel<F>(pc, pxm, c, 0, key);
+            const V vxn = in_x ? AR::add(vxo_v, dlx) : vxo_v;
+            V vxp = AR::shfl_down(vxn);
+            if (e_hi) {
+                const V vo1 = AR::in(xev, big);
+                vxp = (m_vx1 && zin) ? AR::add(vo1, AR::template vdel<F>(AR::in(xep, big), pc, c, 0, key)) : vo1;
+                if (last_x) a.Vx2[oX + 1] = xev;  // face nx is outside @inn(Vx)
+            }
+            // Vz on face z + 1
+            const bool in_z = m_vz && z + 1 <= nz - 1;
+            const V vzo_v = AR::in(vzo, big);
+            pnv = AR::in(pn, big);
+            const V dlz = AR::template vdel<F>(pnv, pc, c, 2, key);
+            vzn = in_z ? AR::add(vzo_v, dlz) : vzo_v;
+            // P
+            const V dlp = AR::template pdel<F>(AR::sub(vxp, vxn), AR::sub(vyn1, vyn0), AR::sub(vzn, vzc), c, key);
+            if (xv) {
+                a.Vy2[oY] = st0;
+                a.Vx2[oX] = in_x ? AR::store(vxo, vxn, dlx) : vxo;
+                a.Vz2[oP + sP] = in_z ? AR::store(vzo, vzn, dlz) : vzo;
+                a.P2[oP] = AR::store(pr, AR::add(pc, dlp), dlp);
+            }
+        };
+        uint32_t key = 0xFFFFFFFFu;
+        plane(std::true_type{}, &key);
+        if constexpr (AR::kRetest)
+            if (__any_sync(0xFFFFFFFFu, key < c.lo)) plane(std::false_type{}, &key);
         vzc = vzn;
         pc = pnv;
         pr = pn;
@@ -324,12 +349,15 @@ int acoustic_step(const ps_array& Vx, const ps_array& Vy, const ps_array& Vz, co
     if (P.dtype == PS_F32) {
         if (fp64_mode != PS_FP64_IEEE) return fail(PS_ERR_UNSUPPORTED, "ps_acoustic3d_step: fp64_mode needs FP64 arrays");
         // FP32: the scalars are FP32 numbers, dt/ρ and dt·k evaluated in FP32 (Float32 Data.Number)
-        AcuIeee<float>::C c{(float)dt / (float)rho, (float)dt * (float)k,
-                            {make_div((float)dx), make_div((float)dy), make_div((float)dz)}};
+        const float h[3] = {(float)dx, (float)dy, (float)dz};
+        AcuIeee<float>::C c{(float)dt / (float)rho, (float)dt * (float)k, {}, 0u};
+        c.lo = make_div3(h, c.h);
         return launch_acoustic<AcuIeee<float>>(Vx, Vy, Vz, P, Vx2, Vy2, Vz2, P2, c, st, s);
     }
     if (fp64_mode == PS_FP64_IEEE) {
-        AcuIeee<double>::C c{dt / rho, dt * k, {make_div(dx), make_div(dy), make_div(dz)}};
+        const double h[3] = {dx, dy, dz};
+        AcuIeee<double>::C c{dt / rho, dt * k, {}, 0u};
+        c.lo = make_div3(h, c.h);
         return launch_acoustic<AcuIeee<double>>(Vx, Vy, Vz, P, Vx2, Vy2, Vz2, P2, c, st, s);
     }
     if (fp64_mode != PS_FP64_SPLIT)

@@ -4,7 +4,11 @@
 #include <cuda.h>  // CUtensorMap and its enums only; the driver is reached through cudart
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
+#include <algorithm>
+#include <cmath>
+#include <limits>
 #include <utility>
 
 #include "ps_gb300.h"
@@ -190,60 +194,170 @@ __device__ __forceinline__ void ordered_tile_done(const TileOrder& o) {
 // ---------------------------------------------------------------------------------------
 // Division by a number known on the host, correctly rounded.
 // ---------------------------------------------------------------------------------------
-// Markstein's method (P. W. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", IBM J. Res. Develop. 34 (1990) 111-119): with y = RN(1/b) and a quotient
-// q within one ulp of a/b, the remainder r = a - b q is exact in one FMA and RN(q + r y) = RN(a/b).
-// The first quotient RN(a y) can be 1.5 ulps off, so one FMA correction brings it within an ulp and
-// a second gives the correctly rounded quotient: 1 multiply + 4 FMAs against the general division's
-// reciprocal iteration and slow-path test. Dividends outside [lo, hi] (tiny, huge, non-finite; zero
-// is a * y, with the quotient's sign) take the IEEE division; for divisors outside [2^-20, 2^20]
-// (FP32) or [2^-60, 2^60] (FP64) the host sets lo > hi and every division takes it. lo keeps the
-// quotient normal and the remainder a - bq, a multiple of 2^(e(a) - 2p + 1), representable
-// (subnormal remainders are exact); hi keeps a*y and the quotient finite. Results equal a / b bit
-// for bit (checked against the IEEE division by ps_check_division).
+// Method of N. Brisebarre, J.-M. Muller and S. K. Raina ("Accelerating correctly rounded floating-point
+// division when the divisor is known in advance", IEEE Trans. Computers 53 (2004) 1069-1072): with
+// 1/b held as yh + yl, RN(a yh + RN(a yl)) -- one multiply and one FMA -- equals RN(a/b) unless a/b
+// lies within about 2^-2p of a midpoint between neighbouring p-bit numbers. Such dividends are few
+// and computable: with integer significands A, B in [2^(p-1), 2^p) and a midpoint M/2^p (A >= B) or
+// M/2^(p+1) (A < B), the distance is |k| / (2^p B) or |k| / (2^(p+1) B), k = 2^p A - M B (2^(p+1) A - M B)
+// != 0, so they solve a linear congruence for each small k. make_div solves it, tries the scheme on
+// each solution against the IEEE division and moves yl by an ulp until all agree (significands
+// enter only, so that covers every exponent). yh is 1/b rounded towards zero, so yl has its sign
+// and a zero dividend keeps the quotient's sign; yl is never 0, so infinities pass too.
+//
+// Dividends below `lo` in magnitude, where a yl or the quotient could be subnormal (zeros
+// excepted), take div_slow; so do all dividends of divisors outside [2^-20, 2^20] (FP32) or
+// [2^-60, 2^60] (FP64), and of the 3 % of divisors for which no yl within an ulp passes (a wider search
+// finds no more of them). Large dividends, infinities and NaN need no test: the quotient overflows
+// where a/b does. The test is on integer keys (zero has the largest) and costs no FP64 instruction;
+// the FP64 division is 2 FP64 instructions instead of 7 (GB300 issues 2 FP64 per clock per SM).
+//
+// div_slow, for a divisor without a pair: Markstein's method (P. W. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Develop. 34 (1990)
+// 111-119): with y = RN(1/b) and a quotient q within one ulp of a/b, the remainder r = a - b q is
+// exact in one FMA and RN(q + r y) = RN(a/b). The first quotient RN(a y) can be 1.5 ulps off, so one
+// correction brings it within an ulp and a second rounds it correctly: 1 multiply + 4 FMAs, for
+// dividends that keep a y and the quotient normal and the remainder, a multiple of 2^(e(a) - 2p + 1),
+// representable. Everything else there is the IEEE division. Results equal a / b bit for bit (checked
+// against the IEEE division by ps_check_division).
 template <typename T>
 struct DivC {
-    T b, y, lo, hi;
+    T b, yh, yl;
+    uint32_t lo;   // div_key of the smallest dividend of the fast path
+    uint32_t fix;  // no pair: yh = RN(1/b), yl = 0 (exact for zeros, the only dividends let through)
 };
+
+// Key of a dividend: grows with |a|, largest for zeros.
+__host__ __device__ __forceinline__ uint32_t div_key_bits(uint32_t hi, uint32_t rest) {
+    return (hi << 1) + (rest ? 0u : 0xFFFFFFFFu);
+}
+__device__ __forceinline__ uint32_t div_key(float a) { return div_key_bits(__float_as_uint(a), 0u); }
+__device__ __forceinline__ uint32_t div_key(double a) {
+    return div_key_bits((uint32_t)__double2hiint(a), (uint32_t)__double2loint(a));
+}
+
+// Whether RN(a yh + RN(a yl)) = RN(a/b) for every dividend that can fail: b = B in [2^(p-1), 2^p).
+template <typename T>
+inline bool div_pair_exact(T b, T yh, T yl) {
+    constexpr int p = sizeof(T) == 4 ? 24 : 53;
+    const uint64_t B = (uint64_t)b;
+    int t = 0;
+    while (!((B >> t) & 1)) t++;
+    const uint64_t Bo = B >> t;
+    uint64_t inv = Bo;  // Bo^-1 mod 2^64 (Newton)
+    for (int i = 0; i < 6; i++) inv *= 2 - Bo * inv;
+    // relative error of the pair: at most 3/2 ulp(yl) (yl rounded, then moved by one ulp), half an ulp of
+    // a yl and 2^-2p / 4 from its underflow, together 8.25 2^-2p at most (|yl| <= 2^(1-p) yh): |k| < 17 for
+    // A < B, half of that for A >= B
+    for (int side = 0; side < 2; side++) {
+        const int m = p + side;  // midpoints M / 2^m, M odd in (2^p, 2^(p+1))
+        for (int k = -20; k <= 20; k++) {
+            if (k == 0 || t > 4 || (k & ((1 << t) - 1))) continue;  // k is a multiple of 2^t
+            // M Bo = -k / 2^t (mod 2^(m - t)): 2^t or 2^(t+1) values of M below 2^(p+1)
+            const uint64_t mod = 1ull << (m - t);
+            const uint64_t M0 = ((uint64_t)(-(int64_t)(k >> t)) * inv) & (mod - 1);
+            for (uint64_t M = M0; M < (2ull << p); M += mod) {
+                if (M <= (1ull << p) || !(M & 1)) continue;
+                const __int128 v = (__int128)M * B + k;
+                const uint64_t A = (uint64_t)(v >> m);
+                if (((__int128)A << m) != v || A < (1ull << (p - 1)) || A >= (1ull << p)) continue;
+                if (side == 0 ? A < B : A >= B) continue;
+                const T a = (T)A;
+                if (std::fma(a, yh, a * yl) != a / b) return false;
+            }
+        }
+    }
+    return true;
+}
 template <typename T>
 inline DivC<T> make_div(T b) {
     const T lim = sizeof(T) == 4 ? (T)0x1p20 : (T)0x1p60;
-    const T a = b < 0 ? -b : b;
+    const T ab = std::fabs(b);
     DivC<T> d;
     d.b = b;
-    if (a >= 1 / lim && a <= lim) {
-        d.y = (T)1 / b;
-        d.lo = sizeof(T) == 4 ? (T)0x1p-100 : (T)0x1p-960;
-        d.hi = sizeof(T) == 4 ? (T)0x1p70 : (T)0x1p900;
-    } else {
-        d.y = 0;
-        d.lo = 1;
-        d.hi = 0;
+    d.lo = 0xFFFFFFFFu;  // zeros only: their quotient is a zero, or NaN for a zero or NaN divisor
+    d.yh = ab > 0 ? std::copysign((T)1, b) : std::numeric_limits<T>::quiet_NaN();
+    d.yl = d.yh;
+    d.fix = 0;
+    if (!(ab >= 1 / lim && ab <= lim)) return d;
+    constexpr int p = sizeof(T) == 4 ? 24 : 53;
+    const int e = std::ilogb(ab);
+    const T B = std::ldexp(ab, p - 1 - e);  // the integer significand
+    T yh = (T)1 / B;
+    T r = std::fma(-B, yh, (T)1);  // exact
+    if (r < 0) {
+        yh = std::nextafter(yh, (T)0);
+        r = std::fma(-B, yh, (T)1);
     }
+    // a power of two has r = 0: any yl far below the last place of yh leaves the exact quotient
+    const T y0 = r == 0 ? std::ldexp(yh, -2 * p) : r / B;
+    for (int j = 0; j < 3; j++) {
+        const T yl = j == 0 ? y0 : std::nextafter(y0, j == 1 ? (T)1 : (T)0);
+        if (!(yl > 0) || !div_pair_exact(B, yh, yl)) continue;
+        d.yh = std::copysign(std::ldexp(yh, p - 1 - e), b);
+        d.yl = std::copysign(std::ldexp(yl, p - 1 - e), b);
+        // quotients of 2^-100 (2^-960) and above: a yl is rounded to 2^-50 (2^-113) of the quotient or better
+        const T lo = std::ldexp((T)1, e + 1 - (sizeof(T) == 4 ? 100 : 960));
+        if (sizeof(T) == 4) {
+            uint32_t u;
+            memcpy(&u, &lo, 4);
+            d.lo = div_key_bits(u, 0u);
+        } else {
+            uint64_t u;
+            memcpy(&u, &lo, 8);
+            d.lo = div_key_bits((uint32_t)(u >> 32), 0u);
+        }
+        return d;
+    }
+    d.yh = (T)1 / b;
+    d.yl = 0;
+    d.fix = 1;
     return d;
 }
-__device__ __forceinline__ float div_c(float a, const DivC<float>& d) {
-    const float aa = fabsf(a);
-    if (aa >= d.lo && aa <= d.hi) {
-        float q = a * d.y;
+// The divisors of one kernel and the key every one of them takes without a test; returns that key.
+template <typename T>
+inline uint32_t make_div3(const T b[3], DivC<T> d[3]) {
+    d[0] = make_div(b[0]);
+    d[1] = b[1] == b[0] ? d[0] : make_div(b[1]);
+    d[2] = b[2] == b[0] ? d[0] : b[2] == b[1] ? d[1] : make_div(b[2]);
+    return std::max(d[0].lo, std::max(d[1].lo, d[2].lo));
+}
+__device__ __forceinline__ float div_pair(float a, const DivC<float>& d) { return fmaf(a, d.yh, a * d.yl); }
+__device__ __forceinline__ double div_pair(double a, const DivC<double>& d) { return fma(a, d.yh, a * d.yl); }
+__device__ __forceinline__ float div_slow(float a, const DivC<float>& d) {
+    const uint32_t k = div_key(a);
+    if (d.fix && k >= 0x1AFFFFFFu && k < 0xC5000000u) {  // 2^-100 <= |a| <= 2^70
+        float q = a * d.yh;
         float r = fmaf(-q, d.b, a);
-        q = fmaf(r, d.y, q);
+        q = fmaf(r, d.yh, q);
         r = fmaf(-q, d.b, a);
-        return fmaf(r, d.y, q);
+        return fmaf(r, d.yh, q);
     }
-    return (aa == 0.0f && d.lo <= d.hi) ? a * d.y : a / d.b;
+    return a / d.b;
 }
-__device__ __forceinline__ double div_c(double a, const DivC<double>& d) {
-    const double aa = fabs(a);
-    if (aa >= d.lo && aa <= d.hi) {
-        double q = a * d.y;
+__device__ __forceinline__ double div_slow(double a, const DivC<double>& d) {
+    const uint32_t k = div_key(a);
+    if (d.fix && k >= 0x07DFFFFFu && k < 0xF0600000u) {  // 2^-960 <= |a| <= 2^900
+        double q = a * d.yh;
         double r = fma(-q, d.b, a);
-        q = fma(r, d.y, q);
+        q = fma(r, d.yh, q);
         r = fma(-q, d.b, a);
-        return fma(r, d.y, q);
+        return fma(r, d.yh, q);
     }
-    return (aa == 0.0 && d.lo <= d.hi) ? a * d.y : a / d.b;
+    return a / d.b;
 }
+template <typename T>
+__device__ __forceinline__ T div_c(T a, const DivC<T>& d) {
+    return div_key(a) >= d.lo ? div_pair(a, d) : div_slow(a, d);
+}
+
+// A divisor whose quotients are taken without the test: the smallest key of the dividends is kept in
+// *key, and the caller computes again with DivC where *key came out below its divisors' lo.
+template <typename T>
+struct DivF {
+    const DivC<T>& d;
+    uint32_t* key;
+};
 
 // a / h for statement helpers used with a plain divisor (host or device) or a DivC (device)
 template <typename T>
@@ -253,6 +367,11 @@ __host__ __device__ __forceinline__ T dvd(T a, T h) {
 template <typename T>
 __device__ __forceinline__ T dvd(T a, const DivC<T>& h) {
     return div_c(a, h);
+}
+template <typename T>
+__device__ __forceinline__ T dvd(T a, const DivF<T>& h) {
+    *h.key = min(*h.key, div_key(a));
+    return div_pair(a, h.d);
 }
 
 // ---------------------------------------------------------------------------------------

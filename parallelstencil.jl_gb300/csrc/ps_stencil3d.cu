@@ -371,6 +371,8 @@ template <typename T>
 struct DiffParams {
     T lam, dt, hx, hy, hz;
     DivC<T> q[3];  // the divisors hx*hx, hy*hy, hz*hz of the `/dx^2` form
+    uint32_t lo;   // the smallest dividend key all three take without a test
+    T h2[3];       // hx*hx, hy*hy, hz*hz of the `*_dx^2` form
 };
 
 // One cell of the diffusion statement in form FORM (see ps_diffusion_form). Operation order
@@ -383,10 +385,14 @@ __device__ __forceinline__ T diff_cell(const DiffParams<T>& p, T Tc, T Txm, T Tx
         T d2y = (Typ - Tc) - (Tc - Tym);
         T d2z = (Tzp - Tc) - (Tc - Tzm);
         T s;
-        if constexpr (FORM == PS_DIFF_DIV)
-            s = (div_c(d2x, p.q[0]) + div_c(d2y, p.q[1])) + div_c(d2z, p.q[2]);
-        else
-            s = (d2x * (p.hx * p.hx) + d2y * (p.hy * p.hy)) + d2z * (p.hz * p.hz);
+        if constexpr (FORM == PS_DIFF_DIV) {
+            if (min(div_key(d2x), min(div_key(d2y), div_key(d2z))) >= p.lo)
+                s = (div_pair(d2x, p.q[0]) + div_pair(d2y, p.q[1])) + div_pair(d2z, p.q[2]);
+            else
+                s = (div_c(d2x, p.q[0]) + div_c(d2y, p.q[1])) + div_c(d2z, p.q[2]);
+        } else {
+            s = (d2x * p.h2[0] + d2y * p.h2[1]) + d2z * p.h2[2];
+        }
         return Tc + p.dt * ((p.lam * ci) * s);
     } else {
         T kxp, kxm, kyp, kym, kzp, kzm;
@@ -770,9 +776,19 @@ static dim3 grid3(int64_t wx, int64_t wy, int64_t wz, dim3 blk) {
 }
 
 template <typename T>
-static DiffParams<T> diff_params(double lam, double dt, double hx, double hy, double hz) {
+static DiffParams<T> diff_params(int form, double lam, double dt, double hx, double hy, double hz) {
     const T x = (T)hx, y = (T)hy, z = (T)hz;
-    return DiffParams<T>{(T)lam, (T)dt, x, y, z, {make_div((T)(x * x)), make_div((T)(y * y)), make_div((T)(z * z))}};
+    DiffParams<T> p{};
+    p.lam = (T)lam;
+    p.dt = (T)dt;
+    p.hx = x;
+    p.hy = y;
+    p.hz = z;
+    p.h2[0] = x * x;
+    p.h2[1] = y * y;
+    p.h2[2] = z * z;
+    if (form == PS_DIFF_DIV) p.lo = make_div3(p.h2, p.q);
+    return p;
 }
 
 int launch_diffusion_split(int form, const ps_array& T2, const ps_array& Tin, const ps_array& Ci, const ps_array* lam,
@@ -869,7 +885,7 @@ static int dispatch_diffusion(int form, const ps_array& T2, const ps_array& Tin,
                               const ps_array* lam, double lam_s, double dt, double hx, double hy, double hz,
                               const Box& cb, int memopt, int loopsize, cudaStream_t s, int* d_err,
                               HideReq* hr = nullptr) {
-    DiffParams<T> p = diff_params<T>(lam_s, dt, hx, hy, hz);
+    DiffParams<T> p = diff_params<T>(form, lam_s, dt, hx, hy, hz);
     switch (form) {
     case PS_DIFF_DIV:
         return launch_diffusion<T, PS_DIFF_DIV>(T2, Tin, Ci, nullptr, p, cb, memopt, loopsize, s, d_err, hr);

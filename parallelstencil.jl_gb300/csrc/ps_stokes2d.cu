@@ -68,12 +68,14 @@ template <typename T>
 struct S2P {
     DivC<T> dx, dy;
     T dampX, dampY, Vsc, Ptsc, min_dxy2, max_nxy;
+    uint32_t lo;  // the smallest dividend key both divisors take without a test
 };
 
 template <typename T>
 static S2P<T> s2p(const ps_stokes2d_params& p) {
-    return S2P<T>{make_div((T)p.dx), make_div((T)p.dy), (T)p.dampX,    (T)p.dampY,
-                  (T)p.Vsc,          (T)p.Ptsc,         (T)p.min_dxy2, (T)p.max_nxy};
+    const DivC<T> dx = make_div((T)p.dx), dy = make_div((T)p.dy);
+    return S2P<T>{dx,        dy,        (T)p.dampX,    (T)p.dampY,    (T)p.Vsc,
+                  (T)p.Ptsc, (T)p.min_dxy2, (T)p.max_nxy, std::max(dx.lo, dy.lo)};
 }
 
 #define A2(a, i, j, n0) (a)[(int64_t)(i) + (int64_t)(n0) * (int64_t)(j)]
@@ -218,6 +220,16 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+// Evaluates a statement without testing each dividend, and again with the tests (and the IEEE
+// division where they fail) in the rare case that one of its dividends is too small: one test and one
+// branch per statement instead of one per division.
+#define S2_DIV(stmt)                                                            \
+    do {                                                                        \
+        uint32_t key_ = 0xFFFFFFFFu;                                            \
+        stmt(DivF<T>{p.dx, &key_}, DivF<T>{p.dy, &key_});                       \
+        if (key_ < p.lo) stmt(p.dx, p.dy);                                      \
+    } while (0)
+
 // I: index type (int where every array has fewer than 2^31 elements: fewer instructions per cell).
 // RED: a.red is set (the FP64 sums are compiled in only then: the conversions to double run on the
 // FP64 pipe even when predicated off).
@@ -288,13 +300,17 @@ __global__ void __launch_bounds__(S2_TX* s2_ty<T>()) s2_fused(S2Fused<T> a, S2P<
             T vx0 = sVx[v][u], vx1 = sVx[v][u + 1];  // Vx faces gi, gi+1 of row gj
             T vy0 = sVy[v][u], vy1 = sVy[v + 1][u];  // Vy faces gj, gj+1 of column gi
             T mus = sMus[v][u];
-            T d = s2_divV(vx0, vx1, vy0, vy1, p.dx, p.dy);
+            T d, txx, tyy;
+            auto strain = [&](auto hx, auto hy) {
+                d = s2_divV(vx0, vx1, vy0, vy1, hx, hy);
+                txx = s2_tau_nn(mus, vx0, vx1, d, hx);
+                tyy = s2_tau_nn(mus, vy0, vy1, d, hy);
+            };
+            S2_DIV(strain);
             T dtp = READ_DT ? c_dt[q] : s2_dtPt(p.Ptsc, mus, p.max_nxy);
             T dp = d;
             if constexpr (DEFECT) dp = d + c_f[q];
             T pn = c_p[q] - dtp * dp;
-            T txx = s2_tau_nn(mus, vx0, vx1, d, p.dx);
-            T tyy = s2_tau_nn(mus, vy0, vy1, d, p.dy);
             sP[v][u] = pn;
             sTxx[v][u] = txx;
             sTyy[v][u] = tyy;
@@ -311,8 +327,12 @@ __global__ void __launch_bounds__(S2_TX* s2_ty<T>()) s2_fused(S2Fused<T> a, S2P<
         }
         // corner (gi, gj): between cells gi..gi+1, gj..gj+1
         if (gi >= 0 && gi < nx - 1 && gj >= 0 && gj < ny - 1) {
-            T t = s2_tau_xy(sMus[v][u], sMus[v][u + 1], sMus[v + 1][u], sMus[v + 1][u + 1],
-                            sVx[v + 1][u + 1] - sVx[v][u + 1], sVy[v + 1][u + 1] - sVy[v + 1][u], p.dx, p.dy);
+            T t;
+            auto shear = [&](auto hx, auto hy) {
+                t = s2_tau_xy(sMus[v][u], sMus[v][u + 1], sMus[v + 1][u], sMus[v + 1][u + 1],
+                              sVx[v + 1][u + 1] - sVx[v][u + 1], sVy[v + 1][u + 1] - sVy[v + 1][u], hx, hy);
+            };
+            S2_DIV(shear);
             sTxy[v][u] = t;
             if constexpr (STORE_TMP)
                 if (u >= 1 && v >= 1) a.txy[gi + (nx - 1) * gj] = t;
@@ -327,7 +347,11 @@ __global__ void __launch_bounds__(S2_TX* s2_ty<T>()) s2_fused(S2Fused<T> a, S2P<
     if (xin) {
         T vnew = sVx[v][u];
         if (xinner) {
-            T r = s2_Rx(sTxx[v][u - 1], sTxx[v][u], sTxy[v - 1][u - 1], sTxy[v][u - 1], sP[v][u - 1], sP[v][u], p.dx, p.dy);
+            T r;
+            auto resid = [&](auto hx, auto hy) {
+                r = s2_Rx(sTxx[v][u - 1], sTxx[v][u], sTxy[v - 1][u - 1], sTxy[v][u - 1], sP[v][u - 1], sP[v][u], hx, hy);
+            };
+            S2_DIV(resid);
             if constexpr (DEFECT) r = r + x_f;
             T dv = p.dampX * x_dv + r;
             a.dVxdt[rxi] = dv;
@@ -346,8 +370,12 @@ __global__ void __launch_bounds__(S2_TX* s2_ty<T>()) s2_fused(S2Fused<T> a, S2P<
     if (yin) {
         T vnew = sVy[v][u];
         if (yinner) {
-            T r = s2_Ry_core(sTyy[v - 1][u], sTyy[v][u], sTxy[v - 1][u - 1], sTxy[v - 1][u], sP[v - 1][u], sP[v][u], p.dx,
-                             p.dy);
+            T r;
+            auto resid = [&](auto hx, auto hy) {
+                r = s2_Ry_core(sTyy[v - 1][u], sTyy[v][u], sTxy[v - 1][u - 1], sTxy[v - 1][u], sP[v - 1][u], sP[v][u], hx,
+                               hy);
+            };
+            S2_DIV(resid);
             r = r + y_f;  // the defect source, or the buoyancy average of the two cells
             T dv = p.dampY * y_dv + r;
             a.dVydt[ryi] = dv;

@@ -139,3 +139,13 @@ def test_constant_division_equals_ieee_division(ps, b):
         bad = ctypes.c_int64(-1)
         _lib.call("ps_check_division", float(b), dtype, n, 12345, ctypes.byref(bad), None)
         assert bad.value == 0, (b, dtype, bad.value)
+
+
+@pytest.mark.parametrize("b", [float.fromhex("0x1.6e6c1ep-4"), float.fromhex("0x1.e7a9a78a18f56p-2"),
+                               10.0 / 1022, 1.0 / 1022, 10.0 / 509, 2.0 ** -7, 3.0 * 2.0 ** -9, -(2.0 - 2.0 ** -22),
+                               1.0 + 2.0 ** -22, 2.0 ** -20, 2.0 ** 21])
+def test_division_by_reciprocal_pairs(ps, b):
+    """More divisors of the two-instruction division: grid spacings, powers of two, significands at
+    both ends of a binade, the ends of its range, and divisors that no reciprocal pair serves (the
+    first two, found on the CPU), against the IEEE division as above."""
+    test_constant_division_equals_ieee_division(ps, b)
