@@ -359,6 +359,17 @@ struct DivF {
     uint32_t* key;
 };
 
+// x * 2^k by an integer addition to the exponent (a multiplication is an FP64 instruction). Equal to
+// the product, bit for bit, for zeros and wherever x and x 2^k are normal: *key keeps x's key as
+// DivF does, so small x make the caller compute again, and becomes 0 for |x| >= 2^900, infinities and
+// NaN. lo >= 2^-1019 with the divisors' range, so k >= -2 keeps the result normal.
+__device__ __forceinline__ double scale_pow2(double x, int k, uint32_t* key) {
+    const int hi = __double2hiint(x);
+    const uint32_t kx = div_key(x);
+    *key = min(*key, kx < 0xF0600000u || kx == 0xFFFFFFFFu ? kx : 0u);
+    return __hiloint2double(kx == 0xFFFFFFFFu ? hi : hi + (k << 20), __double2loint(x));
+}
+
 // a / h for statement helpers used with a plain divisor (host or device) or a DivC (device)
 template <typename T>
 __host__ __device__ __forceinline__ T dvd(T a, T h) {

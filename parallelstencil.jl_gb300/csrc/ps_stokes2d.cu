@@ -6,17 +6,16 @@
 //                             below so all paths round identically
 //   one-to-one kernels        compute_timesteps!, compute_P!, compute_τ!, compute_dV!, compute_V!,
 //                             bc_x!, bc_y! -- the drop-in replacements of the six `@parallel` calls
-//   s2_fused                  one whole PT iteration in one kernel: a CTA stages its tile of
-//                             Vx, Vy, Pt, Mus (+1-2 cell halo) in shared memory, recomputes the halo
-//                             of ∇V / Pt / τ, updates dVdτ and V of its own faces and applies the
-//                             free-slip copies. Old/new V and Pt are ping-pong buffers, so results are
-//                             identical to the six-kernel sequence. Optional fused FP64 reduction of
-//                             Σ|Rx|, Σ|Ry|, Σ|∇V| (warp shuffles + one atomicAdd per block).
+//   s2_march                  one whole PT iteration in FP32: warps march along y with the previous row in
+//                             registers and the neighbour columns by shuffles. Old/new V and Pt are
+//                             ping-pong buffers, so results are identical to the six-kernel sequence.
+//                             Optional fused FP64 reduction of Σ|Rx|, Σ|Ry|, Σ|∇V|.
+//   s2_cells, s2_faces        the FP64 iteration in place, one thread per position, the same reductions.
 //   s2_residual64             FP64 residuals of the current state (no pseudo-time update) for the
 //                             defect-correction outer loop.
 //   ps_stokes2d_solve         PT solve to `tol` in FP64 (mode 0) or with FP32 PT sweeps on the
 //                             correction and an FP64 residual / update / convergence check (mode 1).
-//                             Iterations run as CUDA graphs of `nout` fused kernels.
+//                             Iterations run as CUDA graphs of `nout` iterations.
 #include <math.h>
 #include <string.h>
 
@@ -50,10 +49,27 @@ template <typename T, typename H>
 __host__ __device__ __forceinline__ T s2_tau_nn(T mus, T v0, T v1, T divV, H h) {
     return (T(2.0) * mus) * (dvd(v1 - v0, h) - (T(1.0) / T(3.0)) * divV);
 }
+// msum: the four corner viscosities summed in the macro's order ((m00 + m10) + m01) + m11
+template <typename T, typename H>
+__host__ __device__ __forceinline__ T s2_tau_xy_sum(T msum, T dyVx, T dxVy, H dx, H dy) {
+    T av = msum * T(0.25);
+    return (T(2.0) * av) * (T(0.5) * (dvd(dyVx, dy) + dvd(dxVy, dx)));
+}
 template <typename T, typename H>
 __host__ __device__ __forceinline__ T s2_tau_xy(T m00, T m10, T m01, T m11, T dyVx, T dxVy, H dx, H dy) {
-    T av = (((m00 + m10) + m01) + m11) * T(0.25);
-    return (T(2.0) * av) * (T(0.5) * (dvd(dyVx, dy) + dvd(dxVy, dx)));
+    return s2_tau_xy_sum(((m00 + m10) + m01) + m11, dyVx, dxVy, dx, dy);
+}
+// The same two statements in FP64 with the factors 2, 0.25 and 0.5 gathered into one power of two applied
+// to the product (equal bit for bit while nothing on the way is subnormal or overflows: the keys).
+__device__ __forceinline__ double s2_tau_nn(double mus, double v0, double v1, double divV, DivF<double> h) {
+    const double e = dvd(v1 - v0, h) - (1.0 / 3.0) * divV;
+    if ((__double2hiint(mus) & 0x7FFFFFFF) >= 0x78300000) *h.key = 0u;  // |mus| < 2^900: 2 mus is finite
+    return scale_pow2(mus * e, 1, h.key);
+}
+__device__ __forceinline__ double s2_tau_xy_sum(double msum, double dyVx, double dxVy, DivF<double> dx, DivF<double> dy) {
+    const double e = dvd(dyVx, dy) + dvd(dxVy, dx);
+    *dx.key = min(*dx.key, min(div_key(msum), div_key(e)));
+    return scale_pow2(msum * e, -2, dx.key);
 }
 template <typename T, typename H>
 __host__ __device__ __forceinline__ T s2_Rx(T txx_l, T txx_r, T txy_b, T txy_t, T p_l, T p_r, H dx, H dy) {
@@ -169,14 +185,6 @@ __global__ void s2_bc_y_k(T* A, int64_t n0, int64_t n1) {
 // =======================================================================================
 // Fused PT iteration
 // =======================================================================================
-constexpr int S2_TX = 32;
-// tile rows: FP64 16 (the halo it recomputes is FP64-pipe work: 0.366 -> 0.354 ms per 1023^2
-// iteration), FP32 8 (16 measured slower there)
-template <typename T>
-__host__ __device__ constexpr int s2_ty() {
-    return sizeof(T) == 8 ? 16 : 8;
-}
-
 template <typename T>
 struct S2Fused {
     // state in / out (ping-pong) and in-place pseudo-velocities
@@ -190,7 +198,6 @@ struct S2Fused {
     T* dVydt;
     const T* Mus;
     const T* Rog;  // PLAIN: buoyancy (nx, ny); DEFECT: unused
-    // pseudo-time steps read from arrays (drop-in) or recomputed from Mus (solver)
     const T* dtVx;
     const T* dtVy;
     const T* dtPt;
@@ -209,20 +216,208 @@ struct S2Fused {
     int64_t nx, ny;
 };
 
-template <typename T, typename I>
-__device__ __forceinline__ T ldg_or0(const T* a, I i, I j, I n0, I n1) {
-    return (i >= 0 && i < n0 && j >= 0 && j < n1) ? __ldg(a + i + n0 * j) : T(0);
-}
-
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
-// Evaluates a statement without testing each dividend, and again with the tests (and the IEEE
-// division where they fail) in the rare case that one of its dividends is too small: one test and one
-// branch per statement instead of one per division.
+// One PT iteration as a march along y: a warp owns 30 columns (lanes 1..30; lanes 0 and 31 hold the
+// neighbour columns) and `rows` rows. Row j's step computes the cell (c, j) -- ∇V, P, τxx, τyy -- and
+// the corner (c, j-1) above row j-1, then the Vy face (c, j) and, a row late because it needs the
+// corner above it, the Vx face (c, j-1). What the next row needs stays in registers, the values of
+// the columns c - 1 and c + 1 come by shuffles, and row j + 1's loads are issued before row j is
+// computed: no barrier, no shared memory, and only one extra row per segment and two extra columns
+// per strip are computed twice. Quotients are taken without testing their dividends; a warp that met
+// one too small for that computes the row again with the tests (DivF, div_c).
+//
+// Bound: the latency of a row's loads and of its dependent instructions, at 20 warps per SM. Against the
+// 32 x 8 tile kernel before it (window in shared memory, halo computed twice, bounds tests per staged
+// value), per iteration: 1023^2 37.8 -> 16.6 us (3.8 TB/s on 15 words per cell), 511^2 7.8, 63^2 3.5 us,
+// where the launches of successive iterations overlap (programmatic dependent launch).
+//
+// I: index type (int where every array has fewer than 2^31 elements: fewer instructions per cell).
+// RED: a.red is set (the FP64 sums are compiled in only then: the conversions to double run on the
+// FP64 pipe even when predicated off).
+constexpr int S2_W = 4;  // warps per block; five blocks per SM (six or more: 17.7-18.7 us at 1023^2, spills)
+
+template <bool DEFECT, typename T>
+struct S2Row {  // one lane's inputs of a row
+    T vx, vyn, mus, p, dtp, f, xdv, xdt, xf, ydv, ydt, yf;
+};
+
+template <typename T, bool DEFECT, bool STORE_TMP, typename I, bool RED>
+__global__ void __launch_bounds__(32 * S2_W, 5) s2_march(S2Fused<T> a, S2P<T> p, int rows) {
+    const I nx = (I)a.nx, ny = (I)a.ny;
+    const int lane = threadIdx.x;
+    const I c = (I)blockIdx.x * 30 - 1 + lane;
+    const I r0 = ((I)blockIdx.y * S2_W + (I)threadIdx.y) * rows;
+    if (r0 >= ny) return;  // whole warps only: shuffles follow, no barrier
+    const I r1 = r0 + rows < ny ? r0 + rows : ny;
+    grid_dependency_wait();  // the state is read with plain loads: __ldg need not see the kernel before
+    grid_dependents_may_launch();
+    const bool last = r1 == ny;  // this segment also takes the Vy faces ny
+    const bool own = lane >= 1 && lane <= 30;
+    const bool cx = c >= 0 && c < nx, vxx = c >= 0 && c <= nx;
+    const bool xinx = c >= 1 && c <= nx - 1;  // Vx face column with a residual
+    const bool yinx = c >= 1 && c <= nx - 2;  // Vy face column with a residual
+    using Row = S2Row<DEFECT, T>;
+
+    // inputs of row j: cell row j, Vy faces j + 1 (the cell's upper side; faces j are carried), Vx faces of
+    // row j - 1 (finished in this step). Offsets of the next row to load: cells and Vy, Vx, and the
+    // residual arrays of the two faces.
+    I oC = c + nx * (r0 - 1), oX = oC + (r0 - 1), oU = (c - 1) + (nx - 1) * (r0 - 3), oV = (c - 1) + (nx - 2) * (r0 - 2);
+    auto load = [&](I j) {
+        Row r{};
+        const bool cy = j >= 0 && j < ny;
+        if (vxx && cy) r.vx = a.Vx_in[oX];
+        if (cx && j >= -1 && j < ny) r.vyn = a.Vy_in[oC + nx];
+        if (cx && cy) {
+            r.mus = __ldg(a.Mus + oC);
+            if (j < r1) {
+                r.p = a.P_in[oC];
+                r.dtp = __ldg(a.dtPt + oC);
+                if constexpr (DEFECT) r.f = __ldg(a.fp + oC);
+                else r.yf = __ldg(a.Rog + oC);
+            }
+        }
+        if (own && xinx && j > r0 && j >= 2 && j <= ny - 1) {
+            r.xdv = a.dVxdt[oU];
+            r.xdt = __ldg(a.dtVx + oU);
+            if constexpr (DEFECT) r.xf = __ldg(a.fx + oU);
+        }
+        if (own && yinx && j >= r0 && j < r1 && j >= 1) {
+            r.ydv = a.dVydt[oV];
+            r.ydt = __ldg(a.dtVy + oV);
+            if constexpr (DEFECT) r.yf = __ldg(a.fy + oV);
+        }
+        oC += nx;
+        oX += nx + 1;
+        oU += nx - 1;
+        oV += nx - 2;
+        return r;
+    };
+
+    // carried from row j - 1: Vx and its right neighbour, Mus and its pair sum with the right neighbour,
+    // P, τyy, the x parts of Rx, the corner's left neighbour, Rog
+    T vx_m = T(0), vxr_m = T(0), mus2_m = T(0), p_m = T(0), tyy_m = T(0), ax_m = T(0), px_m = T(0),
+      tl_m = T(0), rog_m = T(0);
+    double acc_rx = 0.0, acc_ry = 0.0, acc_div = 0.0;
+
+    T vy0 = (cx && r0 >= 1) ? a.Vy_in[oC] : T(0);  // Vy faces of row r0 - 1
+    Row cur = load(r0 - 1);
+    for (I j = r0 - 1; j <= r1; ++j) {
+        // offsets of row j (load leaves them at the next row)
+        const I qC = oC - nx, qX = oX - (nx + 1), qU = oU - (nx - 1), qV = oV - (nx - 2);
+        Row nxt{};
+        if (j < r1) nxt = load(j + 1);
+        const T vx = cur.vx, vy1 = cur.vyn, mus = cur.mus;
+        const T vxr = __shfl_down_sync(0xFFFFFFFFu, vx, 1);
+        const T vyr = __shfl_down_sync(0xFFFFFFFFu, vy0, 1);
+        const T musr = __shfl_down_sync(0xFFFFFFFFu, mus, 1);
+        T d, pn, txx, tyy, t, tl, ax, px, rx, ry;
+        auto row = [&](auto hx, auto hy) {
+            // cell (c, j)
+            d = s2_divV(vx, vxr, vy0, vy1, hx, hy);
+            T dp = d;
+            if constexpr (DEFECT) dp = d + cur.f;
+            pn = cur.p - cur.dtp * dp;
+            txx = s2_tau_nn(mus, vx, vxr, d, hx);
+            tyy = s2_tau_nn(mus, vy0, vy1, d, hy);
+            // corner (c, j-1): between rows j-1 and j, columns c and c+1
+            t = s2_tau_xy_sum((mus2_m + mus) + musr, vxr - vxr_m, vyr - vy0, hx, hy);
+            // the left neighbours' values
+            const T txl = __shfl_up_sync(0xFFFFFFFFu, txx, 1), pl = __shfl_up_sync(0xFFFFFFFFu, pn, 1);
+            tl = __shfl_up_sync(0xFFFFFFFFu, t, 1);
+            // Vx face (c, j-1), whose x differences were taken in the last step
+            rx = (ax_m + dvd(tl - tl_m, hy)) - px_m;
+            ax = dvd(txx - txl, hx);
+            px = dvd(pn - pl, hx);
+            // Vy face (c, j)
+            ry = (dvd(tyy - tyy_m, hy) + dvd(t - tl, hx)) - dvd(pn - p_m, hy);
+        };
+        uint32_t key = 0xFFFFFFFFu;
+        row(DivF<T>{p.dx, &key}, DivF<T>{p.dy, &key});
+        if (__any_sync(0xFFFFFFFFu, key < p.lo)) row(p.dx, p.dy);
+
+        if (own && j >= r0) {
+            if (cx && j < r1) {  // cell (c, j), P
+                a.P_out[qC] = pn;
+                if constexpr (STORE_TMP) {
+                    a.divV[qC] = d;
+                    a.txx[qC] = txx;
+                    a.tyy[qC] = tyy;
+                }
+                if constexpr (RED) acc_div += fabs((double)(DEFECT ? d + cur.f : d));
+            }
+            // corner (c, j-1), 0 <= j-1 < ny-1
+            if constexpr (STORE_TMP)
+                if (j > r0 && j < ny && c >= 0 && c < nx - 1) a.txy[c + (nx - 1) * (j - 1)] = t;
+            // Vx face (c, j-1); bc_y!(Vx): rows 0 and ny-1 copy rows 1 and ny-2
+            if (vxx && j > r0 && j >= 2 && j <= ny - 1) {
+                T vnew = vx_m;
+                if (xinx) {
+                    T r = rx;
+                    if constexpr (DEFECT) r = r + cur.xf;
+                    const T dv = p.dampX * cur.xdv + r;
+                    a.dVxdt[qU] = dv;
+                    if constexpr (STORE_TMP) a.Rx[qU] = r;
+                    if constexpr (RED) acc_rx += fabs((double)r);
+                    vnew = vnew + cur.xdt * dv;
+                }
+                a.Vx_out[qX - (nx + 1)] = vnew;
+                if (j == 2) a.Vx_out[c] = vnew;
+                if (j == ny - 1) a.Vx_out[qX] = vnew;
+            }
+            // Vy face (c, j); bc_x!(Vy): columns 0 and nx-1 copy columns 1 and nx-2
+            if (yinx && (j < r1 || last)) {
+                T vnew = vy0;
+                if (j >= 1 && j <= ny - 1) {
+                    T r = ry;
+                    if constexpr (DEFECT) r = r + cur.yf;
+                    else r = r + (rog_m + cur.yf) * T(0.5);
+                    const T dv = p.dampY * cur.ydv + r;
+                    a.dVydt[qV] = dv;
+                    if constexpr (STORE_TMP) a.Ry[qV] = r;
+                    if constexpr (RED) acc_ry += fabs((double)r);
+                    vnew = vnew + cur.ydt * dv;
+                }
+                a.Vy_out[qC] = vnew;
+                if (c == 1) a.Vy_out[qC - 1] = vnew;
+                if (c == nx - 2) a.Vy_out[qC + 1] = vnew;
+            }
+        }
+        vy0 = vy1;
+        vx_m = vx;
+        vxr_m = vxr;
+        mus2_m = mus + musr;
+        p_m = pn;
+        tyy_m = tyy;
+        ax_m = ax;
+        px_m = px;
+        tl_m = tl;
+        if constexpr (!DEFECT) rog_m = cur.yf;
+        cur = nxt;
+    }
+    if constexpr (RED) {
+        const double s0 = warp_sum(acc_rx), s1 = warp_sum(acc_ry), s2 = warp_sum(acc_div);
+        if (lane == 0) {
+            atomicAdd(a.red, s0);
+            atomicAdd(a.red + 1, s1);
+            atomicAdd(a.red + 2, s2);
+        }
+    }
+}
+
+// The FP64 iteration: two kernels in place, one thread per position and no halo computed twice, because
+// the FP64 pipe bounds it (57 FP64 instructions per cell; the march above issues a sixth more for its
+// extra rows and columns, and its few warps per scheduler leave the pipe idle between dependent
+// instructions). s2_cells: ∇V, P and the stresses; s2_faces: residuals, pseudo-velocities, velocities and
+// the free-slip copies (a face reads no other face's velocity). Per iteration, against a 32 x 16 tile
+// kernel that computes its halo twice: 511^2 82 -> 32.8 us, 1023^2 270 -> 117 us (80 % of the FP64 pipe).
+//
+// S2_DIV evaluates a statement without testing each dividend, and again with the tests (and the IEEE
+// division where they fail) in the rare case that one of its dividends is too small.
 #define S2_DIV(stmt)                                                            \
     do {                                                                        \
         uint32_t key_ = 0xFFFFFFFFu;                                            \
@@ -230,179 +425,108 @@ __device__ __forceinline__ double warp_sum(double v) {
         if (key_ < p.lo) stmt(p.dx, p.dy);                                      \
     } while (0)
 
-// I: index type (int where every array has fewer than 2^31 elements: fewer instructions per cell).
-// RED: a.red is set (the FP64 sums are compiled in only then: the conversions to double run on the
-// FP64 pipe even when predicated off).
-template <typename T, bool DEFECT, bool STORE_TMP, bool READ_DT, typename I, bool RED>
-__global__ void __launch_bounds__(S2_TX* s2_ty<T>()) s2_fused(S2Fused<T> a, S2P<T> p) {
-    constexpr int TX = S2_TX, TY = s2_ty<T>();
-    constexpr int VW = TX + 2, VH = TY + 2;  // staged V / Mus window: [x0-1, x0+TX] x [y0-1, y0+TY]
-    constexpr int CW = TX + 1, CH = TY + 1;  // computed cells / corners: [x0-1, x0+TX) x [y0-1, y0+TY)
-    __shared__ T sVx[VH][VW], sVy[VH][VW], sMus[VH][VW];
-    __shared__ T sP[CH][CW], sTxx[CH][CW], sTyy[CH][CW], sTxy[CH][CW];
-    __shared__ double sred[3][TX * TY / 32];
+// (a + b) * 0.5, the buoyancy average
+template <typename H>
+__device__ __forceinline__ double s2_half_sum(double a, double b, H) {
+    return (a + b) * 0.5;
+}
+__device__ __forceinline__ double s2_half_sum(double a, double b, DivF<double> h) { return scale_pow2(a + b, -1, h.key); }
 
+template <typename I, bool STORE_TMP, bool RED>
+__global__ void __launch_bounds__(256) s2_cells(S2Fused<double> a, S2P<double> p) {
+    using T = double;
     const I nx = (I)a.nx, ny = (I)a.ny;
-    const int tid = threadIdx.y * TX + threadIdx.x;
-    const I x0 = (I)blockIdx.x * TX, y0 = (I)blockIdx.y * TY;
-    constexpr int NC = (CW * CH + TX * TY - 1) / (TX * TY);  // halo-window cells per thread
-
-    // Every global load of the thread is issued before the first barrier (the staged window, the
-    // cells' P / dtPt / defect source, the faces' dVdt / dt / sources), so one memory round trip
-    // covers the iteration instead of three dependent ones.
-    for (int k = tid; k < VW * VH; k += TX * TY) {
-        int u = k % VW, v = k / VW;
-        I gi = x0 - 1 + u, gj = y0 - 1 + v;
-        sVx[v][u] = ldg_or0(a.Vx_in, gi, gj, nx + 1, ny);
-        sVy[v][u] = ldg_or0(a.Vy_in, gi, gj, nx, ny + 1);
-        sMus[v][u] = ldg_or0(a.Mus, gi, gj, nx, ny);
-    }
-    T c_p[NC], c_dt[NC], c_f[NC];
-#pragma unroll
-    for (int q = 0; q < NC; q++) {
-        const int k = tid + q * TX * TY;
-        const I gi = x0 - 1 + k % CW, gj = y0 - 1 + k / CW;
-        const bool in = k < CW * CH && gi >= 0 && gi < nx && gj >= 0 && gj < ny;
-        c_p[q] = in ? __ldg(a.P_in + gi + nx * gj) : T(0);
-        c_dt[q] = (READ_DT && in) ? __ldg(a.dtPt + gi + nx * gj) : T(0);
-        c_f[q] = (DEFECT && in) ? __ldg(a.fp + gi + nx * gj) : T(0);
-    }
-    const int lx = threadIdx.x, ly = threadIdx.y;
-    const I fi = x0 + lx, fj = y0 + ly;
-    const bool xin = fi <= nx && fj < ny, xinner = fi >= 1 && fi <= nx - 1 && fj >= 1 && fj <= ny - 2;
-    const bool yin = fi < nx && fj <= ny, yinner = fi >= 1 && fi <= nx - 2 && fj >= 1 && fj <= ny - 1;
-    const I rxi = (fi - 1) + (nx - 1) * (fj - 1), ryi = (fi - 1) + (nx - 2) * (fj - 1);
-    T x_dv = T(0), x_dt = T(0), x_f = T(0), y_dv = T(0), y_dt = T(0), y_f = T(0);
-    if (xin && xinner) {
-        x_dv = a.dVxdt[rxi];
-        if constexpr (READ_DT) x_dt = __ldg(a.dtVx + rxi);
-        if constexpr (DEFECT) x_f = __ldg(a.fx + rxi);
-    }
-    if (yin && yinner) {
-        y_dv = a.dVydt[ryi];
-        if constexpr (READ_DT) y_dt = __ldg(a.dtVy + ryi);
-        if constexpr (DEFECT)
-            y_f = __ldg(a.fy + ryi);
-        else
-            y_f = (__ldg(a.Rog + fi + nx * (fj - 1)) + __ldg(a.Rog + fi + nx * fj)) * T(0.5);
-    }
-    __syncthreads();
-
-    double acc_div = 0.0;
-    // cells and corners of the halo window
-#pragma unroll
-    for (int q = 0; q < NC; q++) {
-        const int k = tid + q * TX * TY;
-        if (k >= CW * CH) break;
-        int u = k % CW, v = k / CW;  // window cell (u, v) = global cell (x0-1+u, y0-1+v)
-        I gi = x0 - 1 + u, gj = y0 - 1 + v;
-        if (gi >= 0 && gi < nx && gj >= 0 && gj < ny) {
-            T vx0 = sVx[v][u], vx1 = sVx[v][u + 1];  // Vx faces gi, gi+1 of row gj
-            T vy0 = sVy[v][u], vy1 = sVy[v + 1][u];  // Vy faces gj, gj+1 of column gi
-            T mus = sMus[v][u];
-            T d, txx, tyy;
-            auto strain = [&](auto hx, auto hy) {
-                d = s2_divV(vx0, vx1, vy0, vy1, hx, hy);
-                txx = s2_tau_nn(mus, vx0, vx1, d, hx);
-                tyy = s2_tau_nn(mus, vy0, vy1, d, hy);
-            };
-            S2_DIV(strain);
-            T dtp = READ_DT ? c_dt[q] : s2_dtPt(p.Ptsc, mus, p.max_nxy);
-            T dp = d;
-            if constexpr (DEFECT) dp = d + c_f[q];
-            T pn = c_p[q] - dtp * dp;
-            sP[v][u] = pn;
-            sTxx[v][u] = txx;
-            sTyy[v][u] = tyy;
-            bool own = u >= 1 && v >= 1;  // inside [x0, x0+TX) x [y0, y0+TY)
-            if (own) {
-                a.P_out[gi + nx * gj] = pn;
-                if constexpr (STORE_TMP) {
-                    a.divV[gi + nx * gj] = d;
-                    a.txx[gi + nx * gj] = txx;
-                    a.tyy[gi + nx * gj] = tyy;
-                }
-                if constexpr (RED) acc_div += fabs((double)dp);
-            }
-        }
-        // corner (gi, gj): between cells gi..gi+1, gj..gj+1
-        if (gi >= 0 && gi < nx - 1 && gj >= 0 && gj < ny - 1) {
+    const I i = (I)(blockIdx.x * 32 + threadIdx.x), j = (I)(blockIdx.y * 8 + threadIdx.y);
+    grid_dependency_wait();  // the state is read with plain loads: __ldg need not see the kernel before
+    grid_dependents_may_launch();
+    double acc = 0.0;
+    if (i < nx && j < ny) {
+        const I c = i + nx * j, cx = c + j;  // Vx rows have nx + 1 faces
+        const T vx0 = a.Vx_out[cx], vx1 = a.Vx_out[cx + 1], vy0 = a.Vy_out[c], vy1 = a.Vy_out[c + nx];
+        const T mus = __ldg(a.Mus + c);
+        T d, txx, tyy;
+        auto strain = [&](auto hx, auto hy) {
+            d = s2_divV(vx0, vx1, vy0, vy1, hx, hy);
+            txx = s2_tau_nn(mus, vx0, vx1, d, hx);
+            tyy = s2_tau_nn(mus, vy0, vy1, d, hy);
+        };
+        S2_DIV(strain);
+        a.P_out[c] = a.P_out[c] - __ldg(a.dtPt + c) * d;
+        a.txx[c] = txx;
+        a.tyy[c] = tyy;
+        if constexpr (STORE_TMP) a.divV[c] = d;
+        if constexpr (RED) acc = fabs(d);
+        if (i < nx - 1 && j < ny - 1) {
+            const T msum = ((mus + __ldg(a.Mus + c + 1)) + __ldg(a.Mus + c + nx)) + __ldg(a.Mus + c + nx + 1);
+            const T dyVx = a.Vx_out[cx + nx + 2] - vx1, dxVy = a.Vy_out[c + nx + 1] - vy1;
             T t;
-            auto shear = [&](auto hx, auto hy) {
-                t = s2_tau_xy(sMus[v][u], sMus[v][u + 1], sMus[v + 1][u], sMus[v + 1][u + 1],
-                              sVx[v + 1][u + 1] - sVx[v][u + 1], sVy[v + 1][u + 1] - sVy[v + 1][u], hx, hy);
-            };
+            auto shear = [&](auto hx, auto hy) { t = s2_tau_xy_sum(msum, dyVx, dxVy, hx, hy); };
             S2_DIV(shear);
-            sTxy[v][u] = t;
-            if constexpr (STORE_TMP)
-                if (u >= 1 && v >= 1) a.txy[gi + (nx - 1) * gj] = t;
+            a.txy[c - j] = t;
         }
-    }
-    __syncthreads();
-
-    // faces of this tile
-    const int u = lx + 1, v = ly + 1;  // window coordinates of cell (fi, fj)
-    double acc_rx = 0.0, acc_ry = 0.0;
-    // ---- Vx face (fi, fj), Vx is (nx+1, ny) ----
-    if (xin) {
-        T vnew = sVx[v][u];
-        if (xinner) {
-            T r;
-            auto resid = [&](auto hx, auto hy) {
-                r = s2_Rx(sTxx[v][u - 1], sTxx[v][u], sTxy[v - 1][u - 1], sTxy[v][u - 1], sP[v][u - 1], sP[v][u], hx, hy);
-            };
-            S2_DIV(resid);
-            if constexpr (DEFECT) r = r + x_f;
-            T dv = p.dampX * x_dv + r;
-            a.dVxdt[rxi] = dv;
-            if constexpr (STORE_TMP) a.Rx[rxi] = r;
-            if constexpr (RED) acc_rx += fabs((double)r);
-            T dt = READ_DT ? x_dt : s2_dtV(p.Vsc, p.min_dxy2, sMus[v][u - 1], sMus[v][u]);
-            vnew = vnew + dt * dv;
-        }
-        // bc_y!(Vx): rows 0 and ny-1 copy rows 1 and ny-2 (written by the owner of the inner row)
-        if (fj >= 1 && fj <= ny - 2) a.Vx_out[fi + (nx + 1) * fj] = vnew;
-        if (fj == 1) a.Vx_out[fi] = vnew;
-        if (fj == ny - 2) a.Vx_out[fi + (nx + 1) * (ny - 1)] = vnew;
-        if (ny <= 2 && (fj == 0 || fj == ny - 1)) a.Vx_out[fi + (nx + 1) * fj] = vnew;  // degenerate grid
-    }
-    // ---- Vy face (fi, fj), Vy is (nx, ny+1) ----
-    if (yin) {
-        T vnew = sVy[v][u];
-        if (yinner) {
-            T r;
-            auto resid = [&](auto hx, auto hy) {
-                r = s2_Ry_core(sTyy[v - 1][u], sTyy[v][u], sTxy[v - 1][u - 1], sTxy[v - 1][u], sP[v - 1][u], sP[v][u], hx,
-                               hy);
-            };
-            S2_DIV(resid);
-            r = r + y_f;  // the defect source, or the buoyancy average of the two cells
-            T dv = p.dampY * y_dv + r;
-            a.dVydt[ryi] = dv;
-            if constexpr (STORE_TMP) a.Ry[ryi] = r;
-            if constexpr (RED) acc_ry += fabs((double)r);
-            T dt = READ_DT ? y_dt : s2_dtV(p.Vsc, p.min_dxy2, sMus[v - 1][u], sMus[v][u]);
-            vnew = vnew + dt * dv;
-        }
-        // bc_x!(Vy): columns 0 and nx-1 copy columns 1 and nx-2
-        if (fi >= 1 && fi <= nx - 2) a.Vy_out[fi + nx * fj] = vnew;
-        if (fi == 1) a.Vy_out[nx * fj] = vnew;
-        if (fi == nx - 2) a.Vy_out[(nx - 1) + nx * fj] = vnew;
-        if (nx <= 2 && (fi == 0 || fi == nx - 1)) a.Vy_out[fi + nx * fj] = vnew;
     }
     if constexpr (RED) {
-        double s0 = warp_sum(acc_rx), s1 = warp_sum(acc_ry), s2 = warp_sum(acc_div);
-        int w = tid >> 5;
-        if ((tid & 31) == 0) {
-            sred[0][w] = s0;
-            sred[1][w] = s1;
-            sred[2][w] = s2;
+        acc = warp_sum(acc);
+        if (threadIdx.x == 0) atomicAdd(a.red + 2, acc);
+    }
+}
+
+template <typename I, bool STORE_TMP, bool RED>
+__global__ void __launch_bounds__(256) s2_faces(S2Fused<double> a, S2P<double> p) {
+    using T = double;
+    const I nx = (I)a.nx, ny = (I)a.ny;
+    const I i = (I)(blockIdx.x * 32 + threadIdx.x), j = (I)(blockIdx.y * 8 + threadIdx.y);
+    grid_dependency_wait();  // the state is read with plain loads: __ldg need not see the kernel before
+    grid_dependents_may_launch();
+    double acc_x = 0.0, acc_y = 0.0;
+    const I c = i + nx * j;  // cell (i, j) and Vy face (i, j)
+    // Vx face (i, j); bc_y!(Vx): rows 0 and ny-1 copy rows 1 and ny-2
+    if (i <= nx && j >= 1 && j <= ny - 2) {
+        const I cx = c + j;
+        T v = a.Vx_out[cx];
+        if (i >= 1 && i <= nx - 1) {
+            const I k = (i - 1) + (nx - 1) * (j - 1);  // residual index, and the corner (i-1, j-1)
+            const T txl = a.txx[c - 1], txr = a.txx[c], tb = a.txy[k], tt = a.txy[k + nx - 1], pl = a.P_out[c - 1],
+                    pr = a.P_out[c];
+            T r;
+            auto resid = [&](auto hx, auto hy) { r = s2_Rx(txl, txr, tb, tt, pl, pr, hx, hy); };
+            S2_DIV(resid);
+            const T dv = p.dampX * a.dVxdt[k] + r;
+            a.dVxdt[k] = dv;
+            if constexpr (STORE_TMP) a.Rx[k] = r;
+            if constexpr (RED) acc_x = fabs(r);
+            v = v + __ldg(a.dtVx + k) * dv;
+            a.Vx_out[cx] = v;
         }
-        __syncthreads();
-        if (tid < 3) {
-            double s = 0.0;
-            for (int k = 0; k < TX * TY / 32; k++) s += sred[tid][k];
-            atomicAdd(a.red + tid, s);
+        if (j == 1) a.Vx_out[i] = v;
+        if (j == ny - 2) a.Vx_out[cx + nx + 1] = v;
+    }
+    // Vy face (i, j); bc_x!(Vy): columns 0 and nx-1 copy columns 1 and nx-2
+    if (i >= 1 && i <= nx - 2 && j <= ny) {
+        T v = a.Vy_out[c];
+        if (j >= 1 && j <= ny - 1) {
+            const I k = (i - 1) + (nx - 2) * (j - 1), kc = (i - 1) + (nx - 1) * (j - 1);
+            const T tb = a.tyy[c - nx], tt = a.tyy[c], tl = a.txy[kc], tr = a.txy[kc + 1], pb = a.P_out[c - nx],
+                    pt = a.P_out[c], g0 = __ldg(a.Rog + c - nx), g1 = __ldg(a.Rog + c);
+            T r;
+            auto resid = [&](auto hx, auto hy) { r = s2_Ry_core(tb, tt, tl, tr, pb, pt, hx, hy) + s2_half_sum(g0, g1, hx); };
+            S2_DIV(resid);
+            const T dv = p.dampY * a.dVydt[k] + r;
+            a.dVydt[k] = dv;
+            if constexpr (STORE_TMP) a.Ry[k] = r;
+            if constexpr (RED) acc_y = fabs(r);
+            v = v + __ldg(a.dtVy + k) * dv;
+            a.Vy_out[c] = v;
+        }
+        if (i == 1) a.Vy_out[c - 1] = v;
+        if (i == nx - 2) a.Vy_out[c + 1] = v;
+    }
+    if constexpr (RED) {
+        acc_x = warp_sum(acc_x);
+        acc_y = warp_sum(acc_y);
+        if (threadIdx.x == 0) {
+            atomicAdd(a.red, acc_x);
+            atomicAdd(a.red + 1, acc_y);
         }
     }
 }
@@ -548,33 +672,67 @@ static void scratch_free(void* p) {
     g_scratch_all.erase(std::remove(g_scratch_all.begin(), g_scratch_all.end(), p), g_scratch_all.end());
 }
 
-template <typename T, bool DEFECT, bool STORE_TMP, bool READ_DT>
-static void launch_fused(const S2Fused<T>& a, const S2P<T>& p, cudaStream_t s) {
-    constexpr int TY = s2_ty<T>();
-    dim3 blk(S2_TX, TY);
-    dim3 grd((unsigned)((a.nx + 1 + S2_TX - 1) / S2_TX), (unsigned)((a.ny + 1 + TY - 1) / TY));
-    // 32-bit indices while the largest array and the tile origins stay below 2^31
-    const bool i32 = (a.nx + 1 + S2_TX) * (a.ny + 1 + TY) < ((int64_t)1 << 31);
+// Rows per warp of the march (each segment computes one extra row): as few as fill the GPU's warps twice
+// over, so that the second round's loads overlap the first round's tail, at least 2, at most 32. 1023^2:
+// 6 rows 16.7 us per iteration, 12 (one round) 19.5, 4 17.9, 24 27.0; 255^2: 2 rows 3.7 us, 4 4.6, 8 6.8.
+static int s2_rows(int64_t ny, int64_t strips, int64_t warps) {
+    const int64_t segs = std::max<int64_t>(1, 2 * warps / strips);
+    return (int)std::min<int64_t>(32, std::max<int64_t>(2, (ny + segs - 1) / segs));
+}
+
+// 32-bit indices while every array's size and the offsets a few rows past it stay below 2^31
+static bool s2_index32(int64_t nx, int64_t ny) { return (nx + 32) * (ny + 4) < ((int64_t)1 << 31); }
+
+// dependent: the kernel before this one on the stream is the previous iteration's
+template <bool DEFECT, bool STORE_TMP>
+static void launch_march(const S2Fused<float>& a, const S2P<float>& p, cudaStream_t s, bool dependent) {
+    auto launch = [&](auto kernel, int& per_sm) {
+        if (!per_sm) per_sm = resident_ctas(kernel, 32 * S2_W, 0);
+        DeviceState* st = nullptr;
+        const int sms = current_state(&st) == PS_OK ? st->num_sms : 1;
+        const int64_t strips = (a.nx + 1 + 29) / 30;
+        const int rows = s2_rows(a.ny, strips, (int64_t)per_sm * sms * S2_W);
+        const int64_t segs = (a.ny + rows - 1) / rows;
+        const dim3 grd((unsigned)strips, (unsigned)((segs + S2_W - 1) / S2_W));
+        if (dependent) launch_dependent(kernel, grd, dim3(32, S2_W), 0, s, a, p, rows);
+        else kernel<<<grd, dim3(32, S2_W), 0, s>>>(a, p, rows);
+    };
+    static int occ[4];
+    const bool i32 = s2_index32(a.nx, a.ny);
     if (a.red) {
-        if (i32) s2_fused<T, DEFECT, STORE_TMP, READ_DT, int, true><<<grd, blk, 0, s>>>(a, p);
-        else s2_fused<T, DEFECT, STORE_TMP, READ_DT, int64_t, true><<<grd, blk, 0, s>>>(a, p);
+        if (i32) launch(s2_march<float, DEFECT, STORE_TMP, int, true>, occ[0]);
+        else launch(s2_march<float, DEFECT, STORE_TMP, int64_t, true>, occ[1]);
     } else {
-        if (i32) s2_fused<T, DEFECT, STORE_TMP, READ_DT, int, false><<<grd, blk, 0, s>>>(a, p);
-        else s2_fused<T, DEFECT, STORE_TMP, READ_DT, int64_t, false><<<grd, blk, 0, s>>>(a, p);
+        if (i32) launch(s2_march<float, DEFECT, STORE_TMP, int, false>, occ[2]);
+        else launch(s2_march<float, DEFECT, STORE_TMP, int64_t, false>, occ[3]);
+    }
+}
+
+// One FP64 iteration in place on the state A (the buffers B are not used).
+template <bool STORE_TMP>
+static void launch_cells_faces(const S2Fused<double>& a, const S2P<double>& p, cudaStream_t s, bool dependent) {
+    const dim3 blk(32, 8), gc = g2(a.nx, a.ny, blk), gf = g2(a.nx + 1, a.ny + 1, blk);
+    auto launch = [&](auto cells, auto faces) {
+        if (dependent) launch_dependent(cells, gc, blk, 0, s, a, p);
+        else cells<<<gc, blk, 0, s>>>(a, p);
+        launch_dependent(faces, gf, blk, 0, s, a, p);
+    };
+    const bool i32 = s2_index32(a.nx, a.ny);
+    if (a.red) {
+        if (i32) launch(s2_cells<int, STORE_TMP, true>, s2_faces<int, STORE_TMP, true>);
+        else launch(s2_cells<int64_t, STORE_TMP, true>, s2_faces<int64_t, STORE_TMP, true>);
+    } else {
+        if (i32) launch(s2_cells<int, STORE_TMP, false>, s2_faces<int, STORE_TMP, false>);
+        else launch(s2_cells<int64_t, STORE_TMP, false>, s2_faces<int64_t, STORE_TMP, false>);
     }
 }
 
 template <typename T>
-static int iterate_dropin(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp, int64_t n_iter, cudaStream_t s) {
-    int64_t nx = f->Pt.n[0], ny = f->Pt.n[1];
-    S2P<T> p = s2p<T>(*pp);
-    size_t bx = (nx + 1) * ny * sizeof(T), by = nx * (ny + 1) * sizeof(T), bp = nx * ny * sizeof(T);
-    void* buf = nullptr;
-    PS_TRY(scratch_alloc(&buf, bx + by + bp + 256));
-    T* Vx_b = static_cast<T*>(buf);
-    T* Vy_b = reinterpret_cast<T*>(static_cast<char*>(buf) + bx);
-    T* P_b = reinterpret_cast<T*>(static_cast<char*>(buf) + bx + by);
+static S2Fused<T> s2_dropin_args(const ps_stokes2d_fields* f) {
     S2Fused<T> a{};
+    a.Vx_in = a.Vx_out = P_<T>(f->Vx);
+    a.Vy_in = a.Vy_out = P_<T>(f->Vy);
+    a.P_in = a.P_out = P_<T>(f->Pt);
     a.Mus = P_<T>(f->Mus);
     a.Rog = P_<T>(f->Rog);
     a.dtVx = P_<T>(f->dtauVx);
@@ -588,26 +746,55 @@ static int iterate_dropin(const ps_stokes2d_fields* f, const ps_stokes2d_params*
     a.txy = P_<T>(f->txy);
     a.Rx = P_<T>(f->Rx);
     a.Ry = P_<T>(f->Ry);
-    a.red = nullptr;
-    a.nx = nx;
-    a.ny = ny;
-    T* A[3] = {P_<T>(f->Vx), P_<T>(f->Vy), P_<T>(f->Pt)};
-    T* B[3] = {Vx_b, Vy_b, P_b};
+    a.nx = f->Pt.n[0];
+    a.ny = f->Pt.n[1];
+    return a;
+}
+
+// n_iter FP64 iterations; the temporaries nothing reads between iterations are stored in the last
+static void s2_iterate64(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp, int64_t n_iter, cudaStream_t s) {
+    const S2P<double> p = s2p<double>(*pp);
+    const S2Fused<double> a = s2_dropin_args<double>(f);
     for (int64_t it = 0; it < n_iter; ++it) {
-        T** in = (it % 2 == 0) ? A : B;
-        T** out = (it % 2 == 0) ? B : A;
+        if (it == n_iter - 1) launch_cells_faces<true>(a, p, s, it > 0);
+        else launch_cells_faces<false>(a, p, s, it > 0);
+    }
+}
+
+// n_iter FP32 iterations between the caller's state and the ping-pong buffers B
+static void s2_iterate32(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp, int64_t n_iter, float* const B[3],
+                         cudaStream_t s) {
+    const S2P<float> p = s2p<float>(*pp);
+    S2Fused<float> a = s2_dropin_args<float>(f);
+    float* const A[3] = {a.Vx_out, a.Vy_out, a.P_out};
+    for (int64_t it = 0; it < n_iter; ++it) {
+        float* const* in = (it % 2 == 0) ? A : B;
+        float* const* out = (it % 2 == 0) ? B : A;
         a.Vx_in = in[0];
         a.Vy_in = in[1];
         a.P_in = in[2];
         a.Vx_out = out[0];
         a.Vy_out = out[1];
         a.P_out = out[2];
-        launch_fused<T, false, true, true>(a, p, s);
+        if (it == n_iter - 1) launch_march<false, true>(a, p, s, it > 0);
+        else launch_march<false, false>(a, p, s, it > 0);
     }
     if (n_iter % 2 == 1) {
-        cudaMemcpyAsync(A[0], B[0], bx, cudaMemcpyDeviceToDevice, s);
-        cudaMemcpyAsync(A[1], B[1], by, cudaMemcpyDeviceToDevice, s);
-        cudaMemcpyAsync(A[2], B[2], bp, cudaMemcpyDeviceToDevice, s);
+        const int64_t n[3] = {numel(f->Vx), numel(f->Vy), numel(f->Pt)};
+        for (int k = 0; k < 3; k++) cudaMemcpyAsync(A[k], B[k], n[k] * sizeof(float), cudaMemcpyDeviceToDevice, s);
+    }
+}
+
+static int iterate_dropin(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp, int64_t n_iter, cudaStream_t s) {
+    void* buf = nullptr;
+    if (f->Pt.dtype == PS_F64) {
+        s2_iterate64(f, pp, n_iter, s);
+    } else {
+        const int64_t n[2] = {numel(f->Vx), numel(f->Vy)};
+        PS_TRY(scratch_alloc(&buf, (n[0] + n[1] + numel(f->Pt)) * sizeof(float) + 256));
+        float* const B[3] = {static_cast<float*>(buf), static_cast<float*>(buf) + n[0],
+                             static_cast<float*>(buf) + n[0] + n[1]};
+        s2_iterate32(f, pp, n_iter, B, s);
     }
     cudaError_t e = cudaStreamSynchronize(s);
     scratch_free(buf);
@@ -616,35 +803,18 @@ static int iterate_dropin(const ps_stokes2d_fields* f, const ps_stokes2d_params*
 }
 
 // ---- solver ---------------------------------------------------------------------------
-// Runs `nout` fused iterations per CUDA graph launch; the last one of each graph accumulates
-// Σ|Rx|, Σ|Ry|, Σ|∇V| into `red`. `n_even` iterations keep the ping-pong parity.
-template <typename T, bool DEFECT>
+// Runs `nout` iterations per CUDA graph launch; the last one of each graph accumulates Σ|Rx|, Σ|Ry|,
+// Σ|∇V| into `red`. nout is even: the FP32 ping-pong ends where it began.
 struct PTRunner {
-    S2Fused<T> a{};
-    S2P<T> p{};
-    T* A[3];
-    T* B[3];
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
-    int64_t nout = 0;
 
-    int build(cudaStream_t s, int64_t nout_) {
-        nout = nout_;
+    // iteration(it, red): enqueues iteration `it` (red: null except in the last)
+    template <typename F>
+    int build(cudaStream_t s, int64_t nout, double* red, F iteration) {
         PS_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        cudaMemsetAsync(a.red, 0, 3 * sizeof(double), s);
-        for (int64_t it = 0; it < nout; ++it) {
-            T** in = (it % 2 == 0) ? A : B;
-            T** out = (it % 2 == 0) ? B : A;
-            S2Fused<T> k = a;
-            k.Vx_in = in[0];
-            k.Vy_in = in[1];
-            k.P_in = in[2];
-            k.Vx_out = out[0];
-            k.Vy_out = out[1];
-            k.P_out = out[2];
-            if (it != nout - 1) k.red = nullptr;
-            launch_fused<T, DEFECT, false, false>(k, p, s);
-        }
+        cudaMemsetAsync(red, 0, 3 * sizeof(double), s);
+        for (int64_t it = 0; it < nout; ++it) iteration(it, it == nout - 1 ? red : nullptr);
         PS_CUDA_TRY(cudaStreamEndCapture(s, &graph));
         PS_CUDA_TRY(cudaGraphInstantiate(&exec, graph, 0));
         return PS_OK;
@@ -657,6 +827,16 @@ struct PTRunner {
     }
 };
 
+// The pseudo-time steps of a solve, computed once (compute_timesteps!) instead of in every iteration.
+template <typename T>
+static void s2_solver_timesteps(S2Fused<T>& a, const S2P<T>& p, T* dtVx, T* dtVy, T* dtPt, cudaStream_t s) {
+    const dim3 blk(32, 8);
+    s2_timesteps_k<T><<<g2(a.nx, a.ny, blk), blk, 0, s>>>(dtVx, dtVy, dtPt, a.Mus, a.nx, a.ny, p);
+    a.dtVx = dtVx;
+    a.dtVy = dtVy;
+    a.dtPt = dtPt;
+}
+
 static double now_s() {
     return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
@@ -664,32 +844,31 @@ static double now_s() {
 static int solve_fp64(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp, double tol, int64_t max_iter,
                       int64_t nout, double max_seconds, ps_solve_stats* st, cudaStream_t s) {
     int64_t nx = f->Pt.n[0], ny = f->Pt.n[1];
-    size_t bx = (nx + 1) * ny * 8, by = nx * (ny + 1) * 8, bp = nx * ny * 8;
+    const int64_t nRx = (nx - 1) * (ny - 2), nRy = (nx - 2) * (ny - 1), nP = nx * ny;
     void* buf = nullptr;
-    PS_TRY(scratch_alloc(&buf, bx + by + bp + 3 * sizeof(double) + 256));
-    char* c = static_cast<char*>(buf);
-    PTRunner<double, false> r;
-    r.p = s2p<double>(*pp);
-    r.a.Mus = P_<double>(f->Mus);
-    r.a.Rog = P_<double>(f->Rog);
-    r.a.dVxdt = P_<double>(f->dVxdtau);
-    r.a.dVydt = P_<double>(f->dVydtau);
-    r.a.red = reinterpret_cast<double*>(c + bx + by + bp);
-    r.a.nx = nx;
-    r.a.ny = ny;
-    r.A[0] = P_<double>(f->Vx);
-    r.A[1] = P_<double>(f->Vy);
-    r.A[2] = P_<double>(f->Pt);
-    r.B[0] = reinterpret_cast<double*>(c);
-    r.B[1] = reinterpret_cast<double*>(c + bx);
-    r.B[2] = reinterpret_cast<double*>(c + bx + by);
-    int rc = r.build(s, nout);
+    // τxx, τyy, τxy, dτVx, dτVy, dτPt and the three sums
+    PS_TRY(scratch_alloc(&buf, (3 * nP + (nx - 1) * (ny - 1) + nRx + nRy + 3) * sizeof(double) + 256));
+    double* c = static_cast<double*>(buf);
+    S2Fused<double> a = s2_dropin_args<double>(f);
+    const S2P<double> p = s2p<double>(*pp);
+    a.txx = c;
+    a.tyy = c + nP;
+    a.txy = c + 2 * nP;
+    double* dt = a.txy + (nx - 1) * (ny - 1);
+    s2_solver_timesteps(a, p, dt, dt + nRx, dt + nRx + nRy, s);
+    double* red = dt + nRx + nRy + nP;
+    PTRunner r;
+    int rc = r.build(s, nout, red, [&](int64_t it, double* rd) {
+        S2Fused<double> k = a;
+        k.red = rd;
+        launch_cells_faces<false>(k, p, s, it > 0);
+    });
     const double nrx = (double)((nx - 1) * (ny - 2)), nry = (double)((nx - 2) * (ny - 1)), nd = (double)(nx * ny);
     double t0 = now_s(), err = INFINITY, h[3];
     int64_t it = 0;
     while (rc == PS_OK && it < max_iter) {
         cudaError_t e = cudaGraphLaunch(r.exec, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(h, r.a.red, sizeof(h), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h, red, sizeof(h), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
             rc = cuda_fail(e, "ps_stokes2d_solve(fp64)");
@@ -708,7 +887,6 @@ static int solve_fp64(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp,
             break;
         }
     }
-    // the state is in A after an even number of iterations (nout is even)
     r.destroy();
     cudaStreamSynchronize(s);
     scratch_free(buf);
@@ -729,20 +907,20 @@ static int solve_mixed(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp
     int64_t nx = f->Pt.n[0], ny = f->Pt.n[1];
     const int64_t nVx = (nx + 1) * ny, nVy = nx * (ny + 1), nP = nx * ny, nRx = (nx - 1) * (ny - 2),
                   nRy = (nx - 2) * (ny - 1);
-    // float buffers: δVx a/b, δVy a/b, δP a/b, dVxdτ, dVydτ, fx, fy, fp, Mus32
-    int64_t counts[12] = {nVx, nVx, nVy, nVy, nP, nP, nRx, nRy, nRx, nRy, nP, nP};
-    size_t off[13];
+    // float buffers: δVx a/b, δVy a/b, δP a/b, dVxdτ, dVydτ, fx, fy, fp, Mus32, dτVx, dτVy, dτPt
+    const int64_t counts[15] = {nVx, nVx, nVy, nVy, nP, nP, nRx, nRy, nRx, nRy, nP, nP, nRx, nRy, nP};
+    size_t off[16];
     off[0] = 0;
-    for (int k = 0; k < 12; k++) off[k + 1] = off[k] + ((counts[k] * 4 + 255) / 256) * 256;
-    size_t total = off[12] + 2 * 3 * sizeof(double) + 256;
+    for (int k = 0; k < 15; k++) off[k + 1] = off[k] + ((counts[k] * 4 + 255) / 256) * 256;
+    size_t total = off[15] + 2 * 3 * sizeof(double) + 256;
     void* buf = nullptr;
     PS_TRY(scratch_alloc(&buf, total));
     char* c = static_cast<char*>(buf);
     auto F = [&](int k) { return reinterpret_cast<float*>(c + off[k]); };
-    double* red_in = reinterpret_cast<double*>(c + off[12]);
+    double* red_in = reinterpret_cast<double*>(c + off[15]);
     double* red_out = red_in + 3;
     int rc = PS_OK;
-    cudaError_t e = cudaMemsetAsync(buf, 0, off[12], s);
+    cudaError_t e = cudaMemsetAsync(buf, 0, off[15], s);
     if (e != cudaSuccess) rc = cuda_fail(e, "memset");
     const double* Mus = P_<double>(f->Mus);
     s2_to_f32<<<256, 256, 0, s>>>(F(11), Mus, nP);
@@ -752,24 +930,31 @@ static int solve_mixed(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp
     s2_bc_y_k<double><<<(unsigned)((nx + 1 + 255) / 256), 256, 0, s>>>(P_<double>(f->Vx), nx + 1, ny);
     s2_bc_x_k<double><<<(unsigned)((ny + 1 + 255) / 256), 256, 0, s>>>(P_<double>(f->Vy), nx, ny + 1);
 
-    PTRunner<float, true> r;
-    r.p = s2p<float>(*pp);
-    r.a.Mus = F(11);
-    r.a.dVxdt = F(6);
-    r.a.dVydt = F(7);
-    r.a.fx = F(8);
-    r.a.fy = F(9);
-    r.a.fp = F(10);
-    r.a.red = red_in;
-    r.a.nx = nx;
-    r.a.ny = ny;
-    r.A[0] = F(0);
-    r.A[1] = F(2);
-    r.A[2] = F(4);
-    r.B[0] = F(1);
-    r.B[1] = F(3);
-    r.B[2] = F(5);
-    if (rc == PS_OK) rc = r.build(s, nout);
+    S2Fused<float> a{};
+    const S2P<float> p32 = s2p<float>(*pp);
+    a.Mus = F(11);
+    a.dVxdt = F(6);
+    a.dVydt = F(7);
+    a.fx = F(8);
+    a.fy = F(9);
+    a.fp = F(10);
+    a.nx = nx;
+    a.ny = ny;
+    s2_solver_timesteps(a, p32, F(12), F(13), F(14), s);
+    PTRunner r;
+    if (rc == PS_OK)
+        rc = r.build(s, nout, red_in, [&](int64_t it, double* rd) {
+            const int i = (int)(it % 2), o = 1 - i;
+            S2Fused<float> k = a;
+            k.Vx_in = F(i);
+            k.Vy_in = F(2 + i);
+            k.P_in = F(4 + i);
+            k.Vx_out = F(o);
+            k.Vy_out = F(2 + o);
+            k.P_out = F(4 + o);
+            k.red = rd;
+            launch_march<true, false>(k, p32, s, it > 0);
+        });
 
     S2P<double> p64 = s2p<double>(*pp);
     const double nrx = (double)nRx, nry = (double)nRy, nd = (double)nP;
@@ -993,8 +1178,7 @@ int ps_stokes2d_iterate(const ps_stokes2d_fields* f, const ps_stokes2d_params* p
     if (!p) return fail(PS_ERR_NULL, "NULL params");
     if (n_iter < 0) return fail(PS_ERR_ARG, "n_iter must be >= 0");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int rc = f->Pt.dtype == PS_F64 ? iterate_dropin<double>(f, p, n_iter, s) : iterate_dropin<float>(f, p, n_iter, s);
-    PS_TRY(rc);
+    PS_TRY(iterate_dropin(f, p, n_iter, s));
     return finish_launch(s, 1, "ps_stokes2d_iterate");
 }
 
@@ -1105,58 +1289,27 @@ void stokes2d_static_forget() {
 
 static size_t round256(size_t b) { return (b + 255) / 256 * 256; }
 
-template <typename T>
 static int iterate_static(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp, int64_t n_iter, cudaStream_t s) {
     const int64_t nx = f->Pt.n[0], ny = f->Pt.n[1];
-    const size_t bx = (nx + 1) * ny * sizeof(T), by = nx * (ny + 1) * sizeof(T), bp = nx * ny * sizeof(T);
+    const size_t es = elsize(f->Pt.dtype), bx = (nx + 1) * ny * es, by = nx * (ny + 1) * es, bp = nx * ny * es;
     const size_t need = round256(bx) + round256(by) + round256(bp);
     if (need > kStaticScratchBytes)
         return fail(PS_ERR_SHAPE,
                     "ps_stokes2d_iterate_static: a %lld x %lld grid needs %zu bytes of scratch; the static buffer "
                     "holds %zu bytes (use ps_stokes2d_iterate)",
                     (long long)nx, (long long)ny, need, kStaticScratchBytes);
+    if (f->Pt.dtype == PS_F64) {  // in place: the limit above is the entry point's, not the kernels'
+        s2_iterate64(f, pp, n_iter, s);
+        return PS_OK;
+    }
     void* base = nullptr;
     PS_TRY(static_scratch(&base));
     char* c = static_cast<char*>(base);
-    T* B[3] = {reinterpret_cast<T*>(c), reinterpret_cast<T*>(c + round256(bx)),
-               reinterpret_cast<T*>(c + round256(bx) + round256(by))};
-    T* A[3] = {P_<T>(f->Vx), P_<T>(f->Vy), P_<T>(f->Pt)};
-    S2P<T> p = s2p<T>(*pp);
-    S2Fused<T> a{};
-    a.Mus = P_<T>(f->Mus);
-    a.Rog = P_<T>(f->Rog);
-    a.dtVx = P_<T>(f->dtauVx);
-    a.dtVy = P_<T>(f->dtauVy);
-    a.dtPt = P_<T>(f->dtauPt);
-    a.dVxdt = P_<T>(f->dVxdtau);
-    a.dVydt = P_<T>(f->dVydtau);
-    a.divV = P_<T>(f->divV);
-    a.txx = P_<T>(f->txx);
-    a.tyy = P_<T>(f->tyy);
-    a.txy = P_<T>(f->txy);
-    a.Rx = P_<T>(f->Rx);
-    a.Ry = P_<T>(f->Ry);
-    a.red = nullptr;
-    a.nx = nx;
-    a.ny = ny;
     // every element of the buffers in use is written before it is read within a call, so the
     // contents left by the previous call never matter
-    for (int64_t it = 0; it < n_iter; ++it) {
-        T** in = (it % 2 == 0) ? A : B;
-        T** out = (it % 2 == 0) ? B : A;
-        a.Vx_in = in[0];
-        a.Vy_in = in[1];
-        a.P_in = in[2];
-        a.Vx_out = out[0];
-        a.Vy_out = out[1];
-        a.P_out = out[2];
-        launch_fused<T, false, true, true>(a, p, s);
-    }
-    if (n_iter % 2 == 1) {
-        PS_CUDA_TRY(cudaMemcpyAsync(A[0], B[0], bx, cudaMemcpyDeviceToDevice, s));
-        PS_CUDA_TRY(cudaMemcpyAsync(A[1], B[1], by, cudaMemcpyDeviceToDevice, s));
-        PS_CUDA_TRY(cudaMemcpyAsync(A[2], B[2], bp, cudaMemcpyDeviceToDevice, s));
-    }
+    float* const B[3] = {reinterpret_cast<float*>(c), reinterpret_cast<float*>(c + round256(bx)),
+                         reinterpret_cast<float*>(c + round256(bx) + round256(by))};
+    s2_iterate32(f, pp, n_iter, B, s);
     return PS_OK;
 }
 
@@ -1171,7 +1324,6 @@ extern "C" int ps_stokes2d_iterate_static(const ps_stokes2d_fields* f, const ps_
     if (!p) return fail(PS_ERR_NULL, "NULL params");
     if (n_iter < 0) return fail(PS_ERR_ARG, "n_iter must be >= 0");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int rc = f->Pt.dtype == PS_F64 ? iterate_static<double>(f, p, n_iter, s) : iterate_static<float>(f, p, n_iter, s);
-    PS_TRY(rc);
+    PS_TRY(iterate_static(f, p, n_iter, s));
     return finish_launch(s, 1, "ps_stokes2d_iterate_static");
 }
