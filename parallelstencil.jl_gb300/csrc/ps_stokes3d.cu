@@ -7,15 +7,11 @@
 //                           by every kernel below so all paths round identically
 //   one-to-one kernels      compute_timesteps!, compute_P!, compute_τ!, compute_dV!, compute_V!,
 //                           bc_x!, bc_y!, bc_z! -- drop-in replacements of the `@parallel` calls
-//   iteration kernels       one PT iteration in three launches:
-//                             s3_Ptau_k  ∇V, Pt and the six stresses of a cell; the normal
-//                                        stresses are indexed so that every thread uses the ∇V
-//                                        of its own cell (no re-read of ∇V from memory),
-//                             s3_dVV_k   residuals, pseudo-velocity and velocity updates,
-//                             s3_bc_k    the six free-slip copies of the loop body at once: the
-//                                        copies along different axes commute, so each boundary
-//                                        value is the composed copy of an interior value.
-//                           Results are bit-identical to the reference's ten-launch loop body.
+//   iteration kernels       one PT iteration in two launches: s3_cells (∇V, Pt and the six stresses) and
+//                           s3_faces (residuals, pseudo-velocities, velocities and the loop body's six
+//                           free-slip copies: copies along different axes commute, so each boundary
+//                           value is the composed copy of an interior value). Results are
+//                           bit-identical to the reference's ten-launch loop body.
 //   ps_stokes3d_solve       the `while err > ε` loop in FP64: CUDA graphs of `nout` iterations
 //                           followed by the FP64 residual norms, checked on the host.
 #include <math.h>
@@ -35,12 +31,16 @@ template <typename T>
 struct S3P {
     DivC<T> dx, dy, dz;  // divisors of the statements (correctly rounded division by host numbers)
     T dampX, dampY, dampZ, Vsc, Ptsc, min_dxyz2, max_nxyz;
+    uint32_t lo;  // the smallest dividend key all three divisors take without a test
 };
 
 template <typename T>
 static S3P<T> s3p(const ps_stokes3d_params& p) {
-    return S3P<T>{make_div((T)p.dx), make_div((T)p.dy), make_div((T)p.dz), (T)p.dampX,     (T)p.dampY,
-                  (T)p.dampZ,        (T)p.Vsc,          (T)p.Ptsc,         (T)p.min_dxyz2, (T)p.max_nxyz};
+    const T h[3] = {(T)p.dx, (T)p.dy, (T)p.dz};
+    DivC<T> d[3];
+    const uint32_t lo = make_div3(h, d);
+    return S3P<T>{d[0],       d[1],      d[2],          (T)p.dampX,       (T)p.dampY,      (T)p.dampZ,
+                  (T)p.Vsc,   (T)p.Ptsc, (T)p.min_dxyz2, (T)p.max_nxyz, lo};
 }
 
 // Device pointers of the miniapp's arrays (sizes relative to (nx, ny, nz) = size(Pt) as in
@@ -82,16 +82,38 @@ __device__ __forceinline__ T s3_divV(const S3A<T>& a, const S3P<T>& p, I x, I y,
            div_c(a.Vz[I3T(x, y, z + 1, nx, ny)] - a.Vz[I3T(x, y, z, nx, ny)], p.dz);
 }
 // 2.0*μ*(dV/h - 1.0/3.0*∇V)
-template <typename T>
-__device__ __forceinline__ T s3_tnn(T m, T v1, T v0, const DivC<T>& h, T d) {
-    return (T(2.0) * m) * (div_c(v1 - v0, h) - (T(1.0) / T(3.0)) * d);
+// H: DivC<T>, or DivF<T> (quotients without the dividend tests). In FP64 with DivF the factors 2, 0.25
+// and 0.5 are gathered into one power of two applied to the product (scale_pow2).
+template <typename T, typename H>
+__device__ __forceinline__ T s3_tnn(T m, T v1, T v0, H h, T d) {
+    return (T(2.0) * m) * (dvd(v1 - v0, h) - (T(1.0) / T(3.0)) * d);
 }
-// 2.0*@av_..i(μ)*(0.5*(a/ha + b/hb)), the four μ in the macro's order
+__device__ __forceinline__ double s3_tnn(double m, double v1, double v0, DivF<double> h, double d) {
+    const double e = dvd(v1 - v0, h) - (1.0 / 3.0) * d;
+    if ((__double2hiint(m) & 0x7FFFFFFF) >= 0x78300000) *h.key = 0u;  // |m| < 2^900: 2 m is finite
+    return scale_pow2(m * e, 1, h.key);
+}
+// 2.0*@av_..i(μ)*(0.5*(a/ha + b/hb)), msum: the four μ summed in the macro's order
+template <typename T, typename H>
+__device__ __forceinline__ T s3_tsh_sum(T msum, T a, H ha, T b, H hb) {
+    const T av = msum * T(0.25);
+    return (T(2.0) * av) * (T(0.5) * (dvd(a, ha) + dvd(b, hb)));
+}
+__device__ __forceinline__ double s3_tsh_sum(double msum, double a, DivF<double> ha, double b, DivF<double> hb) {
+    const double e = dvd(a, ha) + dvd(b, hb);
+    *ha.key = min(*ha.key, min(div_key(msum), div_key(e)));
+    return scale_pow2(msum * e, -2, ha.key);
+}
 template <typename T>
 __device__ __forceinline__ T s3_tsh(T m0, T m1, T m2, T m3, T a, const DivC<T>& ha, T b, const DivC<T>& hb) {
-    const T av = (((m0 + m1) + m2) + m3) * T(0.25);
-    return (T(2.0) * av) * (T(0.5) * (div_c(a, ha) + div_c(b, hb)));
+    return s3_tsh_sum(((m0 + m1) + m2) + m3, a, ha, b, hb);
 }
+// (a + b) * 0.5, the buoyancy average
+template <typename T, typename H>
+__device__ __forceinline__ T s3_half_sum(T a, T b, H) {
+    return (a + b) * T(0.5);
+}
+__device__ __forceinline__ double s3_half_sum(double a, double b, DivF<double> h) { return scale_pow2(a + b, -1, h.key); }
 
 template <typename T, typename I = int64_t>
 __device__ __forceinline__ void s3_txy(const S3A<T>& a, const S3P<T>& p, I x, I y, I z) {
@@ -301,41 +323,225 @@ __global__ void s3_bc_axis_k(T* A, int64_t n0, int64_t n1, int64_t n2, int ax) {
 }
 
 // ---- iteration kernels ---------------------------------------------------------------------
-// compute_P! and compute_τ! of cell (x, y, z): τxx, τyy, τzz are written at the index whose ∇V
-// is this cell's, τxy, τxz, τyz at the cell's own index.
-template <typename T, int MODE = S3_PLAIN, typename I = int64_t>
-__global__ void s3_Ptau_k(S3A<T> a, S3P<T> p) {
-    S3_IDXT;
-    const I c = I3T(x, y, z, nx, ny);
-    const T d = s3_divV<T, I>(a, p, x, y, z);
-    if constexpr (MODE == S3_DEFECT) {  // the correction's continuity residual includes the outer one
-        const T dp = d + a.fp[c];
-        a.divV[c] = dp;
-        a.Pt[c] = a.Pt[c] - a.dtPt[c] * dp;
-    } else {
-        a.divV[c] = d;
-        if constexpr (MODE == S3_PLAIN) a.Pt[c] = a.Pt[c] - a.dtPt[c] * d;
+// One iteration in two in-place kernels, one thread per position. s3_cells: ∇V, Pt and the stresses of a
+// cell and of the edges at its upper sides; s3_faces: residuals, pseudo-velocities, velocities of the
+// faces at the cell's lower sides and the free-slip copies (the thread of an inner face writes the
+// boundary faces that copy it; no face reads another face's velocity). Every load of a thread is issued
+// before its arithmetic. Quotients are taken without testing their dividends; a thread that met one too
+// small for that computes its position again with the tests. STORE: ∇V (s3_cells) and R (s3_faces) are
+// stored too; nothing reads them between iterations.
+//
+// Bound: instruction issue -- half of it address arithmetic -- and latency at half occupancy (FP32), FP64
+// pipe (FP64). Per iteration, against a test and a branch per division, ∇V and R stored every time and
+// the copies in a third launch: FP32 127^3 106 -> 66 us, 255^3 768 -> 482 us, FP64 127^3 0.97 -> 0.45 ms.
+// Measured slower in FP32 at 127^3: sweeps of 4 planes per thread with the shared values in registers
+// (70 us), two or four columns per thread (73, 92), 40 or 32 registers for more warps (spills; 88, 130).
+template <typename T>
+constexpr int s3_blocks() {  // blocks per SM: 64 registers in FP32, 80 in FP64
+    return sizeof(T) == 4 ? 4 : 3;
+}
+template <typename T, int MODE, typename I, bool STORE>
+__global__ void __launch_bounds__(256, s3_blocks<T>()) s3_cells(S3A<T> a, S3P<T> p) {
+    const I nx = (I)a.nx, ny = (I)a.ny, nz = (I)a.nz;
+    const I x = (I)(blockIdx.x * 32 + threadIdx.x), y = (I)(blockIdx.y * 8 + threadIdx.y), z = (I)blockIdx.z;
+    grid_dependency_wait();  // the state is read with plain loads: __ldg need not see the kernel before
+    grid_dependents_may_launch();
+    if (x >= nx || y >= ny) return;
+    const bool x1 = x < nx - 1, y1 = y < ny - 1, z1 = z < nz - 1;  // an edge at the upper x / y / z side exists
+    const bool ix = x >= 1 && x1, iy = y >= 1 && y1, iz = z >= 1 && z1;
+    const I sC = nx * ny, c = x + nx * (y + ny * z);
+    const T* const vx = a.Vx + (x + (nx + 1) * (y + ny * z));
+    const T* const vy = a.Vy + (x + nx * (y + (ny + 1) * z));
+    const T *const vz = a.Vz + c, *const mu = a.Mus + c;
+    // planes z and z + 1 (n)
+    const T vx0 = vx[0], vx1 = vx[1], vy0 = vy[0], vy1 = vy[nx], vz0 = vz[0], vz1 = vz[sC], m00 = __ldg(mu);
+    T vxu = T(0), vyr = T(0), vzr = T(0), vzu = T(0), vx1n = T(0), vy1n = T(0);
+    T m10 = T(0), m01 = T(0), m11 = T(0), m00n = T(0), m10n = T(0), m01n = T(0);
+    if (y1) vxu = vx[1 + (nx + 1)];
+    if (x1) vyr = vy[nx + 1];
+    if (x1) vzr = vz[sC + 1];
+    if (y1) vzu = vz[sC + nx];
+    if (x1) m10 = __ldg(mu + 1);
+    if (y1) m01 = __ldg(mu + nx);
+    if (x1 && y1) m11 = __ldg(mu + nx + 1);
+    if (z1) {
+        vx1n = vx[1 + (nx + 1) * ny];
+        vy1n = vy[nx + nx * (ny + 1)];
+        m00n = __ldg(mu + sC);
+        if (x1) m10n = __ldg(mu + sC + 1);
+        if (y1) m01n = __ldg(mu + sC + nx);
     }
-    const T m = a.Mus[c];
-    const bool iy = y >= 1 && y <= ny - 2, iz = z >= 1 && z <= nz - 2, ix = x >= 1 && x <= nx - 2;
-    if (iy && iz)
-        a.txx[I3T(x, y - 1, z - 1, nx, ny - 2)] =
-            s3_tnn(m, a.Vx[I3T(x + 1, y, z, nx + 1, ny)], a.Vx[I3T(x, y, z, nx + 1, ny)], p.dx, d);
-    if (ix && iz)
-        a.tyy[I3T(x - 1, y, z - 1, nx - 2, ny)] =
-            s3_tnn(m, a.Vy[I3T(x, y + 1, z, nx, ny + 1)], a.Vy[I3T(x, y, z, nx, ny + 1)], p.dy, d);
-    if (ix && iy)
-        a.tzz[I3T(x - 1, y - 1, z, nx - 2, ny - 2)] =
-            s3_tnn(m, a.Vz[I3T(x, y, z + 1, nx, ny)], a.Vz[I3T(x, y, z, nx, ny)], p.dz, d);
-    if (x < nx - 1 && y < ny - 1 && z < nz - 2) s3_txy<T, I>(a, p, x, y, z);
-    if (x < nx - 1 && y < ny - 2 && z < nz - 1) s3_txz<T, I>(a, p, x, y, z);
-    if (x < nx - 2 && y < ny - 1 && z < nz - 1) s3_tyz<T, I>(a, p, x, y, z);
+    [[maybe_unused]] T pt = T(0), dtp = T(0), f = T(0);
+    if constexpr (MODE != S3_RESIDUAL) {
+        pt = a.Pt[c];
+        dtp = __ldg(a.dtPt + c);
+    }
+    if constexpr (MODE == S3_DEFECT) f = __ldg(a.fp + c);
+    T d, txx = T(0), tyy = T(0), tzz = T(0), txy = T(0), txz = T(0), tyz = T(0);
+    auto cell = [&](auto hx, auto hy, auto hz) {
+        d = (dvd(vx1 - vx0, hx) + dvd(vy1 - vy0, hy)) + dvd(vz1 - vz0, hz);
+        if (iy && iz) txx = s3_tnn(m00, vx1, vx0, hx, d);
+        if (ix && iz) tyy = s3_tnn(m00, vy1, vy0, hy, d);
+        if (ix && iy) tzz = s3_tnn(m00, vz1, vz0, hz, d);
+        if (x1 && y1 && iz) txy = s3_tsh_sum(((m00 + m10) + m01) + m11, vxu - vx1, hy, vyr - vy1, hx);
+        if (x1 && iy && z1) txz = s3_tsh_sum(((m00 + m10) + m00n) + m10n, vx1n - vx1, hz, vzr - vz1, hx);
+        if (ix && y1 && z1) tyz = s3_tsh_sum(((m00 + m01) + m00n) + m01n, vy1n - vy1, hz, vzu - vz1, hy);
+    };
+    uint32_t key = 0xFFFFFFFFu;
+    cell(DivF<T>{p.dx, &key}, DivF<T>{p.dy, &key}, DivF<T>{p.dz, &key});
+    if (key < p.lo) cell(p.dx, p.dy, p.dz);
+    const T dp = MODE == S3_DEFECT ? d + f : d;  // the correction's continuity residual includes the outer one
+    if constexpr (STORE) a.divV[c] = dp;
+    if constexpr (MODE != S3_RESIDUAL) a.Pt[c] = pt - dtp * dp;
+    if (iy && iz) a.txx[x + nx * ((y - 1) + (ny - 2) * (z - 1))] = txx;
+    if (ix && iz) a.tyy[(x - 1) + (nx - 2) * (y + ny * (z - 1))] = tyy;
+    if (ix && iy) a.tzz[(x - 1) + (nx - 2) * ((y - 1) + (ny - 2) * z)] = tzz;
+    if (x1 && y1 && iz) a.txy[x + (nx - 1) * (y + (ny - 1) * (z - 1))] = txy;
+    if (x1 && iy && z1) a.txz[x + (nx - 1) * ((y - 1) + (ny - 2) * z)] = txz;
+    if (ix && y1 && z1) a.tyz[(x - 1) + (nx - 2) * (y + (ny - 1) * z)] = tyz;
 }
 
-template <typename T, int MODE = S3_PLAIN, typename I = int64_t>
-__global__ void s3_dVV_k(S3A<T> a, S3P<T> p) {
-    S3_IDXT;
-    s3_dV<T, MODE, I>(a, p, x, y, z, true);
+template <typename T, int MODE, typename I, bool STORE>
+__global__ void __launch_bounds__(256, s3_blocks<T>()) s3_faces(S3A<T> a, S3P<T> p) {
+    const I nx = (I)a.nx, ny = (I)a.ny, nz = (I)a.nz;
+    const I x = (I)(blockIdx.x * 32 + threadIdx.x), y = (I)(blockIdx.y * 8 + threadIdx.y), z = (I)blockIdx.z;
+    grid_dependency_wait();
+    grid_dependents_may_launch();
+    if (x > nx || y > ny) return;
+    const bool ix = x >= 1 && x <= nx - 2, iy = y >= 1 && y <= ny - 2, iz = z >= 1 && z <= nz - 2;
+    // the faces with a residual: Vx, Vy, Vz (their low x, y, z sides of the cell)
+    const bool du = x >= 1 && x <= nx - 1 && iy && iz, dv = ix && y >= 1 && y <= ny - 1 && iz,
+               dw = ix && iy && z >= 1 && z <= nz - 1;
+    const I sC = nx * ny, c = x + nx * (y + ny * z), sU = (nx - 1) * (ny - 2), sV = (nx - 2) * (ny - 1),
+            sW = (nx - 2) * (ny - 2);
+    T* const vx = a.Vx + (x + (nx + 1) * (y + ny * z));
+    T* const vy = a.Vy + (x + nx * (y + (ny + 1) * z));
+    T *const vz = a.Vz + c, *const pt = a.Pt + c;
+    // residual indices (x-1, y-1, z-1), which are also those of txz at (x-1/2, z-1/2), of tyz at
+    // (y-1/2, z-1/2) and of tzz of the cell z - 1; the other stresses around the faces
+    const I qu = (x - 1) + (nx - 1) * (y - 1) + sU * (z - 1), qv = (x - 1) + (nx - 2) * (y - 1) + sV * (z - 1),
+            qw = (x - 1) + (nx - 2) * (y - 1) + sW * (z - 1);
+    const T* const txx = a.txx + (x + nx * ((y - 1) + (ny - 2) * (z - 1)));
+    const T* const tyy = a.tyy + ((x - 1) + (nx - 2) * (y + ny * (z - 1)));
+    const T* const txy = a.txy + ((x - 1) + (nx - 1) * ((y - 1) + (ny - 1) * (z - 1)));
+    const T *const txz = a.txz + qu, *const tyz = a.tyz + qv, *const tzz = a.tzz + qw;
+    // the differences' operands; pseudo-velocities g, their steps t, velocities v, defect sources f
+    T p0 = T(0), xy = T(0), xz = T(0), xzn = T(0), yz = T(0), yzn = T(0);
+    T xr = T(0), xl = T(0), xyu = T(0), pl = T(0), yu = T(0), yd = T(0), xyr = T(0), pd = T(0);
+    T zu = T(0), zd = T(0), xzr = T(0), yzu = T(0), pb = T(0);
+    [[maybe_unused]] T r0 = T(0), r1 = T(0), ug = T(0), ut = T(0), uv = T(0), uf = T(0), vg = T(0), vt = T(0), vv = T(0),
+                       vf = T(0), wg = T(0), wt = T(0), wv = T(0), wf = T(0);
+    if (du || dv || dw) p0 = pt[0];
+    if (du || dv) xy = txy[0];
+    if (du || dw) xz = txz[0];
+    if (dv || dw) yz = tyz[0];
+    if (du) {
+        xr = txx[0];
+        xl = txx[-1];
+        xyu = txy[nx - 1];
+        xzn = txz[sU];
+        pl = pt[-1];
+        if constexpr (MODE != S3_RESIDUAL) {
+            ug = a.dVx[qu];
+            ut = __ldg(a.dtVx + qu);
+        }
+        if constexpr (MODE == S3_DEFECT) uf = __ldg(a.fx + qu);
+    }
+    if (dv) {
+        yu = tyy[0];
+        yd = tyy[-(nx - 2)];
+        xyr = txy[1];
+        yzn = tyz[sV];
+        pd = pt[-nx];
+        if constexpr (MODE != S3_RESIDUAL) {
+            vg = a.dVy[qv];
+            vt = __ldg(a.dtVy + qv);
+        }
+        if constexpr (MODE == S3_DEFECT) vf = __ldg(a.fy + qv);
+    }
+    if (dw) {
+        zu = tzz[sW];
+        zd = tzz[0];
+        xzr = txz[1];
+        yzu = tyz[nx - 2];
+        pb = pt[-sC];
+        if constexpr (MODE != S3_DEFECT) {
+            r0 = __ldg(a.Rog + (c - sC));
+            r1 = __ldg(a.Rog + c);
+        }
+        if constexpr (MODE != S3_RESIDUAL) {
+            wg = a.dVz[qw];
+            wt = __ldg(a.dtVz + qw);
+        }
+        if constexpr (MODE == S3_DEFECT) wf = __ldg(a.fz + qw);
+    }
+    if constexpr (MODE != S3_RESIDUAL) {
+        if (iy && iz) uv = vx[0];
+        if (ix && iz) vv = vy[0];
+        if (ix && iy) wv = vz[0];
+    }
+    T ru = T(0), rv = T(0), rw = T(0);
+    auto resid = [&](auto hx, auto hy, auto hz) {
+        if (du) ru = ((dvd(xr - xl, hx) + dvd(xyu - xy, hy)) + dvd(xzn - xz, hz)) - dvd(p0 - pl, hx);
+        if (dv) rv = ((dvd(yu - yd, hy) + dvd(xyr - xy, hx)) + dvd(yzn - yz, hz)) - dvd(p0 - pd, hy);
+        if (dw) {
+            rw = ((dvd(zu - zd, hz) + dvd(xzr - xz, hx)) + dvd(yzu - yz, hy)) - dvd(p0 - pb, hz);
+            // the correction's buoyancy is part of the outer residual
+            if constexpr (MODE != S3_DEFECT) rw = rw + s3_half_sum(r0, r1, hz);
+        }
+    };
+    uint32_t key = 0xFFFFFFFFu;
+    resid(DivF<T>{p.dx, &key}, DivF<T>{p.dy, &key}, DivF<T>{p.dz, &key});
+    if (key < p.lo) resid(p.dx, p.dy, p.dz);
+    if constexpr (MODE == S3_DEFECT) {
+        ru = ru + uf;
+        rv = rv + vf;
+        rw = rw + wf;
+    }
+    if constexpr (STORE) {
+        if (du) a.Rx[qu] = ru;
+        if (dv) a.Ry[qv] = rv;
+        if (dw) a.Rz[qw] = rw;
+    }
+    if constexpr (MODE != S3_RESIDUAL) {
+        // the new velocities: old values outside @inn
+        if (du) {
+            const T g = p.dampX * ug + ru;
+            a.dVx[qu] = g;
+            uv = uv + ut * g;
+            vx[0] = uv;
+        }
+        if (dv) {
+            const T g = p.dampY * vg + rv;
+            a.dVy[qv] = g;
+            vv = vv + vt * g;
+            vy[0] = vv;
+        }
+        if (dw) {
+            const T g = p.dampZ * wg + rw;
+            a.dVz[qw] = g;
+            wv = wv + wt * g;
+            vz[0] = wv;
+        }
+        // bc_y!, bc_z!(Vx), bc_x!, bc_z!(Vy), bc_x!, bc_y!(Vz): a boundary face copies the face with its copied
+        // axes clamped into [1, n-2]
+        const int xa = x == 1 ? -1 : 0, xb = x == nx - 2 ? 1 : 0, ya = y == 1 ? -1 : 0, yb = y == ny - 2 ? 1 : 0,
+                  za = z == 1 ? -1 : 0, zb = z == nz - 2 ? 1 : 0;
+        if (xa | xb | ya | yb | za | zb) {
+            if (iy && iz)
+                for (int j = ya; j <= yb; ++j)
+                    for (int k = za; k <= zb; ++k)
+                        if (j || k) vx[j * (nx + 1) + k * ((nx + 1) * ny)] = uv;
+            if (ix && iz)
+                for (int i = xa; i <= xb; ++i)
+                    for (int k = za; k <= zb; ++k)
+                        if (i || k) vy[i + k * (nx * (ny + 1))] = vv;
+            if (ix && iy)
+                for (int i = xa; i <= xb; ++i)
+                    for (int j = ya; j <= yb; ++j)
+                        if (i || j) vz[i + j * nx] = wv;
+        }
+    }
 }
 
 // The loop body's six copies (bc_x!(Vy), bc_x!(Vz), bc_y!(Vx), bc_y!(Vz), bc_z!(Vx), bc_z!(Vy)):
@@ -675,23 +881,27 @@ static dim3 g3(int64_t wx, int64_t wy, int64_t wz) {
     return dim3((unsigned)((wx + 31) / 32), (unsigned)((wy + 7) / 8), (unsigned)wz);
 }
 
-enum S3Kernel { S3_TIMESTEPS, S3_P, S3_TAU, S3_DV, S3_V, S3_PTAU, S3_DVV, S3_BC };
+enum S3Kernel { S3_TIMESTEPS, S3_P, S3_TAU, S3_DV, S3_V, S3_BC };
 
 // The iteration kernels in 32-bit index arithmetic where every array index fits (the largest array,
 // a staggered velocity, has fewer than (nx+1)(ny+1)(nz+1) < 2^31 elements), else 64-bit.
 template <typename T>
 static bool s3_idx32(const S3A<T>& a) {
-    return (a.nx + 1) * (a.ny + 1) * (a.nz + 1) < (int64_t(1) << 31);
+    return (a.nx + 1) * (a.ny + 1) * (a.nz + 3) < (int64_t(1) << 31);  // two planes of slack for the sweeps' offsets
 }
-template <typename T, int MODE>
-static void s3_iteration_kernels(const S3A<T>& a, const S3P<T>& p, dim3 gc, dim3 b, cudaStream_t s) {
-    if (s3_idx32(a)) {
-        s3_Ptau_k<T, MODE, int><<<gc, b, 0, s>>>(a, p);
-        s3_dVV_k<T, MODE, int><<<gc, b, 0, s>>>(a, p);
-    } else {
-        s3_Ptau_k<T, MODE, int64_t><<<gc, b, 0, s>>>(a, p);
-        s3_dVV_k<T, MODE, int64_t><<<gc, b, 0, s>>>(a, p);
-    }
+// One iteration (or, MODE = S3_RESIDUAL, the residual): s3_cells and s3_faces. after: the kernel before
+// them on the stream is an iteration's, whose last wave they may overlap.
+template <typename T, int MODE, bool STORE>
+static void s3_iteration_kernels(const S3A<T>& a, const S3P<T>& p, bool after, cudaStream_t s) {
+    const dim3 b(32, 8, 1);
+    auto launch = [&](auto cells, auto faces) {
+        const dim3 gc = g3(a.nx, a.ny, a.nz), gf = g3(a.nx + 1, a.ny + 1, a.nz + 1);
+        if (after) launch_dependent(cells, gc, b, 0, s, a, p);
+        else cells<<<gc, b, 0, s>>>(a, p);
+        launch_dependent(faces, gf, b, 0, s, a, p);
+    };
+    if (s3_idx32(a)) launch(s3_cells<T, MODE, int, STORE>, s3_faces<T, MODE, int, STORE>);
+    else launch(s3_cells<T, MODE, int64_t, STORE>, s3_faces<T, MODE, int64_t, STORE>);
 }
 
 template <typename T>
@@ -707,14 +917,6 @@ static void s3_launch(S3Kernel k, const S3A<T>& a, const S3P<T>& p, cudaStream_t
     case S3_TAU: s3_tau_k<T><<<gc, b, 0, s>>>(a, p); break;
     case S3_DV: s3_dV_k<T><<<gc, b, 0, s>>>(a, p); break;
     case S3_V: s3_V_k<T><<<gc, b, 0, s>>>(a); break;
-    case S3_PTAU:
-        if (s3_idx32(a)) s3_Ptau_k<T, S3_PLAIN, int><<<gc, b, 0, s>>>(a, p);
-        else s3_Ptau_k<T, S3_PLAIN, int64_t><<<gc, b, 0, s>>>(a, p);
-        break;
-    case S3_DVV:
-        if (s3_idx32(a)) s3_dVV_k<T, S3_PLAIN, int><<<gc, b, 0, s>>>(a, p);
-        else s3_dVV_k<T, S3_PLAIN, int64_t><<<gc, b, 0, s>>>(a, p);
-        break;
     case S3_BC: {
         const int64_t face = std::max(std::max((a.nx + 1) * (a.ny + 1), (a.nx + 1) * (a.nz + 1)), (a.ny + 1) * (a.nz + 1));
         s3_bc_k<T><<<dim3((unsigned)std::min<int64_t>((face + 255) / 256, 1024), 12), 256, 0, s>>>(a);
@@ -723,11 +925,11 @@ static void s3_launch(S3Kernel k, const S3A<T>& a, const S3P<T>& p, cudaStream_t
     }
 }
 
-// n iterations of MODE on the state (a.Vx, a.Vy, a.Vz, a.Pt): pairs of one-launch iterations
-// through the second set B (the state is back in a's arrays after each pair), then the remaining
-// one or two iterations as the three kernels that also store ∇V, τ and R (the reference's loop
-// body leaves them, and the solvers' residual norms read them). With n >= 1 the last iteration
-// always stores. B.Vx.. B.Pt: arrays of the shapes of a's.
+// n iterations of MODE on the state (a.Vx, a.Vy, a.Vz, a.Pt): with one_launch, pairs of one-launch
+// iterations through the second set B (the state is back in a's arrays after each pair), then the
+// remaining ones as the two kernels in place, the last of which also stores ∇V and R (the reference's
+// loop body leaves them, and the solvers' residual norms read them). B.Vx.. B.Pt: arrays of the
+// shapes of a's.
 template <typename T, int MODE>
 static void s3_iterations(const S3A<T>& a, const S3Out<T>& B, const S3P<T>& p, int64_t n, cudaStream_t s,
                           bool one_launch) {
@@ -743,17 +945,13 @@ static void s3_iterations(const S3A<T>& a, const S3Out<T>& B, const S3P<T>& p, i
         s3_fused_launch<T, MODE>(a, toB, p, s);
         s3_fused_launch<T, MODE>(b, toA, p, s);
     }
-    const dim3 b3(32, 8, 1), gc = g3(a.nx, a.ny, a.nz);
-    for (int64_t i = 2 * pairs; i < n; ++i) {
-        s3_iteration_kernels<T, MODE>(a, p, gc, b3, s);
-        s3_launch(S3_BC, a, p, s);
-    }
+    for (int64_t i = 2 * pairs; i + 1 < n; ++i) s3_iteration_kernels<T, MODE, false>(a, p, i > 2 * pairs, s);
+    s3_iteration_kernels<T, MODE, true>(a, p, n - 1 > 2 * pairs, s);
 }
 
 // divV, the stresses and Rx, Ry, Rz of the FP64 state (the reference's statements, no update)
 static void s3_residual(const S3A<double>& a, const S3P<double>& p, cudaStream_t s) {
-    const dim3 b(32, 8, 1), gc = g3(a.nx, a.ny, a.nz);
-    s3_iteration_kernels<double, S3_RESIDUAL>(a, p, gc, b, s);
+    s3_iteration_kernels<double, S3_RESIDUAL, true>(a, p, false, s);
 }
 
 // Library scratch of the iterate entry point: grow-only, one per device and stream.
@@ -1002,15 +1200,6 @@ int ps_stokes3d_iterate_ex(const ps_stokes3d_fields* f, const ps_stokes3d_params
     if (n_iter < 0) return fail(PS_ERR_ARG, "n_iter must be >= 0");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (n_iter == 0) return PS_OK;
-    if (!one_launch) {  // the three storing kernels per iteration, in place
-        for (int64_t it = 0; it < n_iter; ++it) {
-            if (f->Pt.dtype == PS_F64)
-                s3_iterations<double, S3_PLAIN>(s3a<double>(f), S3Out<double>{}, s3p<double>(*p), 1, s, false);
-            else
-                s3_iterations<float, S3_PLAIN>(s3a<float>(f), S3Out<float>{}, s3p<float>(*p), 1, s, false);
-        }
-        return finish_launch(s, 1, "ps_stokes3d_iterate");
-    }
     // the second state set of the one-launch iterations (grow-only library scratch per device and stream)
     const size_t es = elsize(f->Pt.dtype);
     const size_t nb[4] = {(size_t)numel(f->Vx) * es, (size_t)numel(f->Vy) * es, (size_t)numel(f->Vz) * es,
@@ -1021,7 +1210,7 @@ int ps_stokes3d_iterate_ex(const ps_stokes3d_fields* f, const ps_stokes3d_params
         total += (nb[i] + 255) / 256 * 256;
     }
     char* base = nullptr;
-    PS_TRY(s3_scratch(total, &base, s));
+    if (one_launch) PS_TRY(s3_scratch(total, &base, s));
     if (f->Pt.dtype == PS_F64) {
         const S3Out<double> B{reinterpret_cast<double*>(base + off[0]), reinterpret_cast<double*>(base + off[1]),
                               reinterpret_cast<double*>(base + off[2]), reinterpret_cast<double*>(base + off[3])};

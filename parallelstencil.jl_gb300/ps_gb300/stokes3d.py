@@ -3,7 +3,7 @@
 ``Stokes3D`` holds the miniapp's arrays (Stokes3D.jl:89-110) as device arrays in Julia layout and
 exposes the `@parallel` kernels one-to-one (``compute_timesteps``, ``compute_P``, ``compute_tau``,
 ``compute_dV``, ``compute_V``, ``bc``), ``step_reference_sequence()`` (the loop body as the
-miniapp writes it, ten launches), ``iterate(n)`` (the loop body in three launches per
+miniapp writes it, ten launches), ``iterate(n)`` (the loop body in two launches per
 iteration), ``err()`` (Stokes3D.jl:145-146) and ``solve(tol)`` (the `while err > ε` loop in FP64).
 """
 from __future__ import annotations
