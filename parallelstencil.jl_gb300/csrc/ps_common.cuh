@@ -50,7 +50,6 @@ struct DeviceState {
 int current_state(DeviceState** st);
 // Frees library-owned solver scratch (ps_finalize).
 void stokes2d_free_scratch();
-void stokes2d_static_forget();  // drop the cached device addresses of the static scratch array
 void diffusion_free_scratch();
 void adjoint_free_scratch();
 void acoustic_free_scratch();

@@ -401,7 +401,6 @@ int ps_finalize(void) {
     adjoint_free_scratch();
     acoustic_free_scratch();
     stokes3d_free_scratch();
-    stokes2d_static_forget();
     for (int d = 0; d < kMaxDevices; d++) {
         DeviceState& st = g_dev[d];
         if (!st.ready) continue;

@@ -6,11 +6,9 @@
 //                             below so all paths round identically
 //   one-to-one kernels        compute_timesteps!, compute_P!, compute_τ!, compute_dV!, compute_V!,
 //                             bc_x!, bc_y! -- the drop-in replacements of the six `@parallel` calls
-//   s2_march                  one whole PT iteration in FP32: warps march along y with the previous row in
-//                             registers and the neighbour columns by shuffles. Old/new V and Pt are
-//                             ping-pong buffers, so results are identical to the six-kernel sequence.
-//                             Optional fused FP64 reduction of Σ|Rx|, Σ|Ry|, Σ|∇V|.
-//   s2_cells, s2_faces        the FP64 iteration in place, one thread per position, the same reductions.
+//   s2_cells, s2_faces        one whole PT iteration in place, one thread per position; results are
+//                             identical to the six-kernel sequence. Optional fused FP64 reduction of
+//                             Σ|Rx|, Σ|Ry|, Σ|∇V|.
 //   s2_residual64             FP64 residuals of the current state (no pseudo-time update) for the
 //                             defect-correction outer loop.
 //   ps_stokes2d_solve         PT solve to `tol` in FP64 (mode 0) or with FP32 PT sweeps on the
@@ -187,13 +185,10 @@ __global__ void s2_bc_y_k(T* A, int64_t n0, int64_t n1) {
 // =======================================================================================
 template <typename T>
 struct S2Fused {
-    // state in / out (ping-pong) and in-place pseudo-velocities
-    const T* Vx_in;
-    const T* Vy_in;
-    const T* P_in;
-    T* Vx_out;
-    T* Vy_out;
-    T* P_out;
+    // the state and the pseudo-velocities, in place
+    T* Vx;
+    T* Vy;
+    T* P;
     T* dVxdt;
     T* dVydt;
     const T* Mus;
@@ -205,11 +200,11 @@ struct S2Fused {
     const T* fp;  // (nx, ny)
     const T* fx;  // (nx-1, ny-2)
     const T* fy;  // (nx-2, ny-1)
-    // temporaries of the reference (written only if STORE_TMP)
-    T* divV;
     T* txx;
     T* tyy;
     T* txy;
+    // temporaries of the reference (written only if STORE_TMP)
+    T* divV;
     T* Rx;
     T* Ry;
     double* red;  // Σ|Rx|, Σ|Ry|, Σ|∇V| (NULL: no reduction)
@@ -222,199 +217,20 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// One PT iteration as a march along y: a warp owns 30 columns (lanes 1..30; lanes 0 and 31 hold the
-// neighbour columns) and `rows` rows. Row j's step computes the cell (c, j) -- ∇V, P, τxx, τyy -- and
-// the corner (c, j-1) above row j-1, then the Vy face (c, j) and, a row late because it needs the
-// corner above it, the Vx face (c, j-1). What the next row needs stays in registers, the values of
-// the columns c - 1 and c + 1 come by shuffles, and row j + 1's loads are issued before row j is
-// computed: no barrier, no shared memory, and only one extra row per segment and two extra columns
-// per strip are computed twice. Quotients are taken without testing their dividends; a warp that met
-// one too small for that computes the row again with the tests (DivF, div_c).
+// One PT iteration as two kernels in place, one thread per position: s2_cells (∇V, P and the stresses) and
+// s2_faces (residuals, pseudo-velocities, velocities and the free-slip copies; a face reads no other
+// face's velocity). Nothing is computed twice, every load of a thread is issued before its first store,
+// and the constant arrays' loads go out while the kernel before still runs.
 //
-// Bound: the latency of a row's loads and of its dependent instructions, at 20 warps per SM. Against the
-// 32 x 8 tile kernel before it (window in shared memory, halo computed twice, bounds tests per staged
-// value), per iteration: 1023^2 37.8 -> 16.6 us (3.8 TB/s on 15 words per cell), 511^2 7.8, 63^2 3.5 us,
-// where the launches of successive iterations overlap (programmatic dependent launch).
+// Bound: FP64 pipe (FP64: 57 FP64 instructions per cell, 80 % busy), L2 and launches (FP32: 24 words per
+// cell). Per iteration, against one kernel on shared-memory tiles that computed a halo twice and tested
+// every dividend: FP64 511^2 82 -> 32.8 us, 1023^2 270 -> 118 us; FP32 1023^2 37.8 -> 15.4 us, 511^2 6.6 us,
+// 63^2 3.6 us. A march along y with rows in registers and shuffles (one kernel, 15 words per cell) was
+// measured at 16.6, 7.8 and 3.5 us in FP32 and 150 us in FP64 at 1023^2: its few long warps wait on loads
+// and, in FP64, leave the pipe idle.
 //
-// I: index type (int where every array has fewer than 2^31 elements: fewer instructions per cell).
-// RED: a.red is set (the FP64 sums are compiled in only then: the conversions to double run on the
-// FP64 pipe even when predicated off).
-constexpr int S2_W = 4;  // warps per block; five blocks per SM (six or more: 17.7-18.7 us at 1023^2, spills)
-
-template <bool DEFECT, typename T>
-struct S2Row {  // one lane's inputs of a row
-    T vx, vyn, mus, p, dtp, f, xdv, xdt, xf, ydv, ydt, yf;
-};
-
-template <typename T, bool DEFECT, bool STORE_TMP, typename I, bool RED>
-__global__ void __launch_bounds__(32 * S2_W, 5) s2_march(S2Fused<T> a, S2P<T> p, int rows) {
-    const I nx = (I)a.nx, ny = (I)a.ny;
-    const int lane = threadIdx.x;
-    const I c = (I)blockIdx.x * 30 - 1 + lane;
-    const I r0 = ((I)blockIdx.y * S2_W + (I)threadIdx.y) * rows;
-    if (r0 >= ny) return;  // whole warps only: shuffles follow, no barrier
-    const I r1 = r0 + rows < ny ? r0 + rows : ny;
-    grid_dependency_wait();  // the state is read with plain loads: __ldg need not see the kernel before
-    grid_dependents_may_launch();
-    const bool last = r1 == ny;  // this segment also takes the Vy faces ny
-    const bool own = lane >= 1 && lane <= 30;
-    const bool cx = c >= 0 && c < nx, vxx = c >= 0 && c <= nx;
-    const bool xinx = c >= 1 && c <= nx - 1;  // Vx face column with a residual
-    const bool yinx = c >= 1 && c <= nx - 2;  // Vy face column with a residual
-    using Row = S2Row<DEFECT, T>;
-
-    // inputs of row j: cell row j, Vy faces j + 1 (the cell's upper side; faces j are carried), Vx faces of
-    // row j - 1 (finished in this step). Offsets of the next row to load: cells and Vy, Vx, and the
-    // residual arrays of the two faces.
-    I oC = c + nx * (r0 - 1), oX = oC + (r0 - 1), oU = (c - 1) + (nx - 1) * (r0 - 3), oV = (c - 1) + (nx - 2) * (r0 - 2);
-    auto load = [&](I j) {
-        Row r{};
-        const bool cy = j >= 0 && j < ny;
-        if (vxx && cy) r.vx = a.Vx_in[oX];
-        if (cx && j >= -1 && j < ny) r.vyn = a.Vy_in[oC + nx];
-        if (cx && cy) {
-            r.mus = __ldg(a.Mus + oC);
-            if (j < r1) {
-                r.p = a.P_in[oC];
-                r.dtp = __ldg(a.dtPt + oC);
-                if constexpr (DEFECT) r.f = __ldg(a.fp + oC);
-                else r.yf = __ldg(a.Rog + oC);
-            }
-        }
-        if (own && xinx && j > r0 && j >= 2 && j <= ny - 1) {
-            r.xdv = a.dVxdt[oU];
-            r.xdt = __ldg(a.dtVx + oU);
-            if constexpr (DEFECT) r.xf = __ldg(a.fx + oU);
-        }
-        if (own && yinx && j >= r0 && j < r1 && j >= 1) {
-            r.ydv = a.dVydt[oV];
-            r.ydt = __ldg(a.dtVy + oV);
-            if constexpr (DEFECT) r.yf = __ldg(a.fy + oV);
-        }
-        oC += nx;
-        oX += nx + 1;
-        oU += nx - 1;
-        oV += nx - 2;
-        return r;
-    };
-
-    // carried from row j - 1: Vx and its right neighbour, Mus and its pair sum with the right neighbour,
-    // P, τyy, the x parts of Rx, the corner's left neighbour, Rog
-    T vx_m = T(0), vxr_m = T(0), mus2_m = T(0), p_m = T(0), tyy_m = T(0), ax_m = T(0), px_m = T(0),
-      tl_m = T(0), rog_m = T(0);
-    double acc_rx = 0.0, acc_ry = 0.0, acc_div = 0.0;
-
-    T vy0 = (cx && r0 >= 1) ? a.Vy_in[oC] : T(0);  // Vy faces of row r0 - 1
-    Row cur = load(r0 - 1);
-    for (I j = r0 - 1; j <= r1; ++j) {
-        // offsets of row j (load leaves them at the next row)
-        const I qC = oC - nx, qX = oX - (nx + 1), qU = oU - (nx - 1), qV = oV - (nx - 2);
-        Row nxt{};
-        if (j < r1) nxt = load(j + 1);
-        const T vx = cur.vx, vy1 = cur.vyn, mus = cur.mus;
-        const T vxr = __shfl_down_sync(0xFFFFFFFFu, vx, 1);
-        const T vyr = __shfl_down_sync(0xFFFFFFFFu, vy0, 1);
-        const T musr = __shfl_down_sync(0xFFFFFFFFu, mus, 1);
-        T d, pn, txx, tyy, t, tl, ax, px, rx, ry;
-        auto row = [&](auto hx, auto hy) {
-            // cell (c, j)
-            d = s2_divV(vx, vxr, vy0, vy1, hx, hy);
-            T dp = d;
-            if constexpr (DEFECT) dp = d + cur.f;
-            pn = cur.p - cur.dtp * dp;
-            txx = s2_tau_nn(mus, vx, vxr, d, hx);
-            tyy = s2_tau_nn(mus, vy0, vy1, d, hy);
-            // corner (c, j-1): between rows j-1 and j, columns c and c+1
-            t = s2_tau_xy_sum((mus2_m + mus) + musr, vxr - vxr_m, vyr - vy0, hx, hy);
-            // the left neighbours' values
-            const T txl = __shfl_up_sync(0xFFFFFFFFu, txx, 1), pl = __shfl_up_sync(0xFFFFFFFFu, pn, 1);
-            tl = __shfl_up_sync(0xFFFFFFFFu, t, 1);
-            // Vx face (c, j-1), whose x differences were taken in the last step
-            rx = (ax_m + dvd(tl - tl_m, hy)) - px_m;
-            ax = dvd(txx - txl, hx);
-            px = dvd(pn - pl, hx);
-            // Vy face (c, j)
-            ry = (dvd(tyy - tyy_m, hy) + dvd(t - tl, hx)) - dvd(pn - p_m, hy);
-        };
-        uint32_t key = 0xFFFFFFFFu;
-        row(DivF<T>{p.dx, &key}, DivF<T>{p.dy, &key});
-        if (__any_sync(0xFFFFFFFFu, key < p.lo)) row(p.dx, p.dy);
-
-        if (own && j >= r0) {
-            if (cx && j < r1) {  // cell (c, j), P
-                a.P_out[qC] = pn;
-                if constexpr (STORE_TMP) {
-                    a.divV[qC] = d;
-                    a.txx[qC] = txx;
-                    a.tyy[qC] = tyy;
-                }
-                if constexpr (RED) acc_div += fabs((double)(DEFECT ? d + cur.f : d));
-            }
-            // corner (c, j-1), 0 <= j-1 < ny-1
-            if constexpr (STORE_TMP)
-                if (j > r0 && j < ny && c >= 0 && c < nx - 1) a.txy[c + (nx - 1) * (j - 1)] = t;
-            // Vx face (c, j-1); bc_y!(Vx): rows 0 and ny-1 copy rows 1 and ny-2
-            if (vxx && j > r0 && j >= 2 && j <= ny - 1) {
-                T vnew = vx_m;
-                if (xinx) {
-                    T r = rx;
-                    if constexpr (DEFECT) r = r + cur.xf;
-                    const T dv = p.dampX * cur.xdv + r;
-                    a.dVxdt[qU] = dv;
-                    if constexpr (STORE_TMP) a.Rx[qU] = r;
-                    if constexpr (RED) acc_rx += fabs((double)r);
-                    vnew = vnew + cur.xdt * dv;
-                }
-                a.Vx_out[qX - (nx + 1)] = vnew;
-                if (j == 2) a.Vx_out[c] = vnew;
-                if (j == ny - 1) a.Vx_out[qX] = vnew;
-            }
-            // Vy face (c, j); bc_x!(Vy): columns 0 and nx-1 copy columns 1 and nx-2
-            if (yinx && (j < r1 || last)) {
-                T vnew = vy0;
-                if (j >= 1 && j <= ny - 1) {
-                    T r = ry;
-                    if constexpr (DEFECT) r = r + cur.yf;
-                    else r = r + (rog_m + cur.yf) * T(0.5);
-                    const T dv = p.dampY * cur.ydv + r;
-                    a.dVydt[qV] = dv;
-                    if constexpr (STORE_TMP) a.Ry[qV] = r;
-                    if constexpr (RED) acc_ry += fabs((double)r);
-                    vnew = vnew + cur.ydt * dv;
-                }
-                a.Vy_out[qC] = vnew;
-                if (c == 1) a.Vy_out[qC - 1] = vnew;
-                if (c == nx - 2) a.Vy_out[qC + 1] = vnew;
-            }
-        }
-        vy0 = vy1;
-        vx_m = vx;
-        vxr_m = vxr;
-        mus2_m = mus + musr;
-        p_m = pn;
-        tyy_m = tyy;
-        ax_m = ax;
-        px_m = px;
-        tl_m = tl;
-        if constexpr (!DEFECT) rog_m = cur.yf;
-        cur = nxt;
-    }
-    if constexpr (RED) {
-        const double s0 = warp_sum(acc_rx), s1 = warp_sum(acc_ry), s2 = warp_sum(acc_div);
-        if (lane == 0) {
-            atomicAdd(a.red, s0);
-            atomicAdd(a.red + 1, s1);
-            atomicAdd(a.red + 2, s2);
-        }
-    }
-}
-
-// The FP64 iteration: two kernels in place, one thread per position and no halo computed twice, because
-// the FP64 pipe bounds it (57 FP64 instructions per cell; the march above issues a sixth more for its
-// extra rows and columns, and its few warps per scheduler leave the pipe idle between dependent
-// instructions). s2_cells: ∇V, P and the stresses; s2_faces: residuals, pseudo-velocities, velocities and
-// the free-slip copies (a face reads no other face's velocity). Per iteration, against a 32 x 16 tile
-// kernel that computes its halo twice: 511^2 82 -> 32.8 us, 1023^2 270 -> 117 us (80 % of the FP64 pipe).
+// RED: a.red is set (the FP64 sums are compiled in only then: the conversions to double run on the FP64
+// pipe even when predicated off). I: index type (int where every array has fewer than 2^31 elements).
 //
 // S2_DIV evaluates a statement without testing each dividend, and again with the tests (and the IEEE
 // division where they fail) in the rare case that one of its dividends is too small.
@@ -426,101 +242,159 @@ __global__ void __launch_bounds__(32 * S2_W, 5) s2_march(S2Fused<T> a, S2P<T> p,
     } while (0)
 
 // (a + b) * 0.5, the buoyancy average
-template <typename H>
-__device__ __forceinline__ double s2_half_sum(double a, double b, H) {
-    return (a + b) * 0.5;
+template <typename T, typename H>
+__device__ __forceinline__ T s2_half_sum(T a, T b, H) {
+    return (a + b) * T(0.5);
 }
 __device__ __forceinline__ double s2_half_sum(double a, double b, DivF<double> h) { return scale_pow2(a + b, -1, h.key); }
 
-template <typename I, bool STORE_TMP, bool RED>
-__global__ void __launch_bounds__(256) s2_cells(S2Fused<double> a, S2P<double> p) {
-    using T = double;
+// Rows of 32 threads per block. FP32: 8; FP64, bound by the FP64 pipe: 2, which spreads a small grid more
+// evenly over the SMs (8 rows -> 2: 255^2 11.4 -> 10.7 us per iteration, 130^2 7.1 -> 6.3, 1023^2 118 both).
+template <typename T>
+__host__ __device__ constexpr int s2_block_rows() {
+    return sizeof(T) == 4 ? 8 : 2;
+}
+
+template <typename T, bool DEFECT, typename I, bool STORE_TMP, bool RED>
+__global__ void __launch_bounds__(32 * s2_block_rows<T>()) s2_cells(S2Fused<T> a, S2P<T> p) {
     const I nx = (I)a.nx, ny = (I)a.ny;
-    const I i = (I)(blockIdx.x * 32 + threadIdx.x), j = (I)(blockIdx.y * 8 + threadIdx.y);
+    const I i = (I)(blockIdx.x * 32 + threadIdx.x), j = (I)(blockIdx.y * s2_block_rows<T>() + threadIdx.y);
+    const I c = i + nx * j, cx = c + j;  // Vx rows have nx + 1 faces
+    const bool cell = i < nx && j < ny, corner = i < nx - 1 && j < ny - 1;
+    // what no iteration writes, while the kernel before this one still runs
+    T m00 = T(0), m10 = T(0), m01 = T(0), m11 = T(0), dtp = T(0);
+    [[maybe_unused]] T f = T(0);
+    if (cell) {
+        m00 = __ldg(a.Mus + c);
+        dtp = __ldg(a.dtPt + c);
+        if constexpr (DEFECT) f = __ldg(a.fp + c);
+    }
+    if (corner) {
+        m10 = __ldg(a.Mus + c + 1);
+        m01 = __ldg(a.Mus + c + nx);
+        m11 = __ldg(a.Mus + c + nx + 1);
+    }
     grid_dependency_wait();  // the state is read with plain loads: __ldg need not see the kernel before
     grid_dependents_may_launch();
+    T vx0 = T(0), vx1 = T(0), vy0 = T(0), vy1 = T(0), pt = T(0), vxu = T(0), vyr = T(0);
+    if (cell) {
+        vx0 = a.Vx[cx];
+        vx1 = a.Vx[cx + 1];
+        vy0 = a.Vy[c];
+        vy1 = a.Vy[c + nx];
+        pt = a.P[c];
+    }
+    if (corner) {
+        vxu = a.Vx[cx + nx + 2];
+        vyr = a.Vy[c + nx + 1];
+    }
     double acc = 0.0;
-    if (i < nx && j < ny) {
-        const I c = i + nx * j, cx = c + j;  // Vx rows have nx + 1 faces
-        const T vx0 = a.Vx_out[cx], vx1 = a.Vx_out[cx + 1], vy0 = a.Vy_out[c], vy1 = a.Vy_out[c + nx];
-        const T mus = __ldg(a.Mus + c);
-        T d, txx, tyy;
-        auto strain = [&](auto hx, auto hy) {
-            d = s2_divV(vx0, vx1, vy0, vy1, hx, hy);
-            txx = s2_tau_nn(mus, vx0, vx1, d, hx);
-            tyy = s2_tau_nn(mus, vy0, vy1, d, hy);
-        };
-        S2_DIV(strain);
-        a.P_out[c] = a.P_out[c] - __ldg(a.dtPt + c) * d;
+    T d, txx, tyy, txy;
+    auto stresses = [&](auto hx, auto hy) {
+        d = s2_divV(vx0, vx1, vy0, vy1, hx, hy);
+        txx = s2_tau_nn(m00, vx0, vx1, d, hx);
+        tyy = s2_tau_nn(m00, vy0, vy1, d, hy);
+        txy = s2_tau_xy_sum(((m00 + m10) + m01) + m11, vxu - vx1, vyr - vy1, hx, hy);
+    };
+    S2_DIV(stresses);
+    if (cell) {
+        T dp = d;
+        if constexpr (DEFECT) dp = d + f;
+        a.P[c] = pt - dtp * dp;
         a.txx[c] = txx;
         a.tyy[c] = tyy;
         if constexpr (STORE_TMP) a.divV[c] = d;
-        if constexpr (RED) acc = fabs(d);
-        if (i < nx - 1 && j < ny - 1) {
-            const T msum = ((mus + __ldg(a.Mus + c + 1)) + __ldg(a.Mus + c + nx)) + __ldg(a.Mus + c + nx + 1);
-            const T dyVx = a.Vx_out[cx + nx + 2] - vx1, dxVy = a.Vy_out[c + nx + 1] - vy1;
-            T t;
-            auto shear = [&](auto hx, auto hy) { t = s2_tau_xy_sum(msum, dyVx, dxVy, hx, hy); };
-            S2_DIV(shear);
-            a.txy[c - j] = t;
-        }
+        if constexpr (RED) acc = fabs((double)dp);
     }
+    if (corner) a.txy[c - j] = txy;
     if constexpr (RED) {
         acc = warp_sum(acc);
         if (threadIdx.x == 0) atomicAdd(a.red + 2, acc);
     }
 }
 
-template <typename I, bool STORE_TMP, bool RED>
-__global__ void __launch_bounds__(256) s2_faces(S2Fused<double> a, S2P<double> p) {
-    using T = double;
+template <typename T, bool DEFECT, typename I, bool STORE_TMP, bool RED>
+__global__ void __launch_bounds__(32 * s2_block_rows<T>()) s2_faces(S2Fused<T> a, S2P<T> p) {
     const I nx = (I)a.nx, ny = (I)a.ny;
-    const I i = (I)(blockIdx.x * 32 + threadIdx.x), j = (I)(blockIdx.y * 8 + threadIdx.y);
-    grid_dependency_wait();  // the state is read with plain loads: __ldg need not see the kernel before
+    const I i = (I)(blockIdx.x * 32 + threadIdx.x), j = (I)(blockIdx.y * s2_block_rows<T>() + threadIdx.y);
+    const I c = i + nx * j, cx = c + j;  // cell and Vy face (i, j), Vx face (i, j)
+    const I kx = (i - 1) + (nx - 1) * (j - 1), ky = (i - 1) + (nx - 2) * (j - 1);  // residuals; kx: corner (i-1, j-1) too
+    const bool colx = i <= nx && j >= 1 && j <= ny - 2, fx = colx && i >= 1 && i <= nx - 1;  // Vx faces, with a residual
+    const bool coly = i >= 1 && i <= nx - 2 && j <= ny, fy = coly && j >= 1 && j <= ny - 1;
+    // what no iteration writes, while the kernel before this one still runs
+    T xt = T(0), yt = T(0), g0 = T(0), g1 = T(0);
+    [[maybe_unused]] T xf = T(0);
+    if (fx) {
+        xt = __ldg(a.dtVx + kx);
+        if constexpr (DEFECT) xf = __ldg(a.fx + kx);
+    }
+    if (fy) {
+        yt = __ldg(a.dtVy + ky);
+        if constexpr (DEFECT) {
+            g0 = __ldg(a.fy + ky);
+        } else {
+            g0 = __ldg(a.Rog + c - nx);
+            g1 = __ldg(a.Rog + c);
+        }
+    }
+    grid_dependency_wait();
     grid_dependents_may_launch();
+    T xr = T(0), xl = T(0), s00 = T(0), s01 = T(0), s10 = T(0), p0 = T(0), pl = T(0), pd = T(0), yu = T(0), yd = T(0);
+    T xg = T(0), yg = T(0), vx = T(0), vy = T(0);
+    if (fx || fy) {
+        s00 = a.txy[kx];
+        p0 = a.P[c];
+    }
+    if (fx) {
+        xr = a.txx[c];
+        xl = a.txx[c - 1];
+        s01 = a.txy[kx + (nx - 1)];
+        pl = a.P[c - 1];
+        xg = a.dVxdt[kx];
+    }
+    if (fy) {
+        yu = a.tyy[c];
+        yd = a.tyy[c - nx];
+        s10 = a.txy[kx + 1];
+        pd = a.P[c - nx];
+        yg = a.dVydt[ky];
+    }
+    if (colx) vx = a.Vx[cx];
+    if (coly) vy = a.Vy[c];
     double acc_x = 0.0, acc_y = 0.0;
-    const I c = i + nx * j;  // cell (i, j) and Vy face (i, j)
+    T rx, ry;
+    auto resid = [&](auto hx, auto hy) {
+        rx = s2_Rx(xl, xr, s00, s01, pl, p0, hx, hy);
+        ry = s2_Ry_core(yd, yu, s00, s10, pd, p0, hx, hy);
+        if constexpr (!DEFECT) ry = ry + s2_half_sum(g0, g1, hx);
+    };
+    S2_DIV(resid);
+    if constexpr (DEFECT) {
+        rx = rx + xf;
+        ry = ry + g0;
+    }
     // Vx face (i, j); bc_y!(Vx): rows 0 and ny-1 copy rows 1 and ny-2
-    if (i <= nx && j >= 1 && j <= ny - 2) {
-        const I cx = c + j;
-        T v = a.Vx_out[cx];
-        if (i >= 1 && i <= nx - 1) {
-            const I k = (i - 1) + (nx - 1) * (j - 1);  // residual index, and the corner (i-1, j-1)
-            const T txl = a.txx[c - 1], txr = a.txx[c], tb = a.txy[k], tt = a.txy[k + nx - 1], pl = a.P_out[c - 1],
-                    pr = a.P_out[c];
-            T r;
-            auto resid = [&](auto hx, auto hy) { r = s2_Rx(txl, txr, tb, tt, pl, pr, hx, hy); };
-            S2_DIV(resid);
-            const T dv = p.dampX * a.dVxdt[k] + r;
-            a.dVxdt[k] = dv;
-            if constexpr (STORE_TMP) a.Rx[k] = r;
-            if constexpr (RED) acc_x = fabs(r);
-            v = v + __ldg(a.dtVx + k) * dv;
-            a.Vx_out[cx] = v;
-        }
-        if (j == 1) a.Vx_out[i] = v;
-        if (j == ny - 2) a.Vx_out[cx + nx + 1] = v;
+    if (fx) {
+        const T dv = p.dampX * xg + rx;
+        a.dVxdt[kx] = dv;
+        if constexpr (STORE_TMP) a.Rx[kx] = rx;
+        if constexpr (RED) acc_x = fabs((double)rx);
+        vx = vx + xt * dv;
+        a.Vx[cx] = vx;
     }
+    if (colx && j == 1) a.Vx[i] = vx;
+    if (colx && j == ny - 2) a.Vx[cx + nx + 1] = vx;
     // Vy face (i, j); bc_x!(Vy): columns 0 and nx-1 copy columns 1 and nx-2
-    if (i >= 1 && i <= nx - 2 && j <= ny) {
-        T v = a.Vy_out[c];
-        if (j >= 1 && j <= ny - 1) {
-            const I k = (i - 1) + (nx - 2) * (j - 1), kc = (i - 1) + (nx - 1) * (j - 1);
-            const T tb = a.tyy[c - nx], tt = a.tyy[c], tl = a.txy[kc], tr = a.txy[kc + 1], pb = a.P_out[c - nx],
-                    pt = a.P_out[c], g0 = __ldg(a.Rog + c - nx), g1 = __ldg(a.Rog + c);
-            T r;
-            auto resid = [&](auto hx, auto hy) { r = s2_Ry_core(tb, tt, tl, tr, pb, pt, hx, hy) + s2_half_sum(g0, g1, hx); };
-            S2_DIV(resid);
-            const T dv = p.dampY * a.dVydt[k] + r;
-            a.dVydt[k] = dv;
-            if constexpr (STORE_TMP) a.Ry[k] = r;
-            if constexpr (RED) acc_y = fabs(r);
-            v = v + __ldg(a.dtVy + k) * dv;
-            a.Vy_out[c] = v;
-        }
-        if (i == 1) a.Vy_out[c - 1] = v;
-        if (i == nx - 2) a.Vy_out[c + 1] = v;
+    if (fy) {
+        const T dv = p.dampY * yg + ry;
+        a.dVydt[ky] = dv;
+        if constexpr (STORE_TMP) a.Ry[ky] = ry;
+        if constexpr (RED) acc_y = fabs((double)ry);
+        vy = vy + yt * dv;
+        a.Vy[c] = vy;
     }
+    if (coly && i == 1) a.Vy[c - 1] = vy;
+    if (coly && i == nx - 2) a.Vy[c + 1] = vy;
     if constexpr (RED) {
         acc_x = warp_sum(acc_x);
         acc_y = warp_sum(acc_y);
@@ -672,46 +546,13 @@ static void scratch_free(void* p) {
     g_scratch_all.erase(std::remove(g_scratch_all.begin(), g_scratch_all.end(), p), g_scratch_all.end());
 }
 
-// Rows per warp of the march (each segment computes one extra row): as few as fill the GPU's warps twice
-// over, so that the second round's loads overlap the first round's tail, at least 2, at most 32. 1023^2:
-// 6 rows 16.7 us per iteration, 12 (one round) 19.5, 4 17.9, 24 27.0; 255^2: 2 rows 3.7 us, 4 4.6, 8 6.8.
-static int s2_rows(int64_t ny, int64_t strips, int64_t warps) {
-    const int64_t segs = std::max<int64_t>(1, 2 * warps / strips);
-    return (int)std::min<int64_t>(32, std::max<int64_t>(2, (ny + segs - 1) / segs));
-}
-
 // 32-bit indices while every array's size and the offsets a few rows past it stay below 2^31
 static bool s2_index32(int64_t nx, int64_t ny) { return (nx + 32) * (ny + 4) < ((int64_t)1 << 31); }
 
-// dependent: the kernel before this one on the stream is the previous iteration's
-template <bool DEFECT, bool STORE_TMP>
-static void launch_march(const S2Fused<float>& a, const S2P<float>& p, cudaStream_t s, bool dependent) {
-    auto launch = [&](auto kernel, int& per_sm) {
-        if (!per_sm) per_sm = resident_ctas(kernel, 32 * S2_W, 0);
-        DeviceState* st = nullptr;
-        const int sms = current_state(&st) == PS_OK ? st->num_sms : 1;
-        const int64_t strips = (a.nx + 1 + 29) / 30;
-        const int rows = s2_rows(a.ny, strips, (int64_t)per_sm * sms * S2_W);
-        const int64_t segs = (a.ny + rows - 1) / rows;
-        const dim3 grd((unsigned)strips, (unsigned)((segs + S2_W - 1) / S2_W));
-        if (dependent) launch_dependent(kernel, grd, dim3(32, S2_W), 0, s, a, p, rows);
-        else kernel<<<grd, dim3(32, S2_W), 0, s>>>(a, p, rows);
-    };
-    static int occ[4];
-    const bool i32 = s2_index32(a.nx, a.ny);
-    if (a.red) {
-        if (i32) launch(s2_march<float, DEFECT, STORE_TMP, int, true>, occ[0]);
-        else launch(s2_march<float, DEFECT, STORE_TMP, int64_t, true>, occ[1]);
-    } else {
-        if (i32) launch(s2_march<float, DEFECT, STORE_TMP, int, false>, occ[2]);
-        else launch(s2_march<float, DEFECT, STORE_TMP, int64_t, false>, occ[3]);
-    }
-}
-
-// One FP64 iteration in place on the state A (the buffers B are not used).
-template <bool STORE_TMP>
-static void launch_cells_faces(const S2Fused<double>& a, const S2P<double>& p, cudaStream_t s, bool dependent) {
-    const dim3 blk(32, 8), gc = g2(a.nx, a.ny, blk), gf = g2(a.nx + 1, a.ny + 1, blk);
+// One iteration. dependent: the kernel before it on the stream is the previous iteration's.
+template <typename T, bool DEFECT, bool STORE_TMP>
+static void launch_cells_faces(const S2Fused<T>& a, const S2P<T>& p, cudaStream_t s, bool dependent) {
+    const dim3 blk(32, s2_block_rows<T>()), gc = g2(a.nx, a.ny, blk), gf = g2(a.nx + 1, a.ny + 1, blk);
     auto launch = [&](auto cells, auto faces) {
         if (dependent) launch_dependent(cells, gc, blk, 0, s, a, p);
         else cells<<<gc, blk, 0, s>>>(a, p);
@@ -719,20 +560,20 @@ static void launch_cells_faces(const S2Fused<double>& a, const S2P<double>& p, c
     };
     const bool i32 = s2_index32(a.nx, a.ny);
     if (a.red) {
-        if (i32) launch(s2_cells<int, STORE_TMP, true>, s2_faces<int, STORE_TMP, true>);
-        else launch(s2_cells<int64_t, STORE_TMP, true>, s2_faces<int64_t, STORE_TMP, true>);
+        if (i32) launch(s2_cells<T, DEFECT, int, STORE_TMP, true>, s2_faces<T, DEFECT, int, STORE_TMP, true>);
+        else launch(s2_cells<T, DEFECT, int64_t, STORE_TMP, true>, s2_faces<T, DEFECT, int64_t, STORE_TMP, true>);
     } else {
-        if (i32) launch(s2_cells<int, STORE_TMP, false>, s2_faces<int, STORE_TMP, false>);
-        else launch(s2_cells<int64_t, STORE_TMP, false>, s2_faces<int64_t, STORE_TMP, false>);
+        if (i32) launch(s2_cells<T, DEFECT, int, STORE_TMP, false>, s2_faces<T, DEFECT, int, STORE_TMP, false>);
+        else launch(s2_cells<T, DEFECT, int64_t, STORE_TMP, false>, s2_faces<T, DEFECT, int64_t, STORE_TMP, false>);
     }
 }
 
 template <typename T>
 static S2Fused<T> s2_dropin_args(const ps_stokes2d_fields* f) {
     S2Fused<T> a{};
-    a.Vx_in = a.Vx_out = P_<T>(f->Vx);
-    a.Vy_in = a.Vy_out = P_<T>(f->Vy);
-    a.P_in = a.P_out = P_<T>(f->Pt);
+    a.Vx = P_<T>(f->Vx);
+    a.Vy = P_<T>(f->Vy);
+    a.P = P_<T>(f->Pt);
     a.Mus = P_<T>(f->Mus);
     a.Rog = P_<T>(f->Rog);
     a.dtVx = P_<T>(f->dtauVx);
@@ -751,60 +592,18 @@ static S2Fused<T> s2_dropin_args(const ps_stokes2d_fields* f) {
     return a;
 }
 
-// n_iter FP64 iterations; the temporaries nothing reads between iterations are stored in the last
-static void s2_iterate64(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp, int64_t n_iter, cudaStream_t s) {
-    const S2P<double> p = s2p<double>(*pp);
-    const S2Fused<double> a = s2_dropin_args<double>(f);
-    for (int64_t it = 0; it < n_iter; ++it) {
-        if (it == n_iter - 1) launch_cells_faces<true>(a, p, s, it > 0);
-        else launch_cells_faces<false>(a, p, s, it > 0);
-    }
-}
-
-// n_iter FP32 iterations between the caller's state and the ping-pong buffers B
-static void s2_iterate32(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp, int64_t n_iter, float* const B[3],
-                         cudaStream_t s) {
-    const S2P<float> p = s2p<float>(*pp);
-    S2Fused<float> a = s2_dropin_args<float>(f);
-    float* const A[3] = {a.Vx_out, a.Vy_out, a.P_out};
-    for (int64_t it = 0; it < n_iter; ++it) {
-        float* const* in = (it % 2 == 0) ? A : B;
-        float* const* out = (it % 2 == 0) ? B : A;
-        a.Vx_in = in[0];
-        a.Vy_in = in[1];
-        a.P_in = in[2];
-        a.Vx_out = out[0];
-        a.Vy_out = out[1];
-        a.P_out = out[2];
-        if (it == n_iter - 1) launch_march<false, true>(a, p, s, it > 0);
-        else launch_march<false, false>(a, p, s, it > 0);
-    }
-    if (n_iter % 2 == 1) {
-        const int64_t n[3] = {numel(f->Vx), numel(f->Vy), numel(f->Pt)};
-        for (int k = 0; k < 3; k++) cudaMemcpyAsync(A[k], B[k], n[k] * sizeof(float), cudaMemcpyDeviceToDevice, s);
-    }
-}
-
-static int iterate_dropin(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp, int64_t n_iter, cudaStream_t s) {
-    void* buf = nullptr;
-    if (f->Pt.dtype == PS_F64) {
-        s2_iterate64(f, pp, n_iter, s);
-    } else {
-        const int64_t n[2] = {numel(f->Vx), numel(f->Vy)};
-        PS_TRY(scratch_alloc(&buf, (n[0] + n[1] + numel(f->Pt)) * sizeof(float) + 256));
-        float* const B[3] = {static_cast<float*>(buf), static_cast<float*>(buf) + n[0],
-                             static_cast<float*>(buf) + n[0] + n[1]};
-        s2_iterate32(f, pp, n_iter, B, s);
-    }
-    cudaError_t e = cudaStreamSynchronize(s);
-    scratch_free(buf);
-    if (e != cudaSuccess) return cuda_fail(e, "ps_stokes2d_iterate");
-    return PS_OK;
+// n_iter iterations; the temporaries nothing reads between iterations are stored in the last
+template <typename T>
+static void s2_iterate(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp, int64_t n_iter, cudaStream_t s) {
+    const S2P<T> p = s2p<T>(*pp);
+    const S2Fused<T> a = s2_dropin_args<T>(f);
+    for (int64_t it = 0; it + 1 < n_iter; ++it) launch_cells_faces<T, false, false>(a, p, s, it > 0);
+    if (n_iter > 0) launch_cells_faces<T, false, true>(a, p, s, n_iter > 1);
 }
 
 // ---- solver ---------------------------------------------------------------------------
 // Runs `nout` iterations per CUDA graph launch; the last one of each graph accumulates Σ|Rx|, Σ|Ry|,
-// Σ|∇V| into `red`. nout is even: the FP32 ping-pong ends where it began.
+// Σ|∇V| into `red`.
 struct PTRunner {
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
@@ -861,7 +660,7 @@ static int solve_fp64(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp,
     int rc = r.build(s, nout, red, [&](int64_t it, double* rd) {
         S2Fused<double> k = a;
         k.red = rd;
-        launch_cells_faces<false>(k, p, s, it > 0);
+        launch_cells_faces<double, false, false>(k, p, s, it > 0);
     });
     const double nrx = (double)((nx - 1) * (ny - 2)), nry = (double)((nx - 2) * (ny - 1)), nd = (double)(nx * ny);
     double t0 = now_s(), err = INFINITY, h[3];
@@ -907,8 +706,8 @@ static int solve_mixed(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp
     int64_t nx = f->Pt.n[0], ny = f->Pt.n[1];
     const int64_t nVx = (nx + 1) * ny, nVy = nx * (ny + 1), nP = nx * ny, nRx = (nx - 1) * (ny - 2),
                   nRy = (nx - 2) * (ny - 1);
-    // float buffers: δVx a/b, δVy a/b, δP a/b, dVxdτ, dVydτ, fx, fy, fp, Mus32, dτVx, dτVy, dτPt
-    const int64_t counts[15] = {nVx, nVx, nVy, nVy, nP, nP, nRx, nRy, nRx, nRy, nP, nP, nRx, nRy, nP};
+    // float buffers: δVx, δVy, δP, dVxdτ, dVydτ, fx, fy, fp, Mus32, dτVx, dτVy, dτPt, τxx, τyy, τxy
+    const int64_t counts[15] = {nVx, nVy, nP, nRx, nRy, nRx, nRy, nP, nP, nRx, nRy, nP, nP, nP, (nx - 1) * (ny - 1)};
     size_t off[16];
     off[0] = 0;
     for (int k = 0; k < 15; k++) off[k + 1] = off[k] + ((counts[k] * 4 + 255) / 256) * 256;
@@ -923,7 +722,7 @@ static int solve_mixed(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp
     cudaError_t e = cudaMemsetAsync(buf, 0, off[15], s);
     if (e != cudaSuccess) rc = cuda_fail(e, "memset");
     const double* Mus = P_<double>(f->Mus);
-    s2_to_f32<<<256, 256, 0, s>>>(F(11), Mus, nP);
+    s2_to_f32<<<256, 256, 0, s>>>(F(8), Mus, nP);
     // The corrections keep the free-slip copies (bc_y!(Vx), bc_x!(Vy)) of the state they are added
     // to, so a start state that violates them (an externally supplied guess) would keep its
     // violation: apply the copies once, as the first FP64 PT iteration would.
@@ -932,28 +731,27 @@ static int solve_mixed(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp
 
     S2Fused<float> a{};
     const S2P<float> p32 = s2p<float>(*pp);
-    a.Mus = F(11);
-    a.dVxdt = F(6);
-    a.dVydt = F(7);
-    a.fx = F(8);
-    a.fy = F(9);
-    a.fp = F(10);
+    a.Vx = F(0);
+    a.Vy = F(1);
+    a.P = F(2);
+    a.dVxdt = F(3);
+    a.dVydt = F(4);
+    a.fx = F(5);
+    a.fy = F(6);
+    a.fp = F(7);
+    a.Mus = F(8);
+    a.txx = F(12);
+    a.tyy = F(13);
+    a.txy = F(14);
     a.nx = nx;
     a.ny = ny;
-    s2_solver_timesteps(a, p32, F(12), F(13), F(14), s);
+    s2_solver_timesteps(a, p32, F(9), F(10), F(11), s);
     PTRunner r;
     if (rc == PS_OK)
         rc = r.build(s, nout, red_in, [&](int64_t it, double* rd) {
-            const int i = (int)(it % 2), o = 1 - i;
             S2Fused<float> k = a;
-            k.Vx_in = F(i);
-            k.Vy_in = F(2 + i);
-            k.P_in = F(4 + i);
-            k.Vx_out = F(o);
-            k.Vy_out = F(2 + o);
-            k.P_out = F(4 + o);
             k.red = rd;
-            launch_march<true, false>(k, p32, s, it > 0);
+            launch_cells_faces<float, true, false>(k, p32, s, it > 0);
         });
 
     S2P<double> p64 = s2p<double>(*pp);
@@ -966,7 +764,7 @@ static int solve_mixed(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp
         // FP64 residual of the outer state -> fx, fy, fp (float) and err
         cudaMemsetAsync(red_out, 0, 3 * sizeof(double), s);
         s2_residual64<<<grd, blk, 0, s>>>(P_<double>(f->Vx), P_<double>(f->Vy), P_<double>(f->Pt), Mus,
-                                          P_<double>(f->Rog), F(10), F(8), F(9), red_out, nx, ny, p64);
+                                          P_<double>(f->Rog), F(7), F(5), F(6), red_out, nx, ny, p64);
         e = cudaMemcpyAsync(h, red_out, sizeof(h), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
@@ -986,7 +784,7 @@ static int solve_mixed(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp
         }
         ++outer;
         // inner FP32 PT on the correction, from zero
-        cudaMemsetAsync(c, 0, off[8], s);  // δV, δP (a and b), dVxdτ, dVydτ
+        cudaMemsetAsync(c, 0, off[5], s);  // δV, δP, dVxdτ, dVydτ
         double target = std::max(err * inner_rtol, tol * 0.25);
         double ierr = INFINITY;
         while (it < max_iter) {
@@ -1009,10 +807,10 @@ static int solve_mixed(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp
             if (ierr > 0.98 * prev && ierr < err * 0.5) break;
         }
         if (rc != PS_OK) break;
-        // FP64 update of the outer state with the FP32 correction (in A after nout even)
+        // FP64 update of the outer state with the FP32 correction
         s2_axpy32<<<256, 256, 0, s>>>(P_<double>(f->Vx), F(0), nVx);
-        s2_axpy32<<<256, 256, 0, s>>>(P_<double>(f->Vy), F(2), nVy);
-        s2_axpy32<<<256, 256, 0, s>>>(P_<double>(f->Pt), F(4), nP);
+        s2_axpy32<<<256, 256, 0, s>>>(P_<double>(f->Vy), F(1), nVy);
+        s2_axpy32<<<256, 256, 0, s>>>(P_<double>(f->Pt), F(2), nP);
     }
     r.destroy();
     cudaStreamSynchronize(s);
@@ -1178,7 +976,8 @@ int ps_stokes2d_iterate(const ps_stokes2d_fields* f, const ps_stokes2d_params* p
     if (!p) return fail(PS_ERR_NULL, "NULL params");
     if (n_iter < 0) return fail(PS_ERR_ARG, "n_iter must be >= 0");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    PS_TRY(iterate_dropin(f, p, n_iter, s));
+    if (f->Pt.dtype == PS_F64) s2_iterate<double>(f, p, n_iter, s);
+    else s2_iterate<float>(f, p, n_iter, s);
     return finish_launch(s, 1, "ps_stokes2d_iterate");
 }
 
@@ -1241,75 +1040,27 @@ int ps_stokes2d_solve(const ps_stokes2d_fields* f, const ps_stokes2d_params* p, 
 
 
 // =======================================================================================
-// ps_stokes2d_iterate_static: the fused PT iteration without any device allocation.
-//
-// ps_stokes2d_iterate needs three ping-pong buffers (the old/new Vx, Vy, Pt) and allocates them
-// per call. Some hosts cannot let a library allocate device memory: an application whose device
-// memory is fully owned by its own pool allocator (CUDA.jl's memory pool, a framework caching
-// allocator), where a cudaMalloc behind its back fails or fragments the pool, and code that must
-// not call cudaFree, which synchronises the whole device. This variant takes its ping-pong buffers
-// from a fixed device array compiled into the library instead.
-//
-// The array is file-scope, kStaticScratchBytes (16 MiB) on every device that loads the library,
-// held until process exit. Host code must not pass the array's name to a kernel (on the host it
-// is only a stand-in symbol): its device address is looked up once per device with
-// cudaGetSymbolAddress, on the first call on that device, with that device current, and cached.
-// The cache belongs to the device's current context: ps_finalize clears it, so that after a
-// context is torn down (ps_finalize, then cudaDeviceReset) the next call looks the address up again.
+// ps_stokes2d_iterate_static: the PT iteration for callers that cannot let a library allocate device
+// memory: an application whose device memory is fully owned by its own pool allocator (CUDA.jl's memory
+// pool, a framework caching allocator), where a cudaMalloc behind its back fails or fragments the pool,
+// and code that must not call cudaFree, which synchronises the whole device. The iteration works in
+// place, so neither entry point allocates; this one keeps the bound on the grid that its callers know.
 // =======================================================================================
 namespace ps {
 
 constexpr size_t kStaticScratchBytes = size_t(16) << 20;
-static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
-
-static constexpr int kStaticMaxDevices = 64;
-static void* g_static_scratch_addr[kStaticMaxDevices] = {};
-static std::mutex g_static_mutex;
-
-// Device address of g_static_scratch on the current device (looked up once per device).
-static int static_scratch(void** out) {
-    int dev = -1;
-    PS_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kStaticMaxDevices) return fail(PS_ERR_ARG, "device %d out of range", dev);
-    std::lock_guard<std::mutex> lock(g_static_mutex);
-    if (!g_static_scratch_addr[dev]) {
-        void* p = nullptr;
-        cudaError_t e = cudaGetSymbolAddress(&p, g_static_scratch);
-        if (e != cudaSuccess || !p) return cuda_fail(e, "cudaGetSymbolAddress(static scratch)");
-        g_static_scratch_addr[dev] = p;
-    }
-    *out = g_static_scratch_addr[dev];
-    return PS_OK;
-}
-
-void stokes2d_static_forget() {
-    std::lock_guard<std::mutex> lock(g_static_mutex);
-    for (int d = 0; d < kStaticMaxDevices; d++) g_static_scratch_addr[d] = nullptr;
-}
 
 static size_t round256(size_t b) { return (b + 255) / 256 * 256; }
 
-static int iterate_static(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp, int64_t n_iter, cudaStream_t s) {
+static int check_static_bound(const ps_stokes2d_fields* f) {
     const int64_t nx = f->Pt.n[0], ny = f->Pt.n[1];
-    const size_t es = elsize(f->Pt.dtype), bx = (nx + 1) * ny * es, by = nx * (ny + 1) * es, bp = nx * ny * es;
-    const size_t need = round256(bx) + round256(by) + round256(bp);
+    const size_t es = elsize(f->Pt.dtype);
+    const size_t need = round256((nx + 1) * ny * es) + round256(nx * (ny + 1) * es) + round256(nx * ny * es);
     if (need > kStaticScratchBytes)
         return fail(PS_ERR_SHAPE,
-                    "ps_stokes2d_iterate_static: a %lld x %lld grid needs %zu bytes of scratch; the static buffer "
-                    "holds %zu bytes (use ps_stokes2d_iterate)",
+                    "ps_stokes2d_iterate_static: the state of a %lld x %lld grid is %zu bytes; the static buffer "
+                    "bound is %zu bytes (use ps_stokes2d_iterate)",
                     (long long)nx, (long long)ny, need, kStaticScratchBytes);
-    if (f->Pt.dtype == PS_F64) {  // in place: the limit above is the entry point's, not the kernels'
-        s2_iterate64(f, pp, n_iter, s);
-        return PS_OK;
-    }
-    void* base = nullptr;
-    PS_TRY(static_scratch(&base));
-    char* c = static_cast<char*>(base);
-    // every element of the buffers in use is written before it is read within a call, so the
-    // contents left by the previous call never matter
-    float* const B[3] = {reinterpret_cast<float*>(c), reinterpret_cast<float*>(c + round256(bx)),
-                         reinterpret_cast<float*>(c + round256(bx) + round256(by))};
-    s2_iterate32(f, pp, n_iter, B, s);
     return PS_OK;
 }
 
@@ -1324,6 +1075,8 @@ extern "C" int ps_stokes2d_iterate_static(const ps_stokes2d_fields* f, const ps_
     if (!p) return fail(PS_ERR_NULL, "NULL params");
     if (n_iter < 0) return fail(PS_ERR_ARG, "n_iter must be >= 0");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    PS_TRY(iterate_static(f, p, n_iter, s));
+    PS_TRY(check_static_bound(f));
+    if (f->Pt.dtype == PS_F64) s2_iterate<double>(f, p, n_iter, s);
+    else s2_iterate<float>(f, p, n_iter, s);
     return finish_launch(s, 1, "ps_stokes2d_iterate_static");
 }

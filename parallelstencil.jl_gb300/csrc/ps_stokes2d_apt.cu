@@ -168,38 +168,75 @@ __device__ __forceinline__ void apt_block_add(double v0, double* out0, double v1
 
 #define A2I(a, i, j, n0) (a)[(i) + (n0) * (j)]  // index arithmetic in the index type I
 
+// A thread issues every load before its first store: the arrays' pointers may alias as far as the compiler
+// knows, so a load written after a store waits for it (FP32 1023^2: 15.7 -> 13.1 us per iteration, 8.3 TB/s
+// on the two kernels' 26 words per cell, from L2 mostly). Measured and not kept: two to four rows per
+// thread (13.2-14.2 us), blocks of 128 threads (18.9: twice the blocks to launch) or 512 (16.3 and more).
+
+// Rows of 32 threads per block. FP32: 8; FP64, bound by the FP64 pipe: 4, which spreads a small grid more
+// evenly over the SMs (8 rows -> 4: 255^2 11.6 -> 10.6 us per iteration, 130^2 8.7 -> 7.9, 1023^2 100.5 both).
+template <typename T>
+__host__ __device__ constexpr int apt_block_rows() {
+    return sizeof(T) == 4 ? 8 : 4;
+}
+
 // compute_P_τ!: cells (∇V, Pt, τxx, τyy) and corners (τxy). DEFECT: the correction's sweep
 // (pressure driven by ∇δV + ∇V of the outer state). STORE: write ∇V (and add Σ|∇V| to red).
 // I: index type (int where every array has fewer than 2^31 elements).
 template <typename T, bool DEFECT, bool STORE, typename I>
-__global__ void __launch_bounds__(256) apt_cells_k(AptArrays<T> a) {
+__global__ void __launch_bounds__(32 * apt_block_rows<T>()) apt_cells_k(AptArrays<T> a) {
+    const I ix = (I)blockIdx.x * 32 + (I)threadIdx.x, iy = (I)blockIdx.y * apt_block_rows<T>() + (I)threadIdx.y;
+    const I nx = (I)a.nx, ny = (I)a.ny, c = ix + nx * iy;
+    // the coefficients, which no iteration writes, while the kernel before this one still runs
+    T kP = (T)0, aT = (T)0, bT = (T)0, aTc = (T)0, bTc = (T)0;
+    [[maybe_unused]] T src = (T)0;
+    if (ix < nx && iy < ny) {
+        kP = __ldg(a.kP + c);
+        aT = __ldg(a.aT + c);
+        bT = __ldg(a.bT + c);
+        if constexpr (DEFECT) src = __ldg(a.div0 + c);
+    }
+    if (ix < nx - 1 && iy < ny - 1) {
+        aTc = __ldg(a.aTc + (c - iy));
+        bTc = __ldg(a.bTc + (c - iy));
+    }
     grid_dependency_wait();  // V of the previous iteration's faces kernel
     grid_dependents_may_launch();
-    const I ix = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x, iy = (I)blockIdx.y * (I)blockDim.y + (I)threadIdx.y;
-    const I nx = (I)a.nx, ny = (I)a.ny;
+    T vx0, vx1, vy0, vy1, pt, txx, tyy, vxu, vyr, txy;
+    vx0 = vx1 = vy0 = vy1 = pt = txx = tyy = vxu = vyr = txy = (T)0;
+    if (ix < nx && iy < ny) {
+        vx0 = a.Vx[c + iy];
+        vx1 = a.Vx[c + iy + 1];
+        vy0 = a.Vy[c];
+        vy1 = a.Vy[c + nx];
+        pt = a.Pt[c];
+        txx = a.txx[c];
+        tyy = a.tyy[c];
+    }
+    if (ix < nx - 1 && iy < ny - 1) {
+        vxu = a.Vx[c + iy + 1 + (nx + 1)];
+        vyr = a.Vy[c + nx + 1];
+        txy = a.txy[c - iy];
+    }
     const T third = (T)(1.0 / 3.0), h = (T)0.5;
     double sabs = 0.0;
     if (ix < nx && iy < ny) {
-        const I c = ix + nx * iy;
-        const T dvx = A2I(a.Vx, ix + 1, iy, nx + 1) - A2I(a.Vx, ix, iy, nx + 1);
-        const T dvy = A2I(a.Vy, ix, iy + 1, nx) - A2I(a.Vy, ix, iy, nx);
-        const T d = dvx * a._dx + dvy * a._dy;
+        const T ex = (vx1 - vx0) * a._dx, ey = (vy1 - vy0) * a._dy;
+        const T d = ex + ey;
         const T td = d * third;
         T dp = d;
-        if constexpr (DEFECT) dp = d + a.div0[c];
-        a.Pt[c] = a.Pt[c] - a.kP[c] * dp;
-        a.txx[c] = a.aT[c] * a.txx[c] + a.bT[c] * (dvx * a._dx - td);
-        a.tyy[c] = a.aT[c] * a.tyy[c] + a.bT[c] * (dvy * a._dy - td);
+        if constexpr (DEFECT) dp = d + src;
+        a.Pt[c] = pt - kP * dp;
+        a.txx[c] = aT * txx + bT * (ex - td);
+        a.tyy[c] = aT * tyy + bT * (ey - td);
         if constexpr (STORE) {
             a.divV[c] = dp;
             sabs = fabs((double)dp);
         }
-        if (ix < nx - 1 && iy < ny - 1) {
-            const I k = ix + (nx - 1) * iy;
-            const T e = h * ((A2I(a.Vx, ix + 1, iy + 1, nx + 1) - A2I(a.Vx, ix + 1, iy, nx + 1)) * a._dy +
-                             (A2I(a.Vy, ix + 1, iy + 1, nx) - A2I(a.Vy, ix, iy + 1, nx)) * a._dx);
-            a.txy[k] = a.aTc[k] * a.txy[k] + a.bTc[k] * e;
-        }
+    }
+    if (ix < nx - 1 && iy < ny - 1) {
+        const T e = h * ((vxu - vx1) * a._dy + (vyr - vy1) * a._dx);
+        a.txy[c - iy] = aTc * txy + bTc * e;
     }
     if constexpr (STORE) {
         if (a.red) apt_block_add(sabs, a.red + 2);
@@ -210,48 +247,72 @@ __global__ void __launch_bounds__(256) apt_cells_k(AptArrays<T> a) {
 // bc_x!(Vy). DEFECT adds the outer state's FP64 residual as source. STORE: write Rx, Ry (and add
 // Σ|Rx|, Σ|Ry| to red).
 template <typename T, bool DEFECT, bool STORE, bool UPDATE, typename I>
-__global__ void __launch_bounds__(256) apt_faces_k(AptArrays<T> a) {
+__global__ void __launch_bounds__(32 * apt_block_rows<T>()) apt_faces_k(AptArrays<T> a) {
+    const I ix = (I)blockIdx.x * 32 + (I)threadIdx.x, iy = (I)blockIdx.y * apt_block_rows<T>() + (I)threadIdx.y;
+    const I nx = (I)a.nx, ny = (I)a.ny, c = ix + nx * iy;
+    const T h = (T)0.5;
+    // the steps and sources, which no iteration writes, while the kernel before this one still runs
+    const bool fx = ix < nx - 1 && iy < ny - 2, fy = ix < nx - 2 && iy < ny - 1;
+    [[maybe_unused]] T dtx = (T)0, dty = (T)0, srcx = (T)0, srcy = (T)0;
+    if (fx) {
+        if constexpr (UPDATE) dtx = __ldg(a.dtVx + (c - iy));
+        if constexpr (DEFECT) srcx = __ldg(a.rx0 + (c - iy));
+    }
+    if (fy) {
+        if constexpr (UPDATE) dty = __ldg(a.dtVy + (c - 2 * iy));
+        if constexpr (DEFECT) srcy = __ldg(a.ry0 + (c - 2 * iy));
+        else srcy = (__ldg(a.Rog + c + 1) + __ldg(a.Rog + c + 1 + nx)) * h;
+    }
     grid_dependency_wait();  // τ and Pt of the cells kernel
     grid_dependents_may_launch();
-    const I ix = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x, iy = (I)blockIdx.y * (I)blockDim.y + (I)threadIdx.y;
-    const I nx = (I)a.nx, ny = (I)a.ny;
-    const T h = (T)0.5;
+    // around the Vx face (ix + 1, iy + 1) and the Vy face (ix + 1, iy + 1)
+    T xr, xl, yu, yd, s00, s01, s10, p01, p11, p10, vx, vy;
+    xr = xl = yu = yd = s00 = s01 = s10 = p01 = p11 = p10 = vx = vy = (T)0;
+    if (fx || fy) {
+        s00 = a.txy[c - iy];
+        p11 = a.Pt[c + nx + 1];
+    }
+    if (fx) {
+        xr = a.txx[c + nx + 1];
+        xl = a.txx[c + nx];
+        s01 = a.txy[c - iy + (nx - 1)];
+        p01 = a.Pt[c + nx];
+        if constexpr (UPDATE) vx = a.Vx[c + iy + nx + 2];
+    }
+    if (fy) {
+        yu = a.tyy[c + nx + 1];
+        yd = a.tyy[c + 1];
+        s10 = a.txy[c - iy + 1];
+        p10 = a.Pt[c + 1];
+        if constexpr (UPDATE) vy = a.Vy[c + nx + 1];
+    }
     double sx = 0.0, sy = 0.0;
-    if (ix < nx - 1 && iy < ny - 2) {
-        const I k = ix + (nx - 1) * iy;
-        T R = ((A2I(a.txx, ix + 1, iy + 1, nx) - A2I(a.txx, ix, iy + 1, nx)) * a._dx +
-               (A2I(a.txy, ix, iy + 1, nx - 1) - A2I(a.txy, ix, iy, nx - 1)) * a._dy) -
-              (A2I(a.Pt, ix + 1, iy + 1, nx) - A2I(a.Pt, ix, iy + 1, nx)) * a._dx;
-        if constexpr (DEFECT) R = R + a.rx0[k];
+    if (fx) {
+        T res = ((xr - xl) * a._dx + (s01 - s00) * a._dy) - (p11 - p01) * a._dx;
+        if constexpr (DEFECT) res = res + srcx;
         if constexpr (STORE) {
-            a.Rx[k] = R;
-            sx = fabs((double)R);
+            a.Rx[c - iy] = res;
+            sx = fabs((double)res);
         }
         if constexpr (UPDATE) {
-            const T v = A2I(a.Vx, ix + 1, iy + 1, nx + 1) + a.dtVx[k] * R;
-            A2I(a.Vx, ix + 1, iy + 1, nx + 1) = v;
-            if (iy == 0) A2I(a.Vx, ix + 1, 0, nx + 1) = v;
-            if (iy == ny - 3) A2I(a.Vx, ix + 1, ny - 1, nx + 1) = v;
+            const T v = vx + dtx * res;
+            a.Vx[c + iy + nx + 2] = v;
+            if (iy == 0) a.Vx[ix + 1] = v;
+            if (iy == ny - 3) a.Vx[c + iy + 2 * nx + 3] = v;
         }
     }
-    if (ix < nx - 2 && iy < ny - 1) {
-        const I k = ix + (nx - 2) * iy;
-        T R = (((A2I(a.tyy, ix + 1, iy + 1, nx) - A2I(a.tyy, ix + 1, iy, nx)) * a._dy +
-                (A2I(a.txy, ix + 1, iy, nx - 1) - A2I(a.txy, ix, iy, nx - 1)) * a._dx) -
-               (A2I(a.Pt, ix + 1, iy + 1, nx) - A2I(a.Pt, ix + 1, iy, nx)) * a._dy);
-        if constexpr (DEFECT)
-            R = R + a.ry0[k];
-        else
-            R = R + (A2I(a.Rog, ix + 1, iy, nx) + A2I(a.Rog, ix + 1, iy + 1, nx)) * h;
+    if (fy) {
+        T res = ((yu - yd) * a._dy + (s10 - s00) * a._dx) - (p11 - p10) * a._dy;
+        res = res + srcy;  // the outer state's residual, or the buoyancy average of the two cells
         if constexpr (STORE) {
-            a.Ry[k] = R;
-            sy = fabs((double)R);
+            a.Ry[c - 2 * iy] = res;
+            sy = fabs((double)res);
         }
         if constexpr (UPDATE) {
-            const T v = A2I(a.Vy, ix + 1, iy + 1, nx) + a.dtVy[k] * R;
-            A2I(a.Vy, ix + 1, iy + 1, nx) = v;
-            if (ix == 0) A2I(a.Vy, 0, iy + 1, nx) = v;
-            if (ix == nx - 3) A2I(a.Vy, nx - 1, iy + 1, nx) = v;
+            const T v = vy + dty * res;
+            a.Vy[c + nx + 1] = v;
+            if (ix == 0) a.Vy[c + nx] = v;
+            if (ix == nx - 3) a.Vy[c + nx + 2] = v;
         }
     }
     if constexpr (UPDATE) {
@@ -391,7 +452,7 @@ static bool apt_i32(int64_t nx, int64_t ny) {  // 32-bit indices: every array an
 
 template <typename T, bool DEFECT, bool STORE, typename I>
 static void apt_launch_iteration_i(const AptArrays<T>& a, cudaStream_t s, bool after_kernel) {
-    const dim3 blk(32, 8);
+    const dim3 blk(32, apt_block_rows<T>());
     const dim3 grd = apt_grid(a.nx, a.ny, blk);
     // each kernel may start while the kernel before it ends (programmatic dependent launch; it waits
     // for that kernel's stores before reading); after_kernel = false: the stream's last operation
@@ -438,10 +499,11 @@ static void apt_residual64(AptArrays<double> a, const double* Mus, double* const
     const dim3 grd = apt_grid(a.nx, a.ny, blk);
     cudaMemsetAsync(red, 0, 3 * sizeof(double), s);
     apt_res_cells_k<<<grd, blk, 0, s>>>(a, Mus);
+    const dim3 fblk(32, apt_block_rows<double>()), fgrd = apt_grid(a.nx, a.ny, fblk);
     if (apt_i32(a.nx, a.ny))
-        apt_faces_k<double, false, true, false, int><<<grd, blk, 0, s>>>(a);
+        apt_faces_k<double, false, true, false, int><<<fgrd, fblk, 0, s>>>(a);
     else
-        apt_faces_k<double, false, true, false, int64_t><<<grd, blk, 0, s>>>(a);
+        apt_faces_k<double, false, true, false, int64_t><<<fgrd, fblk, 0, s>>>(a);
 }
 
 static double apt_err(const double h[3], int64_t nx, int64_t ny) {
@@ -691,12 +753,13 @@ int ps_stokes2d_apt_iterate(const ps_stokes2d_apt_fields* f, const ps_stokes2d_a
     PS_TRY(check_apt_params(p));
     if (n_iter < 0) return fail(PS_ERR_ARG, "n_iter must be >= 0");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    for (int64_t it = 0; it < n_iter; ++it) {
-        if (f->Pt.dtype == PS_F64)
-            apt_launch_iteration<double, false, true>(apt_arrays<double>(f, p), s, it > 0);
-        else
-            apt_launch_iteration<float, false, true>(apt_arrays<float>(f, p), s, it > 0);
-    }
+    auto iterate = [&](auto a) {  // ∇V, Rx and Ry, which nothing reads between iterations, from the last
+        using T = std::remove_const_t<std::remove_pointer_t<decltype(a.kP)>>;
+        for (int64_t it = 0; it + 1 < n_iter; ++it) apt_launch_iteration<T, false, false>(a, s, it > 0);
+        if (n_iter > 0) apt_launch_iteration<T, false, true>(a, s, n_iter > 1);
+    };
+    if (f->Pt.dtype == PS_F64) iterate(apt_arrays<double>(f, p));
+    else iterate(apt_arrays<float>(f, p));
     return finish_launch(s, 1, "ps_stokes2d_apt_iterate");
 }
 

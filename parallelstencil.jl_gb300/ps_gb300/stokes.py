@@ -4,7 +4,7 @@
 and exposes
   - the six `@parallel` kernels one-to-one (``compute_timesteps``, ``compute_P``, ``compute_tau``,
     ``compute_dV``, ``compute_V``, ``bc_x``/``bc_y``),
-  - ``iterate(n)``: n iterations of the loop body with one fused kernel per iteration,
+  - ``iterate(n)``: n iterations of the loop body with two kernels per iteration,
   - ``err()``: max(mean|Rx|, mean|Ry|, mean|∇V|) (Stokes2D.jl:119-120),
   - ``solve(tol, mode)``: the `while err > ε` loop in FP64 (mode 0) or with FP32 PT sweeps on the
     defect-correction update and an FP64 residual / update / convergence check (mode 1).
