@@ -90,6 +90,9 @@ bool tma_eligible(const ps_array& a);
 // columns (one 128-byte swizzle row). Reads past the matrix are zero-filled.
 int encode_bf16_rows_sw128(CUtensorMap* map, const void* ptr, uint64_t cols, uint64_t rows, uint32_t box_cols,
                            uint32_t box_rows);
+// Dense bf16 array of `rank` (2..4) dimensions, dims[0] fastest; the box's first extent is one swizzle row of
+// 64 bytes (32 elements) or 128 bytes (64). Reads outside the array are zero-filled.
+int encode_bf16_box(CUtensorMap* map, const void* ptr, int rank, const uint64_t* dims, const uint32_t* box);
 
 // z-sweep length for loopsize = 0: a launch of cta_xy CTAs per z-block over wz planes with
 // `slots` CTAs resident at once (occupancy x SMs) loses the idle part of its last wave and

@@ -251,6 +251,26 @@ int encode_bf16_rows_sw128(CUtensorMap* map, const void* ptr, uint64_t cols, uin
     return PS_OK;
 }
 
+int encode_bf16_box(CUtensorMap* map, const void* ptr, int rank, const uint64_t* dims, const uint32_t* box) {
+    if (!g_encode) return fail(PS_ERR_NOT_INIT, "TMA encoder unavailable (ps_init not called)");
+    if (rank < 2 || rank > 4 || (box[0] != 32 && box[0] != 64)) return fail(PS_ERR_ARG, "invalid bf16 TMA box");
+    if ((reinterpret_cast<uintptr_t>(ptr) & 15) || (dims[0] * 2) % 16) return fail(PS_ERR_ALIGN, "bf16 array not TMA-eligible");
+    cuuint64_t d[4], st[3], stride = 2;
+    cuuint32_t bx[4], es[4] = {1, 1, 1, 1};
+    for (int i = 0; i < rank; i++) {
+        if (dims[i] == 0 || box[i] == 0 || box[i] > 256) return fail(PS_ERR_ARG, "invalid bf16 TMA box");
+        d[i] = dims[i];
+        bx[i] = box[i];
+        stride *= dims[i];
+        if (i + 1 < rank) st[i] = stride;
+    }
+    CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(ptr), d, st, bx, es,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, box[0] == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(PS_ERR_CUDA, "cuTensorMapEncodeTiled (bf16) failed (CUresult %d)", (int)r);
+    return PS_OK;
+}
+
 // ps_check_division: div_c against the IEEE division. Dividend i: FP32 -- significand i mod 2^23,
 // exponent and sign from i / 2^23 (every significand in each listed binade, both signs); FP64 --
 // a hashed 52-bit significand, exponent and sign from the hash too. The first 64 indices are

@@ -1,12 +1,12 @@
 // ps_nn_net.cu -- the learned warm start's network: a 4-level conv encoder-decoder (U-Net) in bf16
 // with FP32 accumulation, trained and run entirely by this library's kernels.
 //
-// Layout: activations NHWC (channels contiguous), bf16. A 3x3 convolution ("same" padding) is
-//   col  = im2col(x)                  [P][kpad]  (P = B*H*W, kpad = round_up(9*cin, 8), zero tail)
-//   y    = relu(col * W^T + b)        tcgen05 GEMM, bias/ReLU/bf16 fused in the epilogue
+// Layout: activations NHWC (channels contiguous), bf16. A 3x3 convolution ("same" padding) is an implicit
+// GEMM on the tensor cores (ps_nn_conv.cu; bias, ReLU and bf16 in its epilogue); the two-channel first layer
+// and the 1x1 last one, too short in K or N for them, are one pixel per thread
 // and its backward pass
 //   dz   = dy * (y > 0)  (bf16; the bias gradient is summed in FP32 in the same kernel)
-//   dW  += dz^T * col    (GEMM over K = P, split-K with FP32 atomics; col built transposed)
+//   dW  += dz^T * col    (GEMM over K = P, split-K with FP32 atomics; the column matrix built transposed)
 //   dcol = dz * W        (GEMM, B operand = W^T); dx = col2im(dcol) (gather, no atomics).
 // Network (base 32 channels, input 2: log10 viscosity and rho*g; output 3: P, Vx, Vy at cells):
 //   enc: [conv3 c->c, conv3 c->c] at 1, 1/4, 1/16, 1/64 resolution (c = 32, 64, 128, 256; 4x4 average
@@ -35,20 +35,12 @@ typedef __nv_bfloat16 bf16;
 static inline unsigned nblk(int64_t n, int t = 256) { return (unsigned)std::min<int64_t>((n + t - 1) / t, 1 << 20); }
 #define GSTRIDE(i, n) for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
-// col[p][k] of a 3x3 "same" convolution over x [B][H][W][C], or (ldp > 0) colT[k][p] with row stride
-// ldp >= P and zero columns P..ldp
+// colT[k][p] of a 3x3 "same" convolution over x [B][H][W][C], row stride ldp >= P, zero columns P..ldp
 __global__ void nn_im2col3_k(const bf16* __restrict__ x, int64_t P, int H, int W, int C, int kpad, bf16* col,
                              int64_t ldp) {
-    const int64_t n = (ldp > 0 ? ldp : P) * kpad;
+    const int64_t n = ldp * kpad;
     GSTRIDE(i, n) {
-        int64_t p, k;
-        if (ldp > 0) {
-            k = i / ldp;
-            p = i - k * ldp;
-        } else {
-            p = i / kpad;
-            k = i - p * kpad;
-        }
+        const int64_t k = i / ldp, p = i - k * ldp;
         const int tap = (int)(k / C), c = (int)(k - (int64_t)tap * C);
         bf16 v = __float2bfloat16(0.0f);
         if (tap < 9 && p < P) {
@@ -122,21 +114,35 @@ __global__ void nn_transpose_k(const bf16* __restrict__ in, int64_t R, int C, in
     }
 }
 
-// f x f average pooling of x [B][H][W][C] -> [B][H/f][W/f][C] (FP32 sum row by row, bf16 result)
+// f x f average pooling of x [B][H][W][C] -> [B][H/f][W/f][C] (FP32 sum row by row, bf16 result); a thread
+// takes 8 channels (16 bytes), C % 8 == 0
 __global__ void nn_pool_k(const bf16* __restrict__ x, int64_t B, int H, int W, int C, int f, bf16* y) {
-    const int h = H / f, w = W / f;
-    const int64_t n = B * h * w * C;
+    const int h = H / f, w = W / f, C8 = C / 8;
+    const int64_t n = B * h * w * C8;
     const float inv = 1.0f / (float)(f * f);
     GSTRIDE(i, n) {
-        const int c = (int)(i % C);
-        const int64_t q = i / C;
+        const int c = (int)(i % C8);
+        const int64_t q = i / C8;
         const int xx = (int)(q % w), yy = (int)((q / w) % h);
         const int64_t b = q / ((int64_t)w * h);
-        const bf16* s = x + ((b * H + (int64_t)f * yy) * W + (int64_t)f * xx) * C + c;
-        float v = 0.0f;
+        const uint4* s = reinterpret_cast<const uint4*>(x + ((b * H + (int64_t)f * yy) * W + (int64_t)f * xx) * C) + c;
+        float v[8] = {};
         for (int r = 0; r < f; r++)
-            for (int k = 0; k < f; k++) v += __bfloat162float(s[((int64_t)r * W + k) * C]);
-        y[i] = __float2bfloat16_rn(v * inv);
+            for (int k = 0; k < f; k++) {
+                const uint4 u = __ldg(s + ((int64_t)r * W + k) * C8);
+                const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const float2 t = __bfloat1622float2(h2[e]);
+                    v[2 * e] += t.x;
+                    v[2 * e + 1] += t.y;
+                }
+            }
+        uint4 o;
+        __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+        for (int e = 0; e < 4; e++) oh[e] = __floats2bfloat162_rn(v[2 * e] * inv, v[2 * e + 1] * inv);
+        reinterpret_cast<uint4*>(y)[i] = o;
     }
 }
 // dx [B][H][W][C] (+)= dy [B][H/f][W/f][C] / f^2 broadcast
@@ -154,16 +160,92 @@ __global__ void nn_pool_bwd_k(const float* __restrict__ dy, int64_t B, int H, in
         dx[i] = accumulate ? dx[i] + v : v;
     }
 }
-// y[b][Y][X][coff + c] = x[b][Y/f][X/f][c]   (x: [B][H/f][W/f][C], y row stride ldy)
-__global__ void nn_up_k(const bf16* __restrict__ x, int64_t B, int H, int W, int C, int f, bf16* y, int ldy, int coff) {
-    const int h = H / f, w = W / f;
-    const int64_t n = B * H * W * C;
+// k[b][Y][X] = the Cl channels of low[b][Y/f][X/f], then the Cs channels of skip[b][Y][X] (16 bytes per thread;
+// Cl, Cs % 8 == 0)
+__global__ void nn_upcat_k(const bf16* __restrict__ low, int Cl, const bf16* __restrict__ skip, int Cs, int64_t B, int H,
+                           int W, int f, bf16* k) {
+    const int h = H / f, w = W / f, Cl8 = Cl / 8, Cs8 = Cs / 8, C8 = Cl8 + Cs8;
+    const int64_t n = B * H * W * C8;
     GSTRIDE(i, n) {
-        const int c = (int)(i % C);
-        const int64_t q = i / C;
-        const int xx = (int)(q % W), yy = (int)((q / W) % H);
-        const int64_t b = q / ((int64_t)W * H);
-        y[q * ldy + coff + c] = x[((b * h + yy / f) * w + xx / f) * C + c];
+        const int c = (int)(i % C8);
+        const int64_t q = i / C8;
+        uint4 v;
+        if (c < Cl8) {
+            const int xx = (int)(q % W), yy = (int)((q / W) % H);
+            const int64_t b = q / ((int64_t)W * H);
+            v = __ldg(reinterpret_cast<const uint4*>(low) + ((b * h + yy / f) * w + xx / f) * Cl8 + c);
+        } else {
+            v = __ldg(reinterpret_cast<const uint4*>(skip) + q * Cs8 + (c - Cl8));
+        }
+        reinterpret_cast<uint4*>(k)[i] = v;
+    }
+}
+// The first layer: y[p][0..31] = relu(3x3 conv of the two input channels + bias), one pixel per thread
+// (K = 18 is too short for the tensor cores; bound by its 64-byte result per pixel and 576 FMAs)
+__global__ void __launch_bounds__(256, 3) nn_conv_first_k(const bf16* __restrict__ x, const bf16* __restrict__ wgt, int kpad,
+                                                       const float* __restrict__ bias, int64_t B, int H, int W, bf16* y) {
+    __shared__ float4 sw[18][8];  // [tap, channel][output / 4]
+    __shared__ float sb[32];
+    for (int i = threadIdx.x; i < 18 * 32; i += blockDim.x)
+        reinterpret_cast<float*>(sw[i / 32])[i % 32] = __bfloat162float(wgt[(int64_t)(i % 32) * kpad + i / 32]);
+    for (int i = threadIdx.x; i < 32; i += blockDim.x) sb[i] = bias[i];
+    __syncthreads();
+    const int64_t P = B * H * W;
+    GSTRIDE(p, P) {
+        const int xx = (int)(p % W), yy = (int)((p / W) % H);
+        float acc[32];
+#pragma unroll
+        for (int o = 0; o < 32; o++) acc[o] = 0.0f;
+#pragma unroll 1
+        for (int tap = 0; tap < 9; tap++) {
+            const int sy = yy + tap / 3 - 1, sx = xx + tap % 3 - 1;
+            float2 v = make_float2(0.0f, 0.0f);
+            if (sy >= 0 && sy < H && sx >= 0 && sx < W)
+                v = __bfloat1622float2(
+                    reinterpret_cast<const __nv_bfloat162*>(x)[p + (int64_t)(tap / 3 - 1) * W + (tap % 3 - 1)]);
+#pragma unroll
+            for (int o = 0; o < 8; o++) {
+                const float4 a = sw[2 * tap][o], b = sw[2 * tap + 1][o];
+                acc[4 * o] = fmaf(v.y, b.x, fmaf(v.x, a.x, acc[4 * o]));
+                acc[4 * o + 1] = fmaf(v.y, b.y, fmaf(v.x, a.y, acc[4 * o + 1]));
+                acc[4 * o + 2] = fmaf(v.y, b.z, fmaf(v.x, a.z, acc[4 * o + 2]));
+                acc[4 * o + 3] = fmaf(v.y, b.w, fmaf(v.x, a.w, acc[4 * o + 3]));
+            }
+        }
+        uint4 w4[4];
+        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(w4);
+#pragma unroll
+        for (int o = 0; o < 16; o++)
+            h[o] = __floats2bfloat162_rn(fmaxf(acc[2 * o] + sb[2 * o], 0.0f), fmaxf(acc[2 * o + 1] + sb[2 * o + 1], 0.0f));
+#pragma unroll
+        for (int o = 0; o < 4; o++) reinterpret_cast<uint4*>(y + p * 32)[o] = w4[o];
+    }
+}
+// The last layer: y[p][0..2] = W x[p] + bias over 32 channels (FP32 result), one pixel per thread
+__global__ void __launch_bounds__(256) nn_conv_last_k(const bf16* __restrict__ x, const bf16* __restrict__ wgt, int kpad,
+                                                      const float* __restrict__ bias, int64_t P, float* __restrict__ y) {
+    __shared__ float sw[3][32];
+    for (int i = threadIdx.x; i < 96; i += blockDim.x) sw[i / 32][i % 32] = __bfloat162float(wgt[(int64_t)(i / 32) * kpad + i % 32]);
+    __syncthreads();
+    const float b0 = bias[0], b1 = bias[1], b2 = bias[2];
+    GSTRIDE(p, P) {
+        float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint4 u = __ldg(reinterpret_cast<const uint4*>(x + p * 32) + q);
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const float2 t = __bfloat1622float2(h[e]);
+                const int c = 8 * q + 2 * e;
+                a0 = fmaf(t.y, sw[0][c + 1], fmaf(t.x, sw[0][c], a0));
+                a1 = fmaf(t.y, sw[1][c + 1], fmaf(t.x, sw[1][c], a1));
+                a2 = fmaf(t.y, sw[2][c + 1], fmaf(t.x, sw[2][c], a2));
+            }
+        }
+        y[3 * p] = a0 + b0;
+        y[3 * p + 1] = a1 + b1;
+        y[3 * p + 2] = a2 + b2;
     }
 }
 // dx[b][y][x][c] = sum over the f x f children of dk[.][coff + c] (dk row stride ldk)
@@ -183,9 +265,8 @@ __global__ void nn_up_bwd_k(const float* __restrict__ dk, int ldk, int coff, int
         dx[i] = v;
     }
 }
-// dst[p][doff + c] = src[p][soff + c] (bf16 or FP32 copies of channel ranges)
-template <typename T>
-__global__ void nn_copy_ch_k(const T* __restrict__ src, int lds, int soff, int64_t P, int C, T* dst, int ldd, int doff) {
+// dst[p][doff + c] = src[p][soff + c] (copies of channel ranges)
+__global__ void nn_copy_ch_k(const float* __restrict__ src, int lds, int soff, int64_t P, int C, float* dst, int ldd, int doff) {
     const int64_t n = P * C;
     GSTRIDE(i, n) {
         const int64_t p = i / C;
@@ -325,7 +406,7 @@ struct NNet {
     bf16 *x0, *a[15], *p1, *p2, *p3, *k2, *k1, *k0;
     float *y, *ga[15], *gp1, *gp2, *gp3, *gk2, *gk1, *gk0;
     // scratch
-    bf16 *col, *colT, *dz, *dzT;
+    bf16 *colT, *dz, *dzT;
     float* dcol;
     double* loss;
     float* dsc;  // device copy of scales
@@ -450,7 +531,6 @@ static int nn_create(NNet* n, int H, int W, int Bmax, uint64_t seed) {
         colmax = std::max(colmax, Pk * n->conv[i].kpad);
         dzmax = std::max(dzmax, Pk * (int64_t)n->conv[i].ldt);
     }
-    PS_TRY(nn_alloc_t(n, &n->col, colmax));
     PS_TRY(nn_alloc_t(n, &n->colT, colmax));
     PS_TRY(nn_alloc_t(n, &n->dcol, colmax));
     PS_TRY(nn_alloc_t(n, &n->dz, dzmax));
@@ -466,23 +546,15 @@ static int nn_create(NNet* n, int H, int W, int Bmax, uint64_t seed) {
 
 // y = act(conv(x)); x [P][cin] bf16 at resolution (h, w); y bf16 [P][cout] (or FP32 for the last layer)
 static int nn_conv_fwd(NNet* n, Conv& L, const bf16* x, int B, int h, int w, void* y, cudaStream_t s, int* err) {
+    (void)n;
     const int64_t P = (int64_t)B * h * w;
-    GemmEpilogue e{};
-    e.M = P;
-    e.N = L.cout;
-    e.ldc = L.cout;
-    e.alpha = 1.0f;
-    e.bias = L.b;
-    e.relu = L.relu;
-    e.out_bf16 = L.relu;  // hidden layers bf16, output layer FP32
-    e.outh = static_cast<bf16*>(y);
-    e.outf = static_cast<float*>(y);
-    const bf16* A = x;
-    if (L.k == 3) {
-        nn_im2col3_k<<<nblk(P * L.kpad), 256, 0, s>>>(x, P, h, w, L.cin, (int)L.kpad, n->col, 0);
-        A = n->col;
-    }
-    return nn_gemm(A, P, L.W, L.cout, L.kpad, e, 1, s, err);
+    if (L.k == 3 && L.cin % 32 == 0)
+        return nn_conv3_tc(x, B, h, w, L.cin, L.W, L.cout, L.b, L.relu, y, s, err);
+    if (L.k == 3)
+        nn_conv_first_k<<<nblk(P), 256, 0, s>>>(x, L.W, (int)L.kpad, L.b, B, h, w, static_cast<bf16*>(y));
+    else
+        nn_conv_last_k<<<nblk(P), 256, 0, s>>>(x, L.W, (int)L.kpad, L.b, P, static_cast<float*>(y));
+    return PS_OK;
 }
 
 // Backward of one layer: dy (FP32 [P][cout] with row stride ldy) -> gW, gb (accumulated) and,
@@ -539,13 +611,13 @@ static int nn_forward(NNet* n, int B, cudaStream_t s, int* err) {
         return nn_conv_fwd(n, L[i], x, B, nn_level_H(n, lev), nn_level_W(n, lev), y, s, err);
     };
     auto pool = [&](const bf16* x, int lev, int C, bf16* y) {
-        nn_pool_k<<<nblk(nn_level_P(n, B, lev + 1) * C), 256, 0, s>>>(x, B, nn_level_H(n, lev), nn_level_W(n, lev), C,
+        nn_pool_k<<<nblk(nn_level_P(n, B, lev + 1) * C / 8), 256, 0, s>>>(x, B, nn_level_H(n, lev), nn_level_W(n, lev), C,
                                                                       f, y);
     };
     auto upcat = [&](const bf16* low, int Cl, const bf16* skip, int Cs, int lev, bf16* k) {
         const int64_t P = nn_level_P(n, B, lev);
-        nn_up_k<<<nblk(P * Cl), 256, 0, s>>>(low, B, nn_level_H(n, lev), nn_level_W(n, lev), Cl, f, k, Cl + Cs, 0);
-        nn_copy_ch_k<bf16><<<nblk(P * Cs), 256, 0, s>>>(skip, Cs, 0, P, Cs, k, Cl + Cs, Cl);
+        nn_upcat_k<<<nblk(P * (Cl + Cs) / 8), 256, 0, s>>>(low, Cl, skip, Cs, B, nn_level_H(n, lev), nn_level_W(n, lev), f,
+                                                           k);
     };
     PS_TRY(cv(0, n->x0, 0, n->a[0]));
     PS_TRY(cv(1, n->a[0], 0, n->a[1]));
@@ -584,7 +656,7 @@ static int nn_backward(NNet* n, const float* dy, cudaStream_t s, int* err) {
         const int64_t P = nn_level_P(n, B, lev), Pl = nn_level_P(n, B, lev + 1);
         nn_up_bwd_k<<<nblk(Pl * Cl), 256, 0, s>>>(gk, Cl + Cs, 0, B, nn_level_H(n, lev), nn_level_W(n, lev), Cl, f,
                                                   glow);
-        nn_copy_ch_k<float><<<nblk(P * Cs), 256, 0, s>>>(gk, Cl + Cs, Cl, P, Cs, gskip, Cs, 0);
+        nn_copy_ch_k<<<nblk(P * Cs), 256, 0, s>>>(gk, Cl + Cs, Cl, P, Cs, gskip, Cs, 0);
     };
     auto poolbwd = [&](const float* gp, int lev, int C, float* gx) {
         nn_pool_bwd_k<<<nblk(nn_level_P(n, B, lev) * C), 256, 0, s>>>(gp, B, nn_level_H(n, lev), nn_level_W(n, lev), C,
