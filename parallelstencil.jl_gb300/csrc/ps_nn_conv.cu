@@ -2,7 +2,8 @@
 // (tcgen05): y[p][n] = act(sum over taps and channels of x[p + tap][c] * W[n][tap][c] + bias[n]), bf16
 // operands, FP32 accumulation in tensor memory, bf16 result. No column matrix is formed: a tap's 128
 // input pixels by KC channels are one 4-D TMA box of the NHWC activations, shifted by the tap, and the
-// pixels outside the image arrive as the zero fill that "same" padding wants.
+// pixels outside the image arrive as the zero fill that "same" padding wants. In layers whose rows fill
+// tiles of 128 pixels the three taps of a kernel row share one load (ROW below).
 //
 // A tile is 128 output pixels -- a box of bw x bh x bb pixels of x, y and image, powers of two chosen on
 // the host so that the fewest tiles cover the layer -- by BN output channels. Persistent and
@@ -13,10 +14,13 @@
 // rings are sized for that; 2 BN accumulator columns each leave tensor memory for both).
 //
 // KC = 64 channels (128-byte swizzle rows) where cin is a multiple of 64, else 32 (64-byte rows).
-// BN: 32 columns for narrow layers; 128 where the layer has tiles enough to fill the GPU, smaller where
-// splitting the channels over more CTAs is what fills it.
+// BN: 64 channels where the layer then still has a tile for every SM, else 32: splitting the channels over more
+// CTAs is what fills the GPU.
 //
-// Bound: L2 -> shared memory (each input value is loaded once per tap). @@
+// Bound: L2 -> shared memory. 8 images of 256^2, GPU time of a layer: 32 -> 32 channels 31 us, 96 -> 32 75 us
+// (41 and 118 with every tap's pixels loaded by themselves); the 64-channel layers at a quarter of the
+// size 10 to 16 us, the 128- and 256-channel ones 7 to 19 us. The whole forward pass: 7.52 ms through
+// column matrices, 0.38 ms now.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -28,12 +32,20 @@
 namespace ps {
 
 constexpr int kConvM = 128;
-template <int BN, int KC>
+// ROW: a tile is 128 pixels of one image row, and a ring stage holds the 130 pixels that the three taps of
+// one kernel row need, loaded once: a tap's A operand is the same block read from one pixel further on
+// (swizzling goes by the address, so a descriptor may start at any row of it), with the weights of the
+// three taps beside it. DEEP: one CTA per SM with twice the stages, for layers with fewer tiles than SMs.
+template <int BN, int KC, bool ROW, bool DEEP>
 struct ConvCfg {
-    static constexpr int ABYTES = kConvM * KC * 2, BBYTES = BN * KC * 2, STAGE = ABYTES + BBYTES;
-    static constexpr int S = (100 * 1024) / STAGE;  // ring stages: 76 to 113 KB, so that two CTAs fit an SM, not three
-    static constexpr int SMEM = S * STAGE + 1024 + 256;
-    static_assert(S >= 3 && SMEM > 77 * 1024 && SMEM < 113 * 1024, "two CTAs per SM");
+    static constexpr int TAPS = ROW ? 3 : 1;  // taps per stage
+    static constexpr int ABOX = (ROW ? kConvM + 2 : kConvM) * KC * 2, ABYTES = (ABOX + 1023) / 1024 * 1024;
+    static constexpr int BBYTES = BN * KC * 2, STAGE = ABYTES + TAPS * BBYTES;
+    // 76 to 113 KB of stages, so that two CTAs fit an SM, not three; DEEP: one
+    static constexpr int S = (DEEP ? 200 * 1024 : 105 * 1024) / STAGE;
+    static constexpr int SMEM = S * STAGE + 1024 + 512;
+    static_assert(S >= 2 && (DEEP ? SMEM > 115 * 1024 && SMEM < 226 * 1024 : SMEM > 77 * 1024 && SMEM < 113 * 1024),
+                  "CTAs per SM");
     static constexpr uint32_t TMEM = 2 * BN;  // two accumulators; two CTAs' columns fit the SM's 512
 };
 
@@ -44,11 +56,11 @@ struct ConvGeom {
     int tx, ty, tn, ntiles;    // tiles along x, y, channels; all tiles
 };
 
-template <int BN, int KC>
+template <int BN, int KC, bool ROW, bool DEEP>
 __global__ void __launch_bounds__(192, 2)
     nn_conv3_k(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB, ConvGeom g,
                const float* __restrict__ bias, int relu, __nv_bfloat16* __restrict__ y, int* __restrict__ err) {
-    using C = ConvCfg<BN, KC>;
+    using C = ConvCfg<BN, KC, ROW, DEEP>;
     constexpr int S = C::S;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem =
@@ -61,7 +73,7 @@ __global__ void __launch_bounds__(192, 2)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     int* counts = reinterpret_cast<int*>(tmem_slot + 1);  // [0] stages filled, [1] stages consumed
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cblk = g.cin / KC, KB = 9 * cblk;  // K blocks of a tile: taps, channel blocks fastest
+    const int cblk = g.cin / KC, KB = 9 / C::TAPS * cblk;  // ring steps of a tile: taps, channel blocks fastest
 
     if (threadIdx.x == 0) {
         prefetch_tensormap(&mA);
@@ -93,7 +105,7 @@ __global__ void __launch_bounds__(192, 2)
         for (int t = blockIdx.x; t < g.ntiles && ok; t += gridDim.x) {
             const int n0 = (t % g.tn) * BN, m = t / g.tn;
             const int x0 = (m % g.tx) << g.lw, y0 = ((m / g.tx) % g.ty) << g.lh, b0 = (m / (g.tx * g.ty)) << g.lb;
-            for (int tap = 0; tap < 9 && ok; tap++)
+            for (int tap = 0; tap < 9 && ok; tap += C::TAPS)
                 for (int cb = 0; cb < cblk; cb++, it++) {
                     const int s = it % S;
                     // stage s was last read by the MMAs of ring step it - S
@@ -102,9 +114,11 @@ __global__ void __launch_bounds__(192, 2)
                         break;
                     }
                     unsigned char* st = smem + s * C::STAGE;
-                    mbar_arrive_expect_tx(&full[s], C::STAGE);
+                    mbar_arrive_expect_tx(&full[s], C::ABOX + C::TAPS * C::BBYTES);
                     tma_load_4d(st, &mA, &full[s], cb * KC, x0 + tap % 3 - 1, y0 + tap / 3 - 1, b0);
-                    tma_load_2d(st + C::ABYTES, &mB, &full[s], tap * g.cin + cb * KC, n0);
+#pragma unroll
+                    for (int d = 0; d < C::TAPS; d++)
+                        tma_load_2d(st + C::ABYTES + d * C::BBYTES, &mB, &full[s], (tap + d) * g.cin + cb * KC, n0);
                 }
         }
         counts[0] = it;
@@ -130,11 +144,15 @@ __global__ void __launch_bounds__(192, 2)
                 }
                 tc_fence_after();
                 const uint32_t sa = smem_u32(smem + s * C::STAGE);
-                const uint64_t da = KC == 64 ? umma_desc_sw128(sa) : umma_desc_sw64(sa);
-                const uint64_t db = KC == 64 ? umma_desc_sw128(sa + C::ABYTES) : umma_desc_sw64(sa + C::ABYTES);
 #pragma unroll
-                for (int k = 0; k < KC / 16; k++)  // K = 16 per MMA: +32 bytes along the swizzled row
-                    tc_mma(d, da + 2 * k, db + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+                for (int e = 0; e < C::TAPS; e++) {
+                    const uint32_t pa = sa + e * KC * 2, pb = sa + C::ABYTES + e * C::BBYTES;
+                    const uint64_t da = KC == 64 ? umma_desc_sw128(pa) : umma_desc_sw64(pa);
+                    const uint64_t db = KC == 64 ? umma_desc_sw128(pb) : umma_desc_sw64(pb);
+#pragma unroll
+                    for (int k = 0; k < KC / 16; k++)  // K = 16 per MMA: +32 bytes along the swizzled row
+                        tc_mma(d, da + 2 * k, db + 2 * k, idesc, (i > 0 || e > 0 || k > 0) ? 1u : 0u);
+                }
                 tc_commit(&empty[s]);
             }
             if (!ok) break;
@@ -195,42 +213,43 @@ __global__ void __launch_bounds__(192, 2)
     if (warp == 0) tc_dealloc(tmem, C::TMEM);
 }
 
-template <int BN, int KC>
-static int conv3_launch(ConvGeom g, const void* x, const void* wgt, const float* bias, int relu, void* y, int sms,
+template <int BN, int KC, bool ROW, bool DEEP>
+static int conv3_launch(const ConvGeom& g, const void* x, const void* wgt, const float* bias, int relu, void* y, int sms,
                         cudaStream_t s, int* d_err) {
-    using C = ConvCfg<BN, KC>;
-    g.tn = g.cout / BN;
-    const int bw = 1 << g.lw, bh = 1 << g.lh, bb = 1 << g.lb;
-    const int64_t nt = (int64_t)g.tx * g.ty * ((g.B + bb - 1) / bb) * g.tn;
-    if (nt > 0x7FFFFFFF - 65536) return fail(PS_ERR_SHAPE, "nn_conv3: layer too large");
-    g.ntiles = (int)nt;
+    using C = ConvCfg<BN, KC, ROW, DEEP>;
     CUtensorMap mA, mB;
     const uint64_t da[4] = {(uint64_t)g.cin, (uint64_t)g.W, (uint64_t)g.H, (uint64_t)g.B};
-    const uint32_t ba[4] = {KC, (uint32_t)bw, (uint32_t)bh, (uint32_t)bb};
+    const uint32_t ba[4] = {KC, ROW ? kConvM + 2u : 1u << g.lw, 1u << g.lh, 1u << g.lb};
     const uint64_t db[2] = {(uint64_t)g.cin * 9, (uint64_t)g.cout};
     const uint32_t b2[2] = {KC, BN};
     PS_TRY(encode_bf16_box(&mA, x, 4, da, ba));
     PS_TRY(encode_bf16_box(&mB, wgt, 2, db, b2));
+    const auto kernel = nn_conv3_k<BN, KC, ROW, DEEP>;
     // every launch sets it: the attribute belongs to the device's current context
-    PS_CUDA_TRY(cudaFuncSetAttribute(nn_conv3_k<BN, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-    const int grid = (int)std::min<int64_t>(nt, 2 * (int64_t)std::max(1, sms));
-    PS_CUDA_TRY(launch_dependent(nn_conv3_k<BN, KC>, dim3((unsigned)grid), dim3(192), (size_t)C::SMEM, s, mA, mB, g, bias,
-                                 relu, static_cast<__nv_bfloat16*>(y), d_err));
+    PS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+    const int grid = std::min(g.ntiles, (DEEP ? 1 : 2) * sms);
+    PS_CUDA_TRY(launch_dependent(kernel, dim3((unsigned)grid), dim3(192), (size_t)C::SMEM, s, mA, mB, g, bias, relu,
+                                 static_cast<__nv_bfloat16*>(y), d_err));
     return PS_OK;
 }
 
 int nn_conv3_tc(const void* x, int B, int H, int W, int cin, const void* wgt, int cout, const float* bias, int relu,
                 void* y, cudaStream_t s, int* d_err) {
     if (cin % 32 || cout % 32 || B < 1 || H < 1 || W < 1) return fail(PS_ERR_SHAPE, "nn_conv3: layer %d -> %d", cin, cout);
+    DeviceState* st = nullptr;
+    PS_TRY(current_state(&st));
     ConvGeom g{};
     g.B = B;
     g.H = H;
     g.W = W;
     g.cin = cin;
     g.cout = cout;
-    // the box of 128 pixels that covers the layer in the fewest tiles; wide boxes first (longer contiguous runs)
+    // Whole rows of 128 pixels where at least three quarters of them are in the image: the input is read three
+    // times instead of nine. Else the box of 128 pixels that covers the layer in the fewest tiles, wide
+    // boxes first (longer contiguous runs).
+    const bool row = W % kConvM == 0 || W % kConvM >= 3 * kConvM / 4 || (W > kConvM && W % kConvM >= kConvM / 2);
     int64_t best = INT64_MAX;
-    for (int lw = 7; lw >= 0; lw--)
+    for (int lw = 7; lw >= (row ? 7 : 0); lw--)
         for (int lh = 7 - lw; lh >= 0; lh--) {
             const int lb = 7 - lw - lh;
             const int64_t tx = (W + (1 << lw) - 1) >> lw, ty = (H + (1 << lh) - 1) >> lh, tb = (B + (1 << lb) - 1) >> lb;
@@ -243,19 +262,24 @@ int nn_conv3_tc(const void* x, int B, int H, int W, int cin, const void* wgt, in
                 g.ty = (int)ty;
             }
         }
-    DeviceState* st = nullptr;
-    PS_TRY(current_state(&st));
-    // 128 channels per tile where that still gives every SM a tile, else 64, else 32
-    const int bn = cout % 128 == 0 && best * (cout / 128) >= st->num_sms  ? 128
-                   : cout % 64 == 0 && best * (cout / 64) >= st->num_sms ? 64
-                                                                         : 32;
-    auto run = [&](auto k) {
+    // 64 channels per tile where that still gives every SM a tile, else 32
+    const int bn = cout % 64 == 0 && best * (cout / 64) >= st->num_sms ? 64 : 32;
+    g.tn = cout / bn;
+    if (best * g.tn > 0x7FFFFFFF - 65536) return fail(PS_ERR_SHAPE, "nn_conv3: layer too large");
+    g.ntiles = (int)(best * g.tn);
+    const bool deep = g.ntiles < st->num_sms;
+    auto run = [&](auto k, auto r, auto d) {
         constexpr int KC = decltype(k)::value;
-        return bn == 128  ? conv3_launch<128, KC>(g, x, wgt, bias, relu, y, st->num_sms, s, d_err)
-               : bn == 64 ? conv3_launch<64, KC>(g, x, wgt, bias, relu, y, st->num_sms, s, d_err)
-                          : conv3_launch<32, KC>(g, x, wgt, bias, relu, y, st->num_sms, s, d_err);
+        constexpr bool R = decltype(r)::value, D = decltype(d)::value;
+        if constexpr (!D)  // (64 channels are taken only where there are tiles for every SM)
+            if (bn == 64) return conv3_launch<64, KC, R, D>(g, x, wgt, bias, relu, y, st->num_sms, s, d_err);
+        return conv3_launch<32, KC, R, D>(g, x, wgt, bias, relu, y, st->num_sms, s, d_err);
     };
-    return cin % 64 == 0 ? run(std::integral_constant<int, 64>{}) : run(std::integral_constant<int, 32>{});
+    auto kc = [&](auto r, auto d) {
+        return cin % 64 == 0 ? run(std::integral_constant<int, 64>{}, r, d) : run(std::integral_constant<int, 32>{}, r, d);
+    };
+    if (deep) return row ? kc(std::true_type{}, std::true_type{}) : kc(std::false_type{}, std::true_type{});
+    return row ? kc(std::true_type{}, std::false_type{}) : kc(std::false_type{}, std::false_type{});
 }
 
 }  // namespace ps

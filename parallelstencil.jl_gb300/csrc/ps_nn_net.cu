@@ -115,21 +115,21 @@ __global__ void nn_transpose_k(const bf16* __restrict__ in, int64_t R, int C, in
 }
 
 // f x f average pooling of x [B][H][W][C] -> [B][H/f][W/f][C] (FP32 sum row by row, bf16 result); a thread
-// takes 8 channels (16 bytes), C % 8 == 0
-__global__ void nn_pool_k(const bf16* __restrict__ x, int64_t B, int H, int W, int C, int f, bf16* y) {
-    const int h = H / f, w = W / f, C8 = C / 8;
-    const int64_t n = B * h * w * C8;
+// takes 8 channels (16 bytes), C % 8 == 0; blocks along x run over rows of the result, along y over a row's values
+__global__ void __launch_bounds__(256) nn_pool_k(const bf16* __restrict__ x, int rows, int h, int w, int C8, int f, bf16* y) {
+    grid_dependency_wait();
+    grid_dependents_may_launch();
+    const int W = w * f, i = (int)(blockIdx.y * 256 + threadIdx.x);
+    if (i >= w * C8) return;
+    const int xx = i / C8, c = i - xx * C8;
     const float inv = 1.0f / (float)(f * f);
-    GSTRIDE(i, n) {
-        const int c = (int)(i % C8);
-        const int64_t q = i / C8;
-        const int xx = (int)(q % w), yy = (int)((q / w) % h);
-        const int64_t b = q / ((int64_t)w * h);
-        const uint4* s = reinterpret_cast<const uint4*>(x + ((b * H + (int64_t)f * yy) * W + (int64_t)f * xx) * C) + c;
+    for (int r0 = blockIdx.x; r0 < rows; r0 += gridDim.x) {  // row r0 averages rows f * r0 .. of the input (H = f h)
+        const uint4* s = reinterpret_cast<const uint4*>(x) + ((int64_t)r0 * f * W + (int64_t)f * xx) * C8 + c;
         float v[8] = {};
         for (int r = 0; r < f; r++)
+#pragma unroll 4
             for (int k = 0; k < f; k++) {
-                const uint4 u = __ldg(s + ((int64_t)r * W + k) * C8);
+                const uint4 u = s[((int64_t)r * W + k) * C8];
                 const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&u);
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
@@ -142,7 +142,7 @@ __global__ void nn_pool_k(const bf16* __restrict__ x, int64_t B, int H, int W, i
         __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
         for (int e = 0; e < 4; e++) oh[e] = __floats2bfloat162_rn(v[2 * e] * inv, v[2 * e + 1] * inv);
-        reinterpret_cast<uint4*>(y)[i] = o;
+        reinterpret_cast<uint4*>(y)[(int64_t)r0 * w * C8 + i] = o;
     }
 }
 // dx [B][H][W][C] (+)= dy [B][H/f][W/f][C] / f^2 broadcast
@@ -161,70 +161,99 @@ __global__ void nn_pool_bwd_k(const float* __restrict__ dy, int64_t B, int H, in
     }
 }
 // k[b][Y][X] = the Cl channels of low[b][Y/f][X/f], then the Cs channels of skip[b][Y][X] (16 bytes per thread;
-// Cl, Cs % 8 == 0)
-__global__ void nn_upcat_k(const bf16* __restrict__ low, int Cl, const bf16* __restrict__ skip, int Cs, int64_t B, int H,
-                           int W, int f, bf16* k) {
-    const int h = H / f, w = W / f, Cl8 = Cl / 8, Cs8 = Cs / 8, C8 = Cl8 + Cs8;
-    const int64_t n = B * H * W * C8;
-    GSTRIDE(i, n) {
-        const int c = (int)(i % C8);
-        const int64_t q = i / C8;
-        uint4 v;
+// Cl8, Cs8: channels / 8). Blocks along x run over the f-row groups of the result, along y over a row's
+// values: the position in a row and its division are one thread's for all its rows, a value of low is loaded
+// once for its f rows. Bound by its stores (8 images of 256^2, 64 + 32 channels: 65 us with one 64-bit
+// index per value, 28 now).
+__global__ void __launch_bounds__(256) nn_upcat_k(const bf16* __restrict__ low, int Cl8, const bf16* __restrict__ skip,
+                                                  int Cs8, int groups, int W, int f, bf16* k) {
+    grid_dependency_wait();
+    grid_dependents_may_launch();
+    const int C8 = Cl8 + Cs8, w = W / f, i = (int)(blockIdx.y * 256 + threadIdx.x);
+    if (i >= W * C8) return;
+    const int xx = i / C8, c = i - xx * C8, lx = xx / f * Cl8 + c, sx = xx * Cs8 + c - Cl8;
+    for (int g = blockIdx.x; g < groups; g += gridDim.x) {
+        uint4* d = reinterpret_cast<uint4*>(k) + (int64_t)g * f * W * C8 + i;
         if (c < Cl8) {
-            const int xx = (int)(q % W), yy = (int)((q / W) % H);
-            const int64_t b = q / ((int64_t)W * H);
-            v = __ldg(reinterpret_cast<const uint4*>(low) + ((b * h + yy / f) * w + xx / f) * Cl8 + c);
+            const uint4 v = reinterpret_cast<const uint4*>(low)[(int64_t)g * w * Cl8 + lx];
+            for (int r = 0; r < f; r++) d[(int64_t)r * W * C8] = v;
         } else {
-            v = __ldg(reinterpret_cast<const uint4*>(skip) + q * Cs8 + (c - Cl8));
+            const uint4* s = reinterpret_cast<const uint4*>(skip) + (int64_t)g * f * W * Cs8 + sx;
+#pragma unroll 4
+            for (int r = 0; r < f; r++) d[(int64_t)r * W * C8] = s[(int64_t)r * W * Cs8];
         }
-        reinterpret_cast<uint4*>(k)[i] = v;
     }
 }
-// The first layer: y[p][0..31] = relu(3x3 conv of the two input channels + bias), one pixel per thread
-// (K = 18 is too short for the tensor cores; bound by its 64-byte result per pixel and 576 FMAs)
-__global__ void __launch_bounds__(256, 3) nn_conv_first_k(const bf16* __restrict__ x, const bf16* __restrict__ wgt, int kpad,
-                                                       const float* __restrict__ bias, int64_t B, int H, int W, bf16* y) {
+// The first layer: y[p][0..31] = relu(3x3 conv of the two input channels + bias). K = 18 is too short for the
+// tensor cores. A thread takes 16 of the 32 outputs of 4 pixels a block's width apart, so that a 16-byte
+// weight load from shared memory feeds 16 FMAs (one pixel with 32 outputs per thread: 4 FMAs per load, bound by
+// shared memory, 40 us for 8 images of 256^2; now 30).
+constexpr int kFirstPix = 4;
+__global__ void __launch_bounds__(256, 2) nn_conv_first_k(const bf16* __restrict__ x, const bf16* __restrict__ wgt, int kpad,
+                                                       const float* __restrict__ bias, int64_t P, int H, int W, bf16* y) {
     __shared__ float4 sw[18][8];  // [tap, channel][output / 4]
     __shared__ float sb[32];
+    grid_dependency_wait();
+    grid_dependents_may_launch();
     for (int i = threadIdx.x; i < 18 * 32; i += blockDim.x)
         reinterpret_cast<float*>(sw[i / 32])[i % 32] = __bfloat162float(wgt[(int64_t)(i % 32) * kpad + i / 32]);
     for (int i = threadIdx.x; i < 32; i += blockDim.x) sb[i] = bias[i];
     __syncthreads();
-    const int64_t P = B * H * W;
-    GSTRIDE(p, P) {
-        const int xx = (int)(p % W), yy = (int)((p / W) % H);
-        float acc[32];
+    const int half = threadIdx.x & 1, o4 = 4 * half;
+    const int64_t p0 = blockIdx.x * (int64_t)(kFirstPix * 128) + (threadIdx.x >> 1);
+    const __nv_bfloat162* x2 = reinterpret_cast<const __nv_bfloat162*>(x);
+    int xx[kFirstPix], yy[kFirstPix];
 #pragma unroll
-        for (int o = 0; o < 32; o++) acc[o] = 0.0f;
+    for (int j = 0; j < kFirstPix; j++) {
+        const int64_t p = p0 + j * 128, q = p / W;
+        xx[j] = p < P ? (int)(p - q * W) : -2;  // -2: no tap of it is in the image
+        yy[j] = (int)(q % H);
+    }
+    float acc[kFirstPix][16] = {};
 #pragma unroll 1
-        for (int tap = 0; tap < 9; tap++) {
-            const int sy = yy + tap / 3 - 1, sx = xx + tap % 3 - 1;
-            float2 v = make_float2(0.0f, 0.0f);
-            if (sy >= 0 && sy < H && sx >= 0 && sx < W)
-                v = __bfloat1622float2(
-                    reinterpret_cast<const __nv_bfloat162*>(x)[p + (int64_t)(tap / 3 - 1) * W + (tap % 3 - 1)]);
+    for (int ty = -1; ty <= 1; ty++)
+#pragma unroll 1
+        for (int tx = -1; tx <= 1; tx++) {
+            float2 v[kFirstPix];
 #pragma unroll
-            for (int o = 0; o < 8; o++) {
-                const float4 a = sw[2 * tap][o], b = sw[2 * tap + 1][o];
-                acc[4 * o] = fmaf(v.y, b.x, fmaf(v.x, a.x, acc[4 * o]));
-                acc[4 * o + 1] = fmaf(v.y, b.y, fmaf(v.x, a.y, acc[4 * o + 1]));
-                acc[4 * o + 2] = fmaf(v.y, b.z, fmaf(v.x, a.z, acc[4 * o + 2]));
-                acc[4 * o + 3] = fmaf(v.y, b.w, fmaf(v.x, a.w, acc[4 * o + 3]));
+            for (int j = 0; j < kFirstPix; j++) {
+                const bool in = (unsigned)(xx[j] + tx) < (unsigned)W && (unsigned)(yy[j] + ty) < (unsigned)H;
+                v[j] = in ? __bfloat1622float2(x2[p0 + j * 128 + ty * W + tx]) : make_float2(0.0f, 0.0f);
+            }
+            const int tap = 3 * (ty + 1) + tx + 1;
+#pragma unroll
+            for (int o = 0; o < 4; o++) {
+                const float4 a = sw[2 * tap][o4 + o], b = sw[2 * tap + 1][o4 + o];
+#pragma unroll
+                for (int j = 0; j < kFirstPix; j++) {
+                    float* c = acc[j] + 4 * o;
+                    c[0] = fmaf(v[j].y, b.x, fmaf(v[j].x, a.x, c[0]));
+                    c[1] = fmaf(v[j].y, b.y, fmaf(v[j].x, a.y, c[1]));
+                    c[2] = fmaf(v[j].y, b.z, fmaf(v[j].x, a.z, c[2]));
+                    c[3] = fmaf(v[j].y, b.w, fmaf(v[j].x, a.w, c[3]));
+                }
             }
         }
-        uint4 w4[4];
+#pragma unroll
+    for (int j = 0; j < kFirstPix; j++) {
+        if (xx[j] < 0) continue;
+        uint4 w4[2];
         __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(w4);
 #pragma unroll
-        for (int o = 0; o < 16; o++)
-            h[o] = __floats2bfloat162_rn(fmaxf(acc[2 * o] + sb[2 * o], 0.0f), fmaxf(acc[2 * o + 1] + sb[2 * o + 1], 0.0f));
-#pragma unroll
-        for (int o = 0; o < 4; o++) reinterpret_cast<uint4*>(y + p * 32)[o] = w4[o];
+        for (int o = 0; o < 8; o++)
+            h[o] = __floats2bfloat162_rn(fmaxf(acc[j][2 * o] + sb[16 * half + 2 * o], 0.0f),
+                                         fmaxf(acc[j][2 * o + 1] + sb[16 * half + 2 * o + 1], 0.0f));
+        uint4* d = reinterpret_cast<uint4*>(y + (p0 + j * 128) * 32 + 16 * half);
+        d[0] = w4[0];
+        d[1] = w4[1];
     }
 }
 // The last layer: y[p][0..2] = W x[p] + bias over 32 channels (FP32 result), one pixel per thread
 __global__ void __launch_bounds__(256) nn_conv_last_k(const bf16* __restrict__ x, const bf16* __restrict__ wgt, int kpad,
                                                       const float* __restrict__ bias, int64_t P, float* __restrict__ y) {
     __shared__ float sw[3][32];
+    grid_dependency_wait();
+    grid_dependents_may_launch();
     for (int i = threadIdx.x; i < 96; i += blockDim.x) sw[i / 32][i % 32] = __bfloat162float(wgt[(int64_t)(i / 32) * kpad + i % 32]);
     __syncthreads();
     const float b0 = bias[0], b1 = bias[1], b2 = bias[2];
@@ -232,7 +261,7 @@ __global__ void __launch_bounds__(256) nn_conv_last_k(const bf16* __restrict__ x
         float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            const uint4 u = __ldg(reinterpret_cast<const uint4*>(x + p * 32) + q);
+            const uint4 u = reinterpret_cast<const uint4*>(x + p * 32)[q];
             const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
 #pragma unroll
             for (int e = 0; e < 4; e++) {
@@ -276,6 +305,16 @@ __global__ void nn_copy_ch_k(const float* __restrict__ src, int lds, int soff, i
 }
 __global__ void nn_f32_to_bf16_k(const float* __restrict__ a, int64_t n, bf16* b) {
     GSTRIDE(i, n) b[i] = __float2bfloat16_rn(a[i]);
+}
+// the same for the network's input: 4 values per thread (n % 4 == 0; 16-byte aligned arrays)
+__global__ void __launch_bounds__(256) nn_input_k(const float4* __restrict__ a, int64_t n4, uint2* b) {
+    grid_dependency_wait();
+    grid_dependents_may_launch();
+    GSTRIDE(i, n4) {
+        const float4 v = a[i];
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+        b[i] = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+    }
 }
 // weighted mean squared error: loss += sum w (y - t)^2 * scale, dy = 2 w (y - t) * scale
 __global__ void nn_mse_k(const float* __restrict__ y, const float* __restrict__ t, const float* __restrict__ w,
@@ -551,9 +590,11 @@ static int nn_conv_fwd(NNet* n, Conv& L, const bf16* x, int B, int h, int w, voi
     if (L.k == 3 && L.cin % 32 == 0)
         return nn_conv3_tc(x, B, h, w, L.cin, L.W, L.cout, L.b, L.relu, y, s, err);
     if (L.k == 3)
-        nn_conv_first_k<<<nblk(P), 256, 0, s>>>(x, L.W, (int)L.kpad, L.b, B, h, w, static_cast<bf16*>(y));
+        PS_CUDA_TRY(launch_dependent(nn_conv_first_k, dim3((unsigned)((P + kFirstPix * 128 - 1) / (kFirstPix * 128))), dim3(256),
+                                     0, s, x, L.W, (int)L.kpad, L.b, P, h, w, static_cast<bf16*>(y)));
     else
-        nn_conv_last_k<<<nblk(P), 256, 0, s>>>(x, L.W, (int)L.kpad, L.b, P, static_cast<float*>(y));
+        PS_CUDA_TRY(launch_dependent(nn_conv_last_k, dim3(nblk(P)), dim3(256), 0, s, x, L.W, (int)L.kpad, L.b, P,
+                                     static_cast<float*>(y)));
     return PS_OK;
 }
 
@@ -604,6 +645,18 @@ static int nn_conv_bwd(NNet* n, Conv& L, const bf16* x, const bf16* yact, const 
     return PS_OK;
 }
 
+// the bf16 copy of an FP32 input of count values (a multiple of 4); a caller's array may be aligned to its type only
+static int nn_input(const float* x, int64_t count, bf16* x0, cudaStream_t s) {
+    if ((uintptr_t)x % 16 == 0) {
+        PS_CUDA_TRY(launch_dependent(nn_input_k, dim3(nblk(count / 4)), dim3(256), 0, s, reinterpret_cast<const float4*>(x),
+                                     count / 4, reinterpret_cast<uint2*>(x0)));
+    } else {
+        nn_f32_to_bf16_k<<<nblk(count), 256, 0, s>>>(x, count, x0);
+        PS_CUDA_TRY(cudaGetLastError());
+    }
+    return PS_OK;
+}
+
 static int nn_forward(NNet* n, int B, cudaStream_t s, int* err) {
     const int c = n->base, f = n->pf;
     auto& L = n->conv;
@@ -611,32 +664,33 @@ static int nn_forward(NNet* n, int B, cudaStream_t s, int* err) {
         return nn_conv_fwd(n, L[i], x, B, nn_level_H(n, lev), nn_level_W(n, lev), y, s, err);
     };
     auto pool = [&](const bf16* x, int lev, int C, bf16* y) {
-        nn_pool_k<<<nblk(nn_level_P(n, B, lev + 1) * C / 8), 256, 0, s>>>(x, B, nn_level_H(n, lev), nn_level_W(n, lev), C,
-                                                                      f, y);
+        const int h = nn_level_H(n, lev + 1), w = nn_level_W(n, lev + 1);
+        return launch_dependent(nn_pool_k, dim3((unsigned)std::min(B * h, 1 << 20), (unsigned)((w * (C / 8) + 255) / 256)), dim3(256),
+                                0, s, x, B * h, h, w, C / 8, f, y);
     };
     auto upcat = [&](const bf16* low, int Cl, const bf16* skip, int Cs, int lev, bf16* k) {
-        const int64_t P = nn_level_P(n, B, lev);
-        nn_upcat_k<<<nblk(P * (Cl + Cs) / 8), 256, 0, s>>>(low, Cl, skip, Cs, B, nn_level_H(n, lev), nn_level_W(n, lev), f,
-                                                           k);
+        const int groups = B * nn_level_H(n, lev + 1), W = nn_level_W(n, lev);
+        return launch_dependent(nn_upcat_k, dim3((unsigned)std::min(groups, 1 << 20), (unsigned)((W * ((Cl + Cs) / 8) + 255) / 256)),
+                                dim3(256), 0, s, low, Cl / 8, skip, Cs / 8, groups, W, f, k);
     };
     PS_TRY(cv(0, n->x0, 0, n->a[0]));
     PS_TRY(cv(1, n->a[0], 0, n->a[1]));
-    pool(n->a[1], 0, c, n->p1);
+    PS_CUDA_TRY(pool(n->a[1], 0, c, n->p1));
     PS_TRY(cv(2, n->p1, 1, n->a[2]));
     PS_TRY(cv(3, n->a[2], 1, n->a[3]));
-    pool(n->a[3], 1, 2 * c, n->p2);
+    PS_CUDA_TRY(pool(n->a[3], 1, 2 * c, n->p2));
     PS_TRY(cv(4, n->p2, 2, n->a[4]));
     PS_TRY(cv(5, n->a[4], 2, n->a[5]));
-    pool(n->a[5], 2, 4 * c, n->p3);
+    PS_CUDA_TRY(pool(n->a[5], 2, 4 * c, n->p3));
     PS_TRY(cv(6, n->p3, 3, n->a[6]));
     PS_TRY(cv(7, n->a[6], 3, n->a[7]));
-    upcat(n->a[7], 8 * c, n->a[5], 4 * c, 2, n->k2);
+    PS_CUDA_TRY(upcat(n->a[7], 8 * c, n->a[5], 4 * c, 2, n->k2));
     PS_TRY(cv(8, n->k2, 2, n->a[8]));
     PS_TRY(cv(9, n->a[8], 2, n->a[9]));
-    upcat(n->a[9], 4 * c, n->a[3], 2 * c, 1, n->k1);
+    PS_CUDA_TRY(upcat(n->a[9], 4 * c, n->a[3], 2 * c, 1, n->k1));
     PS_TRY(cv(10, n->k1, 1, n->a[10]));
     PS_TRY(cv(11, n->a[10], 1, n->a[11]));
-    upcat(n->a[11], 2 * c, n->a[1], c, 0, n->k0);
+    PS_CUDA_TRY(upcat(n->a[11], 2 * c, n->a[1], c, 0, n->k0));
     PS_TRY(cv(12, n->k0, 0, n->a[12]));
     PS_TRY(cv(13, n->a[12], 0, n->a[13]));
     PS_TRY(cv(14, n->a[13], 0, n->y));
@@ -790,7 +844,7 @@ int ps_nn_forward(void* net, const float* x, int32_t B, float* y, void* stream) 
     NNet* n = as_net(net);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int64_t P0 = nn_level_P(n, B, 0);
-    nn_f32_to_bf16_k<<<nblk(P0 * 2), 256, 0, s>>>(x, P0 * 2, n->x0);
+    PS_TRY(nn_input(x, P0 * 2, n->x0, s));
     PS_TRY(nn_forward(n, B, s, st->d_err));
     if (y) PS_CUDA_TRY(cudaMemcpyAsync(y, n->y, P0 * 3 * sizeof(float), cudaMemcpyDeviceToDevice, s));
     return finish_launch(s, 1, "ps_nn_forward");
@@ -831,7 +885,7 @@ int ps_nn_train_step(void* net, const float* x, const float* t, const float* w, 
     NNet* n = as_net(net);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int64_t P0 = nn_level_P(n, B, 0);
-    nn_f32_to_bf16_k<<<nblk(P0 * 2), 256, 0, s>>>(x, P0 * 2, n->x0);
+    PS_TRY(nn_input(x, P0 * 2, n->x0, s));
     PS_TRY(nn_forward(n, B, s, st->d_err));
     PS_CUDA_TRY(cudaMemsetAsync(n->loss, 0, sizeof(double), s));
     nn_mse_k<<<nblk(P0 * 3), 256, 0, s>>>(n->y, t, w, P0, 3, 1.0f / (float)(P0 * 3), n->ga[14], n->loss);
@@ -967,7 +1021,7 @@ int ps_stokes2d_warm_start(void* net, const ps_stokes2d_fields* f, int32_t nvali
     const int64_t P0 = (int64_t)n->H * n->W;
     nn_ws_input_k<<<nblk(P0), 256, 0, s>>>(static_cast<const double*>(f->Mus.ptr), static_cast<const double*>(f->Rog.ptr),
                                            (int)nx, (int)ny, n->H, n->W, nvalid, n->dsc, n->ws_x);
-    nn_f32_to_bf16_k<<<nblk(P0 * 2), 256, 0, s>>>(n->ws_x, P0 * 2, n->x0);
+    PS_TRY(nn_input(n->ws_x, P0 * 2, n->x0, s));
     PS_TRY(nn_forward(n, 1, s, st->d_err));
     const int64_t tot = nx * ny + (nx + 1) * ny + nx * (ny + 1);
     nn_ws_output_k<<<nblk(tot), 256, 0, s>>>(n->y, n->H, n->W, nvalid, (int)nx, (int)ny, n->dsc,

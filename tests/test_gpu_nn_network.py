@@ -131,3 +131,26 @@ def test_save_load_roundtrip(ps, tmp_path):
     y1 = net2.forward(x).cpu().numpy()
     # saved weights are bf16 (what the forward pass uses), so the outputs agree exactly
     assert np.array_equal(y0, y1)
+
+
+@pytest.mark.parametrize("H,W,B", [(64, 64, 1), (64, 128, 1), (64, 192, 3), (64, 512, 1), (64, 512, 10), (64, 256, 19),
+                                   (192, 64, 5)])
+def test_forward_over_tile_shapes(ps, H, W, B):
+    """Layers narrower and wider than a tile of 128 pixels, ragged row tiles, batches that share a tile or leave
+    one part empty, more and fewer tiles than SMs: the first and the last image against the reference, with
+    the tolerance of test_network_forward_matches_reference; an input that is aligned to its type only gives
+    the same bytes."""
+    import torch
+
+    from oracle.nn_reference import Reference
+
+    net, x = _setup(ps, H, W, B, seed=H + W + B)
+    y = net.forward(x).cpu().numpy()
+    ends = [0, B - 1]
+    with torch.no_grad():
+        yr = Reference(net.get_params()).forward(x[ends].cpu()).numpy()
+    for i, b in enumerate(ends):
+        assert _relerr(y[b], yr[i]) <= 2e-2, (b, _relerr(y[b], yr[i]))
+    odd = torch.empty(x.numel() + 1, device="cuda")[1:].view(x.shape)
+    odd.copy_(x)
+    assert np.array_equal(net.forward(odd).cpu().numpy(), y)
