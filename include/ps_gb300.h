@@ -503,6 +503,9 @@ int ps_jit_launch(void* kernel, const ps_array* arrays, int32_t narrays, const d
 int ps_jit_launch_ex(void* kernel, const ps_array* arrays, int32_t narrays, const double* scalars, int32_t nscalars,
                      const int64_t lo[3], const int64_t count[3], const int32_t threads[3], int64_t shmem,
                      const int32_t loop[3], void* stream, int sync);
+/* Blocks of `threads` threads with `shmem` bytes of dynamic shared memory that one SM holds of a compiled kernel
+ * at once (what a sweep's length per thread is chosen by). */
+int ps_jit_blocks_per_sm(void* kernel, int32_t threads, int64_t shmem, int32_t* blocks);
 /* The memopt z-sweep of a run-time compiled 3-D `@parallel` kernel with its read-only stencil
  * arrays staged plane by plane in shared memory by TMA (src/memopt.jl:190-573 caches the same
  * arrays in registers and shared memory; launched by src/parallel.jl:451-596). The kernel must be

@@ -51,7 +51,9 @@ static ModuleLoadDataFn g_load = nullptr;
 static ModuleGetFunctionFn g_getfn = nullptr;
 static ModuleUnloadFn g_unload = nullptr;
 static LaunchKernelFn g_launch = nullptr;
+typedef CUresult (*OccupancyFn)(int*, CUfunction, int, size_t);
 static FuncSetAttributeFn g_setattr = nullptr;
+static OccupancyFn g_occupancy = nullptr;
 static std::mutex g_jit_mutex;
 
 template <typename F>
@@ -74,6 +76,7 @@ static int jit_driver() {
     PS_TRY(driver_fn("cuModuleGetFunction", &g_getfn));
     PS_TRY(driver_fn("cuModuleUnload", &g_unload));
     PS_TRY(driver_fn("cuFuncSetAttribute", &g_setattr));
+    PS_TRY(driver_fn("cuOccupancyMaxActiveBlocksPerMultiprocessor", &g_occupancy));
     PS_TRY(driver_fn("cuLaunchKernel", &g_launch));
     return PS_OK;
 }
@@ -136,6 +139,22 @@ int ps_jit_compile(const char* source, const char* entry, void** kernel) {
     }
     cudaGetDevice(&k->device);
     *kernel = k;
+    return PS_OK;
+}
+
+int ps_jit_blocks_per_sm(void* kernel, int32_t threads, int64_t shmem, int32_t* blocks) {
+    DeviceState* st = nullptr;
+    PS_TRY(current_state(&st));
+    if (!kernel || !blocks) return fail(PS_ERR_NULL, "ps_jit_blocks_per_sm: NULL argument");
+    if (threads < 1 || threads > 1024 || shmem < 0 || shmem > 227 * 1024)
+        return fail(PS_ERR_ARG, "ps_jit_blocks_per_sm: 1 to 1024 threads and at most 227 KB of dynamic shared memory");
+    JitKernel* k = static_cast<JitKernel*>(kernel);
+    int dev = -1, n = 0;
+    cudaGetDevice(&dev);
+    if (dev != k->device) return fail(PS_ERR_ARG, "ps_jit_blocks_per_sm: kernel compiled for device %d", k->device);
+    const CUresult r = g_occupancy(&n, k->fn, threads, (size_t)shmem);
+    if (r != CUDA_SUCCESS) return fail(PS_ERR_CUDA, "ps_jit_blocks_per_sm: the occupancy query failed (CUresult %d)", (int)r);
+    *blocks = n;
     return PS_OK;
 }
 

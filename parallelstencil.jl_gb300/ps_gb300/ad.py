@@ -38,10 +38,12 @@ from . import _lib
 from ._lib import PSArray
 from .core import ArgumentError, descriptor, require_initialized, stream_handle
 from .fd import AV, DIFF, DIFF2, HARM, MAXLOC, MINLOC, SEL
-from .jit import _MATH, JitKernel, _Gen, _lit, array_ndims, uses_kernel_language
+from .jit import (MAX_ARRAYS, MAX_SCALARS, VALUE_HELPERS, _MATH, JitKernel, _Gen, _lit, array_ndims, blocks_per_sm,
+                  sweep_chunk, uses_kernel_language)
 from .kernels import ranges_to_box
 
 MODES = ("reverse", "forward")
+SWEEP_MIN = 1 << 19  # points from which FP32 reverse kernels sweep
 _ONE = "((R)1.0)"
 _LITERAL = re.compile(r"^\(\(R\)[-+0-9.eE]+\)$")  # a number literal of the kernel's type
 _SCALAR = re.compile(r"^s[0-9]+$")                  # a scalar argument
@@ -97,6 +99,7 @@ class _AdGen(_Gen):
         self.dvars = []      # registers with an adjoint (b...) or tangent (t...)
         self.tape = []       # (executed flag, nodes, store) per statement, in execution order
         self.nodes = None
+        self.fresh = set()   # registers of the current statement whose adjoint nothing has been added to
         self.cur = {}        # real local variable -> its current value
         self.cache = None    # loads of one `@parallel` statement: (array, offsets) -> value
         self.keys = {}       # array -> access keys (offsets / index expressions) of all its accesses
@@ -485,7 +488,7 @@ class _AdGen(_Gen):
 
         def acc(x, expr):
             if x is not None and x.var:
-                lines.append(f"b{x.code} += {expr};")
+                lines.append(self.add(x.code, expr))
         if op == "load":
             name, ivs = aux
             k = self.aidx[name]
@@ -527,6 +530,23 @@ class _AdGen(_Gen):
             acc(a, f"{bo} * {self.dfun(op, A, O)}")
         return lines
 
+    def add(self, v, expr):
+        """Addition to the adjoint of register v; the first one of its statement sets it (an addition to zero is an
+        instruction of its own: 60 of the 140 of the FP64 flux step, whose time is the FP64 pipe's)."""
+        first = v in self.fresh
+        self.fresh.discard(v)
+        return f"b{v} {'' if first else '+'}= {expr};"
+
+    def only_here(self, entry):
+        """Registers of a statement whose adjoints receive nothing from the other statements."""
+        mine = {o.code for _, o, _, _ in self.tape[entry][1]}
+        for i, (_, nodes, store) in enumerate(self.tape):
+            if i != entry:
+                mine -= {x.code for _, _, ins, _ in nodes for x in ins}
+                if store is not None:
+                    mine.discard(store[2].code)
+        return mine
+
     def is_shared(self, name):
         """Whether other threads may touch the shadow elements this thread touches: unless every
         access of the array in the kernel goes to one index of the thread's own (the same offsets /
@@ -545,7 +565,9 @@ class _AdGen(_Gen):
 
     def reverse_lines(self):
         out = []
-        for f, nodes, store in reversed(self.tape):
+        for entry in reversed(range(len(self.tape))):
+            f, nodes, store = self.tape[entry]
+            self.fresh = self.only_here(entry)
             blk = []
             if store is not None:
                 name, i3, rhs = store
@@ -553,7 +575,7 @@ class _AdGen(_Gen):
                     continue
                 k = self.aidx[name]
                 g = f"ad_take(d{k}, n{k}_0, n{k}_1, n{k}_2, {i3[0]}, {i3[1]}, {i3[2]})"
-                blk.append(f"b{rhs.code} += (R){g};" if rhs.var else f"(void){g};")
+                blk.append(self.add(rhs.code, f"(R){g}") if rhs.var else f"(void){g};")
             for op, o, ins, aux in reversed(nodes):
                 blk += self.adjoint(op, o, ins, aux)
             if blk:
@@ -587,6 +609,370 @@ class _AdGen(_Gen):
         return super().types(real) + "\n" + _HELPERS
 
 
+class _NoSweep(Exception):
+    """The sweep form does not apply to this kernel; one point per thread is generated instead."""
+
+
+class _AdSweepGen(_AdGen):
+    """Reverse kernel of a 2-D or 3-D `@parallel` definition as a sweep along the last dimension.
+
+    With one point per thread every value read from a duplicated array is an atomic addition of its own to
+    that array's shadow: 14 per cell for the 3-D flux step with a conductivity array, and their index
+    arithmetic and bounds checks, which is what the kernel spends its time on. Here a thread sums what
+    flows to an element before it touches memory:
+
+    - a thread keeps the contributions of its point in registers, one per array and offset;
+    - those along x move to the thread of the element's column by warp shuffles, those along y through
+      shared memory (two buffers in turn, one barrier per plane);
+    - those along the sweep accumulate in registers until the sweep has passed the element, which then
+      takes one atomic addition. Elements at the edge of a warp's rows, of a block's columns and of a
+      chunk of the sweep take one from each side.
+
+    So the flux step makes 2 additions per cell, and 4 one-lane ones per row and plane of a warp. The order
+    in which an element's contributions are added was never fixed (atomics) and still is not.
+
+    The values of arrays that the kernel only reads are loaded while the plane before is worked on, and handed from
+    offset to offset along the sweep (left to itself the compiler sank the loads to their uses, where each
+    waited for the one before: 390 us).
+
+    Every access must be at fixed offsets from the thread's point; the caller (sweep_fits) has checked
+    that all of them lie in their arrays, so nothing is checked here, and that 32-bit indices do.
+    192^3, FP32: 477 us per launch with one point per thread, 100 so (10 words per cell take 42)."""
+
+    TX, TY = 32, 8            # block of the 3-D form; 2-D: 128 x 1, whose warps exchange nothing
+    SMEM = 40 * 1024          # bound on the exchange buffers
+
+    def __init__(self, kd, ndims, dup):
+        if kd.kind != "parallel" or ndims not in (2, 3):
+            raise _NoSweep
+        super().__init__(kd, ndims, dup, "reverse")
+        self.access = set()   # (array, offset, left-hand array, its mask): what sweep_fits checks
+        self.lhs = None
+        self.regs = {}        # statement's left-hand side -> {(read-only array, offset) -> register}
+        self.early = None     # the taken shadow's element, where it can be loaded with them
+
+    # ---- accesses: `p<k>` points to the thread's point of array k
+    def ref(self, name, o, p="p"):
+        k = self.aidx[name]
+        o = tuple(o) + (0,) * (3 - len(o))
+        if self.lhs is None:
+            raise _NoSweep
+        self.access.add((name, o) + self.lhs)
+        return f"{p}{k}[{o[0]} + n{k}_0 * ({o[1]} + n{k}_1 * {o[2]})]"
+
+    def val(self, name, o):
+        if name in self.temps:
+            return super().val(name, o)
+        if name not in self.aidx:
+            raise ArgumentError(f"unknown array {name}")
+        return self.load(name, o[:self.nd])
+
+    def load(self, name, ix):
+        if any(not isinstance(x, int) for x in ix):
+            raise _NoSweep
+        r = self.ref(name, ix)
+        return f"__ldg(&{r})" if name in self.read_only else r
+
+    def leaf(self, name, idx, key=None):
+        if key is None or key[0] != "o":
+            raise _NoSweep
+        self.key(name, key)
+        code = self.ahead(name, key[1]) if name in self.read_only else self.load(name, key[1])
+        return self.node("load", code, [], aux=(name, key[1])) if name in self.dup else self.const(code)
+
+    def ahead(self, name, o):
+        """The register that holds a read-only array's value, loaded while the plane before was worked on."""
+        self.ref(name, o)
+        o = tuple(o) + (0,) * (3 - len(o))
+        regs = self.regs.setdefault(self.lhs, {})
+        return regs.setdefault((name, o), "L%d_%d" % (list(self.regs).index(self.lhs), len(regs)))
+
+    def condition(self, lhs, ahead=""):
+        """The statement's left-hand condition at this plane, or at the next (ahead = " + 1")."""
+        name, li = lhs
+        k, zd = self.aidx[name], self.nd - 1
+        t3 = ("tx", "ty", "tz")
+        return "in_ && " + " && ".join(f"{t3[d]}{ahead if d == zd else ''} < n{k}_{d} - {2 * ((li >> d) & 1)}"
+                                       for d in range(self.nd))
+
+    def plane_loads(self):
+        """(declarations and the first plane's loads, loads of the next plane, their hand-over)"""
+        zd = self.nd - 1
+        first, nxt, hand = [], [], []
+        for lhs, regs in self.regs.items():
+            start, later = [], []
+            for (name, o), r in regs.items():
+                k = self.aidx[name]
+                at = f"{o[0]} + n{k}_0 * ({o[1]} + n{k}_1 * {o[2]})"
+                first.append(f"    E {r} = 0;")
+                start.append(f"{r} = __ldg(&p{k}[{at}]);")
+                up = regs.get((name, o[:zd] + (o[zd] + 1,) + o[zd + 1:]))
+                nxt.append(f"    E N{r} = {up or '0'};")
+                if not up:
+                    later.append(f"N{r} = __ldg(&p{k}[st{k}_ + {at}]);")
+                hand.append(f"    {r} = N{r};")
+            if self.early and lhs == self.early[0]:
+                k, at = self.early[1:]
+                first.append("    E g_ = 0;")
+                start.append(f"g_ = e{k}[{at}];")
+                nxt.append("    E Ng_ = 0;")
+                later.append(f"Ng_ = e{k}[st{k}_ + {at}];")
+                hand.append("    g_ = Ng_;")
+            first.append(f"    if ({self.condition(lhs)}) {{ {' '.join(start)} }}")
+            nxt.append(f"    if ({self.condition(lhs, ' + 1')} && {'xyz'[zd]}n_ < z1_) {{ {' '.join(later)} }}")
+        return first, nxt, hand
+
+    def store(self, name, idx, rhs):
+        o = self.lhs_offset
+        self.emit(f"{self.ref(name, o)} = (E)({rhs.code});")
+        self.written.add(name)
+        return (name, o, rhs)
+
+    def _stmt(self, s, ind):
+        t = s.targets[0] if isinstance(s, ast.Assign) and len(s.targets) == 1 else None
+        if isinstance(s, ast.Pass) or isinstance(s, ast.Return) and s.value is None and s is self.kd.body[-1]:
+            return
+        if not (isinstance(t, ast.Subscript) and isinstance(t.value, ast.Name) and t.value.id.startswith("__lhs_")):
+            raise _NoSweep
+        sel, name = t.value.id[6:], t.slice.id
+        if sel in self.sels and name in self.aidx:
+            li = self.sels[sel]
+            self.lhs = (name, li)
+            self.lhs_offset = tuple((li >> d) & 1 for d in range(self.nd))
+        super()._stmt(s, ind)
+        self.lhs = None
+
+    # ---- reverse sweep
+    def adjoint(self, op, out, ins, aux):
+        if op == "load":
+            name, o = aux
+            k, b = self.aidx[name], f"b{out.code}"
+            if self.is_shared(name):
+                c = self.contribution(name, o)
+                lines = [f"{c} += (E){b};"]
+            else:
+                self.lhs = self.lhs_of[out.code]
+                lines = [f"{self.ref(name, o, 'e')} += (E){b};"]
+                self.lhs = None
+            return lines
+        return super().adjoint(op, out, ins, aux)
+
+    def contribution(self, name, o):
+        o = tuple(o) + (0,) * (3 - len(o))
+        if max(abs(x) for x in o) > 8:
+            raise _NoSweep
+        self.contrib.setdefault(name, set()).add(o)
+        return "c%d_%d_%d_%d" % ((self.aidx[name],) + tuple(x + 8 for x in o))
+
+    def reverse_lines(self):
+        out = []
+        self.contrib = {}
+        for entry in reversed(range(len(self.tape))):
+            f, nodes, store = self.tape[entry]
+            if store is None:
+                raise _NoSweep
+            name, o, rhs = store
+            if name not in self.dup:
+                continue
+            self.fresh = self.only_here(entry)
+            li = sum(x << d for d, x in enumerate(o))
+            self.lhs_of = {n[1].code: (name, li) for n in nodes}
+            self.lhs = (name, li)
+            r = self.ref(name, o, "e")
+            self.lhs = None
+            if len(self.tape) == 1 and self.regs:  # read with the loads of the plane
+                self.early = ((name, li), self.aidx[name], r[r.index("[") + 1:-1])
+                blk = [f"{r} = (E)0;"]
+            else:
+                blk = [f"g_ = {r}; {r} = (E)0;"]
+            if rhs.var:
+                blk.append(self.add(rhs.code, "(R)g_"))
+            for op, out_, ins, aux in reversed(nodes):
+                blk += self.adjoint(op, out_, ins, aux)
+            out += [f"    if ({f}) {{"] + ["        " + x for x in blk] + ["    }"]
+        return out
+
+    def body_lines(self):
+        fw = []
+        for s in self.kd.body:
+            fw += self.stmt(s, 1)
+        self.check_races()
+        rev = self.reverse_lines()
+        # an offset that one value has needs no sum
+        text = "\n".join(rev)
+        for name, offs in self.contrib.items():
+            for o in offs:
+                c = self.contribution(name, o)
+                if text.count(f"{c} += ") == 1:
+                    text = text.replace(f"{c} += ", f"{c} = ")
+        return fw + text.split("\n")
+
+    # ---- sums over the threads of a block and the planes of a chunk
+    def exchange(self, real):
+        """(declarations before the sweep, code at the end of a plane, code after the sweep, buffers)"""
+        es = {"double": 8, "float": 4}[real]
+        pre, put, get, post, nb = [], [], [], [], 0
+        zd = self.nd - 1
+        for name in self.dup:
+            if name not in self.contrib:
+                continue
+            k, offs = self.aidx[name], self.contrib[name]
+
+            def at(dx, dy, dz):
+                return f"e{k} + ({dx} + n{k}_0 * ({dy} + n{k}_1 * {dz}))"
+
+            def off(dx, dy, w):
+                return (dx, dy, w) if self.nd == 3 else (dx, w, 0)
+
+            groups = {}  # sweep offset -> {dy -> [dx]} (dy = 0 in 2-D)
+            for o in offs:
+                groups.setdefault(o[zd], {}).setdefault(o[1] if self.nd == 3 else 0, []).append(o[0])
+            mode_x = [o[0] for o in offs]
+            x0 = max(sorted(set(mode_x)), key=mode_x.count)
+            mode_y = [o[1] for o in offs] if self.nd == 3 else [0]
+            y0 = max(sorted(set(mode_y)), key=mode_y.count)
+            if max(abs(d - x0) for d in mode_x) > 8 or max(abs(d - y0) for d in mode_y) >= self.TY:
+                raise _NoSweep
+            wlo, whi = min(groups), max(groups)
+            for w in range(wlo, whi + 1):
+                q = f"q{k}_{w - wlo}"
+                pre.append(f"    E {q} = 0;")
+                for dy, dxs in sorted(groups.get(w, {}).items()):
+                    h = f"h{k}_{w - wlo}_{dy + 8}"
+
+                    def c(dx):
+                        return self.contribution(name, off(dx, dy, w))
+                    put.append(f"    E {h} = {c(x0) if x0 in dxs else '(E)0'};")
+                    for dx in sorted(dxs):
+                        s = dx - x0
+                        if s == 0:
+                            continue
+                        up = "up" if s > 0 else "down"
+                        put.append(f"    {{ const E r_ = __shfl_{up}_sync(0xFFFFFFFFu, {c(dx)}, {abs(s)}); "
+                                   f"if (lane_ {'>= %d' % s if s > 0 else '< %d' % (32 + s)}) {h} += r_; }}")
+                        if s > 0 and x0 - s in dxs:
+                            continue  # with its mirror image
+                        if x0 - s in dxs:  # both edges of the row in one addition
+                            m = x0 - s
+                            put.append(f"    if (lane_ < {-s} || lane_ >= {32 + s}) {{ const bool l_ = lane_ < {-s}; "
+                                       f"const E v_ = l_ ? {c(dx)} : {c(m)}; "
+                                       f"if (v_ != (E)0) ad_red(l_ ? {at(*off(dx, dy, w))} : {at(*off(m, dy, w))}, v_); }}")
+                        else:
+                            edge = f"lane_ >= {32 - s}" if s > 0 else f"lane_ < {-s}"
+                            put.append(f"    if ({edge} && {c(dx)} != (E)0) ad_red({at(*off(dx, dy, w))}, {c(dx)});")
+                    if dy == y0:
+                        get.append(f"    {q} += {h};")
+                        continue
+                    t = dy - y0  # to the row t further on
+                    put.append(f"    xs_[par_][{nb}][threadIdx.y][lane_] = {h};")
+                    edge = f"threadIdx.y >= {self.TY - t}" if t > 0 else f"threadIdx.y < {-t}"
+                    inside = f"threadIdx.y >= {t}" if t > 0 else f"threadIdx.y < {self.TY + t}"
+                    put.append(f"    if ({edge} && {h} != (E)0) ad_red({at(*off(x0, dy, w))}, {h});")
+                    get.append(f"    if ({inside}) {q} += xs_[par_][{nb}][threadIdx.y - ({t})][lane_];")
+                    nb += 1
+            first = at(*off(x0, y0, wlo))
+            get.append(f"    if (q{k}_0 != (E)0) ad_red({first}, q{k}_0);")
+            for j in range(whi - wlo):
+                get.append(f"    q{k}_{j} = q{k}_{j + 1};")
+                post.append(f"    if (q{k}_{j} != (E)0) ad_red(e{k} + (long long)({j}) * st{k}_ + "
+                            f"({x0} + n{k}_0 * ({off(x0, y0, wlo)[1]} + n{k}_1 * {off(x0, y0, wlo)[2]})), q{k}_{j});")
+            get.append(f"    q{k}_{whi - wlo} = 0;")
+        if 2 * nb * self.TX * self.TY * es > self.SMEM:
+            raise _NoSweep
+        return pre, put, get, post, nb
+
+    def source(self, real):
+        kd, nd = self.kd, self.nd
+        self.reg = "d" if real == "double" else "f"
+        self.collect_temps()
+        self.infer_locals(kd.body)
+        if self.locals:
+            raise _NoSweep
+        body = self.body_lines()
+        pre, put, get, post, nb = self.exchange(real)
+        first, nxt, hand = self.plane_loads()
+        zd = nd - 1
+        decl, step = [], []
+        t0 = ["tx", "ty", "0"] if nd == 3 else ["tx", "0", "0"]
+        t0[zd] = "z0_"
+        for name, k in self.aidx.items():
+            decl.append(f"    const int n{k}_0 = (int)g.n[{k}][0], n{k}_1 = (int)g.n[{k}][1], n{k}_2 = (int)g.n[{k}][2];")
+            decl.append(f"    const int st{k}_ = {f'n{k}_0 * n{k}_1' if nd == 3 else f'n{k}_0'};")
+            decl.append(f"    E* p{k} = (E*)g.a[{k}] + ({t0[0]} + (long long)n{k}_0 * ({t0[1]} + (long long)n{k}_1 * {t0[2]}));")
+            step.append(f"p{k} += st{k}_;")
+        for name in self.dup:
+            k = self.aidx[name]
+            decl.append(f"    E* e{k} = (E*)g.a[{self.didx[name]}] + ({t0[0]} + (long long)n{k}_0 * ({t0[1]} + (long long)n{k}_1 * {t0[2]}));")
+            step.append(f"e{k} += st{k}_;")
+        for name, k in self.sidx.items():
+            ty = "long long" if name in kd.int_scalars else "R"
+            decl.append(f"    {ty} s{k} = ({ty})g.s[{k}];")
+            if ty == "R":  # kept in a register: converted again on every plane it would cost an FP64 instruction each
+                decl.append(f"    asm volatile(\"\" : \"+{self.reg}\"(s{k}));")
+        regs = []
+        init = {"R": "0", "long long": "0", "bool": "false"}
+        for v, ctype in self.vars:
+            regs.append(f"    {ctype} {v} = {init[ctype]};")
+        for v in self.dvars:
+            regs.append(f"    R b{v} = 0;")
+        if not self.early:
+            regs.append("    E g_ = 0;")
+        for name, offs in self.contrib.items():
+            for o in sorted(offs):
+                regs.append(f"    E {self.contribution(name, o)} = 0;")
+        # every thread of the grid stays for the shuffles and barriers: the columns outside the ranges
+        # execute no statement
+        body = [ln.replace("if (", "if (in_ && ", 1) if ln.startswith("    if (tx < ") else ln for ln in body]
+        xs = f"    __shared__ E xs_[2][{nb}][{self.TY}][{self.TX}];\n    int par_ = 0;" if nb else ""
+        sync = ["    __syncthreads();"] if nb else []
+        flip = ["    par_ ^= 1;"] if nb else []
+        zblk = "z" if nd == 3 else "y"
+        yb = "(int)(blockIdx.y * blockDim.y + threadIdx.y)" if nd == 3 else "0"
+        tsweep = "tz" if nd == 3 else "ty"
+        ypos = "\n    const int ty = (int)g.lo[1] + uy;" if nd == 3 else ""
+        return f"""// reverse derivative of parallel {kd.name} ({nd}-D, {real}, sweep) -- generated by ps_gb300.ad
+{self.types(real)}
+struct ps_jit_args {{ void* a[{MAX_ARRAYS}]; long long n[{MAX_ARRAYS}][3]; double s[{MAX_SCALARS}]; long long lo[3]; long long cnt[3]; int* err; long long smem; long long loop; unsigned* ocnt; int ord[10]; }};
+{VALUE_HELPERS}
+__device__ __forceinline__ void ad_red(E* p, E v) {{ asm volatile("red.global.add.{'f64' if real == 'double' else 'f32'} [%0], %1;" :: "l"(__cvta_generic_to_global(p)), "{self.reg}"(v) : "memory"); }}
+extern "C" __global__ void __launch_bounds__({self.TX * self.TY if nd == 3 else 128}) ps_jit_entry(const ps_jit_args g) {{
+{xs}
+    const int lane_ = threadIdx.x & 31;
+    const int ux = (int)(blockIdx.x * blockDim.x + threadIdx.x), uy = {yb};
+    const bool in_ = ux < g.cnt[0]{" && uy < g.cnt[1]" if nd == 3 else ""};
+    const int tx = (int)g.lo[0] + ux;{ypos}
+    const int z0_ = (int)(g.lo[{zd}] + blockIdx.{zblk} * g.loop);
+    const int z1_ = (int)(min((long long)z0_ + g.loop, g.lo[{zd}] + g.cnt[{zd}]));
+{chr(10).join(decl + pre + [ln.replace(f"{tsweep} <", "z0_ <") for ln in first])}
+    for (int {tsweep} = z0_; {tsweep} < z1_; ++{tsweep}) {{
+    const int {'xyz'[zd]}n_ = {tsweep} + 1;
+{chr(10).join(nxt + regs + body + put + sync + get + flip + hand)}
+    {" ".join(step)}
+    }}
+{chr(10).join(post)}
+}}
+"""
+
+    def types(self, real):
+        return _Gen.types(self, real)
+
+
+def sweep_fits(spans, dims, lo, cnt, nd):
+    """Whether every access of a sweep kernel lies in its array, for all points of the box (lo, cnt) at which
+    its statement runs, and 32-bit indices reach every element. spans: (array, left-hand array, its mask,
+    least and largest offsets); dims: array -> extents."""
+    big = 2 ** 31 - 2 ** 20
+    if any(n[0] * n[1] * n[2] >= big for n in dims.values()) or max(lo[d] + cnt[d] for d in range(3)) >= big:
+        return False
+    for name, lhs, li, omin, omax in spans:
+        n, m = dims[name], dims[lhs]
+        for d in range(nd):
+            end = min(lo[d] + cnt[d], m[d] - 2 * ((li >> d) & 1))
+            if end > lo[d] and (lo[d] + omin[d] < 0 or end - 1 + omax[d] >= n[d]):
+                return False
+    return all(lo[d] == 0 for d in range(nd, 3))
+
+
 def generate(kd, ndims, dtype, dup, mode="reverse"):
     """CUDA C of the derivative kernel of `kd` (arrays `dup` duplicated; their shadows follow the
     primal arrays in the argument list)."""
@@ -612,6 +998,46 @@ def _pairs(kernel: JitKernel, args, grad):
             raise ArgumentError(f"∇: {n} appears twice")
         dup[n] = s
     return dup
+
+
+def _handle(kernel, key, source):
+    if key not in kernel._handles:
+        h = ctypes.c_void_p()
+        _lib.call("ps_jit_compile", source().encode(), b"ps_jit_entry", ctypes.byref(h))
+        kernel._handles[key] = h
+    return kernel._handles[key]
+
+
+def generate_sweep(kd, ndims, dtype, dup):
+    """(CUDA C, accesses) of the reverse kernel's sweep form, or None where it does not apply."""
+    try:
+        gen = _AdSweepGen(kd, ndims, set(dup))
+        src = gen.source(dtype)
+    except _NoSweep:
+        return None
+    spans = {}  # (array, left-hand array, its mask) -> least and largest offset per dimension
+    for name, o, lhs, li in gen.access:
+        lo, hi = spans.setdefault((name, lhs, li), (list(o), list(o)))
+        for d in range(3):
+            lo[d], hi[d] = min(lo[d], o[d]), max(hi[d], o[d])
+    return src, [k + v for k, v in sorted(spans.items())]
+
+
+def _sweep_handle(kernel, ndims, dt, order, descs, lo, cnt):
+    """(handle, blocks per SM) of the sweep form for a launch over the box (lo, cnt), or None."""
+    key = ("ad_sweep", tuple(order), ndims, dt)
+    if key not in kernel._sweeps:
+        kernel._sweeps[key] = generate_sweep(kernel.kd, ndims, dt, order)
+    if kernel._sweeps[key] is None:
+        return None
+    src, spans = kernel._sweeps[key][:2]
+    dims = {n: tuple(d.n) for n, d in zip(kernel.kd.arrays, descs)}
+    if not sweep_fits(spans, dims, lo, cnt, ndims):
+        return None
+    h = _handle(kernel, key, lambda: src)
+    if len(kernel._sweeps[key]) == 2:
+        kernel._sweeps[key] += (blocks_per_sm(h, _AdSweepGen.TX * _AdSweepGen.TY if ndims == 3 else 128),)
+    return h, kernel._sweeps[key][2]
 
 
 def parallel_grad(kernel: JitKernel, args, grad, ad_mode="reverse", ranges=None, stream=None, sync=True,
@@ -665,16 +1091,26 @@ def parallel_grad(kernel: JitKernel, args, grad, ad_mode="reverse", ranges=None,
         if min(lo) < 0:
             raise ArgumentError("ranges must start at index 1 or above")
         cnt = [max(0, hi[d] - lo[d]) for d in range(3)]
-    key = ("ad", ad_mode, tuple(order), ndims, dt)
-    if key not in kernel._handles:
-        src = generate(kernel.kd, ndims, dt, order, ad_mode)
-        h = ctypes.c_void_p()
-        _lib.call("ps_jit_compile", src.encode(), b"ps_jit_entry", ctypes.byref(h))
-        kernel._handles[key] = h
-    h = kernel._handles[key]
+    h = None
+    loop = [1, 1, 1]
+    # FP32 sweeps: 192^3 477 us per launch with one point per thread, 100 so; 2-D 4096^2 994, 111. In FP64 both
+    # forms are bound by the FP64 pipe, where the sweep's own sums cost more than the additions they save
+    # (200^3: 1.90 ms against 1.41). Below SWEEP_MIN points a launch is shorter than its way through the
+    # host, which the sweep's checks make longer (24 x 30 x 26: 58 us without them, 68 with).
+    if ad_mode == "reverse" and dt == "float" and nthreads is None and nblocks is None and ndims in (2, 3) and \
+            cnt[0] * cnt[1] * cnt[2] >= SWEEP_MIN:
+        h = _sweep_handle(kernel, ndims, dt, order, descs, lo, cnt)
+        if h is not None:
+            h, resident = h
+            threads = [_AdSweepGen.TX, _AdSweepGen.TY, 1] if ndims == 3 else [128, 1, 1]
+            cols = -(-cnt[0] // threads[0]) * (-(-cnt[1] // threads[1]) if ndims == 3 else 1)
+            loop[ndims - 1] = sweep_chunk(cnt[ndims - 1], max(1, cols), resident, 3, 256)
+    if h is None:
+        h = _handle(kernel, ("ad", ad_mode, tuple(order), ndims, dt),
+                    lambda: generate(kernel.kd, ndims, dt, order, ad_mode))
     alld = descs + sdescs
     A = (PSArray * len(alld))(*alld)
     S = (ctypes.c_double * max(1, len(scal)))(*[float(x) for x in scal])
     _lib.call("ps_jit_launch_ex", h, A, len(alld), S, len(scal), (ctypes.c_int64 * 3)(*lo),
-              (ctypes.c_int64 * 3)(*cnt), (ctypes.c_int32 * 3)(*threads), 0, (ctypes.c_int32 * 3)(1, 1, 1),
+              (ctypes.c_int64 * 3)(*cnt), (ctypes.c_int32 * 3)(*threads), 0, (ctypes.c_int32 * 3)(*loop),
               stream_handle(stream), int(bool(sync)))

@@ -40,6 +40,7 @@ from __future__ import annotations
 import ast
 import copy
 import ctypes
+import functools
 import io
 import numbers
 import re
@@ -60,6 +61,7 @@ _lib.register("ps_jit_launch_ex", [ctypes.c_void_p, ctypes.POINTER(PSArray), cty
                                    ctypes.POINTER(ctypes.c_double), ctypes.c_int32, ctypes.POINTER(ctypes.c_int64),
                                    ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int32), ctypes.c_int64,
                                    ctypes.POINTER(ctypes.c_int32), ctypes.c_void_p, ctypes.c_int])
+_lib.register("ps_jit_blocks_per_sm", [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.POINTER(ctypes.c_int32)])
 _lib.register("ps_jit_hide_communication", [ctypes.c_void_p, ctypes.POINTER(PSArray), ctypes.c_int32,
                                             ctypes.POINTER(ctypes.c_double), ctypes.c_int32,
                                             ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int32),
@@ -74,7 +76,8 @@ _lib.register("ps_jit_destroy", [ctypes.c_void_p])
 
 MAX_ARRAYS = MAX_SCALARS = 32
 TMA_RING_BYTES = 64 * 1024  # shared memory for the plane ring of a TMA sweep (sets the planes in flight)
-RESIDENT_THREADS = 152 * 2048  # threads a GB300 holds at once (152 SMs x 2048)
+SMS = 152
+RESIDENT_THREADS = SMS * 2048  # threads a GB300 holds at once (152 SMs x 2048)
 # kernel-language macros (src/ParallelKernel/kernel_language.jl): a kernel that uses any of them
 # keeps one point per thread (a sweep would change what @threadIdx, @sharedMem and barriers see)
 _KERNEL_LANGUAGE = {"__m_" + m for m in ("threadIdx", "blockIdx", "blockDim", "gridDim", "sharedMem", "sync_threads",
@@ -439,6 +442,42 @@ def parse(src: str) -> KernelDef:
 # ---- code generation -----------------------------------------------------------------------
 def _lit(v):
     return f"((R){float(v)!r})"
+
+
+# Julia's max / min and Bool * number on the kernel's type
+VALUE_HELPERS = r"""template <typename T> struct jl_f64 { static constexpr bool v = false; };
+template <> struct jl_f64<double> { static constexpr bool v = true; };
+template <typename T> struct jl_f32 { static constexpr bool v = false; };
+template <> struct jl_f32<float> { static constexpr bool v = true; };
+__device__ __forceinline__ long long jl_key(long long b) { return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFLL); }
+__device__ __forceinline__ bool jl_nanb(long long b) { return (b & 0x7FFFFFFFFFFFFFFFLL) > 0x7FF0000000000000LL; }
+// Julia's max / min (NaN-propagating, -0.0 < 0.0); doubles compare as integer keys (the FP64 pipe is slow)
+// and a NaN operand is returned itself; floats use max.NaN / min.NaN (the same bits as the subtraction
+// form, whose NaN is the canonical one)
+template <typename T>
+__device__ __forceinline__ T jl_maxt(T x, T y) {
+    if constexpr (jl_f64<T>::v) {
+        const long long bx = __double_as_longlong(x), by = __double_as_longlong(y);
+        const T r = jl_key(bx) >= jl_key(by) ? x : y;
+        return jl_nanb(bx) ? x : jl_nanb(by) ? y : r;
+    } else if constexpr (jl_f32<T>::v) {
+        float d; asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(x), "f"(y)); return d;
+    } else { T d = x - y; T r = signbit(d) ? y : x; return (isnan(x) || isnan(y)) ? d : r; }
+}
+template <typename T>
+__device__ __forceinline__ T jl_mint(T x, T y) {
+    if constexpr (jl_f64<T>::v) {
+        const long long bx = __double_as_longlong(x), by = __double_as_longlong(y);
+        const T r = jl_key(bx) < jl_key(by) ? x : y;
+        return jl_nanb(bx) ? x : jl_nanb(by) ? y : r;
+    } else if constexpr (jl_f32<T>::v) {
+        float d; asm("min.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(x), "f"(y)); return d;
+    } else { T d = x - y; T r = signbit(d) ? x : y; return (isnan(x) || isnan(y)) ? d : r; }
+}
+__device__ __forceinline__ R jl_max(R x, R y) { return jl_maxt<R>(x, y); }
+__device__ __forceinline__ R jl_min(R x, R y) { return jl_mint<R>(x, y); }
+__device__ __forceinline__ R jl_bmul(bool b, R x) { return b ? x : copysign((R)0, x); }
+"""
 
 
 class _Gen:
@@ -1227,39 +1266,7 @@ __device__ __forceinline__ void jl_sts(E* a, long long n0, long long n1, long lo
     const long long l = i + n0 * (j + n1 * k);
     if (a && jl_in(n0, n1, n2, i, j, k) && l < cap) a[l] = v; else atomicOr(err, 1); }}
 __device__ __forceinline__ unsigned jl_laneid() {{ unsigned l; asm volatile("mov.u32 %0, %%laneid;" : "=r"(l)); return l; }}
-template <typename T> struct jl_f64 {{ static constexpr bool v = false; }};
-template <> struct jl_f64<double> {{ static constexpr bool v = true; }};
-template <typename T> struct jl_f32 {{ static constexpr bool v = false; }};
-template <> struct jl_f32<float> {{ static constexpr bool v = true; }};
-__device__ __forceinline__ long long jl_key(long long b) {{ return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFLL); }}
-__device__ __forceinline__ bool jl_nanb(long long b) {{ return (b & 0x7FFFFFFFFFFFFFFFLL) > 0x7FF0000000000000LL; }}
-// Julia's max / min (NaN-propagating, -0.0 < 0.0); doubles compare as integer keys (the FP64 pipe is slow)
-// and a NaN operand is returned itself; floats use max.NaN / min.NaN (the same bits as the subtraction
-// form, whose NaN is the canonical one)
-template <typename T>
-__device__ __forceinline__ T jl_maxt(T x, T y) {{
-    if constexpr (jl_f64<T>::v) {{
-        const long long bx = __double_as_longlong(x), by = __double_as_longlong(y);
-        const T r = jl_key(bx) >= jl_key(by) ? x : y;
-        return jl_nanb(bx) ? x : jl_nanb(by) ? y : r;
-    }} else if constexpr (jl_f32<T>::v) {{
-        float d; asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(x), "f"(y)); return d;
-    }} else {{ T d = x - y; T r = signbit(d) ? y : x; return (isnan(x) || isnan(y)) ? d : r; }}
-}}
-template <typename T>
-__device__ __forceinline__ T jl_mint(T x, T y) {{
-    if constexpr (jl_f64<T>::v) {{
-        const long long bx = __double_as_longlong(x), by = __double_as_longlong(y);
-        const T r = jl_key(bx) < jl_key(by) ? x : y;
-        return jl_nanb(bx) ? x : jl_nanb(by) ? y : r;
-    }} else if constexpr (jl_f32<T>::v) {{
-        float d; asm("min.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(x), "f"(y)); return d;
-    }} else {{ T d = x - y; T r = signbit(d) ? x : y; return (isnan(x) || isnan(y)) ? d : r; }}
-}}
-__device__ __forceinline__ R jl_max(R x, R y) {{ return jl_maxt<R>(x, y); }}
-__device__ __forceinline__ R jl_min(R x, R y) {{ return jl_mint<R>(x, y); }}
-__device__ __forceinline__ R jl_bmul(bool b, R x) {{ return b ? x : copysign((R)0, x); }}
-extern "C" __global__ void {bounds}ps_jit_entry({'const __grid_constant__ ps_jit_targs t_' if self.tma else 'const ps_jit_args g'}) {{
+{VALUE_HELPERS}extern "C" __global__ void {bounds}ps_jit_entry({'const __grid_constant__ ps_jit_targs t_' if self.tma else 'const ps_jit_args g'}) {{
     extern __shared__ __align__({128 if self.tma else 16}) unsigned char ps_smem[];
 {'    const ps_jit_args& g = t_.g;' + chr(10) if self.tma else ''}{head}    const long long {udecl};
 {guard}
@@ -1270,6 +1277,32 @@ extern "C" __global__ void {bounds}ps_jit_entry({'const __grid_constant__ ps_jit
 {zpost}
 {tail}}}
 """
+
+
+def blocks_per_sm(handle, threads, shmem=0):
+    """Blocks of a compiled kernel that one SM holds at once."""
+    n = ctypes.c_int32()
+    _lib.call("ps_jit_blocks_per_sm", handle, int(threads), int(shmem), ctypes.byref(n))
+    return max(1, n.value)
+
+
+@functools.lru_cache(maxsize=256)
+def sweep_chunk(n, columns, resident, start, most=64):
+    """Indices per thread of a sweep over n of them, `columns` blocks beside each other, `resident` blocks of it
+    on an SM: a launch takes as long as its fullest SM, so it is the length for which the number of
+    waves times the indices of a block (and `start` more for its first loads and its ends) is the least;
+    the longest of equals, at most `most`. A fixed length leaves a last wave nearly empty at some
+    sizes (480 blocks of 64 planes on 456 places take twice the time of one wave)."""
+    best = None
+    for chunks in range(-(-n // most), n + 1):
+        ls = -(-n // chunks)
+        waves = -(-columns * -(-n // ls) // (SMS * resident))
+        cost = waves * (ls + start)
+        if best is None or cost < best[0]:
+            best = (cost, ls)
+        if ls <= 2 or waves > 16:  # many waves: no better for shorter ones
+            break
+    return best[1] if best else 1
 
 
 class _NoTma(Exception):
@@ -1461,6 +1494,7 @@ class JitKernel:
         self._kernel_language = uses_kernel_language(self.kd)
         self.name, self.nargs = self.kd.name, len(self.kd.args)
         self._handles = {}
+        self._sweeps = {}  # sweep forms of the reverse kernel (ps_gb300.ad)
         self._collective = {}
         self._layouts = {}  # TMA stage layout of each TMA-variant handle (None: the plain sweep was generated)
 

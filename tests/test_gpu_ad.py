@@ -179,3 +179,64 @@ def test_misfit_gradient_32_through_generated_reverse_kernels(ps):
         ps.parallel(k, scratch, states[s], Ci, lam, dt, *h, grad=((scratch, lamb), (states[s], Tb), (lam, glam)))
         lamb.add_(Tb)
     assert _rel(ps.to_host(glam), ps.to_host(g_h)) <= 1e-10
+
+
+_SWEPT = {  # source, dimensions, arrays (one point shorter: True), differentiated arrays, scalars
+    "flux_lam": (K.KERNELS["diffusion_flux_lam"][0], 3, {"T2": False, "T": False, "Ci": False, "lam": False},
+                 ("T2", "T", "lam"), (0.01, 1.3, 0.9, 1.1)),
+    "corners": ("""@parallel function c!(R, S, A, B, c)
+    @all(R) = @av(A) * @d_xa(B) + c*@av(B)
+    @all(S) = @all(R) * @av_yza(B) - @d_xa(A)
+    return
+end""", 3, {"R": True, "S": True, "A": False, "B": False}, ("R", "S", "A", "B"), (0.4,)),
+    "heat_2d": ("""@parallel function h!(T2, T, K, Ci, dt)
+    @all(qx) = -@av_xi(K)*@d_xi(T)
+    @all(qy) = -@av_yi(K)*@d_yi(T)
+    @inn(T2) = @inn(T) - dt*@inn(Ci)*(@d_xa(qx) + @d_ya(qy))
+    return
+end""", 2, {"T2": False, "T": False, "K": False, "Ci": False}, ("T2", "T", "K"), (0.1,)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(_SWEPT))
+@pytest.mark.parametrize("n", [(3, 3, 3), (34, 10, 5), (35, 9, 41), (64, 17, 4), (31, 33, 300), (130, 5, 7)])
+def test_reverse_sweep_equals_one_point_per_thread(ps, monkeypatch, name, n, dtype=np.float32):
+    """The reverse kernel's sweep form (the default in FP32) against one point per thread (`nthreads` given): blocks,
+    rows and chunks of the sweep that end inside and at their edges, parts of the box, columns without a
+    statement. Primal stores and taken shadows are the same bytes; an element's sum of at most 27
+    contributions differs by at most 2 * 27 roundings of partial sums, taken as within twice the largest
+    result: 128 * eps of it."""
+    monkeypatch.setattr(ps.ad, "SWEEP_MIN", 0)
+    src, nd, short, dup, scal = _SWEPT[name]
+    n = n[:nd]
+    rng = np.random.default_rng(sum(n))
+    size = {a: tuple(m - s for m in n) for a, s in short.items()}
+    host = {a: np.asfortranarray((0.5 + rng.random(size[a])).astype(dtype)) for a in short}
+    sh = {a: np.asfortranarray(rng.standard_normal(size[a]).astype(dtype)) for a in dup}
+    taken = [a for a in dup if a in ("T2", "R", "S")]
+    for ranges in (None, [(1, max(1, m - 2)) for m in n], [(2, m) for m in n]):
+        got = []
+        for nt in (None, (32, 8, 1)):
+            k = ps.parallel_kernel(src, nd)
+            dev = {a: ps.from_host(host[a]) for a in short}
+            shd = {a: ps.from_host(sh[a]) for a in dup}
+            ps.parallel(k, *dev.values(), *scal, grad=tuple((dev[a], shd[a]) for a in dup), ranges=ranges, nthreads=nt)
+            assert any(h[0] == ("ad" if nt else "ad_sweep") for h in k._handles)
+            got.append(({a: ps.to_host(dev[a]) for a in short}, {a: ps.to_host(shd[a]) for a in dup}))
+        for a in short:
+            assert np.array_equal(got[0][0][a], got[1][0][a]), (a, ranges)
+        for a in dup:
+            if a in taken:
+                assert np.array_equal(got[0][1][a], got[1][1][a]), (a, ranges)
+            else:
+                assert _rel(got[0][1][a], got[1][1][a]) <= 128 * np.finfo(dtype).eps, (a, ranges)
+
+
+def test_reverse_out_of_bounds_is_reported(ps, monkeypatch):
+    """A kernel that reads past an array keeps the checked form and its error (the sweep form checks nothing)."""
+    monkeypatch.setattr(ps.ad, "SWEEP_MIN", 0)
+    k = ps.parallel_kernel(_SWEPT["corners"][0], 3)
+    a = {x: ps.from_host(np.ones((8, 7, 6), np.float32, order="F")) for x in "RSAB"}
+    with pytest.raises(Exception, match="out-of-bounds"):
+        ps.parallel(k, *a.values(), 0.5, grad=((a["A"], ps.from_host(np.ones((8, 7, 6), np.float32, order="F"))),))
+    assert ("ad_sweep", ("A",), 3, "float") not in k._handles
