@@ -152,6 +152,11 @@ int ps_jit_blocks_per_sm(void* kernel, int32_t threads, int64_t shmem, int32_t* 
     int dev = -1, n = 0;
     cudaGetDevice(&dev);
     if (dev != k->device) return fail(PS_ERR_ARG, "ps_jit_blocks_per_sm: kernel compiled for device %d", k->device);
+    if (shmem > k->smem_opt_in) {
+        if (g_setattr(k->fn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)shmem) != CUDA_SUCCESS)
+            return fail(PS_ERR_ARG, "ps_jit_blocks_per_sm: %lld bytes of dynamic shared memory not available", (long long)shmem);
+        k->smem_opt_in = (int)shmem;
+    }
     const CUresult r = g_occupancy(&n, k->fn, threads, (size_t)shmem);
     if (r != CUDA_SUCCESS) return fail(PS_ERR_CUDA, "ps_jit_blocks_per_sm: the occupancy query failed (CUresult %d)", (int)r);
     *blocks = n;

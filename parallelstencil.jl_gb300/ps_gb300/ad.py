@@ -1104,7 +1104,7 @@ def parallel_grad(kernel: JitKernel, args, grad, ad_mode="reverse", ranges=None,
             h, resident = h
             threads = [_AdSweepGen.TX, _AdSweepGen.TY, 1] if ndims == 3 else [128, 1, 1]
             cols = -(-cnt[0] // threads[0]) * (-(-cnt[1] // threads[1]) if ndims == 3 else 1)
-            loop[ndims - 1] = sweep_chunk(cnt[ndims - 1], max(1, cols), resident, 3, 256)
+            loop[ndims - 1] = sweep_chunk(cnt[ndims - 1], max(1, cols), resident, 3)
     if h is None:
         h = _handle(kernel, ("ad", ad_mode, tuple(order), ndims, dt),
                     lambda: generate(kernel.kd, ndims, dt, order, ad_mode))

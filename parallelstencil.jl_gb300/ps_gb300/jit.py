@@ -513,6 +513,11 @@ class _Gen:
         self.tma = bool(tma) and self.zloop and ndims == 3 and not self.ordered
         self.staged = {}
         self.layout = None
+        # a body of FD statements alone (all that definitions of this kind usually have) runs statement by
+        # statement over a thread's columns, with 32-bit indices (see tma_resolve)
+        self.flat = self.tma and all(_is_sel_assign(x) or isinstance(x, ast.Pass) or
+                                     (isinstance(x, ast.Return) and x.value is None and x is kd.body[-1]) for x in kd.body)
+        self.flat_stmts = []
         written = set()
         for n in ast.walk(ast.Module(body=kd.body, type_ignores=[])):
             if isinstance(n, ast.Assign):
@@ -603,6 +608,12 @@ class _Gen:
             if ro and (name, along(o, -1)) in keys:
                 self.persist.append(f"    R P{j}_{var[1:]} = 0;")
                 ups.append(f"{p}    P{j}_{var[1:]} = {var};")
+        if self.flat:
+            def part(c, z):
+                return " && ".join(x for x in c.split(" && ") if x and x.startswith("tz") == z) or "true"
+            box = box if self.checked else ""
+            self.flat_stmts.append((part(cond, False), part(cond, True), part(box, False), part(box, True), loads + [store]))
+            return []
         self.persist.append(f"    bool pr{j} = false;")
         inner = loads + [store] + ups + [f"{p}    pr{j} = true;"]
         if not self.checked or not box:
@@ -789,12 +800,12 @@ class _Gen:
                 a, d = e.args
                 if a.id in self.shared:
                     return f"sm{self.shared[a.id]}_n{int(d.value) - 1}"
-                return f"n{self.aidx[a.id]}_{int(d.value) - 1}"
+                return f"{'(long long)' if self.flat else ''}n{self.aidx[a.id]}_{int(d.value) - 1}"
             if f == "sizeof":  # sizeof(eltype(A)): bytes per element of the kernel's number type
                 return "((long long)sizeof(E))"
             if f == "length" and e.args[0].id in self.aidx:
                 k = self.aidx[e.args[0].id]
-                return f"(n{k}_0 * n{k}_1 * n{k}_2)"
+                return f"({'(long long)' if self.flat else ''}n{k}_0 * n{k}_1 * n{k}_2)"
             if f in ("max", "min"):
                 if self.etype(e) == "int":
                     r = E(e.args[0], "int")
@@ -1085,7 +1096,8 @@ class _Gen:
         smem = stages * off + 8 * stages
         if smem > 200 * 1024:
             raise _NoTma()
-        return {"arrays": arrays, "zl": zl, "span": span, "stages": stages, "stage": off, "smem": smem, "xc": xc,
+        ry = 2 if self.flat and es == 4 else 1  # rows per thread: their values share loads and the step's overhead
+        return {"arrays": arrays, "zl": zl, "span": span, "stages": stages, "stage": off, "smem": smem, "xc": xc, "ry": ry,
                 "tx_bytes": sum(a["bx"] * a["by"] * es for a in arrays)}
 
     def tma_resolve(self, body):
@@ -1097,14 +1109,70 @@ class _Gen:
         def sub(m):
             k, ox, oy, oz = (int(x) for x in m.groups())
             a = by_k[k]
-            return (f"((const E*)(jt_p{oz - L['zl']} + {a['off']}))[(threadIdx.y + {oy - a['ys']}) * {a['bx']} + "
+            return (f"((const E*)(jt_p{oz - L['zl']} + {a['off']}))[(jt_ly + {oy - a['ys']}) * {a['bx']} + "
                     f"(jt_lx + {ox - a['xs']})]")
         pat = re.compile(r"__TMA\[(\d+),(-?\d+),(-?\d+),(-?\d+)\]__")
-        head = ["    if (!jt_to) {", "    #pragma unroll",
+        if self.flat:
+            return self.tma_flat(lambda line: pat.sub(sub, line))
+        head = ["    const int jt_ly = (int)threadIdx.y;", "    if (!jt_to) {", "    #pragma unroll",
                 f"    for (int jt_xc = 0; jt_xc < {L['xc']}; ++jt_xc) {{",
                 "    const int jt_lx = (int)threadIdx.x + 32 * jt_xc;  // this cell's column in the block's tile",
                 "    const long long tx = (long long)jt_x0 + jt_lx;"]
         return head + [pat.sub(sub, line) for line in body] + ["    }", "    }"]
+
+    def tma_flat(self, resolve):
+        """The statements over a thread's cells (xc columns 32 apart, ry rows). What limits this kernel is its
+        instructions (the flux step, 384 x 320 x 256 FP32: 126 per cell, 174 us, against 74 of memory time),
+        and half of them were 64-bit indices and the 64-bit comparisons of masks and bounds for each cell. So
+        each statement tests its x and y conditions once before the sweep (a bit per cell), its z ones once
+        per step; arrays outside the ring are reached from a pointer to the thread's point of the plane;
+        all cells of a thread are computed without branches between them -- the ring holds the stencils of
+        every cell of a block, with zeros from outside the arrays -- and stored where they run; and two rows
+        per thread share their y loads and fluxes and the step's own instructions. 64 per cell, 88 us (one row
+        per thread 7 % more, four 28 %; one and three planes in flight instead of two 3 % and 12 %)."""
+        xc, ry = self.layout["xc"], self.layout["ry"]
+        cells = xc * ry
+        used = set()
+        ref = re.compile(r"a(\d+)\[\(tx\+(-?\d+)\) \+ n\1_0 \* \(\(ty\+(-?\d+)\) \+ n\1_1 \* \(tz\+(-?\d+)\)\)\]")
+
+        def place(m):
+            used.add(m.group(1))
+            k, ox, oy, oz = m.groups()
+            return f"b{k}_[{ox} + 32 * jt_xc + n{k}_0 * ({oy} + jt_r + n{k}_1 * {oz})]"
+        pre, out = [], ["    if (!jt_to) {"]
+        cell = ["    const int jt_xc = jt_c %% %d, jt_r = jt_c / %d, jt_lx = (int)threadIdx.x + 32 * jt_xc, "
+                "jt_ly = (int)threadIdx.y * %d + jt_r;" % (xc, xc, ry),
+                "    const int tx = jt_x0 + jt_lx, ty = jt_y0 + jt_ly; (void)tx; (void)ty;"]
+        loop = f"    for (int jt_c = 0; jt_c < {cells}; ++jt_c) {{"
+        for j, (cxy, cz, bxy, bz, lines) in enumerate(self.flat_stmts):
+            lines = [resolve(ref.sub(place, ln)) for ln in lines]
+            if any(re.search(r"\ba\d+\[", ln) for ln in lines):
+                raise _NoTma()  # an access outside the thread's neighbourhood
+            lhs, eq, rhs = lines[-1].strip().partition(" = ")
+            val, semi, chk = rhs.partition(";")  # "(E)(value)" and, in split FP64, its range check
+            pre += [f"    unsigned ok{j}_ = 0u, bad{j}_ = 0u;  // cells that run / whose stencil leaves an array",
+                    "    #pragma unroll", loop] + cell + \
+                   [f"    if ({cxy}) {{ if ({bxy}) ok{j}_ |= 1u << jt_c; else bad{j}_ |= 1u << jt_c; }}", "    }"]
+            out += [f"    if ({cz}) {{", f"    const bool in_ = {bz};",
+                    f"    const unsigned m_ = in_ ? ok{j}_ : 0u;",
+                    f"    if (in_ ? bad{j}_ : ok{j}_ | bad{j}_) atomicOr(g.err, 1);",
+                    f"    const bool all_ = m_ == {(1 << cells) - 1}u;"]
+            value = lines[:-1] + [f"    o_[jt_c] = {val};{chk}"]
+            if any(re.search(r"\bb\d+_\[", ln) for ln in lines[:-1]):  # reads a written array: only where it runs
+                value = ["    if (all_ || m_ >> jt_c & 1u) {"] + value + ["    }"]
+            # the ring holds (zeros from outside the arrays in) the stencils of all cells of a block
+            out += ["    if (m_) {", f"    E o_[{cells}];", "    #pragma unroll", loop] + cell + value + \
+                   ["    }", "    if (all_) {", "    #pragma unroll", loop] + cell + [f"    {lhs} = o_[jt_c];", "    }",
+                    "    } else {", "    #pragma unroll", loop] + cell + [f"    if (m_ >> jt_c & 1u) {lhs} = o_[jt_c];", "    }",
+                    "    }", "    }", "    }"]
+        out.append("    }")
+        for k in sorted(used):
+            pre += [f"    const long long pl{k}_ = (long long)n{k}_0 * n{k}_1;",
+                    f"    E* b{k}_ = a{k} + (jt_x0 + (int)threadIdx.x + "
+                    f"(long long)n{k}_0 * (jt_y0 + (int)threadIdx.y * {ry}) + pl{k}_ * jt_z0);"]
+            out.append(f"    b{k}_ += pl{k}_;")
+        self.flat_pre = pre
+        return out
 
     def tma_loop(self):
         """Guard, loop head and loop tail of the TMA sweep: thread 0 keeps a ring of `stages` planes
@@ -1125,7 +1193,7 @@ class _Gen:
         zpre = "\n" + "\n".join(self.persist) + f"""
     unsigned long long* const jt_bar = reinterpret_cast<unsigned long long*>(ps_smem + {S} * {L['stage']});
     const int jt_tid = threadIdx.y * 32 + threadIdx.x;
-    const int jt_x0 = (int)blockIdx.x * {32 * L['xc']}, jt_y0 = (int)blockIdx.y * {self.TMA_TY};
+    const int jt_x0 = (int)blockIdx.x * {32 * L['xc']}, jt_y0 = (int)blockIdx.y * {self.TMA_TY}; (void)uy;
     const int jt_z0 = (int)(blockIdx.z * g.loop);
     const int jt_nk = (int)min(g.loop, g.cnt[2] - (long long)jt_z0), jt_nq = jt_nk + {SP - 1};
     int jt_issued = 0;
@@ -1146,11 +1214,11 @@ class _Gen:
         if (!jt_to) jt_to = !jt_wait(jt_bar + c_, 0u);
         jt_ph ^= 1u << c_;
     }}
+{chr(10).join(self.flat_pre) if self.flat else ''}
     int jt_s = 0;  // stage of plane it_
     int jt_w = {SP - 1};  // stage of the plane this step waits for: it_ + {SP - 1}
     for (int it_ = 0; it_ < jt_nk; ++it_) {{
-    const long long uz = (long long)jt_z0 + it_;
-    const long long tz = uz;
+    const {"int" if self.flat else "long long"} tz = jt_z0 + it_;
     if (!jt_to) jt_to = !jt_wait(jt_bar + jt_w, (jt_ph >> jt_w) & 1u);
     jt_ph ^= 1u << jt_w;
 {planes}"""
@@ -1196,10 +1264,13 @@ class _Gen:
         decl = ["    bool big_ = false;"] if self.split else []
         for name, k in self.aidx.items():
             decl.append(f"    E* const a{k} = (E*)g.a[{k}];")
-            decl.append(f"    const long long n{k}_0 = g.n[{k}][0], n{k}_1 = g.n[{k}][1], n{k}_2 = g.n[{k}][2];")
+            it, ic = ("int", "(int)") if self.flat else ("long long", "")
+            decl.append(f"    const {it} n{k}_0 = {ic}g.n[{k}][0], n{k}_1 = {ic}g.n[{k}][1], n{k}_2 = {ic}g.n[{k}][2];")
         for name, k in self.sidx.items():
             if name in kd.int_scalars:
                 decl.append(f"    const long long s{k} = (long long)g.s[{k}];")
+            elif real == "float" and self.zloop:  # converted once: the compiler would do it again at every index
+                decl.append(f"    R s{k} = (R)g.s[{k}];\n    asm volatile(\"\" : \"+f\"(s{k}));")
             else:
                 decl.append(f"    const R s{k} = {self.wrap(f'g.s[{k}]') if self.split else f'(R)g.s[{k}]'};")
         for name, t in self.locals.items():
@@ -1236,7 +1307,7 @@ class _Gen:
             zpost = "    }"
         if self.tma:
             guard, zpre, zpost = self.tma_loop()
-        pos = "const long long " + ", ".join(f"{t[d]} = g.lo[{d}] + {u[d]}" for d in grid)
+        pos = "(void)ux" if self.flat else "const long long " + ", ".join(f"{t[d]} = g.lo[{d}] + {u[d]}" for d in grid)
         # the boundary-first variant: the body in a block that a finished thread jumps past, then the count
         head = "    const uint3 bi = jl_block(g);\n    {\n" if self.ordered else ""
         # the ordered block index and the count raise register use (56 -> 72 for the diffusion step in
@@ -1287,20 +1358,21 @@ def blocks_per_sm(handle, threads, shmem=0):
 
 
 @functools.lru_cache(maxsize=256)
-def sweep_chunk(n, columns, resident, start, most=64):
+def sweep_chunk(n, columns, resident, start, most=256):
     """Indices per thread of a sweep over n of them, `columns` blocks beside each other, `resident` blocks of it
-    on an SM: a launch takes as long as its fullest SM, so it is the length for which the number of
-    waves times the indices of a block (and `start` more for its first loads and its ends) is the least;
-    the longest of equals, at most `most`. A fixed length leaves a last wave nearly empty at some
-    sizes (480 blocks of 64 planes on 456 places take twice the time of one wave)."""
+    on an SM: a launch takes as long as its fullest SM, so it is the length for which that SM's rounds of
+    blocks, times the indices of a block and `start` more for its first loads and its ends, are the least;
+    the longest of equals, at most `most`. A fixed length leaves a round nearly empty at some sizes
+    (384 x 320 x 256 FP32, 120 columns, three blocks on an SM: 132 us with 64 indices, 99 with the 37
+    chosen here)."""
     best = None
     for chunks in range(-(-n // most), n + 1):
         ls = -(-n // chunks)
-        waves = -(-columns * -(-n // ls) // (SMS * resident))
-        cost = waves * (ls + start)
+        rounds = -(-columns * -(-n // ls) // (SMS * resident))
+        cost = rounds * (ls + start)
         if best is None or cost < best[0]:
             best = (cost, ls)
-        if ls <= 2 or waves > 16:  # many waves: no better for shorter ones
+        if ls <= 2 or rounds > 16:  # many rounds: no better for shorter ones
             break
     return best[1] if best else 1
 
@@ -1531,9 +1603,10 @@ class JitKernel:
                                                                              memopt, loopsize, fp64, allow_tma=True)
         if layout is not None:  # the 3-D sweep with its stencil arrays staged by TMA
             maps = [x for a in layout["arrays"] for x in (a["k"], a["bx"], a["by"])]
-            cnt_t = [-(-cnt[0] // layout["xc"]), cnt[1], cnt[2]]  # threads in x: each covers xc columns
+            # threads in x and y: each covers xc columns and ry rows
+            cnt_t = [-(-cnt[0] // layout["xc"]), -(-cnt[1] // layout["ry"]), cnt[2]]
             _lib.call("ps_jit_launch_tma", h, A, nA, S, nS, (ctypes.c_int64 * 3)(*cnt_t),
-                      (ctypes.c_int32 * 3)(32, _Gen.TMA_TY, 1), int(layout["smem"]), int(loop[2]),
+                      (ctypes.c_int32 * 3)(32, _Gen.TMA_TY // layout["ry"], 1), int(layout["smem"]), int(loop[2]),
                       (ctypes.c_int32 * len(maps))(*maps), len(layout["arrays"]), stream_handle(stream),
                       int(bool(sync)))
             self.tma_launches += 1
@@ -1626,8 +1699,13 @@ class JitKernel:
             es = 8 if dt == "double" else 4
             ht = self._handle(ndims, dt, zl, sp, False, tma=True)
             layout = self._layouts[(ndims, dt, zl, sp, "tma")]
-            if layout is not None and all(not ((d.ptr or 0) % 16 or (d.n[0] * es) % 16 or (d.n[0] * d.n[1] * es) % 16)
+            if layout is not None and all(n < 2 ** 31 - 2 ** 16 for d in descs for n in (*d.n, 8 * d.n[0] * d.n[1])) and all(not ((d.ptr or 0) % 16 or (d.n[0] * es) % 16 or (d.n[0] * d.n[1] * es) % 16)
                                           for d in (descs[a["k"]] for a in layout["arrays"])):
+                if not loopsize and "loopsize" not in self.kd.options:
+                    if "resident" not in layout:
+                        layout["resident"] = blocks_per_sm(ht, 32 * _Gen.TMA_TY // layout["ry"], layout["smem"])
+                    cols = -(-cnt[0] // (32 * layout["xc"])) * -(-cnt[1] // _Gen.TMA_TY)
+                    loop[2] = sweep_chunk(max(1, cnt[2]), max(1, cols), layout["resident"], layout["span"])
                 return ht, A, len(descs), S, len(scal), lo, cnt, threads, shmem, loop, layout
         h = self._handle(ndims, dt, zl, sp, ordered)
         if self._collective[(ndims, dt, zl, sp) + (("ordered",) if ordered else ())] and \
