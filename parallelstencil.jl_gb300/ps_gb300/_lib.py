@@ -125,4 +125,6 @@ def check(rc: int) -> None:
 
 
 def call(name: str, *args) -> None:
-    check(getattr(load(), name)(*args))
+    rc = getattr(_lib or load(), name)(*args)
+    if rc != PS_OK:
+        raise PSError(rc, last_error())

@@ -36,9 +36,9 @@ import re
 
 from . import _lib
 from ._lib import PSArray
-from .core import ArgumentError, descriptor, require_initialized, stream_handle
+from .core import ArgumentError, describe, require_initialized, stream_handle
 from .fd import AV, DIFF, DIFF2, HARM, MAXLOC, MINLOC, SEL
-from .jit import (MAX_ARRAYS, MAX_SCALARS, VALUE_HELPERS, _MATH, JitKernel, _Gen, _lit, array_ndims, blocks_per_sm,
+from .jit import (_I32x3, _I64x3, _REALS, MAX_ARRAYS, MAX_SCALARS, VALUE_HELPERS, _MATH, JitKernel, _Gen, _lit, array_ndims, blocks_per_sm,
                   sweep_chunk, uses_kernel_language)
 from .kernels import ranges_to_box
 
@@ -1031,7 +1031,7 @@ def _sweep_handle(kernel, ndims, dt, order, descs, lo, cnt):
     if kernel._sweeps[key] is None:
         return None
     src, spans = kernel._sweeps[key][:2]
-    dims = {n: tuple(d.n) for n, d in zip(kernel.kd.arrays, descs)}
+    dims = {n: d[1] for n, d in zip(kernel.kd.arrays, descs)}
     if not sweep_fits(spans, dims, lo, cnt, ndims):
         return None
     h = _handle(kernel, key, lambda: src)
@@ -1053,24 +1053,24 @@ def parallel_grad(kernel: JitKernel, args, grad, ad_mode="reverse", ranges=None,
     if len(args) != kernel.nargs:
         raise ArgumentError(f"{kernel.name} takes {kernel.nargs} arguments (obtained {len(args)})")
     dup = _pairs(kernel, args, grad)
-    arrs, scal, by_name = [], [], {}
+    arrs, scal = [], []
     for (kind, name), a in zip(kernel.kd.args, args):
-        if kind == "scalar":
-            if not isinstance(a, numbers.Real):
-                raise ArgumentError(f"{kernel.name}: argument {name} is a scalar (obtained {type(a).__name__})")
-            scal.append(a)
-        else:
+        if kind == "array":
             arrs.append(a)
-            by_name[name] = a
-    descs = [descriptor(a) for a in arrs]
+        elif type(a) is float or type(a) is int or isinstance(a, numbers.Real):
+            scal.append(float(a))
+        else:
+            raise ArgumentError(f"{kernel.name}: argument {name} is a scalar (obtained {type(a).__name__})")
+    descs = [describe(a) for a in arrs]
     order = [n for n in kernel.kd.arrays if n in dup]
-    sdescs = [descriptor(dup[n]) for n in order]
+    sdescs = [describe(dup[n]) for n in order]
+    primal = dict(zip(kernel.kd.arrays, descs))
     for n, sd in zip(order, sdescs):
-        pd = descriptor(by_name[n])
-        if tuple(sd.n) != tuple(pd.n) or sd.dtype != pd.dtype:
+        pd = primal[n]
+        if sd[1:] != pd[1:]:
             raise ArgumentError(f"∇: the shadow of {n} must have its shape and number type")
-    dt = {0: "double", 1: "float"}.get(descs[0].dtype) if descs else "double"
-    if dt is None or any(d.dtype != descs[0].dtype for d in descs):
+    dt = _REALS.get(descs[0][2]) if descs else "double"
+    if dt is None or any(d[2] != descs[0][2] for d in descs):
         raise ArgumentError("the array arguments must share one FP64 or FP32 type")
     if len(descs) + len(sdescs) > 32:
         raise ArgumentError("∇: at most 32 arrays and shadows")
@@ -1110,7 +1110,7 @@ def parallel_grad(kernel: JitKernel, args, grad, ad_mode="reverse", ranges=None,
                     lambda: generate(kernel.kd, ndims, dt, order, ad_mode))
     alld = descs + sdescs
     A = (PSArray * len(alld))(*alld)
-    S = (ctypes.c_double * max(1, len(scal)))(*[float(x) for x in scal])
-    _lib.call("ps_jit_launch_ex", h, A, len(alld), S, len(scal), (ctypes.c_int64 * 3)(*lo),
-              (ctypes.c_int64 * 3)(*cnt), (ctypes.c_int32 * 3)(*threads), 0, (ctypes.c_int32 * 3)(*loop),
+    S = (ctypes.c_double * max(1, len(scal)))(*scal)
+    _lib.call("ps_jit_launch_ex", h, A, len(alld), S, len(scal), _I64x3(*lo),
+              _I64x3(*cnt), _I32x3(*threads), 0, _I32x3(*loop),
               stream_handle(stream), int(bool(sync)))

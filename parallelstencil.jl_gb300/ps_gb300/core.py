@@ -209,12 +209,22 @@ def to_host(A) -> np.ndarray:
 
 
 def dtype_code(dtype) -> int:
+    code = _CODES.get(dtype)
+    if code is not None:
+        return code
     torch = _torch()
     if dtype in (torch.float64, np.float64):
-        return _lib.PS_F64
-    if dtype in (torch.float32, np.float32):
-        return _lib.PS_F32
-    raise ArgumentError(f"unsupported element type {dtype}")
+        code = _lib.PS_F64
+    elif dtype in (torch.float32, np.float32):
+        code = _lib.PS_F32
+    else:
+        raise ArgumentError(f"unsupported element type {dtype}")
+    if isinstance(dtype, torch.dtype):
+        _CODES[dtype] = code
+    return code
+
+
+_CODES = {}  # torch dtype -> PS_F64 / PS_F32 (two entries at most)
 
 
 def is_column_major(shape, strides) -> bool:
@@ -226,24 +236,46 @@ def is_column_major(shape, strides) -> bool:
     return True
 
 
-def descriptor(A) -> PSArray:
-    """ps_array descriptor of a device array (dense, column-major, float64/float32)."""
+def describe(A) -> tuple:
+    """(device pointer, extents, type code, 0) of a device array (dense, column-major, float64/float32): the fields
+    of its ps_array descriptor. Launches read extents and types from these, not back from C structures."""
     if A is None:
-        return PSArray(None, (ctypes.c_int64 * 3)(1, 1, 1), _lib.PS_F64, 0)
+        return None, (1, 1, 1), _lib.PS_F64, 0
     if not getattr(A, "is_cuda", False):
         raise ArgumentError("kernel arguments must be device arrays (Data.Array)")
-    shape = tuple(A.shape)
-    if not 1 <= len(shape) <= 3:
-        raise ArgumentError(f"arrays must have 1 to 3 dimensions (obtained {len(shape)})")
+    shape = A.shape
+    nd = len(shape)
+    if not 1 <= nd <= 3:
+        raise ArgumentError(f"arrays must have 1 to 3 dimensions (obtained {nd})")
     if not is_column_major(shape, A.stride()):
         raise ArgumentError("arrays must be dense and column-major (Julia layout); use ps_gb300.zeros/Data.Array")
-    n = list(shape) + [1] * (3 - len(shape))
-    return PSArray(A.data_ptr(), (ctypes.c_int64 * 3)(*n), dtype_code(A.dtype), 0)
+    n = tuple(shape) if nd == 3 else (*shape, 1) if nd == 2 else (shape[0], 1, 1)
+    return A.data_ptr(), n, dtype_code(A.dtype), 0
+
+
+def descriptor(A) -> PSArray:
+    """ps_array descriptor of a device array (see describe)."""
+    return PSArray(*describe(A))
+
+
+def _stream_lookup():
+    """torch's own lookups behind current_stream(): (raw stream of a device, current device), or Nones."""
+    try:
+        import torch
+
+        return torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+    except (ImportError, AttributeError):
+        return None, None
+
+
+_raw_stream, _current_device = _stream_lookup()
 
 
 def stream_handle(stream=None):
     """Raw cudaStream_t of a torch stream (default: the current stream)."""
     if stream is None:
+        if _raw_stream is not None and _torch().cuda.is_initialized():  # 0.4 us; current_stream() 4
+            return ctypes.c_void_p(_raw_stream(_current_device()))
         return ctypes.c_void_p(_torch().cuda.current_stream().cuda_stream)
     if isinstance(stream, int):
         return ctypes.c_void_p(stream)

@@ -49,7 +49,7 @@ from dataclasses import dataclass, field
 
 from . import _lib
 from ._lib import PSArray
-from .core import ArgumentError, descriptor, require_initialized, stream_handle
+from .core import ArgumentError, describe, require_initialized, stream_handle
 from .fd import AV, DIFF, DIFF2, HARM, LHS, MACROS, MAXLOC, MINLOC, SEL
 from .kernels import ranges_to_box
 
@@ -76,6 +76,8 @@ _lib.register("ps_jit_destroy", [ctypes.c_void_p])
 
 MAX_ARRAYS = MAX_SCALARS = 32
 TMA_RING_BYTES = 64 * 1024  # shared memory for the plane ring of a TMA sweep (sets the planes in flight)
+_REALS = {0: "double", 1: "float"}  # PS_F64, PS_F32
+_I64x3, _I32x3 = ctypes.c_int64 * 3, ctypes.c_int32 * 3
 SMS = 152
 RESIDENT_THREADS = SMS * 2048  # threads a GB300 holds at once (152 SMs x 2048)
 # kernel-language macros (src/ParallelKernel/kernel_language.jl): a kernel that uses any of them
@@ -1548,7 +1550,13 @@ def _generate_info(kd: KernelDef, ndims: int, dtype: str, zloop: bool = False, s
 # ---- kernels -----------------------------------------------------------------------------------
 def array_ndims(descs):
     """Rank of a kernel's arrays (the largest; 2-D arrays have n[2] = 1, 1-D arrays n[1] = n[2] = 1)."""
-    return max((3 if d.n[2] > 1 else 2 if d.n[1] > 1 else 1) for d in descs) if descs else 1
+    nd = 1
+    for _, (_, n1, n2), _, _ in descs:
+        if n2 > 1:
+            return 3
+        if n1 > 1:
+            nd = 2
+    return nd
 
 
 class JitKernel:
@@ -1602,17 +1610,19 @@ class JitKernel:
         h, A, nA, S, nS, lo, cnt, threads, shmem, loop, layout = self._config(args, ranges, nblocks, nthreads, shmem,
                                                                              memopt, loopsize, fp64, allow_tma=True)
         if layout is not None:  # the 3-D sweep with its stencil arrays staged by TMA
-            maps = [x for a in layout["arrays"] for x in (a["k"], a["bx"], a["by"])]
+            if "maps" not in layout:
+                maps = [x for a in layout["arrays"] for x in (a["k"], a["bx"], a["by"])]
+                layout["maps"] = (ctypes.c_int32 * len(maps))(*maps)
             # threads in x and y: each covers xc columns and ry rows
             cnt_t = [-(-cnt[0] // layout["xc"]), -(-cnt[1] // layout["ry"]), cnt[2]]
-            _lib.call("ps_jit_launch_tma", h, A, nA, S, nS, (ctypes.c_int64 * 3)(*cnt_t),
-                      (ctypes.c_int32 * 3)(32, _Gen.TMA_TY // layout["ry"], 1), int(layout["smem"]), int(loop[2]),
-                      (ctypes.c_int32 * len(maps))(*maps), len(layout["arrays"]), stream_handle(stream),
+            _lib.call("ps_jit_launch_tma", h, A, nA, S, nS, _I64x3(*cnt_t),
+                      _I32x3(32, _Gen.TMA_TY // layout["ry"], 1), int(layout["smem"]), int(loop[2]),
+                      layout["maps"], len(layout["arrays"]), stream_handle(stream),
                       int(bool(sync)))
             self.tma_launches += 1
             return
-        _lib.call("ps_jit_launch_ex", h, A, nA, S, nS, (ctypes.c_int64 * 3)(*lo), (ctypes.c_int64 * 3)(*cnt),
-                  (ctypes.c_int32 * 3)(*threads), int(shmem or 0), (ctypes.c_int32 * 3)(*loop), stream_handle(stream),
+        _lib.call("ps_jit_launch_ex", h, A, nA, S, nS, _I64x3(*lo), _I64x3(*cnt),
+                  _I32x3(*threads), int(shmem or 0), _I32x3(*loop), stream_handle(stream),
                   int(bool(sync)))
 
     def hide_eligible(self):
@@ -1636,15 +1646,18 @@ class JitKernel:
         require_initialized()
         if len(args) != self.nargs:
             raise ArgumentError(f"{self.name} takes {self.nargs} arguments (obtained {len(args)})")
-        arrs, scal = [], []
+        descs, scal = [], []
         for (kind, name), a in zip(self.kd.args, args):
-            if kind == "scalar" and not isinstance(a, numbers.Real):
+            if kind == "array":
+                descs.append(describe(a))
+            elif type(a) is float or type(a) is int or isinstance(a, numbers.Real):
+                scal.append(float(a))
+            else:
                 raise ArgumentError(f"{self.name}: argument {name} is a scalar (obtained {type(a).__name__})")
-            (arrs if kind == "array" else scal).append(a)
-        descs = [descriptor(a) for a in arrs]
-        dt = {0: "double", 1: "float"}.get(descs[0].dtype) if descs else "double"
-        if dt is None or any(d.dtype != descs[0].dtype for d in descs):
-            raise ArgumentError("the array arguments must share one FP64 or FP32 type")
+        dt = _REALS.get(descs[0][2]) if descs else "double"
+        for d in descs:
+            if dt is None or d[2] != descs[0][2]:
+                raise ArgumentError("the array arguments must share one FP64 or FP32 type")
         ndims = self.ndims or array_ndims(descs)
         lo, cnt = [0, 0, 0], self._extent(descs, ndims)
         threads = [1, 1, 1]
@@ -1690,8 +1703,8 @@ class JitKernel:
         if fp64 not in ("ieee", "split", "split_state", "split_grid"):
             raise ArgumentError("fp64 must be 'ieee' or 'split'")
         sp = fp64 != "ieee" and dt == "double"
-        A = (PSArray * max(1, len(descs)))(*descs)
-        S = (ctypes.c_double * max(1, len(scal)))(*[float(x) for x in scal])
+        A = (PSArray * max(1, len(descs)))(*descs)  # (ctypes fills a structure from its tuple)
+        S = (ctypes.c_double * max(1, len(scal)))(*scal)
         if allow_tma and self.tma and (dt == "float" or self.tma == "always") and zl and ndims == 3 and \
                 not ordered and ranges is None and nblocks is None and nthreads is None and not shmem:
             # the 3-D sweep with its stencil arrays staged by TMA, where every staged array meets TMA's
@@ -1699,10 +1712,12 @@ class JitKernel:
             es = 8 if dt == "double" else 4
             ht = self._handle(ndims, dt, zl, sp, False, tma=True)
             layout = self._layouts[(ndims, dt, zl, sp, "tma")]
-            if layout is not None and all(n < 2 ** 31 - 2 ** 16 for d in descs for n in (*d.n, 8 * d.n[0] * d.n[1])) and all(not ((d.ptr or 0) % 16 or (d.n[0] * es) % 16 or (d.n[0] * d.n[1] * es) % 16)
-                                          for d in (descs[a["k"]] for a in layout["arrays"])):
+            # (and where 32-bit indices reach all of a few planes)
+            if layout is not None and all(max(*n, 8 * n[0] * n[1]) < 2 ** 31 - 2 ** 16 for _, n, _, _ in descs) and \
+                    all(not ((ptr or 0) % 16 or (n[0] * es) % 16 or (n[0] * n[1] * es) % 16)
+                        for ptr, n, _, _ in (descs[a["k"]] for a in layout["arrays"])):
                 if not loopsize and "loopsize" not in self.kd.options:
-                    if "resident" not in layout:
+                    if "resident" not in layout:  # a property of the compiled kernel
                         layout["resident"] = blocks_per_sm(ht, 32 * _Gen.TMA_TY // layout["ry"], layout["smem"])
                     cols = -(-cnt[0] // (32 * layout["xc"])) * -(-cnt[1] // _Gen.TMA_TY)
                     loop[2] = sweep_chunk(max(1, cnt[2]), max(1, cols), layout["resident"], layout["span"])
@@ -1718,10 +1733,16 @@ class JitKernel:
     def _extent(descs, ndims):
         """The `@parallel` grid: the largest extent of the array arguments per dimension
         (src/ParallelKernel/parallel.jl:785-798), 1 beyond ndims."""
-        return [max(int(x.n[d]) for x in descs) if descs and d < ndims else 1 for d in range(3)]
+        if not descs:
+            return [1, 1, 1]
+        n = list(descs[0][1])
+        for d in descs:
+            if d[1] != descs[0][1]:
+                n = list(map(max, n, d[1]))
+        return n[:ndims] + [1] * (3 - ndims)
 
     def grid_extent(self, args):
-        descs = [descriptor(a) for (kind, _), a in zip(self.kd.args, args) if kind == "array"]
+        descs = [describe(a) for (kind, _), a in zip(self.kd.args, args) if kind == "array"]
         return self._extent(descs, self.ndims or array_ndims(descs))
 
     def check(self, stream=None):
