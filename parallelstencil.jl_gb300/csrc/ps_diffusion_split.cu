@@ -495,8 +495,6 @@ __global__ void __launch_bounds__(32 * TY, MINB)
     using C = SplitCfg<LAM, TY, S>;
     constexpr int NHALO = IN64 ? C::HALO * (LAM ? 2 : 1) : 0;
     constexpr int HPT = NHALO > 0 ? (NHALO + 32 * TY - 1) / (32 * TY) : 1;
-    if (*reinterpret_cast<volatile int*>(&run->bad)) return;
-    const int sh = run->shT;
     extern __shared__ __align__(128) unsigned char smem[];
     float2* faceY0 = reinterpret_cast<float2*>(smem + S * C::STAGE);  // 2 x [TY+1][SP_TX]
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + S * C::STAGE + 2 * C::FACE);
@@ -517,6 +515,11 @@ __global__ void __launch_bounds__(32 * TY, MINB)
         fence_mbar_init();
     }
     __syncthreads();
+    // the step before has completed; the next one may set up its blocks while this one runs
+    grid_dependency_wait();
+    grid_dependents_may_launch();
+    if (*reinterpret_cast<volatile int*>(&run->bad)) return;
+    const int sh = run->shT;
     int next_q = 0;
     auto issue = [&](int q) {
         unsigned char* b = slot(q);
@@ -910,8 +913,8 @@ static int launch_grid_variant(const ps_array& Tin, const ps_array& Cs, const ps
         L = auto_loopsize(bx * by, cb.hi[2] - cb.lo[2], (int64_t)occ * st->num_sms);
     }
     dim3 grd((unsigned)bx, (unsigned)by, (unsigned)((cb.hi[2] - cb.lo[2] + L - 1) / L));
-    kernel<<<grd, blk, C::SMEM, s>>>(mT, mL, mC, T2.ptr, p, T2.n[0], T2.n[1], cb, L, d_err, run,
-                                     static_cast<float4*>(Lout), static_cast<float4*>(Cout));
+    PS_CUDA_TRY(launch_dependent(kernel, grd, blk, (size_t)C::SMEM, s, mT, mL, mC, T2.ptr, p, T2.n[0], T2.n[1], cb, L,
+                                 d_err, run, static_cast<float4*>(Lout), static_cast<float4*>(Cout)));
     return PS_OK;
 }
 
@@ -1064,9 +1067,6 @@ __global__ void __launch_bounds__(32 * TY, 2)
                         int64_t nx, int64_t ny, Box cb, int L, int* __restrict__ err, GridRun* __restrict__ run,
                         const GridRun* __restrict__ mrun) {
     using C = AdjCfg<TY, S>;
-    grid_dependents_may_launch();  // glam_boundary_kernel of this step runs beside this kernel
-    if (*reinterpret_cast<volatile int*>(&run->bad) || mrun->bad) return;
-    const int sh = mrun->shT + run->shT;
     extern __shared__ __align__(128) unsigned char smem[];
     float2* faceY0 = reinterpret_cast<float2*>(smem + S * C::STAGE);
     float2* wY0 = reinterpret_cast<float2*>(smem + S * C::STAGE + 2 * C::FACE);
@@ -1089,6 +1089,10 @@ __global__ void __launch_bounds__(32 * TY, 2)
         fence_mbar_init();
     }
     __syncthreads();
+    grid_dependency_wait();        // the step before (or the recomputed states) has completed
+    grid_dependents_may_launch();  // glam_boundary_kernel of this step runs beside this kernel
+    if (*reinterpret_cast<volatile int*>(&run->bad) || *reinterpret_cast<const volatile int*>(&mrun->bad)) return;
+    const int sh = mrun->shT + run->shT;
     int next_q = 0;
     auto issue = [&](int q) {
         unsigned char* b = slot(q);
@@ -1279,7 +1283,8 @@ __global__ void __launch_bounds__(32 * TY, 2)
 __global__ void glam_boundary_kernel(const float2* __restrict__ M, const float2* __restrict__ Tg,
                                      double* __restrict__ glam, dd gc0, dd gc1, dd gc2, int64_t nx, int64_t ny,
                                      int64_t nz, const GridRun* __restrict__ run, const GridRun* __restrict__ mrun) {
-    if (run->bad || mrun->bad) return;
+    grid_dependents_may_launch();  // the next step's blocks may set up
+    const bool skip = run->bad || mrun->bad;
     const int sh = mrun->shT + run->shT;
     const int f = blockIdx.y;  // 0, 1: planes z = 0, nz-1 (all x, y); 2, 3: rows y = 0, ny-1 (z = 1 .. nz-2)
     const int64_t n0 = nx, n1 = f < 2 ? ny : nz - 2;
@@ -1288,7 +1293,7 @@ __global__ void glam_boundary_kernel(const float2* __restrict__ M, const float2*
         const float2 v = a[o];
         return dd{v.x, v.y};
     };
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n0 * n1; t += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n0 * n1 && !skip; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t x = t % n0, v = t / n0;
         const int64_t y = f < 2 ? v : (f == 2 ? 0 : ny - 1), z = f < 2 ? (f == 0 ? 0 : nz - 1) : v + 1;
         const int64_t o = x + nx * (y + ny * z);
@@ -1311,6 +1316,7 @@ __global__ void glam_boundary_kernel(const float2* __restrict__ M, const float2*
         g = dd_add(g, dd_mul(gc2, s3[2]));
         glam[o] = glam[o] + grid_to_f64(f32_to_f64(g.h) + f32_to_f64(g.l), sh);
     }
+    grid_dependency_wait();
 }
 
 template <bool ISO>
@@ -1337,12 +1343,13 @@ static int launch_grid_adj(const ps_array& Min, const ps_array& Ls, const ps_arr
     PS_TRY(current_state(&st));
     const int L = auto_loopsize(bx * by, cb.hi[2] - cb.lo[2], (int64_t)occ * st->num_sms);
     dim3 grd((unsigned)bx, (unsigned)by, (unsigned)((cb.hi[2] - cb.lo[2] + L - 1) / L));
-    kernel<<<grd, dim3(32, TY, 1), C::SMEM, s>>>(mM, mL, mC, mT, static_cast<float2*>(Mout.ptr),
-                                                static_cast<double*>(glam.ptr), p, gc[0], gc[1], gc[2], Mout.n[0],
-                                                Mout.n[1], cb, L, d_err, run, mrun);
+    PS_CUDA_TRY(launch_dependent(kernel, grd, dim3(32, TY, 1), (size_t)C::SMEM, s, mM, mL, mC, mT,
+                                 static_cast<float2*>(Mout.ptr), static_cast<double*>(glam.ptr), p, gc[0], gc[1], gc[2],
+                                 Mout.n[0], Mout.n[1], cb, L, d_err, run, mrun));
     // The boundary rows and planes of glam run beside the kernel above (programmatic dependent
-    // launch without a wait): they read μ and T_n, which the step before completed, and write glam
-    // cells the kernel above does not touch. The next step's launch waits for both.
+    // launch; it starts once every block of that kernel has waited for the step before): they read μ and
+    // T_n, which the step before completed, and write glam cells the kernel above does not touch. They wait
+    // for that kernel at their end, so the next step, which waits for them, waits for both.
     const int64_t nmax = std::max(Mout.n[0] * Mout.n[1], Mout.n[0] * Mout.n[2]);
     const dim3 gb((unsigned)std::min<int64_t>((nmax + 255) / 256, st->num_sms * 4), 4);
     if (launch_dependent(glam_boundary_kernel, gb, dim3(256), 0, s, static_cast<const float2*>(Min.ptr),
