@@ -145,6 +145,9 @@ __global__ void __launch_bounds__(32 * ACU_W, AR::kMinBlocks) acoustic_step_kern
     const int lane = threadIdx.x;
     const I nx = (I)a.nx, ny = (I)a.ny, nz = (I)a.nz;
     const I y = (I)blockIdx.y * ACU_W + (I)threadIdx.y;
+    // the step before has completed (its arrays are read with plain loads); the next one may start as blocks end
+    grid_dependency_wait();
+    grid_dependents_may_launch();
     if (y >= ny) return;  // whole warps only: no block-wide synchronisation follows
     const I x = (I)blockIdx.x * 32 + lane;
     const I z0 = (I)blockIdx.z * Lz;
@@ -284,7 +287,7 @@ int launch_acoustic_i(const ps_array& Vx, const ps_array& Vy, const ps_array& Vz
     int Lz = auto_loopsize(gx * gy, a.nz, (int64_t)slots_per_sm * st->num_sms);
     if ((a.nz + Lz - 1) / Lz > 65535) Lz = (int)((a.nz + 65534) / 65535);
     const dim3 grd((unsigned)gx, (unsigned)gy, (unsigned)((a.nz + Lz - 1) / Lz));
-    acoustic_step_kernel<AR, I><<<grd, blk, 0, s>>>(a, c, Lz, st->d_err);
+    PS_CUDA_TRY(launch_dependent(acoustic_step_kernel<AR, I>, grd, blk, (size_t)0, s, a, c, Lz, st->d_err));
     return PS_OK;
 }
 

@@ -74,7 +74,11 @@ __global__ void __launch_bounds__(32 * TY, MINB) diff3d_split_tma(const __grid_c
                                                                   const int* __restrict__ pred, TileOrder ord) {
     // pred (may be NULL): the launch runs only if *pred is set -- the device-side fallback of a
     // fixed-grid run whose values left the grid
-    if (pred && !*reinterpret_cast<const volatile int*>(pred)) return;
+    if (pred) {  // (first: a launch that does not run costs no set-up)
+        grid_dependency_wait();
+        grid_dependents_may_launch();
+        if (!*reinterpret_cast<const volatile int*>(pred)) return;
+    }
     using C = SplitCfg<LAM, TY, S>;
     // staged arrays converted in place each step: T (unless STATE) and lam (unless PRE)
     constexpr int NCONV = (STATE ? 0 : 1) + ((LAM && !PRE) ? 1 : 0);
@@ -101,6 +105,10 @@ __global__ void __launch_bounds__(32 * TY, MINB) diff3d_split_tma(const __grid_c
         fence_mbar_init();
     }
     __syncthreads();
+    if (!pred) {  // the kernel before has completed; the next one may set up its blocks while this one runs
+        grid_dependency_wait();
+        grid_dependents_may_launch();
+    }
     int next_q = 0;
     auto issue = [&](int q) {
         unsigned char* b = slot(q);
@@ -339,8 +347,12 @@ static int launch_split_variant(const ps_array& Tin, const ps_array& Ci, const p
         hr->nb = ord.nb;
         grd = dim3((unsigned)(bx * by * bz), 1, 1);
     }
-    diff3d_split_tma<LAM, ISO, TY, S, MINB, PRE, STATE><<<grd, blk, C::SMEM, s>>>(
-        mT, mL, mC, static_cast<double*>(T2.ptr), p, T2.n[0], T2.n[1], cb, L, d_err, pred, ord);
+    const auto kernel = diff3d_split_tma<LAM, ISO, TY, S, MINB, PRE, STATE>;
+    if (hr)
+        kernel<<<grd, blk, C::SMEM, s>>>(mT, mL, mC, static_cast<double*>(T2.ptr), p, T2.n[0], T2.n[1], cb, L, d_err, pred, ord);
+    else
+        PS_CUDA_TRY(launch_dependent(kernel, grd, blk, (size_t)C::SMEM, s, mT, mL, mC, static_cast<double*>(T2.ptr), p,
+                                     T2.n[0], T2.n[1], cb, L, d_err, pred, ord));
     return PS_OK;
 }
 

@@ -527,6 +527,9 @@ __global__ void __launch_bounds__(32 * TY) diff3d_zsweep_tma(const __grid_consta
         fence_mbar_init();
     }
     __syncthreads();
+    // the kernel before has completed; the next one may set up its blocks while this one runs
+    grid_dependency_wait();
+    grid_dependents_may_launch();
 
     int next_q = 0;
     auto issue = [&](int q) {
@@ -837,8 +840,12 @@ static int launch_zsweep_tma(const ps_array& T2, const ps_array& Tin, const ps_a
         hr->nb = ord.nb;
         grd = dim3((unsigned)(bx * by * bz), 1, 1);
     }
-    diff3d_zsweep_tma<T, FORM, TY, S><<<grd, blk, Z::SMEM, s>>>(mT, mL, mC, static_cast<T*>(T2.ptr), p, T2.n[0],
-                                                                T2.n[1], cb, L, d_err, ord);
+    const auto kernel = diff3d_zsweep_tma<T, FORM, TY, S>;
+    if (hr)
+        kernel<<<grd, blk, Z::SMEM, s>>>(mT, mL, mC, static_cast<T*>(T2.ptr), p, T2.n[0], T2.n[1], cb, L, d_err, ord);
+    else
+        PS_CUDA_TRY(launch_dependent(kernel, grd, blk, (size_t)Z::SMEM, s, mT, mL, mC, static_cast<T*>(T2.ptr), p, T2.n[0],
+                                     T2.n[1], cb, L, d_err, ord));
     return PS_OK;
 }
 
