@@ -2,9 +2,8 @@
 // with FP32 accumulation, trained and run entirely by this library's kernels.
 //
 // Layout: activations NHWC (channels contiguous), bf16. A 3x3 convolution ("same" padding) is an implicit
-// GEMM on the tensor cores (ps_nn_conv.cu; bias, ReLU and bf16 in its epilogue); the two-channel first layer
-// and the 1x1 last one, too short in K or N for them, are one pixel per thread
-// and its backward pass
+// GEMM on the tensor cores (ps_nn_conv.cu; bias, ReLU and bf16 in its epilogue, on large images also the 1x1
+// output layer), and its backward pass
 //   dz   = dy * (y > 0)  (bf16; the bias gradient is summed in FP32 in the same kernel)
 //   dW  += dz^T * col    (GEMM over K = P, split-K with FP32 atomics; the column matrix built transposed)
 //   dcol = dz * W        (GEMM, B operand = W^T); dx = col2im(dcol) (gather, no atomics).
@@ -182,70 +181,6 @@ __global__ void __launch_bounds__(256) nn_upcat_k(const bf16* __restrict__ low, 
 #pragma unroll 4
             for (int r = 0; r < f; r++) d[(int64_t)r * W * C8] = s[(int64_t)r * W * Cs8];
         }
-    }
-}
-// The first layer: y[p][0..31] = relu(3x3 conv of the two input channels + bias). K = 18 is too short for the
-// tensor cores. A thread takes 16 of the 32 outputs of 4 pixels a block's width apart, so that a 16-byte
-// weight load from shared memory feeds 16 FMAs (one pixel with 32 outputs per thread: 4 FMAs per load, bound by
-// shared memory, 40 us for 8 images of 256^2; now 30).
-constexpr int kFirstPix = 4;
-__global__ void __launch_bounds__(256, 2) nn_conv_first_k(const bf16* __restrict__ x, const bf16* __restrict__ wgt, int kpad,
-                                                       const float* __restrict__ bias, int64_t P, int H, int W, bf16* y) {
-    __shared__ float4 sw[18][8];  // [tap, channel][output / 4]
-    __shared__ float sb[32];
-    grid_dependency_wait();
-    grid_dependents_may_launch();
-    for (int i = threadIdx.x; i < 18 * 32; i += blockDim.x)
-        reinterpret_cast<float*>(sw[i / 32])[i % 32] = __bfloat162float(wgt[(int64_t)(i % 32) * kpad + i / 32]);
-    for (int i = threadIdx.x; i < 32; i += blockDim.x) sb[i] = bias[i];
-    __syncthreads();
-    const int half = threadIdx.x & 1, o4 = 4 * half;
-    const int64_t p0 = blockIdx.x * (int64_t)(kFirstPix * 128) + (threadIdx.x >> 1);
-    const __nv_bfloat162* x2 = reinterpret_cast<const __nv_bfloat162*>(x);
-    int xx[kFirstPix], yy[kFirstPix];
-#pragma unroll
-    for (int j = 0; j < kFirstPix; j++) {
-        const int64_t p = p0 + j * 128, q = p / W;
-        xx[j] = p < P ? (int)(p - q * W) : -2;  // -2: no tap of it is in the image
-        yy[j] = (int)(q % H);
-    }
-    float acc[kFirstPix][16] = {};
-#pragma unroll 1
-    for (int ty = -1; ty <= 1; ty++)
-#pragma unroll 1
-        for (int tx = -1; tx <= 1; tx++) {
-            float2 v[kFirstPix];
-#pragma unroll
-            for (int j = 0; j < kFirstPix; j++) {
-                const bool in = (unsigned)(xx[j] + tx) < (unsigned)W && (unsigned)(yy[j] + ty) < (unsigned)H;
-                v[j] = in ? __bfloat1622float2(x2[p0 + j * 128 + ty * W + tx]) : make_float2(0.0f, 0.0f);
-            }
-            const int tap = 3 * (ty + 1) + tx + 1;
-#pragma unroll
-            for (int o = 0; o < 4; o++) {
-                const float4 a = sw[2 * tap][o4 + o], b = sw[2 * tap + 1][o4 + o];
-#pragma unroll
-                for (int j = 0; j < kFirstPix; j++) {
-                    float* c = acc[j] + 4 * o;
-                    c[0] = fmaf(v[j].y, b.x, fmaf(v[j].x, a.x, c[0]));
-                    c[1] = fmaf(v[j].y, b.y, fmaf(v[j].x, a.y, c[1]));
-                    c[2] = fmaf(v[j].y, b.z, fmaf(v[j].x, a.z, c[2]));
-                    c[3] = fmaf(v[j].y, b.w, fmaf(v[j].x, a.w, c[3]));
-                }
-            }
-        }
-#pragma unroll
-    for (int j = 0; j < kFirstPix; j++) {
-        if (xx[j] < 0) continue;
-        uint4 w4[2];
-        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(w4);
-#pragma unroll
-        for (int o = 0; o < 8; o++)
-            h[o] = __floats2bfloat162_rn(fmaxf(acc[j][2 * o] + sb[16 * half + 2 * o], 0.0f),
-                                         fmaxf(acc[j][2 * o + 1] + sb[16 * half + 2 * o + 1], 0.0f));
-        uint4* d = reinterpret_cast<uint4*>(y + (p0 + j * 128) * 32 + 16 * half);
-        d[0] = w4[0];
-        d[1] = w4[1];
     }
 }
 // The last layer: y[p][0..2] = W x[p] + bias over 32 channels (FP32 result), one pixel per thread
@@ -583,15 +518,22 @@ static int nn_create(NNet* n, int H, int W, int Bmax, uint64_t seed) {
     return PS_OK;
 }
 
-// y = act(conv(x)); x [P][cin] bf16 at resolution (h, w); y bf16 [P][cout] (or FP32 for the last layer)
-static int nn_conv_fwd(NNet* n, Conv& L, const bf16* x, int B, int h, int w, void* y, cudaStream_t s, int* err) {
+// y = act(conv(x)); x [P][cin] bf16 at resolution (h, w); y bf16 [P][cout] (or FP32 for the last layer).
+// next, ynext: the 1x1 layer after it and its result; *fused tells whether it was computed here
+static int nn_conv_fwd(NNet* n, Conv& L, const bf16* x, int B, int h, int w, void* y, cudaStream_t s, int* err,
+                       const Conv* next = nullptr, float* ynext = nullptr, bool* fused = nullptr) {
     (void)n;
     const int64_t P = (int64_t)B * h * w;
-    if (L.k == 3 && L.cin % 32 == 0)
+    if (L.k == 3 && L.cin % 32 == 0) {
+        bool taken = false;
+        PS_TRY(nn_conv3_rows(x, B, h, w, L.cin, L.W, L.cout, L.b, L.relu, y, next ? next->W : nullptr,
+                             next ? (int)next->kpad : 0, next ? next->b : nullptr, ynext, &taken, s, err));
+        if (fused) *fused = taken;
+        if (taken) return PS_OK;
         return nn_conv3_tc(x, B, h, w, L.cin, L.W, L.cout, L.b, L.relu, y, s, err);
+    }
     if (L.k == 3)
-        PS_CUDA_TRY(launch_dependent(nn_conv_first_k, dim3((unsigned)((P + kFirstPix * 128 - 1) / (kFirstPix * 128))), dim3(256),
-                                     0, s, x, L.W, (int)L.kpad, L.b, P, h, w, static_cast<bf16*>(y)));
+        PS_TRY(nn_conv3_first(x, P, h, w, L.W, (int)L.kpad, L.b, y, s, err));
     else
         PS_CUDA_TRY(launch_dependent(nn_conv_last_k, dim3(nblk(P)), dim3(256), 0, s, x, L.W, (int)L.kpad, L.b, P,
                                      static_cast<float*>(y)));
@@ -692,8 +634,9 @@ static int nn_forward(NNet* n, int B, cudaStream_t s, int* err) {
     PS_TRY(cv(11, n->a[10], 1, n->a[11]));
     PS_CUDA_TRY(upcat(n->a[11], 2 * c, n->a[1], c, 0, n->k0));
     PS_TRY(cv(12, n->k0, 0, n->a[12]));
-    PS_TRY(cv(13, n->a[12], 0, n->a[13]));
-    PS_TRY(cv(14, n->a[13], 0, n->y));
+    bool fused = false;
+    PS_TRY(nn_conv_fwd(n, L[13], n->a[12], B, n->H, n->W, n->a[13], s, err, &L[14], n->y, &fused));
+    if (!fused) PS_TRY(cv(14, n->a[13], 0, n->y));
     PS_CUDA_TRY(cudaGetLastError());
     n->lastB = B;
     return PS_OK;
