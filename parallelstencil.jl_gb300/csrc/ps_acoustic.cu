@@ -145,9 +145,8 @@ __global__ void __launch_bounds__(32 * ACU_W, AR::kMinBlocks) acoustic_step_kern
     const int lane = threadIdx.x;
     const I nx = (I)a.nx, ny = (I)a.ny, nz = (I)a.nz;
     const I y = (I)blockIdx.y * ACU_W + (I)threadIdx.y;
-    // the step before has completed (its arrays are read with plain loads); the next one may start as blocks end
+    // the step before has completed (its arrays are read with plain loads)
     grid_dependency_wait();
-    grid_dependents_may_launch();
     if (y >= ny) return;  // whole warps only: no block-wide synchronisation follows
     const I x = (I)blockIdx.x * 32 + lane;
     const I z0 = (I)blockIdx.z * Lz;

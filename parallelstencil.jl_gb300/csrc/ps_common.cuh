@@ -395,6 +395,12 @@ __device__ __forceinline__ T dvd(T a, const DivF<T>& h) {
 // kernel before it on the stream finishes its last wave; it waits in grid_dependency_wait() (a
 // no-op in an ordinary launch) until that kernel has completed and its stores are visible, so
 // every read of data the previous kernel wrote must come after the wait.
+//
+// A kernel that calls grid_dependents_may_launch() lets the next one's blocks in while its own run. That is for
+// kernels meant to run beside each other: in a chain the early blocks take the places that come free
+// first, and the SMs are loaded unevenly for the rest of the launch (accelerated Stokes2D iteration, FP64
+// 350^2: 19.7 us with the call, 14.8 without, 18.4 in ordinary launches; FP32 300 x 411 5.6 and 4.6).
+// Without it the next kernel's blocks start as the last of this one's finish.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;"); }

@@ -76,7 +76,6 @@ __global__ void __launch_bounds__(32 * TY, MINB) diff3d_split_tma(const __grid_c
     // fixed-grid run whose values left the grid
     if (pred) {  // (first: a launch that does not run costs no set-up)
         grid_dependency_wait();
-        grid_dependents_may_launch();
         if (!*reinterpret_cast<const volatile int*>(pred)) return;
     }
     using C = SplitCfg<LAM, TY, S>;
@@ -105,10 +104,7 @@ __global__ void __launch_bounds__(32 * TY, MINB) diff3d_split_tma(const __grid_c
         fence_mbar_init();
     }
     __syncthreads();
-    if (!pred) {  // the kernel before has completed; the next one may set up its blocks while this one runs
-        grid_dependency_wait();
-        grid_dependents_may_launch();
-    }
+    if (!pred) grid_dependency_wait();  // the kernel before has completed
     int next_q = 0;
     auto issue = [&](int q) {
         unsigned char* b = slot(q);
@@ -527,9 +523,7 @@ __global__ void __launch_bounds__(32 * TY, MINB)
         fence_mbar_init();
     }
     __syncthreads();
-    // the step before has completed; the next one may set up its blocks while this one runs
-    grid_dependency_wait();
-    grid_dependents_may_launch();
+    grid_dependency_wait();  // the step before has completed
     if (*reinterpret_cast<volatile int*>(&run->bad)) return;
     const int sh = run->shT;
     int next_q = 0;

@@ -98,7 +98,6 @@ __global__ void __launch_bounds__(192, 2)
     const uint32_t tmem = *tmem_slot;
     // the previous layer's activations
     grid_dependency_wait();
-    grid_dependents_may_launch();
 
     if (threadIdx.x == 0) {  // TMA producer
         int it = 0;
@@ -310,7 +309,6 @@ __global__ void __launch_bounds__(192, 2)
     const uint32_t tmem = *tmem_slot;
     // the previous layer's activations
     grid_dependency_wait();
-    grid_dependents_may_launch();
     if (last.y) {
         for (int i = threadIdx.x; i < 96; i += blockDim.x) sw[i] = __bfloat162float(last.w[(i / 32) * last.kpad + i % 32]);
         __syncthreads();
@@ -515,7 +513,6 @@ __global__ void __launch_bounds__(128, kFirstCtas)
     tc_fence_after();
     const uint32_t tmem = slot;
     grid_dependency_wait();
-    grid_dependents_may_launch();
     if (t < 32) sbias[t] = bias[t];
     for (int i = t; i < 32 * 32; i += 128) {  // weights [output][k], zero beyond 18
         const int n = i >> 5, k = i & 31;

@@ -117,7 +117,6 @@ __global__ void nn_transpose_k(const bf16* __restrict__ in, int64_t R, int C, in
 // takes 8 channels (16 bytes), C % 8 == 0; blocks along x run over rows of the result, along y over a row's values
 __global__ void __launch_bounds__(256) nn_pool_k(const bf16* __restrict__ x, int rows, int h, int w, int C8, int f, bf16* y) {
     grid_dependency_wait();
-    grid_dependents_may_launch();
     const int W = w * f, i = (int)(blockIdx.y * 256 + threadIdx.x);
     if (i >= w * C8) return;
     const int xx = i / C8, c = i - xx * C8;
@@ -167,7 +166,6 @@ __global__ void nn_pool_bwd_k(const float* __restrict__ dy, int64_t B, int H, in
 __global__ void __launch_bounds__(256) nn_upcat_k(const bf16* __restrict__ low, int Cl8, const bf16* __restrict__ skip,
                                                   int Cs8, int groups, int W, int f, bf16* k) {
     grid_dependency_wait();
-    grid_dependents_may_launch();
     const int C8 = Cl8 + Cs8, w = W / f, i = (int)(blockIdx.y * 256 + threadIdx.x);
     if (i >= W * C8) return;
     const int xx = i / C8, c = i - xx * C8, lx = xx / f * Cl8 + c, sx = xx * Cs8 + c - Cl8;
@@ -188,7 +186,6 @@ __global__ void __launch_bounds__(256) nn_conv_last_k(const bf16* __restrict__ x
                                                       const float* __restrict__ bias, int64_t P, float* __restrict__ y) {
     __shared__ float sw[3][32];
     grid_dependency_wait();
-    grid_dependents_may_launch();
     for (int i = threadIdx.x; i < 96; i += blockDim.x) sw[i / 32][i % 32] = __bfloat162float(wgt[(int64_t)(i / 32) * kpad + i % 32]);
     __syncthreads();
     const float b0 = bias[0], b1 = bias[1], b2 = bias[2];
@@ -244,7 +241,6 @@ __global__ void nn_f32_to_bf16_k(const float* __restrict__ a, int64_t n, bf16* b
 // the same for the network's input: 4 values per thread (n % 4 == 0; 16-byte aligned arrays)
 __global__ void __launch_bounds__(256) nn_input_k(const float4* __restrict__ a, int64_t n4, uint2* b) {
     grid_dependency_wait();
-    grid_dependents_may_launch();
     GSTRIDE(i, n4) {
         const float4 v = a[i];
         const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);

@@ -527,9 +527,7 @@ __global__ void __launch_bounds__(32 * TY) diff3d_zsweep_tma(const __grid_consta
         fence_mbar_init();
     }
     __syncthreads();
-    // the kernel before has completed; the next one may set up its blocks while this one runs
-    grid_dependency_wait();
-    grid_dependents_may_launch();
+    grid_dependency_wait();  // the kernel before has completed
 
     int next_q = 0;
     auto issue = [&](int q) {

@@ -249,7 +249,7 @@ __device__ __forceinline__ T s2_half_sum(T a, T b, H) {
 __device__ __forceinline__ double s2_half_sum(double a, double b, DivF<double> h) { return scale_pow2(a + b, -1, h.key); }
 
 // Rows of 32 threads per block. FP32: 8; FP64, bound by the FP64 pipe: 2, which spreads a small grid more
-// evenly over the SMs (8 rows -> 2: 255^2 11.4 -> 10.7 us per iteration, 130^2 7.1 -> 6.3, 1023^2 118 both).
+// evenly over the SMs (4 rows -> 2: 255^2 11.4 -> 10.5 us per iteration, 130^2 6.9 -> 6.1, 1023^2 118 both).
 template <typename T>
 __host__ __device__ constexpr int s2_block_rows() {
     return sizeof(T) == 4 ? 8 : 2;
@@ -275,7 +275,6 @@ __global__ void __launch_bounds__(32 * s2_block_rows<T>()) s2_cells(S2Fused<T> a
         m11 = __ldg(a.Mus + c + nx + 1);
     }
     grid_dependency_wait();  // the state is read with plain loads: __ldg need not see the kernel before
-    grid_dependents_may_launch();
     T vx0 = T(0), vx1 = T(0), vy0 = T(0), vy1 = T(0), pt = T(0), vxu = T(0), vyr = T(0);
     if (cell) {
         vx0 = a.Vx[cx];
@@ -338,7 +337,6 @@ __global__ void __launch_bounds__(32 * s2_block_rows<T>()) s2_faces(S2Fused<T> a
         }
     }
     grid_dependency_wait();
-    grid_dependents_may_launch();
     T xr = T(0), xl = T(0), s00 = T(0), s01 = T(0), s10 = T(0), p0 = T(0), pl = T(0), pd = T(0), yu = T(0), yd = T(0);
     T xg = T(0), yg = T(0), vx = T(0), vy = T(0);
     if (fx || fy) {

@@ -173,11 +173,11 @@ __device__ __forceinline__ void apt_block_add(double v0, double* out0, double v1
 // on the two kernels' 26 words per cell, from L2 mostly). Measured and not kept: two to four rows per
 // thread (13.2-14.2 us), blocks of 128 threads (18.9: twice the blocks to launch) or 512 (16.3 and more).
 
-// Rows of 32 threads per block. FP32: 8; FP64, bound by the FP64 pipe: 4, which spreads a small grid more
-// evenly over the SMs (8 rows -> 4: 255^2 11.6 -> 10.6 us per iteration, 130^2 8.7 -> 7.9, 1023^2 100.5 both).
+// Rows of 32 threads per block. FP32: 8; FP64, bound by the FP64 pipe: 2, which spreads a small grid more
+// evenly over the SMs (8 rows -> 2: 350^2 17.2 -> 14.7 us per iteration, 255^2 11.1 -> 10.4, 1023^2 100.3 both).
 template <typename T>
 __host__ __device__ constexpr int apt_block_rows() {
-    return sizeof(T) == 4 ? 8 : 4;
+    return sizeof(T) == 4 ? 8 : 2;
 }
 
 // compute_P_τ!: cells (∇V, Pt, τxx, τyy) and corners (τxy). DEFECT: the correction's sweep
@@ -201,7 +201,6 @@ __global__ void __launch_bounds__(32 * apt_block_rows<T>()) apt_cells_k(AptArray
         bTc = __ldg(a.bTc + (c - iy));
     }
     grid_dependency_wait();  // V of the previous iteration's faces kernel
-    grid_dependents_may_launch();
     T vx0, vx1, vy0, vy1, pt, txx, tyy, vxu, vyr, txy;
     vx0 = vx1 = vy0 = vy1 = pt = txx = tyy = vxu = vyr = txy = (T)0;
     if (ix < nx && iy < ny) {
@@ -264,7 +263,6 @@ __global__ void __launch_bounds__(32 * apt_block_rows<T>()) apt_faces_k(AptArray
         else srcy = (__ldg(a.Rog + c + 1) + __ldg(a.Rog + c + 1 + nx)) * h;
     }
     grid_dependency_wait();  // τ and Pt of the cells kernel
-    grid_dependents_may_launch();
     // around the Vx face (ix + 1, iy + 1) and the Vy face (ix + 1, iy + 1)
     T xr, xl, yu, yd, s00, s01, s10, p01, p11, p10, vx, vy;
     xr = xl = yu = yd = s00 = s01 = s10 = p01 = p11 = p10 = vx = vy = (T)0;

@@ -345,7 +345,6 @@ __global__ void __launch_bounds__(256, s3_blocks<T>()) s3_cells(S3A<T> a, S3P<T>
     const I nx = (I)a.nx, ny = (I)a.ny, nz = (I)a.nz;
     const I x = (I)(blockIdx.x * 32 + threadIdx.x), y = (I)(blockIdx.y * 8 + threadIdx.y), z = (I)blockIdx.z;
     grid_dependency_wait();  // the state is read with plain loads: __ldg need not see the kernel before
-    grid_dependents_may_launch();
     if (x >= nx || y >= ny) return;
     const bool x1 = x < nx - 1, y1 = y < ny - 1, z1 = z < nz - 1;  // an edge at the upper x / y / z side exists
     const bool ix = x >= 1 && x1, iy = y >= 1 && y1, iz = z >= 1 && z1;
@@ -406,7 +405,6 @@ __global__ void __launch_bounds__(256, s3_blocks<T>()) s3_faces(S3A<T> a, S3P<T>
     const I nx = (I)a.nx, ny = (I)a.ny, nz = (I)a.nz;
     const I x = (I)(blockIdx.x * 32 + threadIdx.x), y = (I)(blockIdx.y * 8 + threadIdx.y), z = (I)blockIdx.z;
     grid_dependency_wait();
-    grid_dependents_may_launch();
     if (x > nx || y > ny) return;
     const bool ix = x >= 1 && x <= nx - 2, iy = y >= 1 && y <= ny - 2, iz = z >= 1 && z <= nz - 2;
     // the faces with a residual: Vx, Vy, Vz (their low x, y, z sides of the cell)
