@@ -1398,6 +1398,22 @@ __global__ void grid_misfit_kernel(double* mu, const double* Tn,
     if ((threadIdx.x & 31) == 0) atomicAdd(loss, s);
 }
 
+// The six faces of the state `from` copied into the `count` states that lie `stride` values apart from `to`
+// (a step writes inner cells only, so a buffer's faces are set once). blockIdx.z: the buffer.
+__global__ void __launch_bounds__(256) grid_faces_copy_kernel(const float2* __restrict__ from, float2* __restrict__ to,
+                                                             int64_t stride, int64_t nx, int64_t ny, int64_t nz) {
+    float2* out = to + stride * blockIdx.z;
+    const int f = blockIdx.y;  // 0,1: z faces; 2,3: y faces; 4,5: x faces
+    const int64_t n0 = f < 4 ? nx : ny, n1 = f < 2 ? ny : nz;
+    const int64_t fixed = (f & 1) ? (f < 2 ? nz : f < 4 ? ny : nx) - 1 : 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n0 * n1; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t v = i / n0, u = i - v * n0;
+        const int64_t ix = f < 4 ? u : fixed, iy = f < 2 ? v : f < 4 ? fixed : u, iz = f < 2 ? fixed : v;
+        const int64_t o = ix + nx * (iy + ny * iz);
+        out[o] = from[o];
+    }
+}
+
 int grid_misfit_gradient(const ps_array& T0, const ps_array& Tobs, const ps_array& Ci, const ps_array& lam, double dt,
                          double hx, double hy, double hz, int64_t nt, int64_t ce, const ps_array& glam,
                          const ps_array& T_final, double* loss, int64_t* recomputed, bool* redo, cudaStream_t s) {
@@ -1407,7 +1423,7 @@ int grid_misfit_gradient(const ps_array& T0, const ps_array& Tobs, const ps_arra
     *recomputed = 0;
     const int64_t n = numel(T0), n2 = n / 2, nseg = (nt + ce - 1) / ce;
     const size_t bytes = (size_t)n * 8, stride = (bytes + 255) / 256 * 256;
-    const int64_t nbuf = 7 + nseg + ce;  // Cs, Ls, fA, fB, μA, μB, μ64, checkpoints, segment states
+    const int64_t nbuf = 7 + nseg + ce;  // Cs, Ls, μA, μB, μ64, fA, fB, checkpoints, segment states
     if (stride * nbuf + 512 > g_grad_bytes) {
         if (g_grad_scratch) cudaFree(g_grad_scratch);
         g_grad_scratch = nullptr;
@@ -1428,7 +1444,7 @@ int grid_misfit_gradient(const ps_array& T0, const ps_array& Tobs, const ps_arra
         a.ptr = scr + 512 + stride * b;
         return a;
     };
-    ps_array Cs = arr(0), Ls = arr(1), fA = arr(2), fB = arr(3), mA = arr(4), mB = arr(5), mu64 = arr(6);
+    ps_array Cs = arr(0), Ls = arr(1), mA = arr(2), mB = arr(3), mu64 = arr(4), fA = arr(5), fB = arr(6);
     auto ckpt = [&](int64_t i) { return arr(7 + i); };
     auto seg = [&](int64_t j) { return arr(7 + nseg + j); };
     SplitParams p{};
@@ -1450,20 +1466,33 @@ int grid_misfit_gradient(const ps_array& T0, const ps_array& Tobs, const ps_arra
     absmax2_bits_kernel<<<st->num_sms * 4, 256, 0, s>>>(static_cast<const double2*>(T0.ptr),
                                                         static_cast<const double2*>(lam.ptr), n2, &r->maxT, &r->maxL);
     grid_setup_kernel<<<1, 1, 0, s>>>(r, G, 1);
-    to_grid_kernel<<<g, 256, 0, s>>>(static_cast<const double2*>(T0.ptr), static_cast<float4*>(fA.ptr), n2, r, 0);
+    to_grid_kernel<<<g, 256, 0, s>>>(static_cast<const double2*>(T0.ptr), static_cast<float4*>(fB.ptr), n2, r, 0);
     to_grid_kernel<<<g, 256, 0, s>>>(static_cast<const double2*>(lam.ptr), static_cast<float4*>(Ls.ptr), n2, r, 1);
     ci_grid_kernel<<<g, 256, 0, s>>>(static_cast<const double2*>(Ci.ptr), static_cast<float4*>(Cs.ptr), n2, r);
-    // every state buffer holds T0's boundary values (the steps write inner cells only)
-    PS_TRY(copy(fB, fA));
-    for (int64_t j = 1; j < ce && j < nt; j++) PS_TRY(copy(seg(j), fA));
-    // forward with checkpoints
+    // every state buffer holds T0's boundary values (the steps write inner cells only): fA, and the checkpoints and
+    // segment states behind fB, where T0 itself is
+    PS_TRY(copy(ckpt(0), fB));
+    const int64_t nmax = std::max(T0.n[0] * T0.n[1], std::max(T0.n[0] * T0.n[2], T0.n[1] * T0.n[2]));
+    const unsigned gf = (unsigned)std::min<int64_t>((nmax + 255) / 256, 64);
+    auto faces = [&](const ps_array& first, int64_t count) {  // grid.z <= 65535 per launch
+        for (int64_t i = 0; i < count; i += 32768)
+            grid_faces_copy_kernel<<<dim3(gf, 6, (unsigned)std::min<int64_t>(32768, count - i)), 256, 0, s>>>(
+                static_cast<const float2*>(fB.ptr), reinterpret_cast<float2*>(static_cast<char*>(first.ptr) + stride * i),
+                (int64_t)(stride / 8), T0.n[0], T0.n[1], T0.n[2]);
+    };
+    faces(fA, 1);
+    if (nseg > 1) faces(ckpt(1), nseg - 1);
+    if (std::min(ce, nt) > 1) faces(seg(1), std::min(ce, nt) - 1);
+    // forward; a step that reaches a checkpoint writes its state there
+    ps_array cur = ckpt(0);
     for (int64_t it = 0; it < nt; it++) {
-        if (it % ce == 0) PS_TRY(copy(ckpt(it / ce), fA));
-        PS_TRY(step(fA, fB));
-        std::swap(fA, fB);
+        const bool at_ckpt = (it + 1) % ce == 0 && it + 1 < nt;
+        const ps_array next = at_ckpt ? ckpt((it + 1) / ce) : cur.ptr == fA.ptr ? fB : fA;
+        PS_TRY(step(cur, next));
+        cur = next;
     }
     // T_nt in FP64, the misfit, μ_nt on its own grid
-    grid_state_to_f64_kernel<<<g, 256, 0, s>>>(static_cast<const float2*>(fA.ptr), static_cast<double*>(mu64.ptr), n, r);
+    grid_state_to_f64_kernel<<<g, 256, 0, s>>>(static_cast<const float2*>(cur.ptr), static_cast<double*>(mu64.ptr), n, r);
     if (T_final.ptr) PS_TRY(copy(T_final, mu64));
     grid_misfit_kernel<<<g, 256, 0, s>>>(static_cast<double*>(mu64.ptr), static_cast<const double*>(mu64.ptr),
                                          static_cast<const double*>(Tobs.ptr), static_cast<const double*>(Ci.ptr), dt,
@@ -1481,15 +1510,15 @@ int grid_misfit_gradient(const ps_array& T0, const ps_array& Tobs, const ps_arra
     // reverse sweep over the segments
     for (int64_t sidx = nseg - 1; sidx >= 0; sidx--) {
         const int64_t n0 = sidx * ce, n1 = std::min(nt, n0 + ce);
-        PS_TRY(copy(seg(0), ckpt(sidx)));
+        auto state = [&](int64_t j) { return j == 0 ? ckpt(sidx) : seg(j); };
         for (int64_t j = 1; j < n1 - n0; j++) {
-            PS_TRY(step(seg(j - 1), seg(j)));
+            PS_TRY(step(state(j - 1), state(j)));
             (*recomputed)++;
         }
         for (int64_t nn = n1 - 1; nn >= n0; nn--) {
             // glam from μ_{nn+1} and T_nn, and μ_nn, in one sweep
-            PS_TRY(iso ? launch_grid_adj<true>(mA, Ls, Cs, seg(nn - n0), mB, glam, p, c, cells, s, st->d_err, r, rm)
-                       : launch_grid_adj<false>(mA, Ls, Cs, seg(nn - n0), mB, glam, p, c, cells, s, st->d_err, r,
+            PS_TRY(iso ? launch_grid_adj<true>(mA, Ls, Cs, state(nn - n0), mB, glam, p, c, cells, s, st->d_err, r, rm)
+                       : launch_grid_adj<false>(mA, Ls, Cs, state(nn - n0), mB, glam, p, c, cells, s, st->d_err, r,
                                                 rm));
             std::swap(mA, mB);
         }
