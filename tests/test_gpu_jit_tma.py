@@ -109,3 +109,45 @@ def test_tma_sweep_falls_back_for_unaligned_arrays(ps):
     ref = _run(ps, k, "HEAT_LAP", ins, outs, sc, np.float64, memopt=False)
     assert not _used_tma(k)
     assert np.array_equal(got[0], ref[0])
+
+
+# reads the array it writes, beside staged ones: evaluated only where the statement runs
+_ACCUMULATE = """@parallel function accumulate!(A, S, B, c)
+    @inn(A) = @inn(A) + c*(@d2_xi(B) + @d2_yi(B) + @d2_zi(B))
+    @all(S) = @all(S) * c - @all(B)
+    return
+end"""
+
+
+@pytest.mark.parametrize("n", [(4, 3, 3), (36, 17, 4), (128, 8, 300), (132, 9, 5), (260, 31, 67)])
+def test_tma_sweep_ragged_tiles_and_written_arrays(ps, n):
+    """FP32 tiles of 128 x 8 cells, two rows per thread: extents one cell above and below them, thin arrays, sweeps of
+    one and several chunks (the default length and given ones), against one point per thread."""
+    rng = np.random.default_rng(n[0])
+    A, S, B = (rng.standard_normal(n).astype(np.float32) for _ in range(3))
+    k = ps.parallel_kernel(_ACCUMULATE)
+
+    def run(**kw):
+        a, s = _dev(ps, A), _dev(ps, S)
+        ps.parallel(k, a, s, _dev(ps, B), 0.3, **kw)
+        return ps.to_host(a), ps.to_host(s)
+    ref = run(memopt=False)
+    before = k.tma_launches
+    for kw in ({}, {"loopsize": 1}, {"loopsize": 7}):
+        for x, y in zip(run(**kw), ref):
+            assert np.array_equal(x, y), (n, kw)
+    assert k.tma_launches == before + 3
+
+
+@pytest.mark.parametrize("short", [0, 1, 2])
+def test_tma_sweep_reports_a_stencil_that_leaves_an_array(ps, short):
+    """One array is shorter along one dimension than the cells that read it."""
+    from ps_gb300._lib import PSError
+
+    n = [132, 20, 40]
+    m = list(n)
+    m[short] -= 4 if short == 0 else 1
+    k = ps.parallel_kernel(_ACCUMULATE)
+    a = [ps.zeros(*n, dtype=np.float32), ps.zeros(*n, dtype=np.float32), ps.zeros(*m, dtype=np.float32)]
+    with pytest.raises(PSError, match="ps_jit_launch_tma.*BoundsError"):
+        ps.parallel(k, *a, 0.3)
