@@ -861,7 +861,7 @@ def bench_ad(ps, torch, n=256):
         out[tag] = row
         del T, lam, Ci, T2, T2b, Tb, lamb
     torch.cuda.empty_cache()
-    out["config"] = (f"{n}^3, flux form with a conductivity array run-time compiled, one point per thread; "
+    out["config"] = (f"{n}^3, flux form with a conductivity array run-time compiled, FP64 one point per thread, FP32 as a sweep; "
                      "events around 10 launches after 3 warm-up launches")
     out["launches"] = launches
     return out

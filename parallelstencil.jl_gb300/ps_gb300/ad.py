@@ -1043,8 +1043,8 @@ def _sweep_handle(kernel, ndims, dt, order, descs, lo, cnt):
 def parallel_grad(kernel: JitKernel, args, grad, ad_mode="reverse", ranges=None, stream=None, sync=True,
                   nblocks=None, nthreads=None):
     """`@parallel ∇=(A->Ā, ...) [ad_mode=...] kernel!(args...)` for a run-time compiled kernel:
-    launches the derivative kernel over the kernel's own grid (or `ranges` / nblocks .* nthreads),
-    one point per thread. Shadows are arrays of the primals' shapes and number type."""
+    launches the derivative kernel over the kernel's own grid (or `ranges` / nblocks .* nthreads), one
+    point per thread, or as a sweep (_AdSweepGen) in FP32 reverse mode. Shadows are arrays of the primals' shapes and number type."""
     require_initialized()
     if not isinstance(kernel, JitKernel):
         raise ArgumentError("∇ applies to run-time compiled kernels (ps_gb300.parallel_kernel)")

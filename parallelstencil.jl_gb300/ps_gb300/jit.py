@@ -1604,7 +1604,8 @@ class JitKernel:
         `memopt=`, else true) runs 2-D and 3-D `@parallel` kernels as sweeps along the last
         dimension (src/memopt.jl, loopdim 2 and 3) of `loopsize` indices per thread -- by default
         64, as src/parallel.jl:532-543 for compute capability >= 9, halved (down to 2) while the
-        launch would have fewer threads than the GPU holds at once -- with the same results.
+        launch would have fewer threads than the GPU holds at once; TMA sweeps: see sweep_chunk -- with the
+        same results.
         fp64="split" evaluates the arithmetic of FP64 kernels on FP32 pairs (each operation within
         ~2^-46 of its operands' magnitude; GB300 issues FP32 at 64x the FP64 rate)."""
         h, A, nA, S, nS, lo, cnt, threads, shmem, loop, layout = self._config(args, ranges, nblocks, nthreads, shmem,
