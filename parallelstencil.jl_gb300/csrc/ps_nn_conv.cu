@@ -21,7 +21,7 @@
 //
 // Bound: L2 -> shared memory, and for the small layers the chain of launch, loads and MMAs. 8 images of 256^2, GPU
 // time of a layer: the 64-channel layers at a quarter of the size 10 to 16 us, the 128- and 256-channel
-// ones 7 to 19 us. The whole forward pass: 7.52 ms through column matrices, 0.29 ms now.
+// ones 7 to 19 us. The whole forward pass: 7.52 ms through column matrices, 0.26 ms now.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -242,15 +242,22 @@ static int conv3_launch(const ConvGeom& g, const void* x, const void* wgt, const
 // eight; a row's newest output starts with an MMA of its own that does not accumulate.
 // With `last` the 1x1 output layer is computed from the row's rounded activations in the same epilogue.
 // 8 images of 256^2: 32 -> 32 channels 21 us (31 in tiles of nn_conv3_k), 96 -> 32 43 us (75), 32 -> 32 with the
-// output layer 25 us (39, and 15 by itself). Bound by the 64-byte rows of its TMA boxes and the per-row chain of
-// load, MMAs and epilogue, not by a pipe.
+// output layer 25 us (39, and 15 by itself). Bound with 96 channels by the MMAs' operand reads (7 KB of shared
+// memory per 128 x 96 x 16, about 110 cycles), with 32 by the per-row chain of load, MMAs and epilogue.
 constexpr int kAccs = 8;  // accumulators of 32 columns: two CTAs fill the SM's 512
-template <int CB>
+//
+// UB > 0: the first UB blocks of 32 channels are a quarter-size layer's, upsampled to the nearest, which nobody
+// has written out: four more warps copy its row once for every four input rows into two buffers in turn, each
+// pixel to its four (the layout is the one TMA would store); RB blocks come by TMA. The layer over the
+// largest concatenation (64 + 32 channels) so takes 45 us by itself, instead of 28 to write its input and 43.
+template <int RB, int UB>
 struct RowsCfg {
+    static constexpr int CB = RB + UB, THREADS = UB ? 320 : 192;
     static constexpr int ABOX = (kConvM + 2) * 64, ABYTES = (ABOX + 1023) / 1024 * 1024;
     static constexpr int WBYTES = 3 * CB * 3 * 32 * 64;  // [kx][cb][ky][32 outputs] rows of 64 bytes
-    static constexpr int S = CB == 1 ? 8 : 5;
-    static constexpr int SMEM = WBYTES + S * ABYTES + 1024 + 1024;
+    static constexpr int S = UB ? 2 : RB == 1 ? 8 : 5;
+    static constexpr int UBYTES = 2 * UB * ABYTES;
+    static constexpr int SMEM = WBYTES + S * ABYTES + UBYTES + 1024 + 1024;
     static_assert(SMEM > 77 * 1024 && SMEM < 113 * 1024, "two CTAs per SM");
 };
 struct RowsGeom {
@@ -264,20 +271,23 @@ struct LastLayer {  // y[p][0..2] = W a[p] + b over the 32 channels; y NULL: non
     float* y;
 };
 
-template <int CB>
-__global__ void __launch_bounds__(192, 2)
+template <int RB, int UB>
+__global__ void __launch_bounds__(RowsCfg<RB, UB>::THREADS, 2)
     nn_conv3_rows_k(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB, RowsGeom g,
-                    const float* __restrict__ bias, int relu, __nv_bfloat16* __restrict__ y, LastLayer last,
-                    int* __restrict__ err) {
-    using C = RowsCfg<CB>;
-    constexpr int S = C::S, CIN = 32 * CB;
+                    const uint4* __restrict__ low, const float* __restrict__ bias, int relu, __nv_bfloat16* __restrict__ y,
+                    LastLayer last, int* __restrict__ err) {
+    using C = RowsCfg<RB, UB>;
+    constexpr int S = C::S, CB = C::CB, CIN = 32 * CB;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem =
         reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* ring = smem + C::WBYTES;
-    uint64_t* full = reinterpret_cast<uint64_t*>(ring + S * C::ABYTES);
+    unsigned char* ups = ring + S * C::ABYTES;  // [2][UB] blocks of upsampled pixels
+    uint64_t* full = reinterpret_cast<uint64_t*>(ups + C::UBYTES);
     uint64_t* empty = full + S;
-    uint64_t* wfull = empty + S;        // the weights have arrived
+    uint64_t* ufull = empty + S;        // [2] a row of upsampled pixels has been written
+    uint64_t* uempty = ufull + 2;       // [2] and read by its last MMAs
+    uint64_t* wfull = uempty + 2;       // the weights have arrived
     uint64_t* afull = wfull + 1;        // [kAccs] an output row's MMAs have completed
     uint64_t* aempty = afull + kAccs;   // [kAccs] its accumulator has been read
     uint64_t* done = aempty + kAccs;
@@ -292,6 +302,10 @@ __global__ void __launch_bounds__(192, 2)
         for (int s = 0; s < S; s++) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
+        }
+        for (int u = 0; u < 2; u++) {
+            mbar_init(&ufull[u], 128);
+            mbar_init(&uempty[u], 1);
         }
         mbar_init(wfull, 1);
         for (int a = 0; a < kAccs; a++) {
@@ -333,7 +347,7 @@ __global__ void __launch_bounds__(192, 2)
         for (int t = blockIdx.x; t < g.jobs && ok; t += gridDim.x) {
             job(t, &x0, &b, &o0, &o1);
             for (int r = o0 - 1; r <= o1 && ok; r++)  // (rows outside the image arrive as zeros)
-                for (int cb = 0; cb < CB; cb++, it++) {
+                for (int cb = 0; cb < RB; cb++, it++) {
                     const int s = it % S;
                     if (it >= S && !mbar_wait_bounded(&empty[s], ((it / S) - 1) & 1)) {
                         ok = false;
@@ -347,10 +361,12 @@ __global__ void __launch_bounds__(192, 2)
         if (!ok) atomicOr(err, DEV_ERR_TMA_TIMEOUT);
     } else if (threadIdx.x == 32) {  // MMA issuer
         int it = 0, n = 0;           // n: sequence number of the CTA's output row o0
+        int ug = 0;                  // upsampled rows taken
         bool ok = mbar_wait_bounded(wfull, 0);
         const uint64_t wdesc = umma_desc_sw64(smem_u32(smem));
         for (int t = blockIdx.x; t < g.jobs && ok; t += gridDim.x) {
             job(t, &x0, &b, &o0, &o1);
+            int row4 = -1;  // the upsampled row in use
             for (int r = o0 - 1; r <= o1 && ok; r++) {
                 const int lo = max(r - 1, o0), hi = min(r + 1, o1 - 1);
                 const bool fresh = hi == r + 1;  // this row starts the accumulator of output row r + 1
@@ -367,20 +383,30 @@ __global__ void __launch_bounds__(192, 2)
                 const uint32_t d0 = tmem + slot * 32, d1 = tmem;
                 const uint64_t b0 = wdesc + (uint64_t)(((lo - r + 1) * 2048) >> 4), b1 = b0 + (uint64_t)((len0 * 2048) >> 4);
                 const uint32_t i0 = umma_idesc_bf16(kConvM, 32 * len0), i1 = umma_idesc_bf16(kConvM, 32 * (len - len0));
-                for (int cb = 0; cb < CB && ok; cb++) ok = mbar_wait_bounded(&full[(it + cb) % S], ((it + cb) / S) & 1);
+                const bool image = r >= 0 && r < g.H;
+                if (UB && image && r / 4 != row4) {
+                    if (row4 >= 0) tc_commit(&uempty[(ug - 1) & 1]);  // arrives when the MMAs on it have completed
+                    row4 = r / 4;
+                    ok = mbar_wait_bounded(&ufull[ug & 1], (ug >> 1) & 1);
+                    ug++;
+                }
+                for (int cb = 0; cb < RB && ok; cb++) ok = mbar_wait_bounded(&full[(it + cb) % S], ((it + cb) / S) & 1);
                 if (!ok) break;
                 tc_fence_after();
+                const int cb0 = UB && !image ? UB : 0;  // zeros above and below the image: the ring's block alone
                 // (kernel column, channel block, 16 channels): each output's sum runs over taps, then channels
 #pragma unroll
                 for (int kx = 0; kx < 3; kx++)
-                    for (int cb = 0; cb < CB; cb++) {
-                        const int s = (it + cb) % S;
-                        const uint64_t a0 = umma_desc_sw64(smem_u32(ring + s * C::ABYTES)) + kx * 4;
+                    for (int cb = cb0; cb < CB; cb++) {
+                        const int s = (it + cb - UB) % S;
+                        const uint64_t a0 =
+                            umma_desc_sw64(smem_u32(cb < UB ? ups + ((ug - 1 & 1) * UB + cb) * C::ABYTES : ring + s * C::ABYTES)) +
+                            kx * 4;
                         const uint64_t w = (uint64_t)(((kx * CB + cb) * 3 * 2048) >> 4);
 #pragma unroll
                         for (int k = 0; k < 2; k++) {  // K = 16 per MMA
                             const uint64_t da = a0 + 2 * k, wk = w + 2 * k;
-                            if (fresh && cb == 0 && kx == 0 && k == 0) {
+                            if (fresh && cb == cb0 && kx == 0 && k == 0) {
                                 // the new row's accumulator is set, the others (one or two, maybe wrapping) added to
                                 const uint32_t one = umma_idesc_bf16(kConvM, 32);
                                 for (int a = lo; a <= r; a++)
@@ -391,16 +417,44 @@ __global__ void __launch_bounds__(192, 2)
                                 if (len > len0) tc_mma(d1, da, b1 + wk, i1, 1u);
                             }
                         }
-                        if (kx == 2) tc_commit(&empty[s]);  // this block has been read by its last MMAs
+                        if (kx == 2 && cb >= UB) tc_commit(&empty[s]);  // this block has been read by its last MMAs
                     }
-                it += CB;
+                it += RB;
                 if (ok && r - 1 >= o0) tc_commit(&afull[(n + r - 1 - o0) % kAccs]);  // output row r - 1 is complete
             }
+            if (UB && row4 >= 0) tc_commit(&uempty[(ug - 1) & 1]);
             n += o1 - o0;
         }
         counts[1] = it;
         if (!ok) atomicOr(err, DEV_ERR_TMA_TIMEOUT);
         tc_commit(done);  // arrives when every MMA issued above has completed
+    } else if (UB && warp >= 6) {  // upsampled pixels: 34 of a low row, 16 bytes of one at a time
+        const int u0 = threadIdx.x - 192, lw = g.W / 4;
+        int n = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < g.jobs && ok; t += gridDim.x) {
+            job(t, &x0, &b, &o0, &o1);
+            const int last4 = min(g.H - 1, o1) / 4;
+            for (int r4 = max(0, o0 - 1) / 4; r4 <= last4; r4++, n++) {
+                if (n >= 2 && !mbar_wait_bounded(&uempty[n & 1], ((n >> 1) - 1) & 1)) {
+                    ok = false;
+                    break;
+                }
+                unsigned char* buf = ups + (n & 1) * UB * C::ABYTES;
+                const uint4* src = low + ((int64_t)b * (g.H / 4) + r4) * lw * (UB * 4);
+                for (int i = u0; i < 34 * UB * 4; i += 128) {
+                    const int j = i / (UB * 4), c = i % (UB * 4), lx = x0 / 4 - 1 + j;
+                    uint4 v = make_uint4(0, 0, 0, 0);
+                    if (lx >= 0 && lx < lw) v = src[lx * (UB * 4) + c];
+                    const int p0 = j == 0 ? 0 : 4 * j - 3, p1 = j == 0 || j == 33 ? p0 : p0 + 3;
+                    for (int p = p0; p <= p1; p++)
+                        *reinterpret_cast<uint4*>(buf + (c >> 2) * C::ABYTES + p * 64 + (((c ^ (p >> 1)) & 3) << 4)) = v;
+                }
+                fence_proxy_async_smem();  // the MMAs read what these threads wrote
+                mbar_arrive1(&ufull[n & 1]);
+            }
+        }
+        if (!ok && lane == 0) atomicOr(err, DEV_ERR_TMA_TIMEOUT);
     } else if (warp >= 2) {  // epilogue: warp w reads TMEM lanes (pixels of the row) 32 (w % 4) .. + 31
         const int q = warp & 3;
         const float low = relu ? 0.0f : -INFINITY;
@@ -468,22 +522,22 @@ __global__ void __launch_bounds__(192, 2)
     if (warp == 0) tc_dealloc(tmem, kAccs * 32);
 }
 
-template <int CB>
-static int conv3_rows_launch(const RowsGeom& g, const void* x, const void* wgt, const float* bias, int relu, void* y,
-                             const LastLayer& last, int sms, cudaStream_t s, int* d_err) {
-    using C = RowsCfg<CB>;
+template <int RB, int UB>
+static int conv3_rows_launch(const RowsGeom& g, const void* x, const void* low, const void* wgt, const float* bias, int relu,
+                             void* y, const LastLayer& last, int sms, cudaStream_t s, int* d_err) {
+    using C = RowsCfg<RB, UB>;
     CUtensorMap mA, mB;
-    const uint64_t da[4] = {32 * CB, (uint64_t)g.W, (uint64_t)g.H, (uint64_t)g.B};
+    const uint64_t da[4] = {32 * RB, (uint64_t)g.W, (uint64_t)g.H, (uint64_t)g.B};
     const uint32_t ba[4] = {32, kConvM + 2, 1, 1};
-    const uint64_t db[2] = {32 * CB * 9, 32};
+    const uint64_t db[2] = {32 * C::CB * 9, 32};
     const uint32_t b2[2] = {32, 32};
     PS_TRY(encode_bf16_box(&mA, x, 4, da, ba));
     PS_TRY(encode_bf16_box(&mB, wgt, 2, db, b2));
-    const auto kernel = nn_conv3_rows_k<CB>;
+    const auto kernel = nn_conv3_rows_k<RB, UB>;
     // every launch sets it: the attribute belongs to the device's current context
     PS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-    PS_CUDA_TRY(launch_dependent(kernel, dim3((unsigned)std::min(g.jobs, 2 * sms)), dim3(192), (size_t)C::SMEM, s, mA, mB,
-                                 g, bias, relu, static_cast<__nv_bfloat16*>(y), last, d_err));
+    PS_CUDA_TRY(launch_dependent(kernel, dim3((unsigned)std::min(g.jobs, 2 * sms)), dim3(C::THREADS), (size_t)C::SMEM, s, mA, mB,
+                                 g, static_cast<const uint4*>(low), bias, relu, static_cast<__nv_bfloat16*>(y), last, d_err));
     return PS_OK;
 }
 
@@ -594,14 +648,15 @@ static bool whole_rows(int W) {
 
 // The layer by rows (see above), with the 1x1 output layer after it; *taken = false (and nothing launched) where
 // it does not apply: other channel counts, narrow images, or too few rows for the walk (with 4 per CTA the
-// input is read 1.5 times; below that the tiles of nn_conv3_k read no more).
-int nn_conv3_rows(const void* x, int B, int H, int W, int cin, const void* wgt, int cout, const float* bias, int relu,
-                  void* y, const void* wlast, int kpad_last, const float* blast, float* ylast, bool* taken,
+// input is read 1.5 times; below that the tiles of nn_conv3_k read no more). low (or NULL): 64 channels of a
+// quarter-size layer that come upsampled before x's 32.
+int nn_conv3_rows(const void* x, const void* low, int B, int H, int W, int cin, const void* wgt, int cout, const float* bias,
+                  int relu, void* y, const void* wlast, int kpad_last, const float* blast, float* ylast, bool* taken,
                   cudaStream_t s, int* d_err) {
     *taken = false;
     DeviceState* st = nullptr;
     PS_TRY(current_state(&st));
-    if (cout != 32 || (cin != 32 && cin != 96) || !whole_rows(W)) return PS_OK;
+    if (cout != 32 || cin != (low ? 96 : 32) || !whole_rows(W) || (low && (H % 4 || W % 4))) return PS_OK;
     const int64_t tx = (W + kConvM - 1) / kConvM, strips = tx * B, ctas = 2 * (int64_t)st->num_sms;
     if (strips * H < 4 * ctas || strips * H > 0x7FFFFFFF - 65536) return PS_OK;
     RowsGeom g{};
@@ -615,8 +670,8 @@ int nn_conv3_rows(const void* x, int B, int H, int W, int cin, const void* wgt, 
     g.jobs = (int)(strips * g.chunks);
     const LastLayer last{static_cast<const __nv_bfloat16*>(wlast), kpad_last, blast, ylast};
     *taken = true;
-    return cin == 32 ? conv3_rows_launch<1>(g, x, wgt, bias, relu, y, last, st->num_sms, s, d_err)
-                     : conv3_rows_launch<3>(g, x, wgt, bias, relu, y, last, st->num_sms, s, d_err);
+    return low ? conv3_rows_launch<1, 2>(g, x, low, wgt, bias, relu, y, last, st->num_sms, s, d_err)
+               : conv3_rows_launch<1, 0>(g, x, nullptr, wgt, bias, relu, y, last, st->num_sms, s, d_err);
 }
 
 int nn_conv3_tc(const void* x, int B, int H, int W, int cin, const void* wgt, int cout, const float* bias, int relu,

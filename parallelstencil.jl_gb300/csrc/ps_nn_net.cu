@@ -374,6 +374,7 @@ struct NNet {
     float scales[8] = {0, 1, 0, 1, 1, 1, 1, 0};  // input offset/scale (2 channels), output scales (3)
     // activations (bf16) and their gradients (FP32)
     bf16 *x0, *a[15], *p1, *p2, *p3, *k2, *k1, *k0;
+    bool k0_whole = false;  // k0 holds the last forward pass's concatenation
     float *y, *ga[15], *gp1, *gp2, *gp3, *gk2, *gk1, *gk0;
     // scratch
     bf16 *colT, *dz, *dzT;
@@ -522,7 +523,7 @@ static int nn_conv_fwd(NNet* n, Conv& L, const bf16* x, int B, int h, int w, voi
     const int64_t P = (int64_t)B * h * w;
     if (L.k == 3 && L.cin % 32 == 0) {
         bool taken = false;
-        PS_TRY(nn_conv3_rows(x, B, h, w, L.cin, L.W, L.cout, L.b, L.relu, y, next ? next->W : nullptr,
+        PS_TRY(nn_conv3_rows(x, nullptr, B, h, w, L.cin, L.W, L.cout, L.b, L.relu, y, next ? next->W : nullptr,
                              next ? (int)next->kpad : 0, next ? next->b : nullptr, ynext, &taken, s, err));
         if (fused) *fused = taken;
         if (taken) return PS_OK;
@@ -595,6 +596,14 @@ static int nn_input(const float* x, int64_t count, bf16* x0, cudaStream_t s) {
     return PS_OK;
 }
 
+// k = low upsampled to level lev, and skip beside it
+static cudaError_t nn_upcat(const NNet* n, int B, const bf16* low, int Cl, const bf16* skip, int Cs, int lev, bf16* k,
+                            cudaStream_t s) {
+    const int groups = B * nn_level_H(n, lev + 1), W = nn_level_W(n, lev);
+    return launch_dependent(nn_upcat_k, dim3((unsigned)std::min(groups, 1 << 20), (unsigned)((W * ((Cl + Cs) / 8) + 255) / 256)),
+                            dim3(256), 0, s, low, Cl / 8, skip, Cs / 8, groups, W, n->pf, k);
+}
+
 static int nn_forward(NNet* n, int B, cudaStream_t s, int* err) {
     const int c = n->base, f = n->pf;
     auto& L = n->conv;
@@ -607,9 +616,7 @@ static int nn_forward(NNet* n, int B, cudaStream_t s, int* err) {
                                 0, s, x, B * h, h, w, C / 8, f, y);
     };
     auto upcat = [&](const bf16* low, int Cl, const bf16* skip, int Cs, int lev, bf16* k) {
-        const int groups = B * nn_level_H(n, lev + 1), W = nn_level_W(n, lev);
-        return launch_dependent(nn_upcat_k, dim3((unsigned)std::min(groups, 1 << 20), (unsigned)((W * ((Cl + Cs) / 8) + 255) / 256)),
-                                dim3(256), 0, s, low, Cl / 8, skip, Cs / 8, groups, W, f, k);
+        return nn_upcat(n, B, low, Cl, skip, Cs, lev, k, s);
     };
     PS_TRY(cv(0, n->x0, 0, n->a[0]));
     PS_TRY(cv(1, n->a[0], 0, n->a[1]));
@@ -628,8 +635,16 @@ static int nn_forward(NNet* n, int B, cudaStream_t s, int* err) {
     PS_CUDA_TRY(upcat(n->a[9], 4 * c, n->a[3], 2 * c, 1, n->k1));
     PS_TRY(cv(10, n->k1, 1, n->a[10]));
     PS_TRY(cv(11, n->a[10], 1, n->a[11]));
-    PS_CUDA_TRY(upcat(n->a[11], 2 * c, n->a[1], c, 0, n->k0));
-    PS_TRY(cv(12, n->k0, 0, n->a[12]));
+    // the largest concatenation: read where its parts lie, and written out by the backward pass, which needs it whole
+    bool apart = false;
+    if (f == 4 && c == 32)
+        PS_TRY(nn_conv3_rows(n->a[1], n->a[11], B, n->H, n->W, L[12].cin, L[12].W, L[12].cout, L[12].b, L[12].relu, n->a[12],
+                             nullptr, 0, nullptr, nullptr, &apart, s, err));
+    n->k0_whole = !apart;
+    if (!apart) {
+        PS_CUDA_TRY(upcat(n->a[11], 2 * c, n->a[1], c, 0, n->k0));
+        PS_TRY(cv(12, n->k0, 0, n->a[12]));
+    }
     bool fused = false;
     PS_TRY(nn_conv_fwd(n, L[13], n->a[12], B, n->H, n->W, n->a[13], s, err, &L[14], n->y, &fused));
     if (!fused) PS_TRY(cv(14, n->a[13], 0, n->y));
@@ -657,6 +672,8 @@ static int nn_backward(NNet* n, const float* dy, cudaStream_t s, int* err) {
     };
     PS_TRY(bw(14, n->a[13], nullptr, dy, 3, 0, n->ga[13], 0));
     PS_TRY(bw(13, n->a[12], n->a[13], n->ga[13], c, 0, n->ga[12], 0));
+    if (!n->k0_whole) PS_CUDA_TRY(nn_upcat(n, B, n->a[11], 2 * c, n->a[1], c, 0, n->k0, s));
+    n->k0_whole = true;
     PS_TRY(bw(12, n->k0, n->a[12], n->ga[12], c, 0, n->gk0, 0));
     catbwd(n->gk0, 2 * c, c, 0, n->ga[11], n->ga[1]);
     PS_TRY(bw(11, n->a[10], n->a[11], n->ga[11], 2 * c, 1, n->ga[10], 0));
