@@ -374,7 +374,7 @@ struct NNet {
     float scales[8] = {0, 1, 0, 1, 1, 1, 1, 0};  // input offset/scale (2 channels), output scales (3)
     // activations (bf16) and their gradients (FP32)
     bf16 *x0, *a[15], *p1, *p2, *p3, *k2, *k1, *k0;
-    bool k0_whole = false;  // k0 holds the last forward pass's concatenation
+    int k0_images = 0;  // the first so many images of k0 hold the concatenation of a[11] and a[1]
     float *y, *ga[15], *gp1, *gp2, *gp3, *gk2, *gk1, *gk0;
     // scratch
     bf16 *colT, *dz, *dzT;
@@ -640,7 +640,7 @@ static int nn_forward(NNet* n, int B, cudaStream_t s, int* err) {
     if (f == 4 && c == 32)
         PS_TRY(nn_conv3_rows(n->a[1], n->a[11], B, n->H, n->W, L[12].cin, L[12].W, L[12].cout, L[12].b, L[12].relu, n->a[12],
                              nullptr, 0, nullptr, nullptr, &apart, s, err));
-    n->k0_whole = !apart;
+    n->k0_images = apart ? 0 : std::max(n->k0_images, B);
     if (!apart) {
         PS_CUDA_TRY(upcat(n->a[11], 2 * c, n->a[1], c, 0, n->k0));
         PS_TRY(cv(12, n->k0, 0, n->a[12]));
@@ -672,8 +672,8 @@ static int nn_backward(NNet* n, const float* dy, cudaStream_t s, int* err) {
     };
     PS_TRY(bw(14, n->a[13], nullptr, dy, 3, 0, n->ga[13], 0));
     PS_TRY(bw(13, n->a[12], n->a[13], n->ga[13], c, 0, n->ga[12], 0));
-    if (!n->k0_whole) PS_CUDA_TRY(nn_upcat(n, B, n->a[11], 2 * c, n->a[1], c, 0, n->k0, s));
-    n->k0_whole = true;
+    if (n->k0_images < B) PS_CUDA_TRY(nn_upcat(n, B, n->a[11], 2 * c, n->a[1], c, 0, n->k0, s));
+    n->k0_images = std::max(n->k0_images, B);
     PS_TRY(bw(12, n->k0, n->a[12], n->ga[12], c, 0, n->gk0, 0));
     catbwd(n->gk0, 2 * c, c, 0, n->ga[11], n->ga[1]);
     PS_TRY(bw(11, n->a[10], n->a[11], n->ga[11], 2 * c, 1, n->ga[10], 0));

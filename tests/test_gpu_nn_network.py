@@ -154,3 +154,23 @@ def test_forward_over_tile_shapes(ps, H, W, B):
     odd = torch.empty(x.numel() + 1, device="cuda")[1:].view(x.shape)
     odd.copy_(x)
     assert np.array_equal(net.forward(odd).cpu().numpy(), y)
+
+
+def test_gradients_where_the_forward_pass_keeps_the_concatenation_apart(ps):
+    """Many large rows: the forward pass does not write the largest concatenation, the backward pass does. The same
+    images one at a time take the other path (too few rows): summed, their gradients are the batch's up to
+    FP32 summation order (<= 5e-3 per layer, the bound of test_network_gradients_per_layer's first part)."""
+    import torch
+
+    net, x = _setup(ps, 64, 256, 19, seed=6)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    dy = torch.randn(19, 64, 256, 3, device="cuda", generator=g)
+    net.zero_grad()
+    net.forward(x)
+    net.backward(dy)
+    whole = net.get_grads()
+    net.zero_grad()
+    for i in range(19):
+        net.forward(x[i:i + 1])
+        net.backward(dy[i:i + 1])
+    assert max(max(e) for e in _layer_errors(whole, net.get_grads())) <= 5e-3
