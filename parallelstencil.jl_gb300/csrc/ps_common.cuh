@@ -117,6 +117,10 @@ inline int auto_loopsize(int64_t cta_xy, int64_t wz, int64_t slots) {
     return best;
 }
 
+// Row blocks that one launch dimension holds. Kernels with blocks of few rows run taller grids in their
+// 64-bit variants, whose blocks have 8.
+constexpr int64_t kGridY = 65535;
+
 // CTAs of `kernel` resident per SM (queried once per kernel by the caller's static cache).
 template <typename K>
 inline int resident_ctas(K kernel, int threads, int smem) {

@@ -933,7 +933,7 @@ static int launch_grid_tile(const ps_array& Tin, const ps_array& Cs, const ps_ar
         L = pick.L;
         if constexpr (!OUT64 && !IN64 && TY == kGridRows) {
             const GridPick six = grid_pick(cb, kGridRowsMiddle, 4, st->num_sms);
-            if (six.cost < 1.02 * pick.cost)
+            if (six.cost < 1.02 * pick.cost && cb.hi[1] - cb.lo[1] <= 65535 * kGridRowsMiddle)
                 return launch_grid_tile<LAM, ISO, OUT64, IN64, kGridRowsMiddle>(Tin, Cs, Ls, T2, p, cb, 0, s, d_err, run, Lout, Cout);
         }
     }

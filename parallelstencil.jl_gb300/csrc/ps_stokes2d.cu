@@ -250,15 +250,15 @@ __device__ __forceinline__ double s2_half_sum(double a, double b, DivF<double> h
 
 // Rows of 32 threads per block. FP32: 8; FP64, bound by the FP64 pipe: 2, which spreads a small grid more
 // evenly over the SMs (4 rows -> 2: 255^2 11.4 -> 10.5 us per iteration, 130^2 6.9 -> 6.1, 1023^2 118 both).
-template <typename T>
+template <typename T, typename I>
 __host__ __device__ constexpr int s2_block_rows() {
-    return sizeof(T) == 4 ? 8 : 2;
+    return sizeof(T) == 4 || sizeof(I) == 8 ? 8 : 2;
 }
 
 template <typename T, bool DEFECT, typename I, bool STORE_TMP, bool RED>
-__global__ void __launch_bounds__(32 * s2_block_rows<T>()) s2_cells(S2Fused<T> a, S2P<T> p) {
+__global__ void __launch_bounds__(32 * s2_block_rows<T, I>()) s2_cells(S2Fused<T> a, S2P<T> p) {
     const I nx = (I)a.nx, ny = (I)a.ny;
-    const I i = (I)(blockIdx.x * 32 + threadIdx.x), j = (I)(blockIdx.y * s2_block_rows<T>() + threadIdx.y);
+    const I i = (I)(blockIdx.x * 32 + threadIdx.x), j = (I)(blockIdx.y * s2_block_rows<T, I>() + threadIdx.y);
     const I c = i + nx * j, cx = c + j;  // Vx rows have nx + 1 faces
     const bool cell = i < nx && j < ny, corner = i < nx - 1 && j < ny - 1;
     // what no iteration writes, while the kernel before this one still runs
@@ -313,9 +313,9 @@ __global__ void __launch_bounds__(32 * s2_block_rows<T>()) s2_cells(S2Fused<T> a
 }
 
 template <typename T, bool DEFECT, typename I, bool STORE_TMP, bool RED>
-__global__ void __launch_bounds__(32 * s2_block_rows<T>()) s2_faces(S2Fused<T> a, S2P<T> p) {
+__global__ void __launch_bounds__(32 * s2_block_rows<T, I>()) s2_faces(S2Fused<T> a, S2P<T> p) {
     const I nx = (I)a.nx, ny = (I)a.ny;
-    const I i = (I)(blockIdx.x * 32 + threadIdx.x), j = (I)(blockIdx.y * s2_block_rows<T>() + threadIdx.y);
+    const I i = (I)(blockIdx.x * 32 + threadIdx.x), j = (I)(blockIdx.y * s2_block_rows<T, I>() + threadIdx.y);
     const I c = i + nx * j, cx = c + j;  // cell and Vy face (i, j), Vx face (i, j)
     const I kx = (i - 1) + (nx - 1) * (j - 1), ky = (i - 1) + (nx - 2) * (j - 1);  // residuals; kx: corner (i-1, j-1) too
     const bool colx = i <= nx && j >= 1 && j <= ny - 2, fx = colx && i >= 1 && i <= nx - 1;  // Vx faces, with a residual
@@ -550,13 +550,14 @@ static bool s2_index32(int64_t nx, int64_t ny) { return (nx + 32) * (ny + 4) < (
 // One iteration. dependent: the kernel before it on the stream is the previous iteration's.
 template <typename T, bool DEFECT, bool STORE_TMP>
 static void launch_cells_faces(const S2Fused<T>& a, const S2P<T>& p, cudaStream_t s, bool dependent) {
-    const dim3 blk(32, s2_block_rows<T>()), gc = g2(a.nx, a.ny, blk), gf = g2(a.nx + 1, a.ny + 1, blk);
+    const bool i32 = s2_index32(a.nx, a.ny) && a.ny / s2_block_rows<T, int>() < kGridY;
+    const dim3 blk(32, i32 ? s2_block_rows<T, int>() : s2_block_rows<T, int64_t>()), gc = g2(a.nx, a.ny, blk),
+               gf = g2(a.nx + 1, a.ny + 1, blk);
     auto launch = [&](auto cells, auto faces) {
         if (dependent) launch_dependent(cells, gc, blk, 0, s, a, p);
         else cells<<<gc, blk, 0, s>>>(a, p);
         launch_dependent(faces, gf, blk, 0, s, a, p);
     };
-    const bool i32 = s2_index32(a.nx, a.ny);
     if (a.red) {
         if (i32) launch(s2_cells<T, DEFECT, int, STORE_TMP, true>, s2_faces<T, DEFECT, int, STORE_TMP, true>);
         else launch(s2_cells<T, DEFECT, int64_t, STORE_TMP, true>, s2_faces<T, DEFECT, int64_t, STORE_TMP, true>);

@@ -175,17 +175,17 @@ __device__ __forceinline__ void apt_block_add(double v0, double* out0, double v1
 
 // Rows of 32 threads per block. FP32: 8; FP64, bound by the FP64 pipe: 2, which spreads a small grid more
 // evenly over the SMs (8 rows -> 2: 350^2 17.2 -> 14.7 us per iteration, 255^2 11.1 -> 10.4, 1023^2 100.3 both).
-template <typename T>
+template <typename T, typename I>
 __host__ __device__ constexpr int apt_block_rows() {
-    return sizeof(T) == 4 ? 8 : 2;
+    return sizeof(T) == 4 || sizeof(I) == 8 ? 8 : 2;
 }
 
 // compute_P_τ!: cells (∇V, Pt, τxx, τyy) and corners (τxy). DEFECT: the correction's sweep
 // (pressure driven by ∇δV + ∇V of the outer state). STORE: write ∇V (and add Σ|∇V| to red).
 // I: index type (int where every array has fewer than 2^31 elements).
 template <typename T, bool DEFECT, bool STORE, typename I>
-__global__ void __launch_bounds__(32 * apt_block_rows<T>()) apt_cells_k(AptArrays<T> a) {
-    const I ix = (I)blockIdx.x * 32 + (I)threadIdx.x, iy = (I)blockIdx.y * apt_block_rows<T>() + (I)threadIdx.y;
+__global__ void __launch_bounds__(32 * apt_block_rows<T, I>()) apt_cells_k(AptArrays<T> a) {
+    const I ix = (I)blockIdx.x * 32 + (I)threadIdx.x, iy = (I)blockIdx.y * apt_block_rows<T, I>() + (I)threadIdx.y;
     const I nx = (I)a.nx, ny = (I)a.ny, c = ix + nx * iy;
     // the coefficients, which no iteration writes, while the kernel before this one still runs
     T kP = (T)0, aT = (T)0, bT = (T)0, aTc = (T)0, bTc = (T)0;
@@ -246,8 +246,8 @@ __global__ void __launch_bounds__(32 * apt_block_rows<T>()) apt_cells_k(AptArray
 // bc_x!(Vy). DEFECT adds the outer state's FP64 residual as source. STORE: write Rx, Ry (and add
 // Σ|Rx|, Σ|Ry| to red).
 template <typename T, bool DEFECT, bool STORE, bool UPDATE, typename I>
-__global__ void __launch_bounds__(32 * apt_block_rows<T>()) apt_faces_k(AptArrays<T> a) {
-    const I ix = (I)blockIdx.x * 32 + (I)threadIdx.x, iy = (I)blockIdx.y * apt_block_rows<T>() + (I)threadIdx.y;
+__global__ void __launch_bounds__(32 * apt_block_rows<T, I>()) apt_faces_k(AptArrays<T> a) {
+    const I ix = (I)blockIdx.x * 32 + (I)threadIdx.x, iy = (I)blockIdx.y * apt_block_rows<T, I>() + (I)threadIdx.y;
     const I nx = (I)a.nx, ny = (I)a.ny, c = ix + nx * iy;
     const T h = (T)0.5;
     // the steps and sources, which no iteration writes, while the kernel before this one still runs
@@ -444,13 +444,15 @@ static AptArrays<T> apt_arrays(const ps_stokes2d_apt_fields* f, const ps_stokes2
     return a;
 }
 
-static bool apt_i32(int64_t nx, int64_t ny) {  // 32-bit indices: every array and offset below 2^31
-    return (nx + 1 + 32) * (ny + 1 + 8) < ((int64_t)1 << 31);
+// 32-bit indices: every array and offset below 2^31, and no more blocks than a launch dimension holds
+template <typename T>
+static bool apt_i32(int64_t nx, int64_t ny) {
+    return (nx + 1 + 32) * (ny + 1 + 8) < ((int64_t)1 << 31) && ny / apt_block_rows<T, int>() < kGridY;
 }
 
 template <typename T, bool DEFECT, bool STORE, typename I>
 static void apt_launch_iteration_i(const AptArrays<T>& a, cudaStream_t s, bool after_kernel) {
-    const dim3 blk(32, apt_block_rows<T>());
+    const dim3 blk(32, apt_block_rows<T, I>());
     const dim3 grd = apt_grid(a.nx, a.ny, blk);
     // each kernel may start while the kernel before it ends (programmatic dependent launch; it waits
     // for that kernel's stores before reading); after_kernel = false: the stream's last operation
@@ -469,7 +471,7 @@ static void apt_launch_iteration_i(const AptArrays<T>& a, cudaStream_t s, bool a
 
 template <typename T, bool DEFECT, bool STORE>
 static void apt_launch_iteration(const AptArrays<T>& a, cudaStream_t s, bool after_kernel = true) {
-    if (apt_i32(a.nx, a.ny))
+    if (apt_i32<T>(a.nx, a.ny))
         apt_launch_iteration_i<T, DEFECT, STORE, int>(a, s, after_kernel);
     else
         apt_launch_iteration_i<T, DEFECT, STORE, int64_t>(a, s, after_kernel);
@@ -497,8 +499,9 @@ static void apt_residual64(AptArrays<double> a, const double* Mus, double* const
     const dim3 grd = apt_grid(a.nx, a.ny, blk);
     cudaMemsetAsync(red, 0, 3 * sizeof(double), s);
     apt_res_cells_k<<<grd, blk, 0, s>>>(a, Mus);
-    const dim3 fblk(32, apt_block_rows<double>()), fgrd = apt_grid(a.nx, a.ny, fblk);
-    if (apt_i32(a.nx, a.ny))
+    const bool i32 = apt_i32<double>(a.nx, a.ny);
+    const dim3 fblk(32, i32 ? apt_block_rows<double, int>() : apt_block_rows<double, int64_t>()), fgrd = apt_grid(a.nx, a.ny, fblk);
+    if (i32)
         apt_faces_k<double, false, true, false, int><<<fgrd, fblk, 0, s>>>(a);
     else
         apt_faces_k<double, false, true, false, int64_t><<<fgrd, fblk, 0, s>>>(a);

@@ -333,17 +333,25 @@ __global__ void s3_bc_axis_k(T* A, int64_t n0, int64_t n1, int64_t n2, int ax) {
 //
 // Bound: instruction issue -- half of it address arithmetic -- and latency at half occupancy (FP32), FP64
 // pipe (FP64). Per iteration, against a test and a branch per division, ∇V and R stored every time and
-// the copies in a third launch: FP32 127^3 106 -> 66 us, 255^3 768 -> 482 us, FP64 127^3 0.97 -> 0.45 ms.
+// the copies in a third launch: FP32 127^3 106 -> 60 us, 255^3 768 -> 446 us, FP64 127^3 0.97 -> 0.45 ms.
 // Measured slower in FP32 at 127^3: sweeps of 4 planes per thread with the shared values in registers
 // (70 us), two or four columns per thread (73, 92), 40 or 32 registers for more warps (spills; 88, 130).
-template <typename T>
-constexpr int s3_blocks() {  // blocks per SM: 64 registers in FP32, 80 in FP64
-    return sizeof(T) == 4 ? 4 : 3;
+// Rows of 32 threads per block, and blocks per SM the kernels are compiled for: 48 and 56 registers (s3_cells, s3_faces)
+// in FP32, 80 in FP64. Blocks of 8 rows, 4 to an SM (64 registers), took 64.7 us per iteration at 127^3 and 193 at
+// 200 x 200 x 150 in FP32, where these take 59.5 and 176: smaller blocks leave and fill an SM more evenly and
+// fit its registers more tightly; 2 rows the same, 1 and 16 slower, 44 registers and fewer spill.
+template <typename T, typename I>
+__host__ __device__ constexpr int s3_rows() {
+    return sizeof(I) == 8 ? 8 : sizeof(T) == 4 ? 4 : 2;
+}
+template <typename T, typename I>
+constexpr int s3_blocks(bool cells) {
+    return sizeof(I) == 8 ? (sizeof(T) == 4 ? 4 : 3) : sizeof(T) == 4 ? (cells ? 10 : 9) : 12;
 }
 template <typename T, int MODE, typename I, bool STORE>
-__global__ void __launch_bounds__(256, s3_blocks<T>()) s3_cells(S3A<T> a, S3P<T> p) {
+__global__ void __launch_bounds__(32 * s3_rows<T, I>(), s3_blocks<T, I>(true)) s3_cells(S3A<T> a, S3P<T> p) {
     const I nx = (I)a.nx, ny = (I)a.ny, nz = (I)a.nz;
-    const I x = (I)(blockIdx.x * 32 + threadIdx.x), y = (I)(blockIdx.y * 8 + threadIdx.y), z = (I)blockIdx.z;
+    const I x = (I)(blockIdx.x * 32 + threadIdx.x), y = (I)(blockIdx.y * s3_rows<T, I>() + threadIdx.y), z = (I)blockIdx.z;
     grid_dependency_wait();  // the state is read with plain loads: __ldg need not see the kernel before
     if (x >= nx || y >= ny) return;
     const bool x1 = x < nx - 1, y1 = y < ny - 1, z1 = z < nz - 1;  // an edge at the upper x / y / z side exists
@@ -401,9 +409,9 @@ __global__ void __launch_bounds__(256, s3_blocks<T>()) s3_cells(S3A<T> a, S3P<T>
 }
 
 template <typename T, int MODE, typename I, bool STORE>
-__global__ void __launch_bounds__(256, s3_blocks<T>()) s3_faces(S3A<T> a, S3P<T> p) {
+__global__ void __launch_bounds__(32 * s3_rows<T, I>(), s3_blocks<T, I>(false)) s3_faces(S3A<T> a, S3P<T> p) {
     const I nx = (I)a.nx, ny = (I)a.ny, nz = (I)a.nz;
-    const I x = (I)(blockIdx.x * 32 + threadIdx.x), y = (I)(blockIdx.y * 8 + threadIdx.y), z = (I)blockIdx.z;
+    const I x = (I)(blockIdx.x * 32 + threadIdx.x), y = (I)(blockIdx.y * s3_rows<T, I>() + threadIdx.y), z = (I)blockIdx.z;
     grid_dependency_wait();
     if (x > nx || y > ny) return;
     const bool ix = x >= 1 && x <= nx - 2, iy = y >= 1 && y <= ny - 2, iz = z >= 1 && z <= nz - 2;
@@ -891,14 +899,16 @@ static bool s3_idx32(const S3A<T>& a) {
 // them on the stream is an iteration's, whose last wave they may overlap.
 template <typename T, int MODE, bool STORE>
 static void s3_iteration_kernels(const S3A<T>& a, const S3P<T>& p, bool after, cudaStream_t s) {
-    const dim3 b(32, 8, 1);
+    const bool i32 = s3_idx32(a) && a.ny / s3_rows<T, int>() < kGridY;
+    const dim3 b(32, i32 ? s3_rows<T, int>() : s3_rows<T, int64_t>(), 1);
     auto launch = [&](auto cells, auto faces) {
-        const dim3 gc = g3(a.nx, a.ny, a.nz), gf = g3(a.nx + 1, a.ny + 1, a.nz + 1);
+        const dim3 gc((unsigned)((a.nx + 31) / 32), (unsigned)((a.ny + b.y - 1) / b.y), (unsigned)a.nz),
+            gf((unsigned)(a.nx / 32 + 1), (unsigned)(a.ny / b.y + 1), (unsigned)a.nz + 1);
         if (after) launch_dependent(cells, gc, b, 0, s, a, p);
         else cells<<<gc, b, 0, s>>>(a, p);
         launch_dependent(faces, gf, b, 0, s, a, p);
     };
-    if (s3_idx32(a)) launch(s3_cells<T, MODE, int, STORE>, s3_faces<T, MODE, int, STORE>);
+    if (i32) launch(s3_cells<T, MODE, int, STORE>, s3_faces<T, MODE, int, STORE>);
     else launch(s3_cells<T, MODE, int64_t, STORE>, s3_faces<T, MODE, int64_t, STORE>);
 }
 
