@@ -522,9 +522,10 @@ __global__ void __launch_bounds__(32 * TY, MINB)
         for (int s = 0; s < S; s++) mbar_init(&bar[s], 1);
         fence_mbar_init();
     }
-    __syncthreads();
     grid_dependency_wait();  // the step before has completed
-    if (*reinterpret_cast<volatile int*>(&run->bad)) return;
+    // One thread reads the flag for the block (and the barriers are set up): blocks of this launch raise it while
+    // others start, and a block of which only some threads left would wait for loads that nobody issues.
+    if (__syncthreads_or(tid == 0 && *reinterpret_cast<volatile int*>(&run->bad))) return;
     const int sh = run->shT;
     int next_q = 0;
     auto issue = [&](int q) {
@@ -1128,10 +1129,12 @@ __global__ void __launch_bounds__(32 * TY, 2)
         for (int s = 0; s < S; s++) mbar_init(&bar[s], 1);
         fence_mbar_init();
     }
-    __syncthreads();
     grid_dependency_wait();        // the step before (or the recomputed states) has completed
     grid_dependents_may_launch();  // glam_boundary_kernel of this step runs beside this kernel
-    if (*reinterpret_cast<volatile int*>(&run->bad) || *reinterpret_cast<const volatile int*>(&mrun->bad)) return;
+    // (one thread reads the flags for the block, see diff3d_grid_tma)
+    if (__syncthreads_or(tid == 0 && (*reinterpret_cast<volatile int*>(&run->bad) ||
+                                      *reinterpret_cast<const volatile int*>(&mrun->bad))))
+        return;
     const int sh = mrun->shT + run->shT;
     int next_q = 0;
     auto issue = [&](int q) {

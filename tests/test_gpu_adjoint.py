@@ -138,3 +138,22 @@ def test_adjoint_step_split_close_to_ieee(ps):
     for a, b in zip(out["ieee"], out["split"]):
         assert np.abs(a - b).max() <= 1e-13 * np.abs(a).max()
     assert not np.array_equal(out["ieee"][0], out["split"][0])  # a different arithmetic really ran
+
+
+@pytest.mark.parametrize("factor", [60.0, 15.0])
+def test_misfit_gradient_adjoint_leaves_grid_while_blocks_still_start(ps, factor):
+    """The forward run stays on its grid (the state is constant where the scheme is unstable), the adjoint leaves its
+    own in the first rows while later blocks of the same launch still start: the split-pair gradient."""
+    n = (512, 512, 20)
+    T0, Ci, lam, h, dt = _problem(n, seed=14)
+    T0[:, :200, :] = 0.5
+    Ci[:, :4, :] = factor  # dt * Ci * lam * 4 sum(1/h^2) is about a fifth of it (lam is 1 in the middle, 5 at most)
+    T_obs = np.asfortranarray(T0 * (0.9 + 0.1 * np.random.default_rng(15).random(n)))
+    dT0, dobs, dCi, dlam = (ps.from_host(a) for a in (T0, T_obs, Ci, lam))
+    res = {}
+    for fp64 in ("split", "split_grid"):
+        loss, g, st = ps.adjoint.misfit_gradient(dT0, dobs, dCi, dlam, dt, h, 6, checkpoint_every=3, fp64=fp64)
+        res[fp64] = (loss, ps.to_host(g))
+    la, lb = res["split"][0], res["split_grid"][0]  # the loss is an atomic sum: order may differ
+    assert la == lb or abs(la - lb) <= 1e-13 * abs(la), (la, lb)
+    assert np.array_equal(res["split"][1], res["split_grid"][1])

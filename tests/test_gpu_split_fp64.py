@@ -237,3 +237,22 @@ def test_grid_run_growth_in_last_step(ps, oracle):
                    fp64="split_grid")
     e = relerr(ps.to_host(dT), ref)
     assert e <= 1e-12, e
+
+
+@pytest.mark.parametrize("noise", [1.0, 1e-3])
+def test_grid_run_growth_while_blocks_still_start(ps, noise):
+    """Values leave the grid in the first rows only (in the first step, or some steps later), whose blocks end while
+    later blocks of the same launch (more than the GPU holds at once) still start and find the flag raised: the run
+    is redone with split pairs."""
+    n = (512, 512, 20)
+    T, Ci, lam, hs, dt = _setup(n, 3, seed=35)
+    Ci[:, :4, :] = 20.0  # dt * Ci * lam * 8 / h^2 = 11 in these rows: noise grows about tenfold per step
+    T[:, :8, :] = 0.5 + noise * (T[:, :8, :] - 0.5)
+    out = {}
+    for mode in ("split_grid", "split_state"):
+        dT, dT2 = ps.from_host(T), ps.from_host(T)
+        ps.kernels.run(ps.kernels.diffusion3D_step_flux_lam, dT, dT2, ps.from_host(Ci), ps.from_host(lam), dt, *hs,
+                       8, fp64=mode)
+        out[mode] = ps.to_host(dT)
+    assert np.abs(out["split_state"]).max() > 1.0  # left the grid of max|T0| < 1
+    assert np.array_equal(out["split_grid"], out["split_state"])
