@@ -1160,7 +1160,9 @@ class _Gen:
                     f"    if (in_ ? bad{j}_ : ok{j}_ | bad{j}_) atomicOr(g.err, 1);",
                     f"    const bool all_ = m_ == {(1 << cells) - 1}u;"]
             value = lines[:-1] + [f"    o_[jt_c] = {val};{chk}"]
-            if any(re.search(r"\bb\d+_\[", ln) for ln in lines[:-1]):  # reads a written array: only where it runs
+            # only where it runs: a statement that reads a written array, and one on split pairs, whose loads
+            # report values outside the pairs' range (cells that do not run may hold any)
+            if self.split or any(re.search(r"\bb\d+_\[", ln) for ln in lines[:-1]):
                 value = ["    if (all_ || m_ >> jt_c & 1u) {"] + value + ["    }"]
             # the ring holds (zeros from outside the arrays in) the stencils of all cells of a block
             out += ["    if (m_) {", f"    E o_[{cells}];", "    #pragma unroll", loop] + cell + value + \

@@ -151,3 +151,26 @@ def test_tma_sweep_reports_a_stencil_that_leaves_an_array(ps, short):
     a = [ps.zeros(*n, dtype=np.float32), ps.zeros(*n, dtype=np.float32), ps.zeros(*m, dtype=np.float32)]
     with pytest.raises(PSError, match="ps_jit_launch_tma.*BoundsError"):
         ps.parallel(k, *a, 0.3)
+
+
+def test_tma_sweep_split_fp64_range_is_that_of_the_cells_that_run(ps):
+    """Values outside the pairs' range in cells that no running statement reads (the faces of an array read as
+    @inn only) are no error; in a cell that runs they are."""
+    from ps_gb300 import PSError
+
+    n = (64, 40, 33)
+    src, ins, outs, sc = _case(ps, "FLUX_LAM", n, np.float64, np.random.default_rng(44))
+    k = ps.parallel_kernel(src)
+    args = dict(memopt=True, fp64="split")
+    Ci = ps.to_host(ins[1])  # T2, T, Ci, lam
+    ref = _run(ps, k, "FLUX_LAM", ins, outs, sc, np.float64, **args)
+    Ci[[0, -1]], Ci[:, [0, -1]], Ci[:, :, [0, -1]] = 1e300, -1e300, np.inf
+    k.tma = "always"
+    before = k.tma_launches
+    got = _run(ps, k, "FLUX_LAM", [ins[0], _dev(ps, Ci), ins[2]], outs, sc, np.float64, **args)
+    assert k.tma_launches == before + 1
+    assert np.array_equal(got[0], ref[0])
+    Ci[20, 20, 20] = 1e300
+    with pytest.raises(PSError):
+        _run(ps, k, "FLUX_LAM", [ins[0], _dev(ps, Ci), ins[2]], outs, sc, np.float64, **args)
+    k.tma = True
