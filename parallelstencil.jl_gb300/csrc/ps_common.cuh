@@ -379,6 +379,15 @@ __device__ __forceinline__ double scale_pow2(double x, int k, uint32_t* key) {
     return __hiloint2double(kx == 0xFFFFFFFFu ? hi : hi + (k << 20), __double2loint(x));
 }
 
+// 2 a b for a finite 2 a, as the product times two: equal to (2 a) b bit for bit where scale_pow2 is, and a product
+// that underflowed to zero (whose double may not) makes the caller compute again too.
+__device__ __forceinline__ double twice_product(double a, double b, uint32_t* key) {
+    const double x = a * b;
+    if (div_key(x) == 0xFFFFFFFFu && div_key(a) != 0xFFFFFFFFu && div_key(b) != 0xFFFFFFFFu) *key = 0u;
+    if ((__double2hiint(a) & 0x7FFFFFFF) >= 0x78300000) *key = 0u;  // |a| < 2^900: 2 a is finite
+    return scale_pow2(x, 1, key);
+}
+
 // a / h for statement helpers used with a plain divisor (host or device) or a DivC (device)
 template <typename T>
 __host__ __device__ __forceinline__ T dvd(T a, T h) {

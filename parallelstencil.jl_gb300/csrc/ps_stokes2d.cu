@@ -61,8 +61,7 @@ __host__ __device__ __forceinline__ T s2_tau_xy(T m00, T m10, T m01, T m11, T dy
 // to the product (equal bit for bit while nothing on the way is subnormal or overflows: the keys).
 __device__ __forceinline__ double s2_tau_nn(double mus, double v0, double v1, double divV, DivF<double> h) {
     const double e = dvd(v1 - v0, h) - (1.0 / 3.0) * divV;
-    if ((__double2hiint(mus) & 0x7FFFFFFF) >= 0x78300000) *h.key = 0u;  // |mus| < 2^900: 2 mus is finite
-    return scale_pow2(mus * e, 1, h.key);
+    return twice_product(mus, e, h.key);
 }
 __device__ __forceinline__ double s2_tau_xy_sum(double msum, double dyVx, double dxVy, DivF<double> dx, DivF<double> dy) {
     const double e = dvd(dyVx, dy) + dvd(dxVy, dx);

@@ -90,8 +90,7 @@ __device__ __forceinline__ T s3_tnn(T m, T v1, T v0, H h, T d) {
 }
 __device__ __forceinline__ double s3_tnn(double m, double v1, double v0, DivF<double> h, double d) {
     const double e = dvd(v1 - v0, h) - (1.0 / 3.0) * d;
-    if ((__double2hiint(m) & 0x7FFFFFFF) >= 0x78300000) *h.key = 0u;  // |m| < 2^900: 2 m is finite
-    return scale_pow2(m * e, 1, h.key);
+    return twice_product(m, e, h.key);
 }
 // 2.0*@av_..i(μ)*(0.5*(a/ha + b/hb)), msum: the four μ summed in the macro's order
 template <typename T, typename H>

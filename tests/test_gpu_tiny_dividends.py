@@ -90,3 +90,44 @@ def test_diffusion_dividing_by_spacings(ps, oracle, dtn, h, memopt):
     T2 = ps.from_host(T)
     ps.parallel(ps.kernels.diffusion3D_step, T2, ps.from_host(T), ps.from_host(Ci), 1.3, dts, *h, memopt=memopt)
     assert np.array_equal(ps.to_host(T2), ref)
+
+
+def _near_underflow(rng, shape, e0):
+    """Values around 2^e0, of both signs."""
+    return np.asfortranarray(np.ldexp(0.5 + 0.5 * rng.random(shape), rng.integers(e0 - 6, e0 + 7, shape)) *
+                             rng.choice([-1.0, 1.0], shape))
+
+
+def test_stokes2d_stress_underflow(ps, oracle):
+    """Viscosities and velocities whose product is about the smallest subnormal number: 2 mu e may be it where mu e
+    is zero."""
+    from test_gpu_stokes2d import ALL, _pair
+
+    g, o = _pair(ps, oracle, 45, 29, "f64")
+    rng = np.random.default_rng(3)
+    for k, e0 in (("Mus", -500), ("Vx", -575), ("Vy", -575), ("Pt", -575)):
+        v = _near_underflow(rng, o[k].shape, e0)
+        o[k][...] = np.abs(v) if k == "Mus" else v
+        g[k].copy_(ps.from_host(o[k]))
+    g.iterate(1)
+    o.step()
+    assert 50 < np.count_nonzero(np.abs(o["txx"]) == 2.0 ** -1074) < o["txx"].size
+    for k in ALL:
+        assert np.array_equal(g.host(k), o[k]), k
+
+
+def test_stokes3d_stress_underflow(ps, oracle):
+    """As above in 3-D."""
+    from test_gpu_stokes3d import STATE, _pair
+
+    g, o = _pair(ps, oracle, (21, 14, 11), "f64")
+    rng = np.random.default_rng(4)
+    for k, e0 in (("Mus", -500), ("Vx", -575), ("Vy", -575), ("Vz", -575), ("Pt", -575)):
+        v = _near_underflow(rng, o[k].shape, e0)
+        o[k][...] = np.abs(v) if k == "Mus" else v
+        g[k].copy_(ps.from_host(o[k]))
+    g.iterate(1)
+    o.step()
+    assert 50 < np.count_nonzero(np.abs(o["txx"]) == 2.0 ** -1074) < o["txx"].size
+    for k in STATE:
+        assert np.array_equal(g.host(k), o[k]), k
