@@ -233,7 +233,7 @@ template <typename T>
 struct DivC {
     T b, yh, yl;
     uint32_t lo;   // div_key of the smallest dividend of the fast path
-    uint32_t fix;  // no pair: yh = RN(1/b), yl = 0 (exact for zeros, the only dividends let through)
+    uint32_t fix;  // no pair: yh = RN(1/b), yl a zero of its sign (exact for zeros, the only dividends let through)
 };
 
 // Key of a dividend: grows with |a|, largest for zeros.
@@ -319,7 +319,7 @@ inline DivC<T> make_div(T b) {
         return d;
     }
     d.yh = (T)1 / b;
-    d.yl = 0;
+    d.yl = std::copysign((T)0, b);  // (of yh's sign, for a zero quotient's)
     d.fix = 1;
     return d;
 }

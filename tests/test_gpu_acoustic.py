@@ -149,3 +149,10 @@ def test_division_by_reciprocal_pairs(ps, b):
     both ends of a binade, the ends of its range, and divisors that no reciprocal pair serves (the
     first two, found on the CPU), against the IEEE division as above."""
     test_constant_division_equals_ieee_division(ps, b)
+
+
+@pytest.mark.parametrize("b", [-10.0 / 15, -10.0 / 17, -float.fromhex("0x1.6e6c1ep-4"), -float.fromhex("0x1.e7a9a78a18f56p-2")])
+def test_division_by_negative_numbers_without_a_pair(ps, b):
+    """Negative divisors that no reciprocal pair serves (the first and third in FP32, the others in FP64): zero
+    dividends give zeros of the quotient's sign."""
+    test_constant_division_equals_ieee_division(ps, b)
