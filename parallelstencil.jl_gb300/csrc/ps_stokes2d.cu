@@ -249,9 +249,15 @@ __device__ __forceinline__ double s2_half_sum(double a, double b, DivF<double> h
 
 // Rows of 32 threads per block. FP32: 8; FP64, bound by the FP64 pipe: 2, which spreads a small grid more
 // evenly over the SMs (4 rows -> 2: 255^2 11.4 -> 10.5 us per iteration, 130^2 6.9 -> 6.1, 1023^2 118 both).
+// The 64-bit variants, which run grids taller than 65535 such blocks too, have 8 (FP32) and 16 rows: with s2_max_rows
+// their faces are 65535 blocks.
 template <typename T, typename I>
 __host__ __device__ constexpr int s2_block_rows() {
-    return sizeof(T) == 4 || sizeof(I) == 8 ? 8 : 2;
+    return sizeof(I) == 8 && sizeof(T) == 8 ? 16 : sizeof(I) == 8 || sizeof(T) == 4 ? 8 : 2;
+}
+template <typename T>
+constexpr int64_t s2_max_rows() {
+    return kGridY * s2_block_rows<T, int64_t>() - 1;
 }
 
 template <typename T, bool DEFECT, typename I, bool STORE_TMP, bool RED>
@@ -546,6 +552,14 @@ static void scratch_free(void* p) {
 // 32-bit indices while every array's size and the offsets a few rows past it stay below 2^31
 static bool s2_index32(int64_t nx, int64_t ny) { return (nx + 32) * (ny + 4) < ((int64_t)1 << 31); }
 
+// Refused before the first launch, so that no iteration stops halfway.
+template <typename T>
+static int check_rows(int64_t ny, const char* what) {
+    if (ny > s2_max_rows<T>())
+        return fail(PS_ERR_SHAPE, "%s: %lld rows, at most %lld", what, (long long)ny, (long long)s2_max_rows<T>());
+    return PS_OK;
+}
+
 // One iteration. dependent: the kernel before it on the stream is the previous iteration's.
 template <typename T, bool DEFECT, bool STORE_TMP>
 static void launch_cells_faces(const S2Fused<T>& a, const S2P<T>& p, cudaStream_t s, bool dependent) {
@@ -592,11 +606,14 @@ static S2Fused<T> s2_dropin_args(const ps_stokes2d_fields* f) {
 
 // n_iter iterations; the temporaries nothing reads between iterations are stored in the last
 template <typename T>
-static void s2_iterate(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp, int64_t n_iter, cudaStream_t s) {
+static int s2_iterate(const ps_stokes2d_fields* f, const ps_stokes2d_params* pp, int64_t n_iter, cudaStream_t s,
+                      const char* what) {
+    PS_TRY(check_rows<T>(f->Pt.n[1], what));
     const S2P<T> p = s2p<T>(*pp);
     const S2Fused<T> a = s2_dropin_args<T>(f);
     for (int64_t it = 0; it + 1 < n_iter; ++it) launch_cells_faces<T, false, false>(a, p, s, it > 0);
     if (n_iter > 0) launch_cells_faces<T, false, true>(a, p, s, n_iter > 1);
+    return finish_launch(s, 1, what);
 }
 
 // ---- solver ---------------------------------------------------------------------------
@@ -627,7 +644,7 @@ struct PTRunner {
 // The pseudo-time steps of a solve, computed once (compute_timesteps!) instead of in every iteration.
 template <typename T>
 static void s2_solver_timesteps(S2Fused<T>& a, const S2P<T>& p, T* dtVx, T* dtVy, T* dtPt, cudaStream_t s) {
-    const dim3 blk(32, 8);
+    const dim3 blk(32, s2_block_rows<T, int64_t>());
     s2_timesteps_k<T><<<g2(a.nx, a.ny, blk), blk, 0, s>>>(dtVx, dtVy, dtPt, a.Mus, a.nx, a.ny, p);
     a.dtVx = dtVx;
     a.dtVy = dtVy;
@@ -974,9 +991,8 @@ int ps_stokes2d_iterate(const ps_stokes2d_fields* f, const ps_stokes2d_params* p
     if (!p) return fail(PS_ERR_NULL, "NULL params");
     if (n_iter < 0) return fail(PS_ERR_ARG, "n_iter must be >= 0");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (f->Pt.dtype == PS_F64) s2_iterate<double>(f, p, n_iter, s);
-    else s2_iterate<float>(f, p, n_iter, s);
-    return finish_launch(s, 1, "ps_stokes2d_iterate");
+    return f->Pt.dtype == PS_F64 ? s2_iterate<double>(f, p, n_iter, s, "ps_stokes2d_iterate")
+                                 : s2_iterate<float>(f, p, n_iter, s, "ps_stokes2d_iterate");
 }
 
 int ps_stokes2d_err(const ps_stokes2d_fields* f, double out_mean_abs[3], void* stream) {
@@ -1017,6 +1033,7 @@ int ps_stokes2d_solve(const ps_stokes2d_fields* f, const ps_stokes2d_params* p, 
     if (nout < 2 || nout % 2) return fail(PS_ERR_ARG, "nout must be even and >= 2");
     if (!(tol > 0) || max_iter < 0) return fail(PS_ERR_ARG, "invalid tol / max_iter");
     if (mode != 0 && mode != 1) return fail(PS_ERR_ARG, "mode must be 0 (FP64) or 1 (FP32 + FP64 defect correction)");
+    PS_TRY(mode == 0 ? check_rows<double>(ny, "ps_stokes2d_solve") : check_rows<float>(ny, "ps_stokes2d_solve (mixed)"));
     memset(stats, 0, sizeof(*stats));
     // the solver captures CUDA graphs: run on a private stream ordered after `stream`
     cudaStream_t user = static_cast<cudaStream_t>(stream), s;
@@ -1074,7 +1091,6 @@ extern "C" int ps_stokes2d_iterate_static(const ps_stokes2d_fields* f, const ps_
     if (n_iter < 0) return fail(PS_ERR_ARG, "n_iter must be >= 0");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     PS_TRY(check_static_bound(f));
-    if (f->Pt.dtype == PS_F64) s2_iterate<double>(f, p, n_iter, s);
-    else s2_iterate<float>(f, p, n_iter, s);
-    return finish_launch(s, 1, "ps_stokes2d_iterate_static");
+    return f->Pt.dtype == PS_F64 ? s2_iterate<double>(f, p, n_iter, s, "ps_stokes2d_iterate_static")
+                                 : s2_iterate<float>(f, p, n_iter, s, "ps_stokes2d_iterate_static");
 }

@@ -70,3 +70,55 @@ def test_stokes2d_apt(ps, oracle, ny):
     o.step()
     for k in STATE:
         assert np.array_equal(g.host(k), o[k]), k
+
+
+# The largest extents: one more row or plane of faces than of cells must be reached, and beyond them a call is
+# refused as a whole.
+@pytest.mark.parametrize("dtn,ny", [("f64", 524280), ("f64", 1048559), ("f32", 524279)])
+def test_stokes2d_most_rows(ps, oracle, dtn, ny):
+    from ps_gb300.stokes import Stokes2D, Stokes2DParams, inclusion_setup
+    from ps_gb300 import PSError
+    from test_gpu_stokes2d import ALL
+
+    nx, ly = 4, float(ny - 1)
+    Mus, Rog = inclusion_setup(nx, ny, 3.0, ly, dtype=DT[dtn])
+    p = Stokes2DParams(nx, ny, 3.0, ly)
+    g, o = Stokes2D(p, Mus, Rog, dtype=DT[dtn]), oracle.Stokes2D(nx, ny, p.dx, p.dy, Mus, Rog, dtype=DT[dtn])
+    o.compute_timesteps()
+    for k in ("dtauVx", "dtauVy", "dtauPt"):
+        g[k].copy_(ps.from_host(o[k]))
+    _random(ps, g, o, ("Pt", "Vx", "Vy", "dVxdtau", "dVydtau"), dtn)
+    start = {k: o[k].copy(order="F") for k in ("Pt", "Vx", "Vy", "dVxdtau", "dVydtau")}
+    for _ in range(2):
+        o.step()
+    g.iterate(2)
+    for k in ALL:
+        assert np.array_equal(g.host(k), o[k]), k
+    if dtn == "f64":  # the solver, which makes its own pseudo-time steps
+        for k, v in start.items():
+            g[k].copy_(ps.from_host(v))
+        with pytest.raises(PSError):  # two iterations do not reach tol
+            g.solve(tol=1e-30, mode=0, max_iter=2, nout=2)
+        for k in start:
+            assert np.array_equal(g.host(k), o[k]), k
+
+
+@pytest.mark.parametrize("dtn,ny", [("f64", 1048560), ("f32", 524280)])
+def test_stokes2d_too_many_rows_is_refused_whole(ps, dtn, ny):
+    from ps_gb300 import PSError
+    from ps_gb300.stokes import Stokes2D, Stokes2DParams
+
+    nx = 3
+    g = Stokes2D(Stokes2DParams(nx, ny, 2.0, float(ny - 1)), np.ones((nx, ny), order="F", dtype=DT[dtn]),
+                 np.ones((nx, ny), order="F", dtype=DT[dtn]), dtype=DT[dtn])
+    g["Vx"].fill_(1.0)
+    g["Vy"].copy_(ps.rand(nx, ny + 1, dtype=DT[dtn], seed=1))
+    before = {k: g[k].clone() for k in ("Pt", "Vx", "Vy", "txx", "txy")}
+    with pytest.raises(PSError, match="rows"):
+        g.iterate(1)
+    if dtn == "f64":
+        for mode in (0, 1):
+            with pytest.raises(PSError, match="rows"):
+                g.solve(tol=1.0, mode=mode, max_iter=2, nout=2)
+    assert all((g[k] == v).all().item() for k, v in before.items())
+
