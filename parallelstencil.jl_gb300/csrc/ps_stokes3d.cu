@@ -407,12 +407,10 @@ __global__ void __launch_bounds__(32 * s3_rows<T, I>(), s3_blocks<T, I>(true)) s
     if (ix && y1 && z1) a.tyz[(x - 1) + (nx - 2) * (y + (ny - 1) * z)] = tyz;
 }
 
+// The faces at the lower sides of the cell (x, y, z), x <= nx, y <= ny, z <= nz.
 template <typename T, int MODE, typename I, bool STORE>
-__global__ void __launch_bounds__(32 * s3_rows<T, I>(), s3_blocks<T, I>(false)) s3_faces(S3A<T> a, S3P<T> p) {
+__device__ __forceinline__ void s3_face(const S3A<T>& a, const S3P<T>& p, const I x, const I y, const I z) {
     const I nx = (I)a.nx, ny = (I)a.ny, nz = (I)a.nz;
-    const I x = (I)(blockIdx.x * 32 + threadIdx.x), y = (I)(blockIdx.y * s3_rows<T, I>() + threadIdx.y), z = (I)blockIdx.z;
-    grid_dependency_wait();
-    if (x > nx || y > ny) return;
     const bool ix = x >= 1 && x <= nx - 2, iy = y >= 1 && y <= ny - 2, iz = z >= 1 && z <= nz - 2;
     // the faces with a residual: Vx, Vy, Vz (their low x, y, z sides of the cell)
     const bool du = x >= 1 && x <= nx - 1 && iy && iz, dv = ix && y >= 1 && y <= ny - 1 && iz,
@@ -546,6 +544,21 @@ __global__ void __launch_bounds__(32 * s3_rows<T, I>(), s3_blocks<T, I>(false)) 
                     for (int j = ya; j <= yb; ++j)
                         if (i || j) vz[i + j * nx] = wv;
         }
+    }
+}
+
+// One thread per position; the 64-bit variant, which runs the tallest and deepest grids too (ny = 65535 * 8 or nz =
+// 65535 cells have one more row or plane of faces than the launch has blocks), takes the positions a grid further on.
+template <typename T, int MODE, typename I, bool STORE>
+__global__ void __launch_bounds__(32 * s3_rows<T, I>(), s3_blocks<T, I>(false)) s3_faces(S3A<T> a, S3P<T> p) {
+    const I x = (I)(blockIdx.x * 32 + threadIdx.x), y = (I)(blockIdx.y * s3_rows<T, I>() + threadIdx.y), z = (I)blockIdx.z;
+    grid_dependency_wait();
+    if (x > (I)a.nx) return;
+    if constexpr (sizeof(I) == 8) {
+        for (I v = z; v <= (I)a.nz; v += gridDim.z)
+            for (I u = y; u <= (I)a.ny; u += (I)gridDim.y * s3_rows<T, I>()) s3_face<T, MODE, I, STORE>(a, p, x, u, v);
+    } else {
+        if (y <= (I)a.ny) s3_face<T, MODE, I, STORE>(a, p, x, y, z);
     }
 }
 
@@ -898,11 +911,12 @@ static bool s3_idx32(const S3A<T>& a) {
 // them on the stream is an iteration's, whose last wave they may overlap.
 template <typename T, int MODE, bool STORE>
 static void s3_iteration_kernels(const S3A<T>& a, const S3P<T>& p, bool after, cudaStream_t s) {
-    const bool i32 = s3_idx32(a) && a.ny / s3_rows<T, int>() < kGridY;
+    const bool i32 = s3_idx32(a) && a.ny / s3_rows<T, int>() < kGridY && a.nz < kGridY;
     const dim3 b(32, i32 ? s3_rows<T, int>() : s3_rows<T, int64_t>(), 1);
     auto launch = [&](auto cells, auto faces) {
         const dim3 gc((unsigned)((a.nx + 31) / 32), (unsigned)((a.ny + b.y - 1) / b.y), (unsigned)a.nz),
-            gf((unsigned)(a.nx / 32 + 1), (unsigned)(a.ny / b.y + 1), (unsigned)a.nz + 1);
+            gf((unsigned)(a.nx / 32 + 1), (unsigned)std::min<int64_t>(a.ny / b.y + 1, kGridY),
+               (unsigned)std::min<int64_t>(a.nz + 1, kGridY));
         if (after) launch_dependent(cells, gc, b, 0, s, a, p);
         else cells<<<gc, b, 0, s>>>(a, p);
         launch_dependent(faces, gf, b, 0, s, a, p);

@@ -122,3 +122,23 @@ def test_stokes2d_too_many_rows_is_refused_whole(ps, dtn, ny):
                 g.solve(tol=1.0, mode=mode, max_iter=2, nout=2)
     assert all((g[k] == v).all().item() for k, v in before.items())
 
+
+@pytest.mark.parametrize("dtn", ["f64", "f32"])
+@pytest.mark.parametrize("n,one_launch", [((4, 3, 65535), False), ((4, 3, 65535), True), ((3, 4, 65534), False),
+                                          ((4, 524280, 3), False), ((3, 524279, 3), False)])
+def test_stokes3d_largest_extents(ps, oracle, dtn, n, one_launch):
+    from ps_gb300.stokes3d import Stokes3D, Stokes3DParams, inclusion_setup
+    from test_gpu_stokes3d import STATE
+
+    l = tuple(float(m - 1) for m in n)
+    Mus, Rog = inclusion_setup(*n, *l, dtype=DT[dtn])
+    p = Stokes3DParams(*n, *l)
+    g, o = Stokes3D(p, Mus, Rog, dtype=DT[dtn]), oracle.Stokes3D(*n, *p.h, Mus, Rog, dtype=DT[dtn])
+    g.compute_timesteps()
+    o.compute_timesteps()
+    _random(ps, g, o, ("Pt", "Vx", "Vy", "Vz", "dVxdtau", "dVydtau", "dVzdtau"), dtn)
+    g.iterate(3, one_launch=one_launch)
+    for _ in range(3):
+        o.step()
+    for k in STATE:
+        assert np.array_equal(g.host(k), o[k]), k
