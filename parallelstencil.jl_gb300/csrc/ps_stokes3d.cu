@@ -607,6 +607,8 @@ __global__ void s3_bc_k(S3A<T> a) {
 // face writes the boundary faces that copy it (s3_bc_k's clamped source), faces outside the
 // updated range keep their old value. Bit-identical to the one-to-one kernels (same operations on
 // the same operands, in the reference's order).
+// Two CTAs per SM in FP32 (64 registers): left to itself the compiler took 73 and one CTA, 362 us per iteration at
+// 127^3 instead of 208. FP64 (104 registers) fits one.
 constexpr int S3F_TY = 16;
 
 template <typename T>
@@ -615,7 +617,7 @@ struct S3Out {
 };
 
 template <typename T, int MODE>
-__global__ void __launch_bounds__(32 * S3F_TY) s3_fused_k(S3A<T> a, S3Out<T> o, S3P<T> p, int Lz) {
+__global__ void __launch_bounds__(32 * S3F_TY, sizeof(T) == 4 ? 2 : 1) s3_fused_k(S3A<T> a, S3Out<T> o, S3P<T> p, int Lz) {
     static_assert(MODE == S3_PLAIN || MODE == S3_DEFECT, "update modes only");
     __shared__ T sPt[S3F_TY][32], sTxx[S3F_TY][32], sTyy[S3F_TY][32], sTxy[S3F_TY][32];
     __shared__ T sLxz[2][S3F_TY][32], sLyz[2][S3F_TY][32];
