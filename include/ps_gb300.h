@@ -104,8 +104,9 @@ const char* ps_last_error(void);
 int ps_abi_version(void);
 /* Number of CUDA devices visible (0 without a driver). Needs no ps_init. */
 int ps_device_count(int* count);
-/* Self-check of the kernels' division by a number known on the host (Markstein's method: one
- * multiply and four FMAs, correctly rounded) against the IEEE division a / b on the device.
+/* Self-check of the kernels' division by a number known on the host (by the reciprocal as a pair of
+ * numbers, one multiply and one FMA, or Markstein's method; every form, correctly rounded) against
+ * the IEEE division a / b on the device.
  * PS_F32: every significand of 12 binades (from 2^-126 to 2^127) with both signs plus special
  * values; PS_F64: n dividends from a seeded hash plus special values. *mismatches = the number
  * of results whose bits differ (NaNs compare equal). Synchronises. */

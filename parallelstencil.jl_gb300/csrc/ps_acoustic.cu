@@ -56,34 +56,41 @@ struct AcuArrays {
 // IEEE arithmetic in the storage type: the reference's statements as written (the divisions by
 // dx, dy, dz correctly rounded through div_c). The increment form `v + (-x)` equals `v - x`.
 template <typename T>
+struct AcuIeeeC {
+    T dtr, dtk;
+    DivC<T> h[3];
+    uint32_t lo;  // the smallest dividend key all three take without a test
+};
+enum AcuDiv { ACU_UNTESTED, ACU_TESTED, ACU_NOPAIR };  // dvd's DivF, DivC and DivG
+template <typename T, bool PAIR>
 struct AcuIeee {
     using S = T;
     using V = T;
     // CTAs per SM the kernel is compiled for: FP32 fits five (47 registers, no spills), FP64 four
     static constexpr int kMinBlocks = sizeof(T) == 4 ? 5 : 4;
-    static constexpr bool kRetest = true;  // quotients are taken before their dividends are tested
-    struct C {
-        T dtr, dtk;
-        DivC<T> h[3];
-        uint32_t lo;  // the smallest dividend key all three take without a test
-    };
+    // quotients are taken before their dividends are tested, unless a divisor has no pair (PAIR = false)
+    static constexpr bool kRetest = PAIR;
+    static constexpr AcuDiv kFirst = PAIR ? ACU_UNTESTED : ACU_NOPAIR, kAlone = PAIR ? ACU_TESTED : ACU_NOPAIR;
+    using C = AcuIeeeC<T>;
     static __device__ __forceinline__ V in(S x, bool&) { return x; }
     static __device__ __forceinline__ V add(V a, V b) { return a + b; }
     static __device__ __forceinline__ V sub(V a, V b) { return a - b; }
     // `- dt/ρ*@d_i(P)/h`: dt/ρ is one host value (Julia evaluates dt/ρ first)
-    // FAST: without the dividend tests; *key keeps the smallest dividend key (see DivF)
-    template <bool FAST>
+    // *key keeps the smallest dividend key where HOW is ACU_UNTESTED
+    template <AcuDiv HOW>
     static __device__ __forceinline__ V dv(V a, const C& c, int d, uint32_t* key) {
-        return FAST ? dvd(a, DivF<T>{c.h[d], key}) : div_c(a, c.h[d]);
+        if constexpr (HOW == ACU_UNTESTED) return dvd(a, DivF<T>{c.h[d], key});
+        else if constexpr (HOW == ACU_TESTED) return div_c(a, c.h[d]);
+        else return dvd(a, DivG<T>{c.h[d]});
     }
-    template <bool FAST>
+    template <AcuDiv HOW>
     static __device__ __forceinline__ V vdel(V pa, V pb, const C& c, int d, uint32_t* key) {
-        return -dv<FAST>(c.dtr * (pa - pb), c, d, key);
+        return -dv<HOW>(c.dtr * (pa - pb), c, d, key);
     }
     // `- dt*k*(@d_xa(Vx)/dx + @d_ya(Vy)/dy + @d_za(Vz)/dz)`
-    template <bool FAST>
+    template <AcuDiv HOW>
     static __device__ __forceinline__ V pdel(V ax, V ay, V az, const C& c, uint32_t* key) {
-        return -(c.dtk * ((dv<FAST>(ax, c, 0, key) + dv<FAST>(ay, c, 1, key)) + dv<FAST>(az, c, 2, key)));
+        return -(c.dtk * ((dv<HOW>(ax, c, 0, key) + dv<HOW>(ay, c, 1, key)) + dv<HOW>(az, c, 2, key)));
     }
     static __device__ __forceinline__ S store(S, V nv, V) { return nv; }
     static __device__ __forceinline__ V shfl_up(V v) { return __shfl_up_sync(0xFFFFFFFFu, v, 1); }
@@ -97,6 +104,7 @@ struct AcuSplit {
     using V = dd;
     static constexpr int kMinBlocks = 4;
     static constexpr bool kRetest = false;
+    static constexpr AcuDiv kFirst = ACU_TESTED, kAlone = ACU_TESTED;  // (it divides by nothing)
     struct C {
         dd cv[3];  // (dt/ρ)/h_d as h + l, and its remainder r (h + l + r exact to ~2^-72)
         dd ck[3];  // (dt·k)/h_d
@@ -115,12 +123,12 @@ struct AcuSplit {
     static __device__ __forceinline__ V in(S x, bool& big) { return dd_split(x, big); }
     static __device__ __forceinline__ V add(V a, V b) { return dd_add(a, b); }
     static __device__ __forceinline__ V sub(V a, V b) { return dd_sub(a, b); }
-    template <bool FAST>
+    template <AcuDiv>
     static __device__ __forceinline__ V vdel(V pa, V pb, const C& c, int d, uint32_t*) {
         const V m = mulc(dd_sub(pa, pb), c.cv[d], c.cvr[d]);
         return {-m.h, -m.l};
     }
-    template <bool FAST>
+    template <AcuDiv>
     static __device__ __forceinline__ V pdel(V ax, V ay, V az, const C& c, uint32_t*) {
         const V m = dd_add(dd_add(mulc(ax, c.ck[0], c.ckr[0]), mulc(ay, c.ck[1], c.ckr[1])), mulc(az, c.ck[2], c.ckr[2]));
         return {-m.h, -m.l};
@@ -178,7 +186,7 @@ __global__ void __launch_bounds__(32 * ACU_W, AR::kMinBlocks) acoustic_step_kern
         const S vo = xv ? a.Vz[oP] : S(0);
         const bool inner = m_vz && z0 >= 1;
         const S pm = (xv && inner) ? a.P[oP - sP] : S(0);
-        vzc = inner ? AR::add(AR::in(vo, big), AR::template vdel<false>(pc, AR::in(pm, big), c, 2, nullptr))
+        vzc = inner ? AR::add(AR::in(vo, big), AR::template vdel<AR::kAlone>(pc, AR::in(pm, big), c, 2, nullptr))
                     : AR::in(vo, big);
         if (xv && z0 == 0) a.Vz2[oP] = vo;  // face 0 is outside @inn(Vz)
     }
@@ -214,8 +222,8 @@ __global__ void __launch_bounds__(32 * ACU_W, AR::kMinBlocks) acoustic_step_kern
         V vzn, pnv;
         // the new faces of the plane and its P. Quotients are taken without testing their dividends;
         // a warp that met one too small for that evaluates and stores the plane again with the tests.
-        auto plane = [&](auto fast, uint32_t* key) {
-            constexpr bool F = decltype(fast)::value;
+        auto plane = [&](auto how, uint32_t* key) {
+            constexpr AcuDiv F = decltype(how)::value;
             // Vy on faces y and y + 1
             V vyn0 = AR::in(vy0, big), vyn1 = AR::in(vy1, big);
             S st0 = vy0;
@@ -260,9 +268,9 @@ __global__ void __launch_bounds__(32 * ACU_W, AR::kMinBlocks) acoustic_step_kern
             }
         };
         uint32_t key = 0xFFFFFFFFu;
-        plane(std::true_type{}, &key);
+        plane(std::integral_constant<AcuDiv, AR::kFirst>{}, &key);
         if constexpr (AR::kRetest)
-            if (__any_sync(0xFFFFFFFFu, key < c.lo)) plane(std::false_type{}, &key);
+            if (__any_sync(0xFFFFFFFFu, key < c.lo)) plane(std::integral_constant<AcuDiv, ACU_TESTED>{}, &key);
         vzc = vzn;
         pc = pnv;
         pr = pn;
@@ -352,15 +360,17 @@ int acoustic_step(const ps_array& Vx, const ps_array& Vy, const ps_array& Vz, co
         if (fp64_mode != PS_FP64_IEEE) return fail(PS_ERR_UNSUPPORTED, "ps_acoustic3d_step: fp64_mode needs FP64 arrays");
         // FP32: the scalars are FP32 numbers, dt/ρ and dt·k evaluated in FP32 (Float32 Data.Number)
         const float h[3] = {(float)dx, (float)dy, (float)dz};
-        AcuIeee<float>::C c{(float)dt / (float)rho, (float)dt * (float)k, {}, 0u};
+        AcuIeeeC<float> c{(float)dt / (float)rho, (float)dt * (float)k, {}, 0u};
         c.lo = make_div3(h, c.h);
-        return launch_acoustic<AcuIeee<float>>(Vx, Vy, Vz, P, Vx2, Vy2, Vz2, P2, c, st, s);
+        return c.lo != kNoPair ? launch_acoustic<AcuIeee<float, true>>(Vx, Vy, Vz, P, Vx2, Vy2, Vz2, P2, c, st, s)
+                               : launch_acoustic<AcuIeee<float, false>>(Vx, Vy, Vz, P, Vx2, Vy2, Vz2, P2, c, st, s);
     }
     if (fp64_mode == PS_FP64_IEEE) {
         const double h[3] = {dx, dy, dz};
-        AcuIeee<double>::C c{dt / rho, dt * k, {}, 0u};
+        AcuIeeeC<double> c{dt / rho, dt * k, {}, 0u};
         c.lo = make_div3(h, c.h);
-        return launch_acoustic<AcuIeee<double>>(Vx, Vy, Vz, P, Vx2, Vy2, Vz2, P2, c, st, s);
+        return c.lo != kNoPair ? launch_acoustic<AcuIeee<double, true>>(Vx, Vy, Vz, P, Vx2, Vy2, Vz2, P2, c, st, s)
+                               : launch_acoustic<AcuIeee<double, false>>(Vx, Vy, Vz, P, Vx2, Vy2, Vz2, P2, c, st, s);
     }
     if (fp64_mode != PS_FP64_SPLIT)
         return fail(PS_ERR_UNSUPPORTED, "ps_acoustic3d_step: fp64_mode %d (IEEE or SPLIT)", fp64_mode);

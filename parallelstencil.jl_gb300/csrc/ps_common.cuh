@@ -221,6 +221,11 @@ __device__ __forceinline__ void ordered_tile_done(const TileOrder& o) {
 // where a/b does. The test is on integer keys (zero has the largest) and costs no FP64 instruction;
 // the FP64 division is 2 FP64 instructions instead of 7 (GB300 issues 2 FP64 per clock per SM).
 //
+// A launch with a divisor without a pair runs a variant of its kernel that tests every dividend at once (PAIR =
+// false, DivG). Quotients taken untested first, for nothing, and then the tested ones: acoustic FP32 255^3 214 us per step
+// instead of 142 (110 where all have pairs), FP64 1744 instead of 1355 (870); Stokes3D 127^3 FP32 91 instead of
+// 75 (61) per iteration, FP64 1306 instead of 752 (449).
+//
 // div_slow, for a divisor without a pair: Markstein's method (P. W. Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Develop. 34 (1990)
 // 111-119): with y = RN(1/b) and a quotient q within one ulp of a/b, the remainder r = a - b q is
@@ -232,9 +237,16 @@ __device__ __forceinline__ void ordered_tile_done(const TileOrder& o) {
 template <typename T>
 struct DivC {
     T b, yh, yl;
-    uint32_t lo;   // div_key of the smallest dividend of the fast path
-    uint32_t fix;  // no pair: yh = RN(1/b), yl a zero of its sign (exact for zeros, the only dividends let through)
+    uint32_t lo;   // div_key of the smallest dividend of the pair; kNoPair: no pair (zeros only)
+    uint32_t fix;  // no pair, Markstein's method: yh = RN(1/b), yl a zero of its sign (exact for zeros), and the
+                   // number of keys from kMarkstein on that it takes
 };
+constexpr uint32_t kNoPair = 0xFFFFFFFFu;
+// Keys of Markstein's method: 2^-100 <= |a| <= 2^70 (FP32), 2^-960 <= |a| <= 2^900 (FP64).
+template <typename T>
+constexpr uint32_t kMarkstein = sizeof(T) == 4 ? 0x1AFFFFFFu : 0x07DFFFFFu;
+template <typename T>
+constexpr uint32_t kMarksteinEnd = sizeof(T) == 4 ? 0xC5000000u : 0xF0600000u;
 
 // Key of a dividend: grows with |a|, largest for zeros.
 __host__ __device__ __forceinline__ uint32_t div_key_bits(uint32_t hi, uint32_t rest) {
@@ -279,12 +291,20 @@ inline bool div_pair_exact(T b, T yh, T yl) {
     return true;
 }
 template <typename T>
+inline DivC<T> div_without_pair(DivC<T> d) {
+    d.yh = (T)1 / d.b;
+    d.yl = std::copysign((T)0, d.b);  // (of yh's sign, for a zero quotient's)
+    d.lo = kNoPair;
+    d.fix = kMarksteinEnd<T> - kMarkstein<T>;
+    return d;
+}
+template <typename T>
 inline DivC<T> make_div(T b) {
     const T lim = sizeof(T) == 4 ? (T)0x1p20 : (T)0x1p60;
     const T ab = std::fabs(b);
     DivC<T> d;
     d.b = b;
-    d.lo = 0xFFFFFFFFu;  // zeros only: their quotient is a zero, or NaN for a zero or NaN divisor
+    d.lo = kNoPair;  // zeros only: their quotient is a zero, or NaN for a zero or NaN divisor
     d.yh = ab > 0 ? std::copysign((T)1, b) : std::numeric_limits<T>::quiet_NaN();
     d.yl = d.yh;
     d.fix = 0;
@@ -318,41 +338,41 @@ inline DivC<T> make_div(T b) {
         }
         return d;
     }
-    d.yh = (T)1 / b;
-    d.yl = std::copysign((T)0, b);  // (of yh's sign, for a zero quotient's)
-    d.fix = 1;
-    return d;
+    return div_without_pair(d);
 }
-// The divisors of one kernel and the key every one of them takes without a test; returns that key.
+// The divisors of one kernel; returns the key from which all of them take their pairs. Where one has none, it is kNoPair
+// and they all divide by Markstein's method (or IEEE).
 template <typename T>
 inline uint32_t make_div3(const T b[3], DivC<T> d[3]) {
     d[0] = make_div(b[0]);
     d[1] = b[1] == b[0] ? d[0] : make_div(b[1]);
     d[2] = b[2] == b[0] ? d[0] : b[2] == b[1] ? d[1] : make_div(b[2]);
-    return std::max(d[0].lo, std::max(d[1].lo, d[2].lo));
+    const uint32_t lo = std::max(d[0].lo, std::max(d[1].lo, d[2].lo));
+    if (lo == kNoPair)
+        for (int i = 0; i < 3; i++)
+            if (d[i].lo != kNoPair) d[i] = div_without_pair(d[i]);
+    return lo;
 }
 __device__ __forceinline__ float div_pair(float a, const DivC<float>& d) { return fmaf(a, d.yh, a * d.yl); }
 __device__ __forceinline__ double div_pair(double a, const DivC<double>& d) { return fma(a, d.yh, a * d.yl); }
-__device__ __forceinline__ float div_slow(float a, const DivC<float>& d) {
-    const uint32_t k = div_key(a);
-    if (d.fix && k >= 0x1AFFFFFFu && k < 0xC5000000u) {  // 2^-100 <= |a| <= 2^70
-        float q = a * d.yh;
-        float r = fmaf(-q, d.b, a);
-        q = fmaf(r, d.yh, q);
-        r = fmaf(-q, d.b, a);
-        return fmaf(r, d.yh, q);
-    }
-    return a / d.b;
+__device__ __forceinline__ float div_markstein(float a, const DivC<float>& d) {
+    float q = a * d.yh;
+    float r = fmaf(-q, d.b, a);
+    q = fmaf(r, d.yh, q);
+    r = fmaf(-q, d.b, a);
+    return fmaf(r, d.yh, q);
 }
-__device__ __forceinline__ double div_slow(double a, const DivC<double>& d) {
+__device__ __forceinline__ double div_markstein(double a, const DivC<double>& d) {
+    double q = a * d.yh;
+    double r = fma(-q, d.b, a);
+    q = fma(r, d.yh, q);
+    r = fma(-q, d.b, a);
+    return fma(r, d.yh, q);
+}
+template <typename T>
+__device__ __forceinline__ T div_slow(T a, const DivC<T>& d) {
     const uint32_t k = div_key(a);
-    if (d.fix && k >= 0x07DFFFFFu && k < 0xF0600000u) {  // 2^-960 <= |a| <= 2^900
-        double q = a * d.yh;
-        double r = fma(-q, d.b, a);
-        q = fma(r, d.yh, q);
-        r = fma(-q, d.b, a);
-        return fma(r, d.yh, q);
-    }
+    if (d.fix && k >= kMarkstein<T> && k < kMarksteinEnd<T>) return div_markstein(a, d);
     return a / d.b;
 }
 template <typename T>
@@ -367,6 +387,33 @@ struct DivF {
     const DivC<T>& d;
     uint32_t* key;
 };
+// A divisor that has a pair, for kernels that only test (FP32 one-launch Stokes3D iteration at 127^3: 205 us against 209
+// with DivC, whose Markstein branch is one more).
+template <typename T>
+struct DivP {
+    const DivC<T>& d;
+};
+// A divisor of a launch whose divisors have no pairs (make_div3).
+template <typename T>
+struct DivG {
+    const DivC<T>& d;
+};
+// A divisor of either kind, in a kernel that is compiled once for both: keys lo .. lo + span - 1 take its pair or
+// Markstein's method (the README's FP32 diffusion step at 255^3: 102 us with pairs, 113 without; with DivC 112
+// and 134).
+template <typename T>
+struct DivA {
+    const DivC<T>& d;
+    uint32_t lo, span;
+};
+template <typename T>
+inline void div_keys(const DivC<T>& d, uint32_t* lo, uint32_t* span) {
+    *lo = d.fix ? kMarkstein<T> : d.lo == kNoPair ? 0u : d.lo;
+    *span = d.fix ? d.fix : 0u - *lo;
+}
+// What a kernel that tests every dividend once divides by.
+template <typename T, bool PAIR>
+using DivBy = std::conditional_t<PAIR, const DivC<T>&, DivG<T>>;
 
 // x * 2^k by an integer addition to the exponent (a multiplication is an FP64 instruction). Equal to
 // the product, bit for bit, for zeros and wherever x and x 2^k are normal: *key keeps x's key as
@@ -396,6 +443,34 @@ __host__ __device__ __forceinline__ T dvd(T a, T h) {
 template <typename T>
 __device__ __forceinline__ T dvd(T a, const DivC<T>& h) {
     return div_c(a, h);
+}
+// A value that the compiler may not compute with before this point: without it the instructions of an IEEE division
+// that is hardly ever taken are issued beside the quotient that is (3 of them on the FP64 pipe).
+__device__ __forceinline__ float not_ahead(float a) {
+    asm volatile("" : "+f"(a));
+    return a;
+}
+__device__ __forceinline__ double not_ahead(double a) {
+    asm volatile("" : "+d"(a));
+    return a;
+}
+template <typename T>
+__device__ __forceinline__ T dvd(T a, const DivG<T>& h) {
+    const uint32_t k = div_key(a);
+    if (k - kMarkstein<T> < h.d.fix) return div_markstein(a, h.d);
+    if (k == 0xFFFFFFFFu) return a * h.d.yh;
+    return not_ahead(a) / h.d.b;
+}
+template <typename T>
+__device__ __forceinline__ T dvd(T a, const DivP<T>& h) {
+    if (div_key(a) >= h.d.lo) return div_pair(a, h.d);
+    return not_ahead(a) / h.d.b;
+}
+template <typename T>
+__device__ __forceinline__ T dvd(T a, const DivA<T>& h) {
+    const uint32_t k = div_key(a);
+    if (k - h.lo < h.span) return h.d.fix ? div_markstein(a, h.d) : div_pair(a, h.d);
+    return k == 0xFFFFFFFFu ? div_pair(a, h.d) : a / h.d.b;
 }
 template <typename T>
 __device__ __forceinline__ T dvd(T a, const DivF<T>& h) {

@@ -271,7 +271,8 @@ int encode_bf16_box(CUtensorMap* map, const void* ptr, int rank, const uint64_t*
     return PS_OK;
 }
 
-// ps_check_division: div_c against the IEEE division. Dividend i: FP32 -- significand i mod 2^23,
+// ps_check_division: div_c and the kernels' other forms (g: the divisor as one without a pair) against the IEEE
+// division. Dividend i: FP32 -- significand i mod 2^23,
 // exponent and sign from i / 2^23 (every significand in each listed binade, both signs); FP64 --
 // a hashed 52-bit significand, exponent and sign from the hash too. The first 64 indices are
 // special values (zeros, subnormals, extremes, infinities, NaN).
@@ -294,7 +295,7 @@ __device__ T special_dividend(int i) {
     return v[i & 15];
 }
 
-__global__ void check_div32_kernel(DivC<float> d, unsigned long long* bad) {
+__global__ void check_div32_kernel(DivC<float> d, DivC<float> g, uint32_t lo, uint32_t span, unsigned long long* bad) {
     const int64_t n = 12LL * 2 * (1LL << 23);
     unsigned long long local = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -307,13 +308,20 @@ __global__ void check_div32_kernel(DivC<float> d, unsigned long long* bad) {
             const int e = c_exp32[(k >> 1) % 12];
             a = ldexpf(1.0f + (float)m * 0x1p-23f, e) * ((k & 1) ? -1.0f : 1.0f);
         }
-        const float q1 = div_c(a, d), q2 = a / d.b;
-        if (__float_as_uint(q1) != __float_as_uint(q2) && !(isnan(q1) && isnan(q2))) ++local;
+        const float q = a / d.b;
+        auto check = [&](float q1) {
+            if (__float_as_uint(q1) != __float_as_uint(q) && !(isnan(q1) && isnan(q))) ++local;
+        };
+        check(div_c(a, d));
+        check(dvd(a, DivA<float>{d, lo, span}));
+        check(dvd(a, DivG<float>{g}));
+        if (d.lo != kNoPair) check(dvd(a, DivP<float>{d}));
     }
     if (local) atomicAdd(bad, local);
 }
 
-__global__ void check_div64_kernel(DivC<double> d, int64_t n, uint64_t seed, unsigned long long* bad) {
+__global__ void check_div64_kernel(DivC<double> d, DivC<double> g, uint32_t lo, uint32_t span, int64_t n, uint64_t seed,
+                                   unsigned long long* bad) {
     unsigned long long local = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double a;
@@ -324,8 +332,14 @@ __global__ void check_div64_kernel(DivC<double> d, int64_t n, uint64_t seed, uns
             const int e = c_exp64[(h >> 52) % 12];
             a = ldexp(1.0 + (double)(h & ((1ull << 52) - 1)) * 0x1p-52, e) * ((h >> 63) ? -1.0 : 1.0);
         }
-        const double q1 = div_c(a, d), q2 = a / d.b;
-        if (__double_as_longlong(q1) != __double_as_longlong(q2) && !(isnan(q1) && isnan(q2))) ++local;
+        const double q = a / d.b;
+        auto check = [&](double q1) {
+            if (__double_as_longlong(q1) != __double_as_longlong(q) && !(isnan(q1) && isnan(q))) ++local;
+        };
+        check(div_c(a, d));
+        check(dvd(a, DivA<double>{d, lo, span}));
+        check(dvd(a, DivG<double>{g}));
+        if (d.lo != kNoPair) check(dvd(a, DivP<double>{d}));
     }
     if (local) atomicAdd(bad, local);
 }
@@ -346,10 +360,19 @@ int ps_check_division(double b, int32_t dtype, int64_t n, uint64_t seed, int64_t
     PS_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&bad), sizeof(*bad), s));
     PS_CUDA_TRY(cudaMemsetAsync(bad, 0, sizeof(*bad), s));
     const unsigned grid = (unsigned)st->num_sms * 8;
+    auto divisors = [](auto d, auto run) {
+        uint32_t lo, span;
+        div_keys(d, &lo, &span);
+        run(d, d.lo != kNoPair ? div_without_pair(d) : d, lo, span);
+    };
     if (dtype == PS_F32)
-        check_div32_kernel<<<grid, 256, 0, s>>>(make_div<float>((float)b), bad);
+        divisors(make_div((float)b), [&](const DivC<float>& d, const DivC<float>& g, uint32_t lo, uint32_t span) {
+            check_div32_kernel<<<grid, 256, 0, s>>>(d, g, lo, span, bad);
+        });
     else
-        check_div64_kernel<<<grid, 256, 0, s>>>(make_div<double>(b), n, seed, bad);
+        divisors(make_div(b), [&](const DivC<double>& d, const DivC<double>& g, uint32_t lo, uint32_t span) {
+            check_div64_kernel<<<grid, 256, 0, s>>>(d, g, lo, span, n, seed, bad);
+        });
     unsigned long long h = 0;
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, bad, sizeof(h), cudaMemcpyDeviceToHost, s);

@@ -372,6 +372,7 @@ struct DiffParams {
     T lam, dt, hx, hy, hz;
     DivC<T> q[3];  // the divisors hx*hx, hy*hy, hz*hz of the `/dx^2` form
     uint32_t lo;   // the smallest dividend key all three take without a test
+    uint32_t klo[3], span[3];  // see DivA
     T h2[3];       // hx*hx, hy*hy, hz*hz of the `*_dx^2` form
 };
 
@@ -389,7 +390,8 @@ __device__ __forceinline__ T diff_cell(const DiffParams<T>& p, T Tc, T Txm, T Tx
             if (min(div_key(d2x), min(div_key(d2y), div_key(d2z))) >= p.lo)
                 s = (div_pair(d2x, p.q[0]) + div_pair(d2y, p.q[1])) + div_pair(d2z, p.q[2]);
             else
-                s = (div_c(d2x, p.q[0]) + div_c(d2y, p.q[1])) + div_c(d2z, p.q[2]);
+                s = (dvd(d2x, DivA<T>{p.q[0], p.klo[0], p.span[0]}) + dvd(d2y, DivA<T>{p.q[1], p.klo[1], p.span[1]})) +
+                    dvd(d2z, DivA<T>{p.q[2], p.klo[2], p.span[2]});
         } else {
             s = (d2x * p.h2[0] + d2y * p.h2[1]) + d2z * p.h2[2];
         }
@@ -725,9 +727,10 @@ __global__ void __launch_bounds__(32 * TY) diff3d_zsweep_smem(T* __restrict__ T2
 // =======================================================================================
 // acoustic3D (miniapps/acoustic3D.jl:11-21)
 // =======================================================================================
-template <typename T>
+template <typename T, bool PAIR>
 __global__ void acoustic_v_kernel(T* __restrict__ Vx, T* __restrict__ Vy, T* __restrict__ Vz, const T* __restrict__ P,
                                   int64_t nx, int64_t ny, int64_t nz, T dtr, DivC<T> dx, DivC<T> dy, DivC<T> dz) {
+    const DivBy<T, PAIR> hx{dx}, hy{dy}, hz{dz};
     // grid = (nx+1, ny+1, nz+1); each statement masked by @inn of its left-hand array.
     int64_t tx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     int64_t ty = blockIdx.y * (int64_t)blockDim.y + threadIdx.y;
@@ -737,25 +740,26 @@ __global__ void acoustic_v_kernel(T* __restrict__ Vx, T* __restrict__ Vy, T* __r
         if (tx < nx - 1 && ty < ny - 2 && tz < nz - 2) {  // @inn(Vx): Vx is (nx+1, ny, nz)
             int64_t v = (tx + 1) + (nx + 1) * ((ty + 1) + ny * (tz + 1));
             int64_t pc = (tx + 1) + sy * (ty + 1) + sz * (tz + 1);
-            Vx[v] = Vx[v] - div_c(dtr * (P[pc] - P[pc - 1]), dx);
+            Vx[v] = Vx[v] - dvd(dtr * (P[pc] - P[pc - 1]), hx);
         }
         if (tx < nx - 2 && ty < ny - 1 && tz < nz - 2) {  // @inn(Vy): Vy is (nx, ny+1, nz)
             int64_t v = (tx + 1) + nx * ((ty + 1) + (ny + 1) * (tz + 1));
             int64_t pc = (tx + 1) + sy * (ty + 1) + sz * (tz + 1);
-            Vy[v] = Vy[v] - div_c(dtr * (P[pc] - P[pc - sy]), dy);
+            Vy[v] = Vy[v] - dvd(dtr * (P[pc] - P[pc - sy]), hy);
         }
         if (tx < nx - 2 && ty < ny - 2 && tz < nz - 1) {  // @inn(Vz): Vz is (nx, ny, nz+1)
             int64_t v = (tx + 1) + nx * ((ty + 1) + ny * (tz + 1));
             int64_t pc = (tx + 1) + sy * (ty + 1) + sz * (tz + 1);
-            Vz[v] = Vz[v] - div_c(dtr * (P[pc] - P[pc - sz]), dz);
+            Vz[v] = Vz[v] - dvd(dtr * (P[pc] - P[pc - sz]), hz);
         }
     }
 }
 
-template <typename T>
+template <typename T, bool PAIR>
 __global__ void acoustic_p_kernel(T* __restrict__ P, const T* __restrict__ Vx, const T* __restrict__ Vy,
                                   const T* __restrict__ Vz, int64_t nx, int64_t ny, int64_t nz, T dtk, DivC<T> dx,
                                   DivC<T> dy, DivC<T> dz) {
+    const DivBy<T, PAIR> hx{dx}, hy{dy}, hz{dz};
     int64_t ix = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     int64_t iy = blockIdx.y * (int64_t)blockDim.y + threadIdx.y;
     if (ix >= nx || iy >= ny) return;
@@ -764,7 +768,7 @@ __global__ void acoustic_p_kernel(T* __restrict__ P, const T* __restrict__ Vx, c
         T ay = Vy[ix + nx * ((iy + 1) + (ny + 1) * iz)] - Vy[ix + nx * (iy + (ny + 1) * iz)];
         T az = Vz[ix + nx * (iy + ny * (iz + 1))] - Vz[ix + nx * (iy + ny * iz)];
         int64_t pc = ix + nx * (iy + ny * iz);
-        P[pc] = P[pc] - dtk * ((div_c(ax, dx) + div_c(ay, dy)) + div_c(az, dz));
+        P[pc] = P[pc] - dtk * ((dvd(ax, hx) + dvd(ay, hy)) + dvd(az, hz));
     }
 }
 
@@ -788,7 +792,10 @@ static DiffParams<T> diff_params(int form, double lam, double dt, double hx, dou
     p.h2[0] = x * x;
     p.h2[1] = y * y;
     p.h2[2] = z * z;
-    if (form == PS_DIFF_DIV) p.lo = make_div3(p.h2, p.q);
+    if (form == PS_DIFF_DIV) {
+        p.lo = make_div3(p.h2, p.q);
+        for (int d = 0; d < 3; d++) div_keys(p.q[d], &p.klo[d], &p.span[d]);
+    }
     return p;
 }
 
@@ -1239,16 +1246,16 @@ int ps_acoustic3d_v(ps_array Vx, ps_array Vy, ps_array Vz, ps_array P, double dt
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     dim3 blk(32, 8, 1);
     dim3 grd = grid3(nx + 1, ny + 1, nz + 1, blk);
-    if (P.dtype == PS_F64)
-        acoustic_v_kernel<double><<<grd, blk, 0, s>>>(static_cast<double*>(Vx.ptr), static_cast<double*>(Vy.ptr),
-                                                      static_cast<double*>(Vz.ptr), static_cast<const double*>(P.ptr),
-                                                      nx, ny, nz, dt / rho, make_div(dx), make_div(dy),
-                                                      make_div(dz));
-    else
-        acoustic_v_kernel<float><<<grd, blk, 0, s>>>(static_cast<float*>(Vx.ptr), static_cast<float*>(Vy.ptr),
-                                                     static_cast<float*>(Vz.ptr), static_cast<const float*>(P.ptr), nx,
-                                                     ny, nz, (float)dt / (float)rho, make_div((float)dx),
-                                                     make_div((float)dy), make_div((float)dz));
+    auto run = [&](auto t) {
+        using T = decltype(t);
+        const T h[3] = {(T)dx, (T)dy, (T)dz};
+        DivC<T> d[3];
+        const auto kernel = make_div3(h, d) != kNoPair ? acoustic_v_kernel<T, true> : acoustic_v_kernel<T, false>;
+        kernel<<<grd, blk, 0, s>>>(static_cast<T*>(Vx.ptr), static_cast<T*>(Vy.ptr), static_cast<T*>(Vz.ptr),
+                                   static_cast<const T*>(P.ptr), nx, ny, nz, (T)dt / (T)rho, d[0], d[1], d[2]);
+    };
+    if (P.dtype == PS_F64) run(double{});
+    else run(float{});
     return finish_launch(s, sync, "ps_acoustic3d_v");
 }
 
@@ -1270,16 +1277,16 @@ int ps_acoustic3d_p(ps_array P, ps_array Vx, ps_array Vy, ps_array Vz, double dt
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     dim3 blk(32, 8, 1);
     dim3 grd = grid3(nx, ny, nz, blk);
-    if (P.dtype == PS_F64)
-        acoustic_p_kernel<double><<<grd, blk, 0, s>>>(static_cast<double*>(P.ptr), static_cast<const double*>(Vx.ptr),
-                                                      static_cast<const double*>(Vy.ptr),
-                                                      static_cast<const double*>(Vz.ptr), nx, ny, nz, dt * k,
-                                                      make_div(dx), make_div(dy), make_div(dz));
-    else
-        acoustic_p_kernel<float><<<grd, blk, 0, s>>>(static_cast<float*>(P.ptr), static_cast<const float*>(Vx.ptr),
-                                                     static_cast<const float*>(Vy.ptr), static_cast<const float*>(Vz.ptr),
-                                                     nx, ny, nz, (float)dt * (float)k, make_div((float)dx),
-                                                     make_div((float)dy), make_div((float)dz));
+    auto run = [&](auto t) {
+        using T = decltype(t);
+        const T h[3] = {(T)dx, (T)dy, (T)dz};
+        DivC<T> d[3];
+        const auto kernel = make_div3(h, d) != kNoPair ? acoustic_p_kernel<T, true> : acoustic_p_kernel<T, false>;
+        kernel<<<grd, blk, 0, s>>>(static_cast<T*>(P.ptr), static_cast<const T*>(Vx.ptr), static_cast<const T*>(Vy.ptr),
+                                   static_cast<const T*>(Vz.ptr), nx, ny, nz, (T)dt * (T)k, d[0], d[1], d[2]);
+    };
+    if (P.dtype == PS_F64) run(double{});
+    else run(float{});
     return finish_launch(s, sync, "ps_acoustic3d_p");
 }
 

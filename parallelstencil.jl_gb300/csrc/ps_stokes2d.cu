@@ -86,9 +86,11 @@ struct S2P {
 
 template <typename T>
 static S2P<T> s2p(const ps_stokes2d_params& p) {
-    const DivC<T> dx = make_div((T)p.dx), dy = make_div((T)p.dy);
-    return S2P<T>{dx,        dy,        (T)p.dampX,    (T)p.dampY,    (T)p.Vsc,
-                  (T)p.Ptsc, (T)p.min_dxy2, (T)p.max_nxy, std::max(dx.lo, dy.lo)};
+    const T h[3] = {(T)p.dx, (T)p.dy, (T)p.dx};
+    DivC<T> d[3];
+    const uint32_t lo = make_div3(h, d);
+    return S2P<T>{d[0],      d[1],      (T)p.dampX,    (T)p.dampY,    (T)p.Vsc,
+                  (T)p.Ptsc, (T)p.min_dxy2, (T)p.max_nxy, lo};
 }
 
 #define A2(a, i, j, n0) (a)[(int64_t)(i) + (int64_t)(n0) * (int64_t)(j)]
@@ -232,12 +234,17 @@ __device__ __forceinline__ double warp_sum(double v) {
 // pipe even when predicated off). I: index type (int where every array has fewer than 2^31 elements).
 //
 // S2_DIV evaluates a statement without testing each dividend, and again with the tests (and the IEEE
-// division where they fail) in the rare case that one of its dividends is too small.
+// division where they fail) in the rare case that one of its dividends is too small. PAIR: both divisors have a
+// reciprocal pair; without one every dividend is tested from the start (see DivC).
 #define S2_DIV(stmt)                                                            \
     do {                                                                        \
-        uint32_t key_ = 0xFFFFFFFFu;                                            \
-        stmt(DivF<T>{p.dx, &key_}, DivF<T>{p.dy, &key_});                       \
-        if (key_ < p.lo) stmt(p.dx, p.dy);                                      \
+        if constexpr (PAIR) {                                                   \
+            uint32_t key_ = 0xFFFFFFFFu;                                        \
+            stmt(DivF<T>{p.dx, &key_}, DivF<T>{p.dy, &key_});                   \
+            if (key_ < p.lo) stmt(p.dx, p.dy);                                  \
+        } else {                                                                \
+            stmt(DivG<T>{p.dx}, DivG<T>{p.dy});                                 \
+        }                                                                       \
     } while (0)
 
 // (a + b) * 0.5, the buoyancy average
@@ -260,7 +267,7 @@ constexpr int64_t s2_max_rows() {
     return kGridY * s2_block_rows<T, int64_t>() - 1;
 }
 
-template <typename T, bool DEFECT, typename I, bool STORE_TMP, bool RED>
+template <typename T, bool DEFECT, typename I, bool STORE_TMP, bool RED, bool PAIR>
 __global__ void __launch_bounds__(32 * s2_block_rows<T, I>()) s2_cells(S2Fused<T> a, S2P<T> p) {
     const I nx = (I)a.nx, ny = (I)a.ny;
     const I i = (I)(blockIdx.x * 32 + threadIdx.x), j = (I)(blockIdx.y * s2_block_rows<T, I>() + threadIdx.y);
@@ -317,7 +324,7 @@ __global__ void __launch_bounds__(32 * s2_block_rows<T, I>()) s2_cells(S2Fused<T
     }
 }
 
-template <typename T, bool DEFECT, typename I, bool STORE_TMP, bool RED>
+template <typename T, bool DEFECT, typename I, bool STORE_TMP, bool RED, bool PAIR>
 __global__ void __launch_bounds__(32 * s2_block_rows<T, I>()) s2_faces(S2Fused<T> a, S2P<T> p) {
     const I nx = (I)a.nx, ny = (I)a.ny;
     const I i = (I)(blockIdx.x * 32 + threadIdx.x), j = (I)(blockIdx.y * s2_block_rows<T, I>() + threadIdx.y);
@@ -571,13 +578,21 @@ static void launch_cells_faces(const S2Fused<T>& a, const S2P<T>& p, cudaStream_
         else cells<<<gc, blk, 0, s>>>(a, p);
         launch_dependent(faces, gf, blk, 0, s, a, p);
     };
-    if (a.red) {
-        if (i32) launch(s2_cells<T, DEFECT, int, STORE_TMP, true>, s2_faces<T, DEFECT, int, STORE_TMP, true>);
-        else launch(s2_cells<T, DEFECT, int64_t, STORE_TMP, true>, s2_faces<T, DEFECT, int64_t, STORE_TMP, true>);
-    } else {
-        if (i32) launch(s2_cells<T, DEFECT, int, STORE_TMP, false>, s2_faces<T, DEFECT, int, STORE_TMP, false>);
-        else launch(s2_cells<T, DEFECT, int64_t, STORE_TMP, false>, s2_faces<T, DEFECT, int64_t, STORE_TMP, false>);
-    }
+    auto with = [&](auto index, auto red, auto pair) {
+        using I = decltype(index);
+        constexpr bool RED = decltype(red)::value, PAIR = decltype(pair)::value;
+        launch(s2_cells<T, DEFECT, I, STORE_TMP, RED, PAIR>, s2_faces<T, DEFECT, I, STORE_TMP, RED, PAIR>);
+    };
+    auto pairs = [&](auto index, auto red) {
+        if (p.lo != kNoPair) with(index, red, std::true_type{});
+        else with(index, red, std::false_type{});
+    };
+    auto sums = [&](auto index) {
+        if (a.red) pairs(index, std::true_type{});
+        else pairs(index, std::false_type{});
+    };
+    if (i32) sums(int{});
+    else sums(int64_t{});
 }
 
 template <typename T>

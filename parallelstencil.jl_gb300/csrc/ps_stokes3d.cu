@@ -103,8 +103,8 @@ __device__ __forceinline__ double s3_tsh_sum(double msum, double a, DivF<double>
     *ha.key = min(*ha.key, min(div_key(msum), div_key(e)));
     return scale_pow2(msum * e, -2, ha.key);
 }
-template <typename T>
-__device__ __forceinline__ T s3_tsh(T m0, T m1, T m2, T m3, T a, const DivC<T>& ha, T b, const DivC<T>& hb) {
+template <typename T, typename H>
+__device__ __forceinline__ T s3_tsh(T m0, T m1, T m2, T m3, T a, const H& ha, T b, const H& hb) {
     return s3_tsh_sum(((m0 + m1) + m2) + m3, a, ha, b, hb);
 }
 // (a + b) * 0.5, the buoyancy average
@@ -347,7 +347,7 @@ template <typename T, typename I>
 constexpr int s3_blocks(bool cells) {
     return sizeof(I) == 8 ? (sizeof(T) == 4 ? 4 : 3) : sizeof(T) == 4 ? (cells ? 10 : 9) : 12;
 }
-template <typename T, int MODE, typename I, bool STORE>
+template <typename T, int MODE, typename I, bool STORE, bool PAIR>
 __global__ void __launch_bounds__(32 * s3_rows<T, I>(), s3_blocks<T, I>(true)) s3_cells(S3A<T> a, S3P<T> p) {
     const I nx = (I)a.nx, ny = (I)a.ny, nz = (I)a.nz;
     const I x = (I)(blockIdx.x * 32 + threadIdx.x), y = (I)(blockIdx.y * s3_rows<T, I>() + threadIdx.y), z = (I)blockIdx.z;
@@ -393,9 +393,13 @@ __global__ void __launch_bounds__(32 * s3_rows<T, I>(), s3_blocks<T, I>(true)) s
         if (x1 && iy && z1) txz = s3_tsh_sum(((m00 + m10) + m00n) + m10n, vx1n - vx1, hz, vzr - vz1, hx);
         if (ix && y1 && z1) tyz = s3_tsh_sum(((m00 + m01) + m00n) + m01n, vy1n - vy1, hz, vzu - vz1, hy);
     };
-    uint32_t key = 0xFFFFFFFFu;
-    cell(DivF<T>{p.dx, &key}, DivF<T>{p.dy, &key}, DivF<T>{p.dz, &key});
-    if (key < p.lo) cell(p.dx, p.dy, p.dz);
+    if constexpr (PAIR) {
+        uint32_t key = 0xFFFFFFFFu;
+        cell(DivF<T>{p.dx, &key}, DivF<T>{p.dy, &key}, DivF<T>{p.dz, &key});
+        if (key < p.lo) cell(p.dx, p.dy, p.dz);
+    } else {
+        cell(DivG<T>{p.dx}, DivG<T>{p.dy}, DivG<T>{p.dz});
+    }
     const T dp = MODE == S3_DEFECT ? d + f : d;  // the correction's continuity residual includes the outer one
     if constexpr (STORE) a.divV[c] = dp;
     if constexpr (MODE != S3_RESIDUAL) a.Pt[c] = pt - dtp * dp;
@@ -408,7 +412,7 @@ __global__ void __launch_bounds__(32 * s3_rows<T, I>(), s3_blocks<T, I>(true)) s
 }
 
 // The faces at the lower sides of the cell (x, y, z), x <= nx, y <= ny, z <= nz.
-template <typename T, int MODE, typename I, bool STORE>
+template <typename T, int MODE, typename I, bool STORE, bool PAIR>
 __device__ __forceinline__ void s3_face(const S3A<T>& a, const S3P<T>& p, const I x, const I y, const I z) {
     const I nx = (I)a.nx, ny = (I)a.ny, nz = (I)a.nz;
     const bool ix = x >= 1 && x <= nx - 2, iy = y >= 1 && y <= ny - 2, iz = z >= 1 && z <= nz - 2;
@@ -493,9 +497,13 @@ __device__ __forceinline__ void s3_face(const S3A<T>& a, const S3P<T>& p, const 
             if constexpr (MODE != S3_DEFECT) rw = rw + s3_half_sum(r0, r1, hz);
         }
     };
-    uint32_t key = 0xFFFFFFFFu;
-    resid(DivF<T>{p.dx, &key}, DivF<T>{p.dy, &key}, DivF<T>{p.dz, &key});
-    if (key < p.lo) resid(p.dx, p.dy, p.dz);
+    if constexpr (PAIR) {
+        uint32_t key = 0xFFFFFFFFu;
+        resid(DivF<T>{p.dx, &key}, DivF<T>{p.dy, &key}, DivF<T>{p.dz, &key});
+        if (key < p.lo) resid(p.dx, p.dy, p.dz);
+    } else {
+        resid(DivG<T>{p.dx}, DivG<T>{p.dy}, DivG<T>{p.dz});
+    }
     if constexpr (MODE == S3_DEFECT) {
         ru = ru + uf;
         rv = rv + vf;
@@ -549,16 +557,16 @@ __device__ __forceinline__ void s3_face(const S3A<T>& a, const S3P<T>& p, const 
 
 // One thread per position; the 64-bit variant, which runs the tallest and deepest grids too (ny = 65535 * 8 or nz =
 // 65535 cells have one more row or plane of faces than the launch has blocks), takes the positions a grid further on.
-template <typename T, int MODE, typename I, bool STORE>
+template <typename T, int MODE, typename I, bool STORE, bool PAIR>
 __global__ void __launch_bounds__(32 * s3_rows<T, I>(), s3_blocks<T, I>(false)) s3_faces(S3A<T> a, S3P<T> p) {
     const I x = (I)(blockIdx.x * 32 + threadIdx.x), y = (I)(blockIdx.y * s3_rows<T, I>() + threadIdx.y), z = (I)blockIdx.z;
     grid_dependency_wait();
     if (x > (I)a.nx) return;
     if constexpr (sizeof(I) == 8) {
         for (I v = z; v <= (I)a.nz; v += gridDim.z)
-            for (I u = y; u <= (I)a.ny; u += (I)gridDim.y * s3_rows<T, I>()) s3_face<T, MODE, I, STORE>(a, p, x, u, v);
+            for (I u = y; u <= (I)a.ny; u += (I)gridDim.y * s3_rows<T, I>()) s3_face<T, MODE, I, STORE, PAIR>(a, p, x, u, v);
     } else {
-        if (y <= (I)a.ny) s3_face<T, MODE, I, STORE>(a, p, x, y, z);
+        if (y <= (I)a.ny) s3_face<T, MODE, I, STORE, PAIR>(a, p, x, y, z);
     }
 }
 
@@ -608,7 +616,7 @@ __global__ void s3_bc_k(S3A<T> a) {
 // updated range keep their old value. Bit-identical to the one-to-one kernels (same operations on
 // the same operands, in the reference's order).
 // Two CTAs per SM in FP32 (64 registers): left to itself the compiler took 73 and one CTA, 362 us per iteration at
-// 127^3 instead of 208. FP64 (104 registers) fits one.
+// 127^3 instead of 205. FP64 (108 registers) fits one.
 constexpr int S3F_TY = 16;
 
 template <typename T>
@@ -616,8 +624,9 @@ struct S3Out {
     T *Vx, *Vy, *Vz, *Pt;
 };
 
-template <typename T, int MODE>
+template <typename T, int MODE, bool PAIR>
 __global__ void __launch_bounds__(32 * S3F_TY, sizeof(T) == 4 ? 2 : 1) s3_fused_k(S3A<T> a, S3Out<T> o, S3P<T> p, int Lz) {
+    const std::conditional_t<PAIR, DivP<T>, DivG<T>> hx{p.dx}, hy{p.dy}, hz{p.dz};
     static_assert(MODE == S3_PLAIN || MODE == S3_DEFECT, "update modes only");
     __shared__ T sPt[S3F_TY][32], sTxx[S3F_TY][32], sTyy[S3F_TY][32], sTxy[S3F_TY][32];
     __shared__ T sLxz[2][S3F_TY][32], sLyz[2][S3F_TY][32];
@@ -682,19 +691,19 @@ __global__ void __launch_bounds__(32 * S3F_TY, sizeof(T) == 4 ? 2 : 1) s3_fused_
         T pt_new = 0, d = 0, txx = 0, tyy = 0, tzz = 0, txy = 0, lxz = 0, lyz = 0, rog = 0;
         if (plane && cell_xy) {
             const int64_t c = C3(X, Y, k);
-            d = (div_c(vx_r - vx, p.dx) + div_c(vy_u - vy, p.dy)) + div_c(vz_n - vz, p.dz);
+            d = (dvd(vx_r - vx, hx) + dvd(vy_u - vy, hy)) + dvd(vz_n - vz, hz);
             T dp = d;
             if constexpr (MODE == S3_DEFECT) dp = d + a.fp[c];
             pt_new = a.Pt[c] - a.dtPt[c] * dp;
             if constexpr (MODE == S3_PLAIN) rog = a.Rog[c];
-            if (yin && k >= 1 && k <= nz - 2) txx = s3_tnn(m00, vx_r, vx, p.dx, d);
-            if (xin && k >= 1 && k <= nz - 2) tyy = s3_tnn(m00, vy_u, vy, p.dy, d);
-            if (xin && yin) tzz = s3_tnn(m00, vz_n, vz, p.dz, d);
+            if (yin && k >= 1 && k <= nz - 2) txx = s3_tnn(m00, vx_r, vx, hx, d);
+            if (xin && k >= 1 && k <= nz - 2) tyy = s3_tnn(m00, vy_u, vy, hy, d);
+            if (xin && yin) tzz = s3_tnn(m00, vz_n, vz, hz, d);
         }
         if (plane && txy_xy && k >= 1 && k <= nz - 2)
-            txy = s3_tsh(m11, m01, m10, m00, vx - vx_d, p.dy, vy - vy_l, p.dx);
-        if (plane && txz_xy && k <= nz - 2) lxz = s3_tsh(m10, m00, m10_n, m00_n, vx_n - vx, p.dz, vz_n - vzl_n, p.dx);
-        if (plane && tyz_xy && k <= nz - 2) lyz = s3_tsh(m01, m00, m01_n, m00_n, vy_n - vy, p.dz, vz_n - vzd_n, p.dy);
+            txy = s3_tsh(m11, m01, m10, m00, vx - vx_d, hy, vy - vy_l, hx);
+        if (plane && txz_xy && k <= nz - 2) lxz = s3_tsh(m10, m00, m10_n, m00_n, vx_n - vx, hz, vz_n - vzl_n, hx);
+        if (plane && tyz_xy && k <= nz - 2) lyz = s3_tsh(m01, m00, m01_n, m00_n, vy_n - vy, hz, vz_n - vzd_n, hy);
         __syncthreads();  // A: the previous plane's neighbour reads are done
         sPt[ty][tx] = pt_new;
         sTxx[ty][tx] = txx;
@@ -710,7 +719,7 @@ __global__ void __launch_bounds__(32 * S3F_TY, sizeof(T) == 4 ? 2 : 1) s3_fused_
             if (plane && X >= 1 && X <= nx - 1 && yin && k >= 1 && k <= nz - 2) {
                 const T A = txx - sTxx[ty][tx - 1], B = sTxy[ty + 1][tx] - txy, Cc = lxz - lxz_m;
                 const T P = pt_new - sPt[ty][tx - 1];
-                T R = ((div_c(A, p.dx) + div_c(B, p.dy)) + div_c(Cc, p.dz)) - div_c(P, p.dx);
+                T R = ((dvd(A, hx) + dvd(B, hy)) + dvd(Cc, hz)) - dvd(P, hx);
                 if constexpr (MODE == S3_DEFECT) R = R + a.fx[r];
                 const T dv = p.dampX * a.dVx[r] + R;
                 a.dVx[r] = dv;
@@ -721,7 +730,7 @@ __global__ void __launch_bounds__(32 * S3F_TY, sizeof(T) == 4 ? 2 : 1) s3_fused_
                 const int64_t ry = I3(X - 1, Y - 1, k - 1, nx - 2, ny - 1);
                 const T A = tyy - sTyy[ty - 1][tx], B = sTxy[ty][tx + 1] - txy, Cc = lyz - lyz_m;
                 const T P = pt_new - sPt[ty - 1][tx];
-                T R = ((div_c(A, p.dy) + div_c(B, p.dx)) + div_c(Cc, p.dz)) - div_c(P, p.dy);
+                T R = ((dvd(A, hy) + dvd(B, hx)) + dvd(Cc, hz)) - dvd(P, hy);
                 if constexpr (MODE == S3_DEFECT) R = R + a.fy[ry];
                 const T dv = p.dampY * a.dVy[ry] + R;
                 a.dVy[ry] = dv;
@@ -735,10 +744,10 @@ __global__ void __launch_bounds__(32 * S3F_TY, sizeof(T) == 4 ? 2 : 1) s3_fused_
                 const T P = pt_new - pt_m;
                 T R;
                 if constexpr (MODE == S3_DEFECT) {
-                    R = (((div_c(A, p.dz) + div_c(B, p.dx)) + div_c(Cc, p.dy)) - div_c(P, p.dz)) + a.fz[rz];
+                    R = (((dvd(A, hz) + dvd(B, hx)) + dvd(Cc, hy)) - dvd(P, hz)) + a.fz[rz];
                 } else {
                     const T G = (rog_m + rog) * T(0.5);
-                    R = (((div_c(A, p.dz) + div_c(B, p.dx)) + div_c(Cc, p.dy)) - div_c(P, p.dz)) + G;
+                    R = (((dvd(A, hz) + dvd(B, hx)) + dvd(Cc, hy)) - dvd(P, hz)) + G;
                 }
                 const T dv = p.dampZ * a.dVz[rz] + R;
                 a.dVz[rz] = dv;
@@ -781,14 +790,16 @@ __global__ void __launch_bounds__(32 * S3F_TY, sizeof(T) == 4 ? 2 : 1) s3_fused_
 
 template <typename T, int MODE>
 static void s3_fused_launch(const S3A<T>& a, const S3Out<T>& o, const S3P<T>& p, cudaStream_t s) {
-    static int occ = 0;
-    if (!occ) occ = resident_ctas(s3_fused_k<T, MODE>, 32 * S3F_TY, 0);
+    static int occ[2] = {};
+    const bool pair = p.lo != kNoPair;
+    const auto kernel = pair ? s3_fused_k<T, MODE, true> : s3_fused_k<T, MODE, false>;
+    if (!occ[pair]) occ[pair] = resident_ctas(kernel, 32 * S3F_TY, 0);
     DeviceState* st = nullptr;
     current_state(&st);
     const int64_t gx = (a.nx + 1 + 29) / 30, gy = (a.ny + 1 + S3F_TY - 3) / (S3F_TY - 2);
-    int Lz = auto_loopsize(gx * gy, a.nz + 1, (int64_t)occ * (st ? st->num_sms : 152));
+    int Lz = auto_loopsize(gx * gy, a.nz + 1, (int64_t)occ[pair] * (st ? st->num_sms : 152));
     const dim3 grd((unsigned)gx, (unsigned)gy, (unsigned)((a.nz + 1 + Lz - 1) / Lz));
-    s3_fused_k<T, MODE><<<grd, dim3(32, S3F_TY, 1), 0, s>>>(a, o, p, Lz);
+    kernel<<<grd, dim3(32, S3F_TY, 1), 0, s>>>(a, o, p, Lz);
 }
 
 // y32 = (float) x64 (rounding of the outer residual for the FP32 sweeps)
@@ -923,8 +934,13 @@ static void s3_iteration_kernels(const S3A<T>& a, const S3P<T>& p, bool after, c
         else cells<<<gc, b, 0, s>>>(a, p);
         launch_dependent(faces, gf, b, 0, s, a, p);
     };
-    if (i32) launch(s3_cells<T, MODE, int, STORE>, s3_faces<T, MODE, int, STORE>);
-    else launch(s3_cells<T, MODE, int64_t, STORE>, s3_faces<T, MODE, int64_t, STORE>);
+    auto pairs = [&](auto index) {
+        using I = decltype(index);
+        if (p.lo != kNoPair) launch(s3_cells<T, MODE, I, STORE, true>, s3_faces<T, MODE, I, STORE, true>);
+        else launch(s3_cells<T, MODE, I, STORE, false>, s3_faces<T, MODE, I, STORE, false>);
+    };
+    if (i32) pairs(int{});
+    else pairs(int64_t{});
 }
 
 template <typename T>

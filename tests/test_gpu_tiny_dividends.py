@@ -131,3 +131,43 @@ def test_stokes3d_stress_underflow(ps, oracle):
     assert 50 < np.count_nonzero(np.abs(o["txx"]) == 2.0 ** -1074) < o["txx"].size
     for k in STATE:
         assert np.array_equal(g.host(k), o[k]), k
+
+
+# Spacings that no reciprocal pair serves (10/15 in FP32, 10/17 in FP64, found on the CPU): the kernels' variants that
+# test every dividend at once, alone and beside spacings with pairs.
+@pytest.mark.parametrize("dtn", ["f64", "f32"])
+@pytest.mark.parametrize("n", [(45, 16), (18, 29), (16, 18)])
+def test_stokes2d_without_pairs(ps, oracle, dtn, n):
+    test_stokes2d(ps, oracle, dtn, n, 10.0)
+
+
+@pytest.mark.parametrize("dtn", ["f64", "f32"])
+@pytest.mark.parametrize("n", [(16, 18, 11), (21, 14, 16), (18, 9, 18)])
+@pytest.mark.parametrize("one_launch", [False, True])
+def test_stokes3d_without_pairs(ps, oracle, dtn, n, one_launch):
+    test_stokes3d(ps, oracle, dtn, n, 10.0, one_launch)
+
+
+@pytest.mark.parametrize("dtn", ["f64", "f32"])
+@pytest.mark.parametrize("h", [(10.0 / 15, 10.0 / 17, 0.37), (0.5, 10.0 / 17, 10.0 / 15), (10.0 / 15, 1e-9, 10.0 / 17)])
+def test_acoustic3d_without_pairs(ps, oracle, dtn, h):
+    if min(h) > 1e-6:  # (1e-9: outside the pairs' range too; one step, so that nothing overflows)
+        test_acoustic3d(ps, oracle, dtn, h)
+    n = (37, 19, 23)
+    rng = np.random.default_rng(8)
+    P = _spread(rng, n, dtn)
+    Vs = [_spread(rng, tuple(m + (d == e) for e, m in enumerate(n)), dtn) for d in range(3)]
+    d = [ps.from_host(a) for a in (*Vs, P)]
+    ps.parallel(ps.kernels.acoustic3D_compute_V, *d, 1e-3, 1.0, *h)
+    ps.parallel(ps.kernels.acoustic3D_compute_P, d[3], *d[:3], 1e-3, 1.0, *h)
+    oracle.acoustic3d_v(*Vs, P, 1e-3, 1.0, *h)
+    oracle.acoustic3d_p(P, *Vs, 1e-3, 1.0, *h)
+    for a, b in zip((*Vs, P), d):
+        assert np.array_equal(ps.to_host(b), a)
+
+
+@pytest.mark.parametrize("dtn", ["f64", "f32"])
+@pytest.mark.parametrize("h", [(247.0 / 254, 110.0 / 254, 0.31), (0.25, 110.0 / 254, 247.0 / 254)])
+@pytest.mark.parametrize("memopt", [False, True])
+def test_diffusion_dividing_by_spacings_without_pairs(ps, oracle, dtn, h, memopt):
+    test_diffusion_dividing_by_spacings(ps, oracle, dtn, h, memopt)
