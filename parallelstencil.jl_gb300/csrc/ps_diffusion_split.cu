@@ -889,11 +889,13 @@ __global__ void ci_grid_kernel(const double2* __restrict__ in, float4* __restric
     if (big) atomicOr(&r->bad, 1);
 }
 
-// Rows of a grid step's tile, besides 8: tiles of 6 rows, four CTAs per SM instead of three, for the steps
-// between a run's first and last. Both hold 24 rows on an SM; the smaller tile's four groups of warps wait
-// less on each other, which is worth 2 % of a step on most sizes (20 steps of 512^3: 14.42 -> 14.15 ms; 256^3
-// 101.4 -> 99.4 us per step; 384 x 384 x 128 the other way, 111 -> 114) and less than a launch can lose by
-// its last wave, so the one whose fullest SM has less to do is taken.
+// Rows of a grid step's tile: 8, or 6 for the steps between a run's first and last. With a conductivity array three
+// and four CTAs fit an SM, 24 rows both, and the smaller tile's four groups of warps wait less on each other (512^3
+// 660 -> 647 us per step, 256^3 98.2 -> 96.0); without one four and five do, 32 rows and 30. Which is faster is a
+// matter of the last wave too (without an array 512 x 256 x 128: 70 us with 8 rows, 76 with 6; 300^3 120 and 115), so the
+// tile whose fullest SM has no more to do is taken, 6 rows where they are equal. There, over 34 grids of 10^6 to
+// 10^8 cells, 6 rows are 1.3 % faster on average, and from 9 % faster (288 x 340 x 150) to 3.6 % slower (512 x 280 x 70;
+// 384 x 384 x 128 108 -> 111 us): nothing that the model counts tells those apart.
 constexpr int kGridRows = 8, kGridRowsMiddle = 6;
 
 // z-sweep length and relative time of a launch of tiles of `rows` rows: the fullest SM's tiles, their rows and their
@@ -912,15 +914,26 @@ static GridPick grid_pick(const Box& cb, int rows, int occ, int sms) {
     return {L, (double)per_sm * rows * ((double)wz / chunks + 2)};
 }
 
+constexpr int kGridStages = 4;
+template <bool LAM, bool ISO, bool OUT64, bool IN64, int TY>
+constexpr auto grid_kernel() {
+    return diff3d_grid_tma<LAM, ISO, TY, kGridStages, TY == kGridRows ? 3 : 4, OUT64, IN64>;
+}
+template <bool LAM, bool ISO, bool OUT64, bool IN64, int TY>
+static int grid_occupancy() {
+    constexpr int smem = SplitCfg<LAM, TY, kGridStages>::SMEM;
+    cudaFuncSetAttribute(grid_kernel<LAM, ISO, OUT64, IN64, TY>(), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return resident_ctas(grid_kernel<LAM, ISO, OUT64, IN64, TY>(), 32 * TY, smem);
+}
+
 // One step of a grid run. IN64 (first step): Tin, Cs and Ls are the caller's FP64 T, Ci and lam,
 // and the step writes the lam / Ci pairs of its cells to Lout / Cout.
 template <bool LAM, bool ISO, bool OUT64, bool IN64, int TY>
 static int launch_grid_tile(const ps_array& Tin, const ps_array& Cs, const ps_array* Ls, const ps_array& T2,
                             const SplitParams& p, const Box& cb, int L, cudaStream_t s, int* d_err, GridRun* run,
                             void* Lout, void* Cout) {
-    constexpr int S = 4, MINB = TY == kGridRows ? 3 : 4;
-    using C = SplitCfg<LAM, TY, S>;
-    auto kernel = diff3d_grid_tma<LAM, ISO, TY, S, MINB, OUT64, IN64>;
+    using C = SplitCfg<LAM, TY, kGridStages>;
+    const auto kernel = grid_kernel<LAM, ISO, OUT64, IN64, TY>();
     DeviceState* st = nullptr;
     PS_TRY(current_state(&st));
     static bool attr = false;
@@ -933,8 +946,9 @@ static int launch_grid_tile(const ps_array& Tin, const ps_array& Cs, const ps_ar
         const GridPick pick = grid_pick(cb, TY, occ, st->num_sms);
         L = pick.L;
         if constexpr (!OUT64 && !IN64 && TY == kGridRows) {
-            const GridPick six = grid_pick(cb, kGridRowsMiddle, 4, st->num_sms);
-            if (six.cost < 1.02 * pick.cost && cb.hi[1] - cb.lo[1] <= 65535 * kGridRowsMiddle)
+            static const int occ6 = grid_occupancy<LAM, ISO, OUT64, IN64, kGridRowsMiddle>();
+            const GridPick six = grid_pick(cb, kGridRowsMiddle, occ6, st->num_sms);
+            if (six.cost <= pick.cost && cb.hi[1] - cb.lo[1] <= 65535 * kGridRowsMiddle)
                 return launch_grid_tile<LAM, ISO, OUT64, IN64, kGridRowsMiddle>(Tin, Cs, Ls, T2, p, cb, 0, s, d_err, run, Lout, Cout);
         }
     }
