@@ -575,6 +575,7 @@ __global__ void __launch_bounds__(128, kFirstCtas)
     }
     const uint64_t da = umma_desc_sw64(smem_u32(sA)), db = umma_desc_sw64(smem_u32(sB));
     uint32_t phase = 0;
+    bool ok = true;  // of a warp: every wait so far ended (a block stops where one of a warp's gave up)
     for (int64_t p0 = blockIdx.x * (int64_t)128; p0 < P; p0 += gridDim.x * (int64_t)128) {
         const int64_t p = p0 + t, q = p / W;
         const int xx = (int)(p - q * W), yy = (int)(q % H);
@@ -593,7 +594,7 @@ __global__ void __launch_bounds__(128, kFirstCtas)
                 c < 3 ? make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]) : make_uint4(0, 0, 0, 0);
         fence_proxy_async_smem();  // the MMAs read what these threads wrote
         tc_fence_before();         // and overwrite the accumulator they have read
-        __syncthreads();
+        if (!__syncthreads_and(ok)) break;
         if (t == 0) {
             tc_fence_after();
             constexpr uint32_t idesc = umma_idesc_bf16(128, 32);
@@ -602,10 +603,11 @@ __global__ void __launch_bounds__(128, kFirstCtas)
             tc_commit(&bar);
         }
         __syncwarp();
-        const bool done = mbar_wait_bounded(&bar, phase);
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar, phase));
         phase ^= 1;
-        if (!__all_sync(0xffffffffu, done)) {
+        if (!ok) {
             if ((t & 31) == 0) atomicOr(err, DEV_ERR_TMA_TIMEOUT);
+            continue;
         }
         tc_fence_after();
         float a[32];
@@ -625,6 +627,7 @@ __global__ void __launch_bounds__(128, kFirstCtas)
             for (int i = 0; i < 4; i++) reinterpret_cast<uint4*>(y + p * 32)[i] = w[i];
         }
     }
+    if (!ok) mbar_wait_bounded(&bar, phase ^ 1);  // the MMAs in flight, before their accumulator is freed
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tc_dealloc(tmem, 32);
