@@ -341,6 +341,12 @@ class _AdGen(_Gen):
         self.written.add(name)
         return (name, i3, rhs)
 
+    def runs(self, lhs, point=("tx", "ty", "tz")):
+        """The points at which a statement with this left-hand side (array, mask) runs."""
+        name, li = lhs
+        k = self.aidx[name]
+        return " && ".join(f"{point[d]} < n{k}_{d} - {2 * ((li >> d) & 1)}" for d in range(self.nd))
+
     def _stmt(self, s, ind):
         if isinstance(s, ast.If):
             c = self.flag(f"({self.expr(s.test, ctx='auto')})")
@@ -397,10 +403,8 @@ class _AdGen(_Gen):
             if name in self.temps:
                 return
             li = self.sels[sel]
-            k = self.aidx[name]
             t3 = ("tx", "ty", "tz")
-            cond = " && ".join(f"{t3[d]} < n{k}_{d} - {2 * ((li >> d) & 1)}" for d in range(self.nd))
-            self.emit(f"if ({cond}) {{")
+            self.emit(f"if ({self.runs((name, li))}) {{")
             saved = self.ind
             self.ind += "    "
             f = self.begin()
@@ -687,13 +691,16 @@ class _AdSweepGen(_AdGen):
         regs = self.regs.setdefault(self.lhs, {})
         return regs.setdefault((name, o), "L%d_%d" % (list(self.regs).index(self.lhs), len(regs)))
 
-    def condition(self, lhs, ahead=""):
-        """The statement's left-hand condition at this plane, or at the next (ahead = " + 1")."""
-        name, li = lhs
-        k, zd = self.aidx[name], self.nd - 1
-        t3 = ("tx", "ty", "tz")
-        return "in_ && " + " && ".join(f"{t3[d]}{ahead if d == zd else ''} < n{k}_{d} - {2 * ((li >> d) & 1)}"
-                                       for d in range(self.nd))
+    def runs(self, lhs, point=("tx", "ty", "tz")):
+        """Every thread of the grid stays for the shuffles and barriers: the columns outside the ranges (in_ false)
+        execute no statement."""
+        return "in_ && " + super().runs(lhs, point)
+
+    def at_plane(self, z):
+        """This thread's point in plane z of the sweep."""
+        t3 = ["tx", "ty", "tz"]
+        t3[self.nd - 1] = z
+        return t3
 
     def plane_loads(self):
         """(declarations and the first plane's loads, loads of the next plane, their hand-over)"""
@@ -718,8 +725,8 @@ class _AdSweepGen(_AdGen):
                 nxt.append("    E Ng_ = 0;")
                 later.append(f"Ng_ = e{k}[st{k}_ + {at}];")
                 hand.append("    g_ = Ng_;")
-            first.append(f"    if ({self.condition(lhs)}) {{ {' '.join(start)} }}")
-            nxt.append(f"    if ({self.condition(lhs, ' + 1')} && {'xyz'[zd]}n_ < z1_) {{ {' '.join(later)} }}")
+            first.append(f"    if ({self.runs(lhs, self.at_plane('z0_'))}) {{ {' '.join(start)} }}")
+            nxt.append(f"    if ({self.runs(lhs, self.at_plane('zn_'))} && zn_ < z1_) {{ {' '.join(later)} }}")
         return first, nxt, hand
 
     def store(self, name, idx, rhs):
@@ -920,9 +927,6 @@ class _AdSweepGen(_AdGen):
         for name, offs in self.contrib.items():
             for o in sorted(offs):
                 regs.append(f"    E {self.contribution(name, o)} = 0;")
-        # every thread of the grid stays for the shuffles and barriers: the columns outside the ranges
-        # execute no statement
-        body = [ln.replace("if (", "if (in_ && ", 1) if ln.startswith("    if (tx < ") else ln for ln in body]
         xs = f"    __shared__ E xs_[2][{nb}][{self.TY}][{self.TX}];\n    int par_ = 0;" if nb else ""
         sync = ["    __syncthreads();"] if nb else []
         flip = ["    par_ ^= 1;"] if nb else []
@@ -943,9 +947,9 @@ extern "C" __global__ void __launch_bounds__({self.TX * self.TY if nd == 3 else 
     const int tx = (int)g.lo[0] + ux;{ypos}
     const int z0_ = (int)(g.lo[{zd}] + blockIdx.{zblk} * g.loop);
     const int z1_ = (int)(min((long long)z0_ + g.loop, g.lo[{zd}] + g.cnt[{zd}]));
-{chr(10).join(decl + pre + [ln.replace(f"{tsweep} <", "z0_ <") for ln in first])}
+{chr(10).join(decl + pre + first)}
     for (int {tsweep} = z0_; {tsweep} < z1_; ++{tsweep}) {{
-    const int {'xyz'[zd]}n_ = {tsweep} + 1;
+    const int zn_ = {tsweep} + 1;
 {chr(10).join(nxt + regs + body + put + sync + get + flip + hand)}
     {" ".join(step)}
     }}

@@ -154,3 +154,18 @@ def test_generator_refusals(jit, ad, src, dup, msg):
 
     with pytest.raises(ArgumentError, match=msg):
         ad.generate(jit.parse(src), 1, "double", dup, "reverse")
+
+
+@pytest.mark.parametrize("name", ["diffusion_flux_lam", "two_statements_2d"])
+def test_sweep_runs_no_statement_outside_the_box_however_its_lines_are_laid_out(jit, ad, name):
+    """All threads of a sweep's blocks stay for the exchanges, so each condition of a statement has to hold the one
+    that the thread's column is in the box; the generator's indentation is not part of the language."""
+    src, nd, _, dup, _ = K.KERNELS[name]
+    for more in (0, 1, 2):
+        class Gen(ad._AdSweepGen):
+            def stmt(self, s, ind):
+                return super().stmt(s, ind + more)
+
+        code = Gen(jit.parse(src), nd, set(dup)).source("float")
+        tests = [ln for ln in code.splitlines() if "if (" in ln and "tx < n" in ln]
+        assert len(tests) >= 3 and all("in_ && tx < n" in ln for ln in tests), tests
