@@ -1474,7 +1474,7 @@ int grid_misfit_gradient(const ps_array& T0, const ps_array& Tobs, const ps_arra
     *recomputed = 0;
     const int64_t n = numel(T0), n2 = n / 2, nseg = (nt + ce - 1) / ce;
     const size_t bytes = (size_t)n * 8, stride = (bytes + 255) / 256 * 256;
-    const int64_t nbuf = 7 + nseg + ce;  // Cs, Ls, μA, μB, μ64, fA, fB, checkpoints, segment states
+    const int64_t nbuf = 7 + nseg + ce - 1;  // Cs, Ls, μA, μB, μ64, fA, fB, checkpoints, segment states after them
     if (stride * nbuf + 512 > g_grad_bytes) {
         if (g_grad_scratch) cudaFree(g_grad_scratch);
         g_grad_scratch = nullptr;
@@ -1497,7 +1497,7 @@ int grid_misfit_gradient(const ps_array& T0, const ps_array& Tobs, const ps_arra
     };
     ps_array Cs = arr(0), Ls = arr(1), mA = arr(2), mB = arr(3), mu64 = arr(4), fA = arr(5), fB = arr(6);
     auto ckpt = [&](int64_t i) { return arr(7 + i); };
-    auto seg = [&](int64_t j) { return arr(7 + nseg + j); };
+    auto seg = [&](int64_t j) { return arr(7 + nseg + j - 1); };  // j = 1 .. ce - 1
     SplitParams p{};
     double G;
     const bool iso = split_coeffs(PS_DIFF_FLUX_LAM, 0.0, dt, hx, hy, hz, &p, &G);

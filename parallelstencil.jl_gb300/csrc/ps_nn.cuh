@@ -23,14 +23,14 @@ struct GemmEpilogue {
 int nn_gemm(const void* A, int64_t M, const void* B, int64_t N, int64_t K, const GemmEpilogue& e, int split,
             cudaStream_t s, int* d_err);
 
-// y = act(conv3x3(x) + bias), "same" padding: x [B][H][W][cin] bf16 (cin % 32 == 0), W [cout][9 cin] bf16
+// y = relu(conv3x3(x) + bias), "same" padding: x [B][H][W][cin] bf16 (cin % 32 == 0), W [cout][9 cin] bf16
 // (columns tap by tap, channels within a tap; cout % 32 == 0), y [B][H][W][cout] bf16.
 int nn_conv3_first(const void* x, int64_t P, int H, int W, const void* wgt, int kpad, const float* bias, void* y,
                    cudaStream_t s, int* d_err);
 int nn_conv3_rows(const void* x, const void* low, int B, int H, int W, int cin, const void* wgt, int cout, const float* bias,
-                  int relu, void* y, const void* wlast, int kpad_last, const float* blast, float* ylast, bool* taken,
+                  void* y, const void* wlast, int kpad_last, const float* blast, float* ylast, bool* taken,
                   cudaStream_t s, int* d_err);
-int nn_conv3_tc(const void* x, int B, int H, int W, int cin, const void* wgt, int cout, const float* bias, int relu,
+int nn_conv3_tc(const void* x, int B, int H, int W, int cin, const void* wgt, int cout, const float* bias,
                 void* y, cudaStream_t s, int* d_err);
 
 }  // namespace ps

@@ -1,5 +1,5 @@
 // ps_nn_conv.cu -- 3x3 convolutions of the warm-start network as implicit GEMMs on the tensor cores
-// (tcgen05): y[p][n] = act(sum over taps and channels of x[p + tap][c] * W[n][tap][c] + bias[n]), bf16
+// (tcgen05): y[p][n] = relu(sum over taps and channels of x[p + tap][c] * W[n][tap][c] + bias[n]), bf16
 // operands, FP32 accumulation in tensor memory, bf16 result. No column matrix is formed: a tap's 128
 // input pixels by KC channels are one 4-D TMA box of the NHWC activations, shifted by the tap, and the
 // pixels outside the image arrive as the zero fill that "same" padding wants. In layers whose rows fill
@@ -60,7 +60,7 @@ struct ConvGeom {
 template <int BN, int KC, bool ROW, bool DEEP>
 __global__ void __launch_bounds__(192, 2)
     nn_conv3_k(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB, ConvGeom g,
-               const float* __restrict__ bias, int relu, __nv_bfloat16* __restrict__ y, int* __restrict__ err) {
+               const float* __restrict__ bias, __nv_bfloat16* __restrict__ y, int* __restrict__ err) {
     using C = ConvCfg<BN, KC, ROW, DEEP>;
     constexpr int S = C::S;
     extern __shared__ unsigned char smem_raw[];
@@ -188,9 +188,8 @@ __global__ void __launch_bounds__(192, 2)
 #pragma unroll
                 for (int i = 0; i < 16; i += 4) {
                     const float4 bv = __ldg(reinterpret_cast<const float4*>(bias + n0 + c + i));
-                    const float lo = relu ? 0.0f : -INFINITY;
-                    h[i / 2] = __floats2bfloat162_rn(fmaxf(v[i] + bv.x, lo), fmaxf(v[i + 1] + bv.y, lo));
-                    h[i / 2 + 1] = __floats2bfloat162_rn(fmaxf(v[i + 2] + bv.z, lo), fmaxf(v[i + 3] + bv.w, lo));
+                    h[i / 2] = __floats2bfloat162_rn(fmaxf(v[i] + bv.x, 0.0f), fmaxf(v[i + 1] + bv.y, 0.0f));
+                    h[i / 2 + 1] = __floats2bfloat162_rn(fmaxf(v[i + 2] + bv.z, 0.0f), fmaxf(v[i + 3] + bv.w, 0.0f));
                 }
                 if (ok) {
                     reinterpret_cast<uint4*>(o + c)[0] = w[0];
@@ -214,7 +213,7 @@ __global__ void __launch_bounds__(192, 2)
 }
 
 template <int BN, int KC, bool ROW, bool DEEP>
-static int conv3_launch(const ConvGeom& g, const void* x, const void* wgt, const float* bias, int relu, void* y, int sms,
+static int conv3_launch(const ConvGeom& g, const void* x, const void* wgt, const float* bias, void* y, int sms,
                         cudaStream_t s, int* d_err) {
     using C = ConvCfg<BN, KC, ROW, DEEP>;
     CUtensorMap mA, mB;
@@ -228,7 +227,7 @@ static int conv3_launch(const ConvGeom& g, const void* x, const void* wgt, const
     // every launch sets it: the attribute belongs to the device's current context
     PS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
     const int grid = std::min(g.ntiles, (DEEP ? 1 : 2) * sms);
-    PS_CUDA_TRY(launch_dependent(kernel, dim3((unsigned)grid), dim3(192), (size_t)C::SMEM, s, mA, mB, g, bias, relu,
+    PS_CUDA_TRY(launch_dependent(kernel, dim3((unsigned)grid), dim3(192), (size_t)C::SMEM, s, mA, mB, g, bias,
                                  static_cast<__nv_bfloat16*>(y), d_err));
     return PS_OK;
 }
@@ -255,7 +254,7 @@ struct RowsCfg {
     static constexpr int CB = RB + UB, THREADS = UB ? 320 : 192;
     static constexpr int ABOX = (kConvM + 2) * 64, ABYTES = (ABOX + 1023) / 1024 * 1024;
     static constexpr int WBYTES = 3 * CB * 3 * 32 * 64;  // [kx][cb][ky][32 outputs] rows of 64 bytes
-    static constexpr int S = UB ? 2 : RB == 1 ? 8 : 5;
+    static constexpr int S = UB ? 2 : 8;
     static constexpr int UBYTES = 2 * UB * ABYTES;
     static constexpr int SMEM = WBYTES + S * ABYTES + UBYTES + 1024 + 1024;
     static_assert(SMEM > 77 * 1024 && SMEM < 113 * 1024, "two CTAs per SM");
@@ -274,7 +273,7 @@ struct LastLayer {  // y[p][0..2] = W a[p] + b over the 32 channels; y NULL: non
 template <int RB, int UB>
 __global__ void __launch_bounds__(RowsCfg<RB, UB>::THREADS, 2)
     nn_conv3_rows_k(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB, RowsGeom g,
-                    const uint4* __restrict__ low, const float* __restrict__ bias, int relu, __nv_bfloat16* __restrict__ y,
+                    const uint4* __restrict__ low, const float* __restrict__ bias, __nv_bfloat16* __restrict__ y,
                     LastLayer last, int* __restrict__ err) {
     using C = RowsCfg<RB, UB>;
     constexpr int S = C::S, CB = C::CB, CIN = 32 * CB;
@@ -457,7 +456,6 @@ __global__ void __launch_bounds__(RowsCfg<RB, UB>::THREADS, 2)
         if (!ok && lane == 0) atomicOr(err, DEV_ERR_TMA_TIMEOUT);
     } else if (warp >= 2) {  // epilogue: warp w reads TMEM lanes (pixels of the row) 32 (w % 4) .. + 31
         const int q = warp & 3;
-        const float low = relu ? 0.0f : -INFINITY;
         int n = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < g.jobs && ok; t += gridDim.x) {
@@ -484,8 +482,8 @@ __global__ void __launch_bounds__(RowsCfg<RB, UB>::THREADS, 2)
 #pragma unroll
                 for (int i = 0; i < 32; i += 4) {
                     const float4 bv = __ldg(reinterpret_cast<const float4*>(bias + i));
-                    h[i / 2] = __floats2bfloat162_rn(fmaxf(v[i] + bv.x, low), fmaxf(v[i + 1] + bv.y, low));
-                    h[i / 2 + 1] = __floats2bfloat162_rn(fmaxf(v[i + 2] + bv.z, low), fmaxf(v[i + 3] + bv.w, low));
+                    h[i / 2] = __floats2bfloat162_rn(fmaxf(v[i] + bv.x, 0.0f), fmaxf(v[i + 1] + bv.y, 0.0f));
+                    h[i / 2 + 1] = __floats2bfloat162_rn(fmaxf(v[i + 2] + bv.z, 0.0f), fmaxf(v[i + 3] + bv.w, 0.0f));
                 }
                 if (px >= g.W) continue;
                 const int64_t p = ((int64_t)b * g.H + o) * g.W + px;
@@ -523,7 +521,7 @@ __global__ void __launch_bounds__(RowsCfg<RB, UB>::THREADS, 2)
 }
 
 template <int RB, int UB>
-static int conv3_rows_launch(const RowsGeom& g, const void* x, const void* low, const void* wgt, const float* bias, int relu,
+static int conv3_rows_launch(const RowsGeom& g, const void* x, const void* low, const void* wgt, const float* bias,
                              void* y, const LastLayer& last, int sms, cudaStream_t s, int* d_err) {
     using C = RowsCfg<RB, UB>;
     CUtensorMap mA, mB;
@@ -537,7 +535,7 @@ static int conv3_rows_launch(const RowsGeom& g, const void* x, const void* low, 
     // every launch sets it: the attribute belongs to the device's current context
     PS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
     PS_CUDA_TRY(launch_dependent(kernel, dim3((unsigned)std::min(g.jobs, 2 * sms)), dim3(C::THREADS), (size_t)C::SMEM, s, mA, mB,
-                                 g, static_cast<const uint4*>(low), bias, relu, static_cast<__nv_bfloat16*>(y), last, d_err));
+                                 g, static_cast<const uint4*>(low), bias, static_cast<__nv_bfloat16*>(y), last, d_err));
     return PS_OK;
 }
 
@@ -654,7 +652,7 @@ static bool whole_rows(int W) {
 // input is read 1.5 times; below that the tiles of nn_conv3_k read no more). low (or NULL): 64 channels of a
 // quarter-size layer that come upsampled before x's 32.
 int nn_conv3_rows(const void* x, const void* low, int B, int H, int W, int cin, const void* wgt, int cout, const float* bias,
-                  int relu, void* y, const void* wlast, int kpad_last, const float* blast, float* ylast, bool* taken,
+                  void* y, const void* wlast, int kpad_last, const float* blast, float* ylast, bool* taken,
                   cudaStream_t s, int* d_err) {
     *taken = false;
     DeviceState* st = nullptr;
@@ -673,11 +671,11 @@ int nn_conv3_rows(const void* x, const void* low, int B, int H, int W, int cin, 
     g.jobs = (int)(strips * g.chunks);
     const LastLayer last{static_cast<const __nv_bfloat16*>(wlast), kpad_last, blast, ylast};
     *taken = true;
-    return low ? conv3_rows_launch<1, 2>(g, x, low, wgt, bias, relu, y, last, st->num_sms, s, d_err)
-               : conv3_rows_launch<1, 0>(g, x, nullptr, wgt, bias, relu, y, last, st->num_sms, s, d_err);
+    return low ? conv3_rows_launch<1, 2>(g, x, low, wgt, bias, y, last, st->num_sms, s, d_err)
+               : conv3_rows_launch<1, 0>(g, x, nullptr, wgt, bias, y, last, st->num_sms, s, d_err);
 }
 
-int nn_conv3_tc(const void* x, int B, int H, int W, int cin, const void* wgt, int cout, const float* bias, int relu,
+int nn_conv3_tc(const void* x, int B, int H, int W, int cin, const void* wgt, int cout, const float* bias,
                 void* y, cudaStream_t s, int* d_err) {
     if (cin % 32 || cout % 32 || B < 1 || H < 1 || W < 1) return fail(PS_ERR_SHAPE, "nn_conv3: layer %d -> %d", cin, cout);
     DeviceState* st = nullptr;
@@ -717,8 +715,8 @@ int nn_conv3_tc(const void* x, int B, int H, int W, int cin, const void* wgt, in
         constexpr int KC = decltype(k)::value;
         constexpr bool R = decltype(r)::value, D = decltype(d)::value;
         if constexpr (!D)  // (64 channels are taken only where there are tiles for every SM)
-            if (bn == 64) return conv3_launch<64, KC, R, D>(g, x, wgt, bias, relu, y, st->num_sms, s, d_err);
-        return conv3_launch<32, KC, R, D>(g, x, wgt, bias, relu, y, st->num_sms, s, d_err);
+            if (bn == 64) return conv3_launch<64, KC, R, D>(g, x, wgt, bias, y, st->num_sms, s, d_err);
+        return conv3_launch<32, KC, R, D>(g, x, wgt, bias, y, st->num_sms, s, d_err);
     };
     auto kc = [&](auto r, auto d) {
         return cin % 64 == 0 ? run(std::integral_constant<int, 64>{}, r, d) : run(std::integral_constant<int, 32>{}, r, d);

@@ -523,11 +523,11 @@ static int nn_conv_fwd(NNet* n, Conv& L, const bf16* x, int B, int h, int w, voi
     const int64_t P = (int64_t)B * h * w;
     if (L.k == 3 && L.cin % 32 == 0) {
         bool taken = false;
-        PS_TRY(nn_conv3_rows(x, nullptr, B, h, w, L.cin, L.W, L.cout, L.b, L.relu, y, next ? next->W : nullptr,
+        PS_TRY(nn_conv3_rows(x, nullptr, B, h, w, L.cin, L.W, L.cout, L.b, y, next ? next->W : nullptr,
                              next ? (int)next->kpad : 0, next ? next->b : nullptr, ynext, &taken, s, err));
         if (fused) *fused = taken;
         if (taken) return PS_OK;
-        return nn_conv3_tc(x, B, h, w, L.cin, L.W, L.cout, L.b, L.relu, y, s, err);
+        return nn_conv3_tc(x, B, h, w, L.cin, L.W, L.cout, L.b, y, s, err);
     }
     if (L.k == 3)
         PS_TRY(nn_conv3_first(x, P, h, w, L.W, (int)L.kpad, L.b, y, s, err));
@@ -638,7 +638,7 @@ static int nn_forward(NNet* n, int B, cudaStream_t s, int* err) {
     // the largest concatenation: read where its parts lie, and written out by the backward pass, which needs it whole
     bool apart = false;
     if (f == 4 && c == 32)
-        PS_TRY(nn_conv3_rows(n->a[1], n->a[11], B, n->H, n->W, L[12].cin, L[12].W, L[12].cout, L[12].b, L[12].relu, n->a[12],
+        PS_TRY(nn_conv3_rows(n->a[1], n->a[11], B, n->H, n->W, L[12].cin, L[12].W, L[12].cout, L[12].b, n->a[12],
                              nullptr, 0, nullptr, nullptr, &apart, s, err));
     n->k0_images = apart ? 0 : std::max(n->k0_images, B);
     if (!apart) {

@@ -531,11 +531,7 @@ static dim3 g2(int64_t wx, int64_t wy, dim3 b) {
     return dim3((unsigned)((wx + b.x - 1) / b.x), (unsigned)((wy + b.y - 1) / b.y), 1);
 }
 
-// Library-owned scratch for the ping-pong buffers and the solvers (freed by ps_finalize).
-struct Scratch {
-    void* ptr = nullptr;
-    size_t bytes = 0;
-};
+// Library-owned scratch of the solvers (freed by ps_finalize).
 static std::mutex g_scr_mutex;
 static std::vector<void*> g_scratch_all;
 

@@ -60,8 +60,6 @@ struct S3A {
 enum { S3_PLAIN = 0, S3_DEFECT = 1, S3_RESIDUAL = 2 };
 
 #define I3(a, b, c, n0, n1) ((int64_t)(a) + (int64_t)(n0) * ((int64_t)(b) + (int64_t)(n1) * (int64_t)(c)))
-// the same in the index type I of the iteration kernels (32-bit where every array has < 2^31 elements)
-#define I3T(a, b, c, n0, n1) ((I)(a) + (I)(n0) * ((I)(b) + (I)(n1) * (I)(c)))
 
 // ---- statement arithmetic ------------------------------------------------------------------
 template <typename T>
@@ -74,12 +72,12 @@ __device__ __forceinline__ T s3_dtPt(T Ptsc, T m, T mn) {
     return ((Ptsc * T(6.1)) * m) / mn;
 }
 // @d_xa(Vx)/dx + @d_ya(Vy)/dy + @d_za(Vz)/dz at cell (x, y, z)
-template <typename T, typename I = int64_t>
-__device__ __forceinline__ T s3_divV(const S3A<T>& a, const S3P<T>& p, I x, I y, I z) {
-    const I nx = (I)a.nx, ny = (I)a.ny;
-    return (div_c(a.Vx[I3T(x + 1, y, z, nx + 1, ny)] - a.Vx[I3T(x, y, z, nx + 1, ny)], p.dx) +
-            div_c(a.Vy[I3T(x, y + 1, z, nx, ny + 1)] - a.Vy[I3T(x, y, z, nx, ny + 1)], p.dy)) +
-           div_c(a.Vz[I3T(x, y, z + 1, nx, ny)] - a.Vz[I3T(x, y, z, nx, ny)], p.dz);
+template <typename T>
+__device__ __forceinline__ T s3_divV(const S3A<T>& a, const S3P<T>& p, int64_t x, int64_t y, int64_t z) {
+    const int64_t nx = a.nx, ny = a.ny;
+    return (div_c(a.Vx[I3(x + 1, y, z, nx + 1, ny)] - a.Vx[I3(x, y, z, nx + 1, ny)], p.dx) +
+            div_c(a.Vy[I3(x, y + 1, z, nx, ny + 1)] - a.Vy[I3(x, y, z, nx, ny + 1)], p.dy)) +
+           div_c(a.Vz[I3(x, y, z + 1, nx, ny)] - a.Vz[I3(x, y, z, nx, ny)], p.dz);
 }
 // 2.0*μ*(dV/h - 1.0/3.0*∇V)
 // H: DivC<T>, or DivF<T> (quotients without the dividend tests). In FP64 with DivF the factors 2, 0.25
@@ -114,102 +112,35 @@ __device__ __forceinline__ T s3_half_sum(T a, T b, H) {
 }
 __device__ __forceinline__ double s3_half_sum(double a, double b, DivF<double> h) { return scale_pow2(a + b, -1, h.key); }
 
-template <typename T, typename I = int64_t>
-__device__ __forceinline__ void s3_txy(const S3A<T>& a, const S3P<T>& p, I x, I y, I z) {
-    const I nx = (I)a.nx, ny = (I)a.ny;
+template <typename T>
+__device__ __forceinline__ void s3_txy(const S3A<T>& a, const S3P<T>& p, int64_t x, int64_t y, int64_t z) {
+    const int64_t nx = a.nx, ny = a.ny;
     const T* M = a.Mus;
-    a.txy[I3T(x, y, z, nx - 1, ny - 1)] =
-        s3_tsh(M[I3T(x, y, z + 1, nx, ny)], M[I3T(x + 1, y, z + 1, nx, ny)], M[I3T(x, y + 1, z + 1, nx, ny)],
-               M[I3T(x + 1, y + 1, z + 1, nx, ny)],
-               a.Vx[I3T(x + 1, y + 1, z + 1, nx + 1, ny)] - a.Vx[I3T(x + 1, y, z + 1, nx + 1, ny)], p.dy,
-               a.Vy[I3T(x + 1, y + 1, z + 1, nx, ny + 1)] - a.Vy[I3T(x, y + 1, z + 1, nx, ny + 1)], p.dx);
+    a.txy[I3(x, y, z, nx - 1, ny - 1)] =
+        s3_tsh(M[I3(x, y, z + 1, nx, ny)], M[I3(x + 1, y, z + 1, nx, ny)], M[I3(x, y + 1, z + 1, nx, ny)],
+               M[I3(x + 1, y + 1, z + 1, nx, ny)],
+               a.Vx[I3(x + 1, y + 1, z + 1, nx + 1, ny)] - a.Vx[I3(x + 1, y, z + 1, nx + 1, ny)], p.dy,
+               a.Vy[I3(x + 1, y + 1, z + 1, nx, ny + 1)] - a.Vy[I3(x, y + 1, z + 1, nx, ny + 1)], p.dx);
 }
-template <typename T, typename I = int64_t>
-__device__ __forceinline__ void s3_txz(const S3A<T>& a, const S3P<T>& p, I x, I y, I z) {
-    const I nx = (I)a.nx, ny = (I)a.ny;
+template <typename T>
+__device__ __forceinline__ void s3_txz(const S3A<T>& a, const S3P<T>& p, int64_t x, int64_t y, int64_t z) {
+    const int64_t nx = a.nx, ny = a.ny;
     const T* M = a.Mus;
-    a.txz[I3T(x, y, z, nx - 1, ny - 2)] =
-        s3_tsh(M[I3T(x, y + 1, z, nx, ny)], M[I3T(x + 1, y + 1, z, nx, ny)], M[I3T(x, y + 1, z + 1, nx, ny)],
-               M[I3T(x + 1, y + 1, z + 1, nx, ny)],
-               a.Vx[I3T(x + 1, y + 1, z + 1, nx + 1, ny)] - a.Vx[I3T(x + 1, y + 1, z, nx + 1, ny)], p.dz,
-               a.Vz[I3T(x + 1, y + 1, z + 1, nx, ny)] - a.Vz[I3T(x, y + 1, z + 1, nx, ny)], p.dx);
+    a.txz[I3(x, y, z, nx - 1, ny - 2)] =
+        s3_tsh(M[I3(x, y + 1, z, nx, ny)], M[I3(x + 1, y + 1, z, nx, ny)], M[I3(x, y + 1, z + 1, nx, ny)],
+               M[I3(x + 1, y + 1, z + 1, nx, ny)],
+               a.Vx[I3(x + 1, y + 1, z + 1, nx + 1, ny)] - a.Vx[I3(x + 1, y + 1, z, nx + 1, ny)], p.dz,
+               a.Vz[I3(x + 1, y + 1, z + 1, nx, ny)] - a.Vz[I3(x, y + 1, z + 1, nx, ny)], p.dx);
 }
-template <typename T, typename I = int64_t>
-__device__ __forceinline__ void s3_tyz(const S3A<T>& a, const S3P<T>& p, I x, I y, I z) {
-    const I nx = (I)a.nx, ny = (I)a.ny;
+template <typename T>
+__device__ __forceinline__ void s3_tyz(const S3A<T>& a, const S3P<T>& p, int64_t x, int64_t y, int64_t z) {
+    const int64_t nx = a.nx, ny = a.ny;
     const T* M = a.Mus;
-    a.tyz[I3T(x, y, z, nx - 2, ny - 1)] =
-        s3_tsh(M[I3T(x + 1, y, z, nx, ny)], M[I3T(x + 1, y + 1, z, nx, ny)], M[I3T(x + 1, y, z + 1, nx, ny)],
-               M[I3T(x + 1, y + 1, z + 1, nx, ny)],
-               a.Vy[I3T(x + 1, y + 1, z + 1, nx, ny + 1)] - a.Vy[I3T(x + 1, y + 1, z, nx, ny + 1)], p.dz,
-               a.Vz[I3T(x + 1, y + 1, z + 1, nx, ny)] - a.Vz[I3T(x + 1, y, z + 1, nx, ny)], p.dy);
-}
-
-// compute_dV! statements at residual index (x, y, z) and, with update_V, compute_V! at the same
-// index (it reads only the pseudo-velocity just written)
-template <typename T, int MODE = S3_PLAIN, typename I = int64_t>
-__device__ __forceinline__ void s3_dV(const S3A<T>& a, const S3P<T>& p, I x, I y, I z, bool update_V) {
-    const I nx = (I)a.nx, ny = (I)a.ny, nz = (I)a.nz;
-    const T* Pt = a.Pt;
-    if (x < nx - 1 && y < ny - 2 && z < nz - 2) {
-        const I r = I3T(x, y, z, nx - 1, ny - 2);
-        const T A = a.txx[I3T(x + 1, y, z, nx, ny - 2)] - a.txx[I3T(x, y, z, nx, ny - 2)];
-        const T B = a.txy[I3T(x, y + 1, z, nx - 1, ny - 1)] - a.txy[I3T(x, y, z, nx - 1, ny - 1)];
-        const T C = a.txz[I3T(x, y, z + 1, nx - 1, ny - 2)] - a.txz[I3T(x, y, z, nx - 1, ny - 2)];
-        const T P = Pt[I3T(x + 1, y + 1, z + 1, nx, ny)] - Pt[I3T(x, y + 1, z + 1, nx, ny)];
-        T R = ((div_c(A, p.dx) + div_c(B, p.dy)) + div_c(C, p.dz)) - div_c(P, p.dx);
-        if constexpr (MODE == S3_DEFECT) R = R + a.fx[r];
-        a.Rx[r] = R;
-        if constexpr (MODE != S3_RESIDUAL) {
-            const T dv = p.dampX * a.dVx[r] + R;
-            a.dVx[r] = dv;
-            if (update_V) {
-                const I v = I3T(x + 1, y + 1, z + 1, nx + 1, ny);
-                a.Vx[v] = a.Vx[v] + a.dtVx[r] * dv;
-            }
-        }
-    }
-    if (x < nx - 2 && y < ny - 1 && z < nz - 2) {
-        const I r = I3T(x, y, z, nx - 2, ny - 1);
-        const T A = a.tyy[I3T(x, y + 1, z, nx - 2, ny)] - a.tyy[I3T(x, y, z, nx - 2, ny)];
-        const T B = a.txy[I3T(x + 1, y, z, nx - 1, ny - 1)] - a.txy[I3T(x, y, z, nx - 1, ny - 1)];
-        const T C = a.tyz[I3T(x, y, z + 1, nx - 2, ny - 1)] - a.tyz[I3T(x, y, z, nx - 2, ny - 1)];
-        const T P = Pt[I3T(x + 1, y + 1, z + 1, nx, ny)] - Pt[I3T(x + 1, y, z + 1, nx, ny)];
-        T R = ((div_c(A, p.dy) + div_c(B, p.dx)) + div_c(C, p.dz)) - div_c(P, p.dy);
-        if constexpr (MODE == S3_DEFECT) R = R + a.fy[r];
-        a.Ry[r] = R;
-        if constexpr (MODE != S3_RESIDUAL) {
-            const T dv = p.dampY * a.dVy[r] + R;
-            a.dVy[r] = dv;
-            if (update_V) {
-                const I v = I3T(x + 1, y + 1, z + 1, nx, ny + 1);
-                a.Vy[v] = a.Vy[v] + a.dtVy[r] * dv;
-            }
-        }
-    }
-    if (x < nx - 2 && y < ny - 2 && z < nz - 1) {
-        const I r = I3T(x, y, z, nx - 2, ny - 2);
-        const T A = a.tzz[I3T(x, y, z + 1, nx - 2, ny - 2)] - a.tzz[I3T(x, y, z, nx - 2, ny - 2)];
-        const T B = a.txz[I3T(x + 1, y, z, nx - 1, ny - 2)] - a.txz[I3T(x, y, z, nx - 1, ny - 2)];
-        const T C = a.tyz[I3T(x, y + 1, z, nx - 2, ny - 1)] - a.tyz[I3T(x, y, z, nx - 2, ny - 1)];
-        const T P = Pt[I3T(x + 1, y + 1, z + 1, nx, ny)] - Pt[I3T(x + 1, y + 1, z, nx, ny)];
-        T R;
-        if constexpr (MODE == S3_DEFECT) {  // the buoyancy is part of the outer residual fz
-            R = (((div_c(A, p.dz) + div_c(B, p.dx)) + div_c(C, p.dy)) - div_c(P, p.dz)) + a.fz[r];
-        } else {
-            const T G = (a.Rog[I3T(x + 1, y + 1, z, nx, ny)] + a.Rog[I3T(x + 1, y + 1, z + 1, nx, ny)]) * T(0.5);
-            R = (((div_c(A, p.dz) + div_c(B, p.dx)) + div_c(C, p.dy)) - div_c(P, p.dz)) + G;
-        }
-        a.Rz[r] = R;
-        if constexpr (MODE != S3_RESIDUAL) {
-            const T dv = p.dampZ * a.dVz[r] + R;
-            a.dVz[r] = dv;
-            if (update_V) {
-                const I v = I3T(x + 1, y + 1, z + 1, nx, ny);
-                a.Vz[v] = a.Vz[v] + a.dtVz[r] * dv;
-            }
-        }
-    }
+    a.tyz[I3(x, y, z, nx - 2, ny - 1)] =
+        s3_tsh(M[I3(x + 1, y, z, nx, ny)], M[I3(x + 1, y + 1, z, nx, ny)], M[I3(x + 1, y, z + 1, nx, ny)],
+               M[I3(x + 1, y + 1, z + 1, nx, ny)],
+               a.Vy[I3(x + 1, y + 1, z + 1, nx, ny + 1)] - a.Vy[I3(x + 1, y + 1, z, nx, ny + 1)], p.dz,
+               a.Vz[I3(x + 1, y + 1, z + 1, nx, ny)] - a.Vz[I3(x + 1, y, z + 1, nx, ny)], p.dy);
 }
 
 #define S3_IDX                                                                               \
@@ -217,12 +148,6 @@ __device__ __forceinline__ void s3_dV(const S3A<T>& a, const S3P<T>& p, I x, I y
     const int64_t y = blockIdx.y * (int64_t)blockDim.y + threadIdx.y;                        \
     const int64_t z = blockIdx.z;                                                            \
     const int64_t nx = a.nx, ny = a.ny, nz = a.nz;                                           \
-    if (x >= nx || y >= ny || z >= nz) return
-#define S3_IDXT                                                                              \
-    const I x = (I)(blockIdx.x * blockDim.x + threadIdx.x);                                  \
-    const I y = (I)(blockIdx.y * blockDim.y + threadIdx.y);                                  \
-    const I z = (I)blockIdx.z;                                                               \
-    const I nx = (I)a.nx, ny = (I)a.ny, nz = (I)a.nz;                                        \
     if (x >= nx || y >= ny || z >= nz) return
 
 // ---- one-to-one kernels (grid: max extents of the kernel's array arguments) ---------------
@@ -278,7 +203,38 @@ __global__ void s3_tau_k(S3A<T> a, S3P<T> p) {
 template <typename T>
 __global__ void s3_dV_k(S3A<T> a, S3P<T> p) {
     S3_IDX;
-    s3_dV(a, p, x, y, z, false);
+    const T* Pt = a.Pt;
+    if (x < nx - 1 && y < ny - 2 && z < nz - 2) {
+        const int64_t r = I3(x, y, z, nx - 1, ny - 2);
+        const T A = a.txx[I3(x + 1, y, z, nx, ny - 2)] - a.txx[I3(x, y, z, nx, ny - 2)];
+        const T B = a.txy[I3(x, y + 1, z, nx - 1, ny - 1)] - a.txy[I3(x, y, z, nx - 1, ny - 1)];
+        const T C = a.txz[I3(x, y, z + 1, nx - 1, ny - 2)] - a.txz[I3(x, y, z, nx - 1, ny - 2)];
+        const T P = Pt[I3(x + 1, y + 1, z + 1, nx, ny)] - Pt[I3(x, y + 1, z + 1, nx, ny)];
+        const T R = ((div_c(A, p.dx) + div_c(B, p.dy)) + div_c(C, p.dz)) - div_c(P, p.dx);
+        a.Rx[r] = R;
+        a.dVx[r] = p.dampX * a.dVx[r] + R;
+    }
+    if (x < nx - 2 && y < ny - 1 && z < nz - 2) {
+        const int64_t r = I3(x, y, z, nx - 2, ny - 1);
+        const T A = a.tyy[I3(x, y + 1, z, nx - 2, ny)] - a.tyy[I3(x, y, z, nx - 2, ny)];
+        const T B = a.txy[I3(x + 1, y, z, nx - 1, ny - 1)] - a.txy[I3(x, y, z, nx - 1, ny - 1)];
+        const T C = a.tyz[I3(x, y, z + 1, nx - 2, ny - 1)] - a.tyz[I3(x, y, z, nx - 2, ny - 1)];
+        const T P = Pt[I3(x + 1, y + 1, z + 1, nx, ny)] - Pt[I3(x + 1, y, z + 1, nx, ny)];
+        const T R = ((div_c(A, p.dy) + div_c(B, p.dx)) + div_c(C, p.dz)) - div_c(P, p.dy);
+        a.Ry[r] = R;
+        a.dVy[r] = p.dampY * a.dVy[r] + R;
+    }
+    if (x < nx - 2 && y < ny - 2 && z < nz - 1) {
+        const int64_t r = I3(x, y, z, nx - 2, ny - 2);
+        const T A = a.tzz[I3(x, y, z + 1, nx - 2, ny - 2)] - a.tzz[I3(x, y, z, nx - 2, ny - 2)];
+        const T B = a.txz[I3(x + 1, y, z, nx - 1, ny - 2)] - a.txz[I3(x, y, z, nx - 1, ny - 2)];
+        const T C = a.tyz[I3(x, y + 1, z, nx - 2, ny - 1)] - a.tyz[I3(x, y, z, nx - 2, ny - 1)];
+        const T P = Pt[I3(x + 1, y + 1, z + 1, nx, ny)] - Pt[I3(x + 1, y + 1, z, nx, ny)];
+        const T G = (a.Rog[I3(x + 1, y + 1, z, nx, ny)] + a.Rog[I3(x + 1, y + 1, z + 1, nx, ny)]) * T(0.5);
+        const T R = (((div_c(A, p.dz) + div_c(B, p.dx)) + div_c(C, p.dy)) - div_c(P, p.dz)) + G;
+        a.Rz[r] = R;
+        a.dVz[r] = p.dampZ * a.dVz[r] + R;
+    }
 }
 
 template <typename T>
