@@ -484,8 +484,9 @@ __device__ __forceinline__ R jl_bmul(bool b, R x) { return b ? x : copysign((R)0
 
 class _Gen:
     def __init__(self, kd: KernelDef, ndims: int, zloop: bool = False, split: bool = False, ordered: bool = False,
-                 tma: bool = False):
+                 tma: bool = False, form: str = ""):
         self.kd, self.nd = kd, ndims
+        self.args = kd, ndims, zloop, split, ordered, tma
         # the boundary-first variant (ps_jit_hide_communication): its block index comes from the
         # launch's tile order, and every warp counts itself in host-mapped memory at the end
         self.ordered = bool(ordered)
@@ -517,9 +518,10 @@ class _Gen:
         self.layout = None
         # a body of FD statements alone (all that definitions of this kind usually have) runs statement by
         # statement over a thread's columns, with 32-bit indices (see tma_resolve)
-        self.flat = self.tma and all(_is_sel_assign(x) or isinstance(x, ast.Pass) or
+        self.flat = form != "points" and self.tma and all(_is_sel_assign(x) or isinstance(x, ast.Pass) or
                                      (isinstance(x, ast.Return) and x.value is None and x is kd.body[-1]) for x in kd.body)
         self.flat_stmts = []
+        self.cells = form == "cells"
         written = set()
         for n in ast.walk(ast.Module(body=kd.body, type_ignores=[])):
             if isinstance(n, ast.Assign):
@@ -1100,6 +1102,8 @@ class _Gen:
             raise _NoTma()
         ry = 2 if self.flat and es == 4 else 1  # rows per thread: their values share loads and the step's overhead
         return {"arrays": arrays, "zl": zl, "span": span, "stages": stages, "stage": off, "smem": smem, "xc": xc, "ry": ry,
+                "flat": self.flat, "slow": 0, "alone": self.flat, "own": False,
+                "statements": len(self.flat_stmts),
                 "tx_bytes": sum(a["bx"] * a["by"] * es for a in arrays)}
 
     def tma_resolve(self, body):
@@ -1131,8 +1135,15 @@ class _Gen:
         all cells of a thread are computed without branches between them -- the ring holds the stencils of
         every cell of a block, with zeros from outside the arrays -- and stored where they run; and two rows
         per thread share their y loads and fluxes and the step's own instructions. 64 per cell, 88 us (one row
-        per thread 7 % more, four 28 %; one and three planes in flight instead of two 3 % and 12 %)."""
+        per thread 7 % more, four 28 %; one and three planes in flight instead of two 3 % and 12 %).
+
+        What cells that do not run compute, on zeros from outside the arrays, is not only work for nothing: a division by
+        zero, or of zero, takes the slow path of the IEEE division, and eight cells' divisions without branches
+        between them cost registers. See sweep_form for which bodies and arrays are swept so."""
         xc, ry = self.layout["xc"], self.layout["ry"]
+        self.layout["slow"] = sum(slow_operations(st[4][-1]) for st in self.flat_stmts)
+        if self.layout["slow"] > FLAT_SLOW:
+            raise _NotFlat()
         cells = xc * ry
         used = set()
         ref = re.compile(r"a(\d+)\[\(tx\+(-?\d+)\) \+ n\1_0 \* \(\(ty\+(-?\d+)\) \+ n\1_1 \* \(tz\+(-?\d+)\)\)\]")
@@ -1159,13 +1170,26 @@ class _Gen:
                     f"    const unsigned m_ = in_ ? ok{j}_ : 0u;",
                     f"    if (in_ ? bad{j}_ : ok{j}_ | bad{j}_) atomicOr(g.err, 1);",
                     f"    const bool all_ = m_ == {(1 << cells) - 1}u;"]
+            # what it reads of written arrays: all cells' loads (of those that run) before the first value
+            own, ahead = [], []
+            for i, ln in enumerate(lines[:-1]):
+                m = re.fullmatch(r"\s*const R (L\d+) = (b\d+_\[.*\]);", ln)
+                if m:
+                    own.append(f"    E W{m.group(1)}_[{cells}];")
+                    ahead.append(f"    W{m.group(1)}_[jt_c] = (E)0; if (all_ || m_ >> jt_c & 1u) W{m.group(1)}_[jt_c] = {m.group(2)};")
+                    lines[i] = f"    const R {m.group(1)} = W{m.group(1)}_[jt_c];"
+            if own:
+                self.layout["own"] = True
+                own += ["    #pragma unroll", loop] + cell + ahead + ["    }"]
             value = lines[:-1] + [f"    o_[jt_c] = {val};{chk}"]
-            # only where it runs: a statement that reads a written array, and one on split pairs, whose loads
-            # report values outside the pairs' range (cells that do not run may hold any)
-            if self.split or any(re.search(r"\bb\d+_\[", ln) for ln in lines[:-1]):
+            # only where it runs: a statement on split pairs, whose loads report values outside the pairs' range (cells that
+            # do not run may hold any), and see sweep_form
+            if self.cells or self.layout["slow"] > 1 or self.split:
                 value = ["    if (all_ || m_ >> jt_c & 1u) {"] + value + ["    }"]
+            else:
+                self.layout["alone"] = False
             # the ring holds (zeros from outside the arrays in) the stencils of all cells of a block
-            out += ["    if (m_) {", f"    E o_[{cells}];", "    #pragma unroll", loop] + cell + value + \
+            out += ["    if (m_) {", f"    E o_[{cells}];"] + own + ["    #pragma unroll", loop] + cell + value + \
                    ["    }", "    if (all_) {", "    #pragma unroll", loop] + cell + [f"    {lhs} = o_[jt_c];", "    }",
                     "    } else {", "    #pragma unroll", loop] + cell + [f"    if (m_ >> jt_c & 1u) {lhs} = o_[jt_c];", "    }",
                     "    }", "    }", "    }"]
@@ -1258,6 +1282,13 @@ class _Gen:
         return f"typedef {real} R;\ntypedef R E;"
 
     def source(self, real):
+        try:
+            return self.generate(real)
+        except _NotFlat:  # once more, point by point
+            self.__init__(*self.args, form="points")
+            return self.generate(real)
+
+    def generate(self, real):
         kd = self.kd
         self.collect_temps()
         self.infer_locals(kd.body)
@@ -1379,6 +1410,40 @@ def sweep_chunk(n, columns, resident, start, most=256):
         if ls <= 2 or rounds > 16:  # many rounds: no better for shorter ones
             break
     return best[1] if best else 1
+
+
+# Divisions and square roots of one cell up to which a TMA sweep runs statement by statement (_Gen.tma_flat).
+FLAT_SLOW = 2
+
+
+def slow_operations(line):
+    """Divisions (but of two numbers) and square roots in a statement's C text."""
+    number = r"\(\(R\)[-+0-9.eE]+\)|\(R\)[-+0-9.eE]+"
+    return line.count(" / ") - len(re.findall(f"(?:{number}) / (?:{number})", line)) + line.count("sqrt(")
+
+
+def sweep_form(layout, descs, cnt):
+    """The form in which a statement-by-statement TMA sweep (_Gen.tma_flat) runs over these arrays: "" (all cells of a
+    block are computed), "cells" (those that run) or "points" (point by point, the form of bodies with more
+    divisions than FLAT_SLOW). FP32, us per launch in the three forms:
+
+    - no division: 384 x 320 x 256 flux 86 / 124 / 129, 300 x 300 x 100 31 / 42 / 48, 36 x 300 x 300 30 / 29 / 32;
+      but where three quarters of the columns lie outside the arrays, 4 x 2048 x 128 86 / 66 / 67, 16 x 1024 x 64
+      25 / 20 / 21, and three velocity updates in place there 46 / 43 / 36;
+    - one (or a square root): 512^3 196 / 242 / 250 where the columns are all in the arrays, else 300 x 300 x 100
+      32 / 22 / 27, 64 x 512 x 200 33 / 21 / 23;
+    - two (always the cells that run): 512^3 286 / 292 / 292, 256 x 256 x 64 15.4 / 12.8 / 13.7, 300 x 300 x 100 50 / 27 / 31;
+    - more: the README's step with its three quotients 384 x 320 x 256 137 / 124 / 120, 300 x 300 x 100
+      89 / 42 / 44; fluxes with quotients 342 / 252 / 220 and 234 / 85 / 80; @harm 249 / 202 / 168."""
+    width = 32 * layout["xc"]
+    columns = -(-cnt[0] // width) * width
+    if 4 * cnt[0] <= columns:
+        return "points" if layout["own"] else "" if layout["alone"] else "cells"
+    return "cells" if layout["slow"] == 1 and not layout["alone"] and any(n[0] != columns for _, n, _, _ in descs) else ""
+
+
+class _NotFlat(Exception):
+    """The body is not swept statement by statement."""
 
 
 class _NoTma(Exception):
@@ -1533,11 +1598,11 @@ def generate(kd: KernelDef, ndims: int, dtype: str, zloop: bool = False) -> str:
 
 
 def _generate_info(kd: KernelDef, ndims: int, dtype: str, zloop: bool = False, split: bool = False,
-                   ordered: bool = False, tma: bool = False):
+                   ordered: bool = False, tma: bool = False, form: str = ""):
     """(source, uses collectives, TMA layout or None); tma asks for the TMA variant of a 3-D sweep,
-    which falls back to the plain sweep where it does not apply."""
+    which falls back to the plain sweep where it does not apply; form: see sweep_form."""
     if tma:
-        g = _Gen(kd, ndims, zloop, split, ordered, tma=True)
+        g = _Gen(kd, ndims, zloop, split, ordered, tma=True, form=form)
         if g.tma:
             try:
                 src = g.source(dtype)
@@ -1583,11 +1648,12 @@ class JitKernel:
     def source(self, ndims, dtype="double"):
         return generate(self.kd, ndims, dtype)
 
-    def _handle(self, ndims, dtype, zloop=False, split=False, ordered=False, tma=False):
-        key = (ndims, dtype, bool(zloop), bool(split)) + (("ordered",) if ordered else ()) + (("tma",) if tma else ())
+    def _handle(self, ndims, dtype, zloop=False, split=False, ordered=False, tma=False, form=""):
+        key = (ndims, dtype, bool(zloop), bool(split)) + (("ordered",) if ordered else ()) + (("tma",) if tma else ()) + \
+            ((form,) if form else ())
         if key not in self._handles:
             src, self._collective[key], self._layouts[key] = _generate_info(self.kd, ndims, dtype, zloop, split,
-                                                                            ordered, tma)
+                                                                            ordered, tma, form)
             h = ctypes.c_void_p()
             _lib.call("ps_jit_compile", src.encode(), b"ps_jit_entry", ctypes.byref(h))
             self._handles[key] = h
@@ -1715,11 +1781,18 @@ class JitKernel:
             es = 8 if dt == "double" else 4
             ht = self._handle(ndims, dt, zl, sp, False, tma=True)
             layout = self._layouts[(ndims, dt, zl, sp, "tma")]
-            # (and where 32-bit indices reach all of a few planes)
-            if layout is not None and all(max(*n, 8 * n[0] * n[1]) < 2 ** 31 - 2 ** 16 for _, n, _, _ in descs) and \
+            # (and, statement by statement, where 32-bit indices reach all of a few planes)
+            if layout is not None and \
+                    (not layout["flat"] or all(max(*n, 8 * n[0] * n[1]) < 2 ** 31 - 2 ** 16 for _, n, _, _ in descs)) and \
                     all(not ((ptr or 0) % 16 or (n[0] * es) % 16 or (n[0] * n[1] * es) % 16)
                         for ptr, n, _, _ in (descs[a["k"]] for a in layout["arrays"])):
-                if not loopsize and "loopsize" not in self.kd.options:
+                form, statements = sweep_form(layout, descs, cnt) if layout["flat"] else "", layout["statements"]
+                if form:
+                    ht = self._handle(ndims, dt, zl, sp, False, tma=True, form=form)
+                    layout = self._layouts[(ndims, dt, zl, sp, "tma", form)]
+                # (narrow arrays swept point by point keep the short sweeps of many blocks where several statements wait
+                # for memory in each plane: three velocity updates, 8 x 8 x 16384 112 -> 94 us, 16 x 1024 x 64 36 -> 35)
+                if not loopsize and "loopsize" not in self.kd.options and not (form == "points" and statements > 1):
                     if "resident" not in layout:  # a property of the compiled kernel
                         layout["resident"] = blocks_per_sm(ht, 32 * _Gen.TMA_TY // layout["ry"], layout["smem"])
                     cols = -(-cnt[0] // (32 * layout["xc"])) * -(-cnt[1] // _Gen.TMA_TY)

@@ -174,3 +174,41 @@ def test_tma_sweep_split_fp64_range_is_that_of_the_cells_that_run(ps):
     with pytest.raises(PSError):
         _run(ps, k, "FLUX_LAM", [ins[0], _dev(ps, Ci), ins[2]], outs, sc, np.float64, **args)
     k.tma = True
+
+
+def _quotients(d, own):
+    """A stencil statement with d divisions; own: added to the array it writes, beside a second one in place."""
+    terms = ["@d2_xi(B)/h", "c/@inn(B)", "@d2_yi(B)/(h*c)", "@d2_zi(B)/c"]
+    rhs = " + ".join(terms[:d] + [t.split("/")[0] if t[0] == "@" else "c*@inn(B)" for t in terms[d:]])
+    more = "@inn(A) + " if own else ""
+    second = "    @all(S) = @all(S)*c - @all(B)\n" if own else ""
+    return (f"@parallel function quot{d}!(A, S, B, c, h)\n    @inn(A) = {more}{rhs}\n{second}"
+            + ("" if own else "    @all(S) = @all(B)\n") + "    return\nend")
+
+
+@pytest.mark.parametrize("n", [(128, 10, 9), (384, 8, 5), (132, 9, 7), (36, 17, 5), (32, 24, 6), (4, 64, 9)])
+@pytest.mark.parametrize("d", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("own", [False, True])
+def test_tma_sweep_forms_by_divisions_and_columns(ps, d, own, n):
+    """All cells of a block, the cells that run, or point by point, by the divisions of the body and the columns
+    outside the arrays (where divisors are zero): the same results as one point per thread."""
+    rng = np.random.default_rng(d)
+    A, S, B = ((0.5 + rng.random(n)).astype(np.float32) for _ in range(3))
+    B[0] = B[:, -1] = 0.0  # divisors on the faces, which no statement reads as such
+    k = ps.parallel_kernel(_quotients(d, own))
+
+    def run(**kw):
+        a, s = _dev(ps, A), _dev(ps, S)
+        ps.parallel(k, a, s, _dev(ps, B), 0.7, 0.3, **kw)
+        return ps.to_host(a), ps.to_host(s)
+    before = k.tma_launches
+    got = run()
+    assert k.tma_launches == before + 1
+    for x, y in zip(got, run(memopt=False)):
+        assert np.array_equal(x, y)
+    key = (3, "float", True, False, "tma")
+    assert k._layouts[key]["flat"] == (d <= 2)
+    form = "" if d > 2 else "points" if own and n[0] <= 32 else "cells" if d < 2 and n[0] <= 32 or d == 1 and n[0] % 128 else ""
+    if form:  # (one kernel object serves all sizes)
+        assert key + (form,) in k._handles
+

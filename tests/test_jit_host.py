@@ -461,3 +461,28 @@ def test_tma_variant_falls_back_where_it_cannot_apply(jit):
     src = "@parallel function cp!(A, B)\n    @all(A) = @all(A) * 2.0\n    return\nend"
     s, _, layout = jit._generate_info(jit.parse(src), 3, "double", True, False, False, True)
     assert layout is None and "cp.async.bulk.tensor" not in s
+
+
+def test_slow_operations_of_a_statement(jit):
+    """Divisions and square roots of a cell, but not quotients of two numbers."""
+    src = """@parallel function q!(A, B, c)
+    @inn(A) = 1/2*@inn(B) + {}
+    return
+end"""
+    for rhs, n in (("c*@d2_xi(B)", 0), ("@d2_xi(B)/c", 1), ("sqrt(@inn(B))", 1), ("@inn(B)^2/c + inv(@inn(B))", 2)):
+        _, _, L = jit._generate_info(jit.parse(src.format(rhs)), 3, "float", True, False, False, True)
+        assert L["flat"] and L["slow"] == n, rhs
+    _, _, L = jit._generate_info(jit.parse(src.format("@harm(B)")), 3, "float", True, False, False, True)
+    assert not L["flat"]
+
+
+def test_sweep_form(jit):
+    """The cells that run alone in narrow arrays (a quarter of the columns at most; point by point where written
+    arrays are read too) and beside columns outside an array where there is a division."""
+    d = lambda *ns: [(0, (n, 8, 8), 1, 0) for n in ns]  # noqa: E731
+    for slow, ns, own, form in ((0, (384, 384), False, ""), (0, (33, 33), True, ""), (0, (32, 32), False, "cells"),
+                                (0, (4,), True, "points"), (1, (384, 384), True, ""), (1, (384, 383), False, "cells"),
+                                (1, (300,), True, "cells"), (1, (24,), True, "points")):
+        layout = {"xc": 4, "slow": slow, "alone": False, "own": own}
+        assert jit.sweep_form(layout, d(*ns), (max(ns), 8, 8)) == form, (slow, ns)
+    assert jit.sweep_form({"xc": 4, "slow": 2, "alone": True, "own": False}, d(300), (300, 8, 8)) == ""
