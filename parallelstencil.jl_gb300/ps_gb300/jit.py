@@ -1781,12 +1781,13 @@ class JitKernel:
             es = 8 if dt == "double" else 4
             ht = self._handle(ndims, dt, zl, sp, False, tma=True)
             layout = self._layouts[(ndims, dt, zl, sp, "tma")]
-            # (and, statement by statement, where 32-bit indices reach all of a few planes)
             if layout is not None and \
-                    (not layout["flat"] or all(max(*n, 8 * n[0] * n[1]) < 2 ** 31 - 2 ** 16 for _, n, _, _ in descs)) and \
                     all(not ((ptr or 0) % 16 or (n[0] * es) % 16 or (n[0] * n[1] * es) % 16)
                         for ptr, n, _, _ in (descs[a["k"]] for a in layout["arrays"])):
-                form, statements = sweep_form(layout, descs, cnt) if layout["flat"] else "", layout["statements"]
+                form, statements = "", layout["statements"]
+                if layout["flat"]:  # (point by point too where 32-bit indices do not reach all of a few planes)
+                    reach = all(max(*n, 8 * n[0] * n[1]) < 2 ** 31 - 2 ** 16 for _, n, _, _ in descs)
+                    form = sweep_form(layout, descs, cnt) if reach else "points"
                 if form:
                     ht = self._handle(ndims, dt, zl, sp, False, tma=True, form=form)
                     layout = self._layouts[(ndims, dt, zl, sp, "tma", form)]

@@ -212,3 +212,16 @@ def test_tma_sweep_forms_by_divisions_and_columns(ps, d, own, n):
     if form:  # (one kernel object serves all sizes)
         assert key + (form,) in k._handles
 
+
+def test_tma_sweep_of_planes_beyond_32_bit_indices(ps):
+    """Eight planes of more than 2^31 elements: staged by TMA all the same, point by point."""
+    import torch
+
+    n = (16384, 16400, 4)
+    k = ps.parallel_kernel("@parallel function big!(A, B, c)\n    @inn(A) = c*@d2_xi(B) + @d2_zi(B)\n    return\nend")
+    B = ps.rand(*n, dtype=np.float32, seed=3)
+    A, A2 = ps.zeros(*n, dtype=np.float32), ps.zeros(*n, dtype=np.float32)
+    ps.parallel(k, A, B, 0.3)
+    assert k.tma_launches == 1 and (3, "float", True, False, "tma", "points") in k._handles
+    ps.parallel(k, A2, B, 0.3, memopt=False)
+    assert torch.equal(A, A2) and A.any().item()
