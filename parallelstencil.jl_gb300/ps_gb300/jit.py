@@ -1643,19 +1643,26 @@ class JitKernel:
         self._handles = {}
         self._sweeps = {}  # sweep forms of the reverse kernel (ps_gb300.ad)
         self._collective = {}
+        self._sources = {}
         self._layouts = {}  # TMA stage layout of each TMA-variant handle (None: the plain sweep was generated)
 
     def source(self, ndims, dtype="double"):
         return generate(self.kd, ndims, dtype)
 
-    def _handle(self, ndims, dtype, zloop=False, split=False, ordered=False, tma=False, form=""):
+    def _variant(self, ndims, dtype, zloop=False, split=False, ordered=False, tma=False, form=""):
+        """Key of a variant of the kernel, whose source and TMA layout are generated on first use."""
         key = (ndims, dtype, bool(zloop), bool(split)) + (("ordered",) if ordered else ()) + (("tma",) if tma else ()) + \
             ((form,) if form else ())
+        if key not in self._layouts:
+            self._sources[key], self._collective[key], self._layouts[key] = \
+                _generate_info(self.kd, ndims, dtype, zloop, split, ordered, tma, form)
+        return key
+
+    def _handle(self, *args, **kw):
+        key = self._variant(*args, **kw)
         if key not in self._handles:
-            src, self._collective[key], self._layouts[key] = _generate_info(self.kd, ndims, dtype, zloop, split,
-                                                                            ordered, tma, form)
             h = ctypes.c_void_p()
-            _lib.call("ps_jit_compile", src.encode(), b"ps_jit_entry", ctypes.byref(h))
+            _lib.call("ps_jit_compile", self._sources[key].encode(), b"ps_jit_entry", ctypes.byref(h))
             self._handles[key] = h
         return self._handles[key]
 
@@ -1779,8 +1786,10 @@ class JitKernel:
             # the 3-D sweep with its stencil arrays staged by TMA, where every staged array meets TMA's
             # 16-byte rules (base address, x extent and x-y plane in bytes); else the plain sweep
             es = 8 if dt == "double" else 4
-            ht = self._handle(ndims, dt, zl, sp, False, tma=True)
-            layout = self._layouts[(ndims, dt, zl, sp, "tma")]
+            key = (ndims, dt, zl, sp, "tma")
+            if key not in self._layouts:
+                self._variant(ndims, dt, zl, sp, False, tma=True)
+            layout = self._layouts[key]
             if layout is not None and \
                     all(not ((ptr or 0) % 16 or (n[0] * es) % 16 or (n[0] * n[1] * es) % 16)
                         for ptr, n, _, _ in (descs[a["k"]] for a in layout["arrays"])):
@@ -1788,9 +1797,11 @@ class JitKernel:
                 if layout["flat"]:  # (point by point too where 32-bit indices do not reach all of a few planes)
                     reach = all(max(*n, 8 * n[0] * n[1]) < 2 ** 31 - 2 ** 16 for _, n, _, _ in descs)
                     form = sweep_form(layout, descs, cnt) if reach else "points"
-                if form:
-                    ht = self._handle(ndims, dt, zl, sp, False, tma=True, form=form)
-                    layout = self._layouts[(ndims, dt, zl, sp, "tma", form)]
+                    if form:
+                        key += (form,)
+                if key not in self._handles:
+                    self._handle(ndims, dt, zl, sp, False, tma=True, form=form)
+                ht, layout = self._handles[key], self._layouts[key]
                 # (narrow arrays swept point by point keep the short sweeps of many blocks where several statements wait
                 # for memory in each plane: three velocity updates, 8 x 8 x 16384 112 -> 94 us, 16 x 1024 x 64 36 -> 35)
                 if not loopsize and "loopsize" not in self.kd.options and not (form == "points" and statements > 1):
