@@ -1336,11 +1336,13 @@ __global__ void __launch_bounds__(32 * TY, 2)
 }
 
 // glam of the cells in the planes z = 0, nz-1 and the rows y = 0, ny-1 (the rest is done by
-// diff3d_grid_adj_tma): the same face sums from global loads, one thread per cell.
+// diff3d_grid_adj_tma): the same face sums from global loads, one thread per cell. It does not let the next step's
+// blocks in early: they took places beside the running step's blocks, which left SMs with two steps' blocks and others with
+// one (gradient per step, with that / without: 16 x 1024 x 64 161 / 135 us, 256 x 256 x 32 92 / 79, 128^3 63.2 / 62.7,
+// 64^3 20.9 / 21.3).
 __global__ void glam_boundary_kernel(const float2* __restrict__ M, const float2* __restrict__ Tg,
                                      double* __restrict__ glam, dd gc0, dd gc1, dd gc2, int64_t nx, int64_t ny,
                                      int64_t nz, const GridRun* __restrict__ run, const GridRun* __restrict__ mrun) {
-    grid_dependents_may_launch();  // the next step's blocks may set up
     const bool skip = run->bad || mrun->bad;
     const int sh = mrun->shT + run->shT;
     const int f = blockIdx.y;  // 0, 1: planes z = 0, nz-1 (all x, y); 2, 3: rows y = 0, ny-1 (z = 1 .. nz-2)
