@@ -330,7 +330,9 @@ int ps_bc_y2d(ps_array A, void* stream, int sync);
 
 /* n_iter iterations of the PT loop body (compute_P!, compute_τ!, compute_dV!, compute_V!,
  * bc_y!(Vx), bc_x!(Vy); Stokes2D.jl:111-116) with two kernels per iteration, in place. Every array,
- * temporaries included, ends bit-identical to the six-call sequence. Synchronises. */
+ * temporaries included, ends bit-identical to the six-call sequence. At most 1048559 rows (ny) in FP64 and 524279
+ * in FP32 (PS_ERR_SHAPE before anything is written; ps_stokes2d_solve likewise, mode 1 with the FP32 bound).
+ * Synchronises. */
 int ps_stokes2d_iterate(const ps_stokes2d_fields* f, const ps_stokes2d_params* p, int64_t n_iter, void* stream);
 
 /* ps_stokes2d_iterate without any device allocation. This entry point has no counterpart in the

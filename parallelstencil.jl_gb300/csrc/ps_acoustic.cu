@@ -469,7 +469,7 @@ int ps_acoustic3d_run(ps_array Vx, ps_array Vy, ps_array Vz, ps_array P, double 
     if (P.dtype == PS_F64 && fp64_mode == PS_FP64_IEEE) {
         // IEEE FP64 is bound by the FP64 pipe, where the fused kernel's extra face updates (the Vy
         // face of the next row, the Vx face past each warp) cost more than its saved traffic: the
-        // miniapp's two kernels in place (measured 1.73 against 2.50 ms per step at 255^3)
+        // miniapp's two kernels in place (measured 0.87 against 1.30 ms per step at 255^3)
         for (int64_t it = 0; it < nt; ++it) {
             PS_TRY(ps_acoustic3d_v(Vx, Vy, Vz, P, dt, rho, dx, dy, dz, stream, 0));
             PS_TRY(ps_acoustic3d_p(P, Vx, Vy, Vz, dt, k, dx, dy, dz, stream, 0));

@@ -225,8 +225,8 @@ __device__ __forceinline__ double warp_sum(double v) {
 //
 // Bound: FP64 pipe (FP64: 57 FP64 instructions per cell, 80 % busy), L2 and launches (FP32: 24 words per
 // cell). Per iteration, against one kernel on shared-memory tiles that computed a halo twice and tested
-// every dividend: FP64 511^2 82 -> 32.8 us, 1023^2 270 -> 118 us; FP32 1023^2 37.8 -> 15.4 us, 511^2 6.6 us,
-// 63^2 3.6 us. A march along y with rows in registers and shuffles (one kernel, 15 words per cell) was
+// every dividend: FP64 511^2 82 -> 32.8 us, 1023^2 270 -> 118 us; FP32 1023^2 37.8 -> 14.4 us, 511^2 5.7 us,
+// 63^2 3.3 us. A march along y with rows in registers and shuffles (one kernel, 15 words per cell) was
 // measured at 16.6, 7.8 and 3.5 us in FP32 and 150 us in FP64 at 1023^2: its few long warps wait on loads
 // and, in FP64, leave the pipe idle.
 //

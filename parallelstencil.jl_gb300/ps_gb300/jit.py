@@ -1634,7 +1634,8 @@ class JitKernel:
     def __init__(self, src: str, ndims=None):
         self.ndims = ndims
         # 3-D sweeps of FP32 arrays stage their stencil arrays by TMA where the launch allows it
-        # ("always": FP64 too -- slower there: the FP64 kernels are bound by arithmetic, not loads)
+        # ("always": FP64 too -- slower there: those kernels are bound by arithmetic, not loads. us per launch, register sweep
+        # / staged: flux body 384 x 320 x 256 IEEE 2501 / 2580, split 758 / 799, 512^3 split 3043 / 3125)
         self.tma = True
         self.tma_launches = 0  # launches that took the TMA variant
         self.kd = parse(src)
