@@ -282,6 +282,15 @@ def stream_handle(stream=None):
     return ctypes.c_void_p(stream.cuda_stream)
 
 
+def capturing(stream=None) -> bool:
+    """Whether work on the stream is being captured into a CUDA graph."""
+    torch = _torch()
+    if stream is None:
+        return torch.cuda.is_current_stream_capturing()
+    with torch.cuda.stream(torch.cuda.ExternalStream(stream) if isinstance(stream, int) else stream):
+        return torch.cuda.is_current_stream_capturing()
+
+
 def synchronize(stream=None) -> None:
     """`@synchronize()` / `@synchronize(stream)`."""
     _lib.call("ps_synchronize", stream_handle(stream))

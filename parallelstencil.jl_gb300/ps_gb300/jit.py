@@ -49,7 +49,7 @@ from dataclasses import dataclass, field
 
 from . import _lib
 from ._lib import PSArray
-from .core import ArgumentError, describe, require_initialized, stream_handle
+from .core import ArgumentError, capturing, describe, require_initialized, stream_handle
 from .fd import AV, DIFF, DIFF2, HARM, LHS, MACROS, MAXLOC, MINLOC, SEL
 from .kernels import ranges_to_box
 
@@ -1685,7 +1685,7 @@ class JitKernel:
         fp64="split" evaluates the arithmetic of FP64 kernels on FP32 pairs (each operation within
         ~2^-46 of its operands' magnitude; GB300 issues FP32 at 64x the FP64 rate)."""
         h, A, nA, S, nS, lo, cnt, threads, shmem, loop, layout = self._config(args, ranges, nblocks, nthreads, shmem,
-                                                                             memopt, loopsize, fp64, allow_tma=True)
+                                                                             memopt, loopsize, fp64, allow_tma=True, stream=stream)
         if layout is not None:  # the 3-D sweep with its stencil arrays staged by TMA
             if "maps" not in layout:
                 maps = [x for a in layout["arrays"] for x in (a["k"], a["bx"], a["by"])]
@@ -1717,7 +1717,8 @@ class JitKernel:
                   (ctypes.c_int32 * 3)(*threads), (ctypes.c_int32 * 3)(*loop), (ctypes.c_int64 * 3)(*bw), comm_fn,
                   None, stream_handle(stream))
 
-    def _config(self, args, ranges, nblocks, nthreads, shmem, memopt, loopsize, fp64, ordered=False, allow_tma=False):
+    def _config(self, args, ranges, nblocks, nthreads, shmem, memopt, loopsize, fp64, ordered=False, allow_tma=False,
+                stream=None):
         """Handle, argument arrays, launch geometry and TMA stage layout (None: no staging) of one
         launch (see jit_launch); allow_tma picks the TMA variant of a 3-D sweep where it applies."""
         require_initialized()
@@ -1794,12 +1795,19 @@ class JitKernel:
             if layout is not None and \
                     all(not ((ptr or 0) % 16 or (n[0] * es) % 16 or (n[0] * n[1] * es) % 16)
                         for ptr, n, _, _ in (descs[a["k"]] for a in layout["arrays"])):
-                form, statements = "", layout["statements"]
+                form, reach, statements = "", True, layout["statements"]
                 if layout["flat"]:  # (point by point too where 32-bit indices do not reach all of a few planes)
                     reach = all(max(*n, 8 * n[0] * n[1]) < 2 ** 31 - 2 ** 16 for _, n, _, _ in descs)
                     form = sweep_form(layout, descs, cnt) if reach else "points"
-                    if form:
-                        key += (form,)
+                if (key + (form,) if form else key) not in self._handles and capturing(stream):
+                    # nothing can be compiled: a form that another launch compiled, or the plain sweep (one result of all)
+                    forms = ("", "cells", "points") if reach else ("points",)
+                    form = next((f for f in forms if (key + (f,) if f else key) in self._handles),
+                                None if (ndims, dt, zl, sp) in self._handles else form)
+            else:
+                form = None
+            if form is not None:
+                key = key + (form,) if form else key
                 if key not in self._handles:
                     self._handle(ndims, dt, zl, sp, False, tma=True, form=form)
                 ht, layout = self._handles[key], self._layouts[key]

@@ -240,3 +240,25 @@ def test_reverse_out_of_bounds_is_reported(ps, monkeypatch):
     with pytest.raises(Exception, match="out-of-bounds"):
         ps.parallel(k, *a.values(), 0.5, grad=((a["A"], ps.from_host(np.ones((8, 7, 6), np.float32, order="F"))),))
     assert ("ad_sweep", ("A",), 3, "float") not in k._handles
+
+
+@pytest.mark.parametrize("warm,n,nt", [(64, 20, None), (20, 64, None), (64, 64, (32, 8, 1)), (64, 64, None)])
+def test_reverse_sweep_captured_after_a_launch_of_another_size(ps, warm, n, nt):
+    """A launch under capture cannot compile: where the form of its number of points has not run, the other one does."""
+    import torch
+
+    from test_gpu_jit_tma import _captured
+
+    src, nd, _, _, scal = _SWEPT["flux_lam"]
+    k = ps.parallel_kernel(src, nd)
+    dims = {64: (64, 64, 160), 20: (20, 20, 20)}
+    assert 18 ** 3 < ps.ad.SWEEP_MIN <= 62 * 62 * 158
+    make = lambda m: (torch.rand(*reversed(dims[m])) + 0.5).cuda().permute(2, 1, 0)  # noqa: E731
+    arr, bar = ({m: [make(m) for _ in range(4)] for m in (warm, n)} for _ in range(2))
+
+    def run(m, nt=None):
+        ps.parallel_async(k, *arr[m], *scal, grad=tuple(zip(arr[m], bar[m])), nthreads=nt)
+    run(warm)
+    for x, y in _captured(lambda: run(n, nt), arr[n] + bar[n]):
+        # (the forms differ in the order of an element's sum only: the bound above)
+        assert _rel(x.numpy(), y.numpy()) <= 128 * np.finfo(np.float32).eps

@@ -225,3 +225,37 @@ def test_tma_sweep_of_planes_beyond_32_bit_indices(ps):
     assert k.tma_launches == 1 and (3, "float", True, False, "tma", "points") in k._handles
     ps.parallel(k, A2, B, 0.3, memopt=False)
     assert torch.equal(A, A2) and A.any().item()
+
+
+def _captured(f, outs):
+    """The results of f in a graph's replay and of a launch by itself (a tensor's former contents put back before each)."""
+    import torch
+
+    start = [x.clone() for x in outs]
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        f()
+    got = []
+    for run in (graph.replay, f):
+        for x, s in zip(outs, start):
+            x.copy_(s)
+        run()
+        torch.cuda.synchronize()
+        got.append([x.cpu() for x in outs])
+    return zip(*got)
+
+
+@pytest.mark.parametrize("d", [0, 1, 3])
+@pytest.mark.parametrize("warm,n", [(128, 128), (128, 16), (16, 128), (37, 128), (132, 16), (37, 132)])
+def test_tma_sweep_captured_after_a_launch_of_another_size(ps, d, warm, n):
+    """A launch under capture cannot compile the form its size would take: it takes one that is there."""
+    import torch
+
+    k = ps.parallel_kernel(_quotients(d, True))
+    size = {m: [(torch.rand(30, 40, m) + 0.5).cuda().permute(2, 1, 0) for _ in range(2)] for m in (warm, n)}
+    S = {m: torch.zeros_like(a[0]) for m, a in size.items()}
+    run = lambda m: ps.parallel_async(k, size[m][0], S[m], size[m][1], 0.7, 0.3)  # noqa: E731
+    run(warm)
+    for x, y in _captured(lambda: run(n), [size[n][0], S[n]]):
+        assert torch.equal(x, y)
