@@ -1819,8 +1819,11 @@ class JitKernel:
                     cols = -(-cnt[0] // (32 * layout["xc"])) * -(-cnt[1] // _Gen.TMA_TY)
                     loop[2] = sweep_chunk(max(1, cnt[2]), max(1, cols), layout["resident"], layout["span"])
                 return ht, A, len(descs), S, len(scal), lo, cnt, threads, shmem, loop, layout
-        h = self._handle(ndims, dt, zl, sp, ordered)
-        if self._collective[(ndims, dt, zl, sp) + (("ordered",) if ordered else ())] and \
+        key = (ndims, dt, zl, sp, "ordered") if ordered else (ndims, dt, zl, sp)
+        h = self._handles.get(key)
+        if h is None:
+            h = self._handle(ndims, dt, zl, sp, ordered)
+        if self._collective[key] and \
                 any(cnt[d] % threads[d] for d in range(3)):
             raise ArgumentError("a kernel with @sync_threads, shuffles or votes needs ranges that are a multiple of "
                                 f"the thread block (ranges {cnt}, nthreads {threads})")
