@@ -1100,19 +1100,21 @@ def parallel_grad(kernel: JitKernel, args, grad, ad_mode="reverse", ranges=None,
     # forms are bound by the FP64 pipe, where the sweep's own sums cost more than the additions they save
     # (200^3: 1.90 ms against 1.41). Below SWEEP_MIN points a launch is shorter than its way through the
     # host, which the sweep's checks make longer (24 x 30 x 26: 58 us without them, 68 with).
-    # The form of one point per thread is compiled in any case: a launch under capture, where nothing can be
-    # compiled, takes it where the sweep has not run yet.
-    h = _handle(kernel, ("ad", ad_mode, tuple(order), ndims, dt),
-                lambda: generate(kernel.kd, ndims, dt, order, ad_mode))
+    h, points = None, ("ad", ad_mode, tuple(order), ndims, dt)
     if ad_mode == "reverse" and dt == "float" and nthreads is None and nblocks is None and ndims in (2, 3) and \
-            cnt[0] * cnt[1] * cnt[2] >= SWEEP_MIN and \
-            (("ad_sweep", tuple(order), ndims, dt) in kernel._handles or not capturing(stream)):
-        sweep = _sweep_handle(kernel, ndims, dt, order, descs, lo, cnt)
+            cnt[0] * cnt[1] * cnt[2] >= SWEEP_MIN:
+        if ("ad_sweep",) + points[2:] not in kernel._handles:
+            # The form of one point per thread is compiled before the sweep: a launch under capture, where nothing
+            # can be compiled, takes it where the sweep has not run yet.
+            h = _handle(kernel, points, lambda: generate(kernel.kd, ndims, dt, order, ad_mode))
+        sweep = _sweep_handle(kernel, ndims, dt, order, descs, lo, cnt) if h is None or not capturing(stream) else None
         if sweep is not None:
             h, resident = sweep
             threads = [_AdSweepGen.TX, _AdSweepGen.TY, 1] if ndims == 3 else [128, 1, 1]
             cols = -(-cnt[0] // threads[0]) * (-(-cnt[1] // threads[1]) if ndims == 3 else 1)
             loop[ndims - 1] = sweep_chunk(cnt[ndims - 1], max(1, cols), resident, 3)
+    if h is None:
+        h = _handle(kernel, points, lambda: generate(kernel.kd, ndims, dt, order, ad_mode))
     alld = descs + sdescs
     A = (PSArray * len(alld))(*alld)
     S = (ctypes.c_double * max(1, len(scal)))(*scal)

@@ -1791,23 +1791,30 @@ class JitKernel:
             key = (ndims, dt, zl, sp, "tma")
             if key not in self._layouts:
                 self._variant(ndims, dt, zl, sp, False, tma=True)
-            layout = self._layouts[key]
-            if layout is not None and \
-                    all(not ((ptr or 0) % 16 or (n[0] * es) % 16 or (n[0] * n[1] * es) % 16)
-                        for ptr, n, _, _ in (descs[a["k"]] for a in layout["arrays"])):
-                form, reach, statements = "", True, layout["statements"]
-                if layout["flat"]:  # (point by point too where 32-bit indices do not reach all of a few planes)
-                    reach = all(max(*n, 8 * n[0] * n[1]) < 2 ** 31 - 2 ** 16 for _, n, _, _ in descs)
+            layout, form = self._layouts[key], None
+            if layout is not None:
+                for a in layout["arrays"]:
+                    ptr, n, _, _ = descs[a["k"]]
+                    if (ptr or 0) % 16 or n[0] * es % 16 or n[0] * n[1] * es % 16:
+                        break
+                else:
+                    form, reach, statements = "", True, layout["statements"]
+            if form is not None:
+                if layout["flat"]:
+                    for _, n, _, _ in descs:
+                        if max(*n, 8 * n[0] * n[1]) >= 2 ** 31 - 2 ** 16:
+                            reach = False
+                    # (point by point too where 32-bit indices do not reach all of a few planes)
                     form = sweep_form(layout, descs, cnt) if reach else "points"
-                if (key + (form,) if form else key) not in self._handles and capturing(stream):
+                wanted = key + (form,) if form else key
+                if wanted not in self._handles and capturing(stream):
                     # nothing can be compiled: a form that another launch compiled, or the plain sweep (one result of all)
                     forms = ("", "cells", "points") if reach else ("points",)
                     form = next((f for f in forms if (key + (f,) if f else key) in self._handles),
                                 None if (ndims, dt, zl, sp) in self._handles else form)
-            else:
-                form = None
+                    wanted = key + (form,) if form else key
             if form is not None:
-                key = key + (form,) if form else key
+                key = wanted
                 if key not in self._handles:
                     self._handle(ndims, dt, zl, sp, False, tma=True, form=form)
                 ht, layout = self._handles[key], self._layouts[key]
